@@ -63,8 +63,7 @@ size_t b200_qmm_workspace_bytes(int M, int N, int K);
  * Replaces qmm_kernel.py:84-164 `matmul(x, w, s, b, group_size)` as bound at
  * mlx_eagle.py:704-708 and called from mlx_model_fwd_bench.py:69 (rows 8/16/24/32), and the
  * mx.quantized_matmul fallback for other row counts (mlx_model_fwd_bench.py:73).
- *   x        [M,K]   fp16, row-major                       M >= 1 (rows beyond 32 are processed
- *                                                          in passes of 32)
+ *   x        [M,K]   fp16, row-major                       M >= 1
  *   wq       [N,K/8] uint32, element j of a pack in bits 4j..4j+3 (MLX layout)
  *   scales, biases [N,K/64] fp16;  group_size must be 64, K % 128 == 0, N % 8 == 0
  *   bias     [N] fp16 or NULL: added after the fp16 rounding of the product
@@ -133,15 +132,19 @@ size_t b200_qmm_tiled_workspace_bytes(int M, int N, int K);
 int b200_qmm_tiled(const void* x, const void* wt, const void* wt2, const void* bias, const void* extra, void* y,
                    int M, int N, int K, int epilogue, void* workspace, size_t workspace_bytes, void* stream);
 
-/* The same product (plain epilogue: y = fp16(acc) [+ bias, in fp16]) on the tcgen05 tensor cores: sixteen warps
- * expand the packed records (exact q*s+b, rounded once) and write the fp16 weights with tcgen05.st straight into
- * 128-row tiles in tensor memory (the weights never pass through shared memory as fp16), one thread per CTA issues
- * tcgen05.mma (weights from tensor memory, activations read in place from the bulk-copied stage in shared memory)
- * with the accumulator in tensor memory.  Same streaming weight layout; M <= 128 (one weight read serves up to 128
- * token rows: the shape of prompt ingestion), N % 128 == 0, K % 128 == 0.  workspace: b200_qmm_umma_workspace_bytes
- * bytes (the activations in the tensor cores' K-major core-matrix order, written by a relayout kernel that this call
- * launches first, + an error word, int 0 of the workspace, non-zero if a bounded wait gave up; zero it before the
- * first use).  Replaces qmm_kernel.py:79-124 like b200_qmm. */
+/* The same product and epilogues (B200_EPI_NONE / RESIDUAL / SILU_MUL) on the tcgen05 tensor cores, for any number of token
+ * rows: one weight read serves up to 128 of them.  Sixteen warps expand the packed records (exact q*s+b, rounded once) and
+ * write the fp16 weights with tcgen05.st into tiles in tensor memory, one thread per CTA issues tcgen05.mma (weights from
+ * tensor memory, activations from TMA-loaded shared memory) with the accumulators in tensor memory.  Same streaming weight
+ * layout; N % 8 == 0, K % 128 == 0.  workspace: b200_qmm_gemm_workspace_bytes bytes let K be cut as the planner likes (4096 is
+ * enough for no cut; the first 4 KiB zero before first use; the last int of that block is an error flag set if a bounded wait
+ * gives up).  b200_qmm takes this path too beyond 32 rows, on row-major weights.  Replaces qmm_kernel.py:79-124 like b200_qmm. */
+size_t b200_qmm_gemm_workspace_bytes(int M, int N, int K, int epilogue);
+int b200_qmm_gemm(const void* x, const void* wt, const void* wt2, const void* bias, const void* extra, void* y,
+                  int M, int N, int K, int epilogue, void* workspace, size_t workspace_bytes, void* stream);
+
+/* The plain product of b200_qmm_gemm for M <= 128 and N % 128 == 0, with the error word in int 0 of a workspace of
+ * b200_qmm_umma_workspace_bytes bytes (zero the first 4 KiB before the first use). */
 size_t b200_qmm_umma_workspace_bytes(int M, int K);
 int b200_qmm_umma(const void* x, const void* w_tiled, const void* bias, void* y, int M, int N, int K,
                   void* workspace, size_t workspace_bytes, void* stream);

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <utility>
 
 #include "b200_eagle.h"
@@ -46,6 +47,19 @@ inline void launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t 
     cfg.attrs = attr;
     cfg.numAttrs = g_use_pdl ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+
+// Lets `kern` use `bytes` of dynamic shared memory: a per-device attribute, set once per device (`done`: one bit each, a static
+// of the caller's).
+template <typename F>
+inline bool allow_smem(F kern, size_t bytes, std::atomic<uint64_t>& done) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    const uint64_t bit = 1ull << (dev & 63);
+    if (done.load(std::memory_order_acquire) & bit) return true;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return false;
+    done.fetch_or(bit, std::memory_order_release);
+    return true;
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }

@@ -209,7 +209,7 @@ struct Ctx {
 
 // Ring waits of this kernel: up to 2^20 polls of <= 1 us each (about a second) before giving up.
 __device__ __forceinline__ bool fwd_wait(uint32_t bar, uint32_t parity) {
-    return mbar_wait_timed(bar, parity, 1u << 20, 1000u);
+    return mbar_wait(bar, parity, 1u << 20);
 }
 
 __device__ __forceinline__ size_t xt_index(int tok, int n, int mp) {

@@ -32,19 +32,21 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
         if (mbar_try_wait(bar, parity)) return true;
     return false;
 }
-// Same, with an explicit per-poll suspend hint (nanoseconds), so that the bound is a time bound:
-// at most `polls` x `hint_ns` (plus scheduling) before the wait gives up.
-__device__ __forceinline__ bool mbar_wait_timed(uint32_t bar, uint32_t parity, uint32_t polls, uint32_t hint_ns) {
-    for (uint32_t i = 0; i < polls; i++) {
-        uint32_t ok;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity), "r"(hint_ns)
-            : "memory");
-        if (ok) return true;
-    }
+// Same, with the iteration limit given: a poll that does not find the phase complete suspends the thread for up to about a
+// microsecond, so the limit is a time limit.  (Without a suspend-time hint a complete phase is seen in 14 cycles and a
+// suspended thread is back ~60 cycles after the arrival; with a hint the same two took 100 and 75 to 100 cycles.)
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t polls) {
+    for (uint32_t i = 0; i < polls; i++)
+        if (mbar_try_wait(bar, parity)) return true;
     return false;
+}
+// One lane of a converged warp.  A branch on this keeps the compiler's knowledge that everything else is warp-uniform, so the
+// descriptors and addresses of tcgen05.mma and of copies stay in uniform registers: an MMA issues every 19 cycles instead of
+// every 45 behind `if (lane == 0)`.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}\n" : "=r"(p));
+    return p != 0;
 }
 __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),

@@ -20,6 +20,7 @@
 //     workspace and the last CTA of a row tile adds them in split order (deterministic) and runs
 //     the epilogue (bias / residual add / SiLU-gate multiply).
 #include "qmm_common.cuh"
+#include "qmm_gemm.cuh"
 
 namespace b200 {
 namespace {
@@ -408,7 +409,10 @@ extern "C" {
 
 size_t b200_qmm_workspace_bytes(int M, int N, int K) {
     if (M < 1 || N < 8 || K < b200::kChunkK || (K % b200::kChunkK) != 0) return 0;
-    if (M > 32) M = 32;
+    if (M > 32) {
+        const size_t part = b200::qmm_gemm_partial_bytes(M, N, K, false);
+        return part ? b200::kCounterBytes + part : 0;
+    }
     size_t need = 0;
     for (int dual = 0; dual < 2; dual++) {
         b200::Plan pl = b200::make_plan(M, N, K, dual != 0, -1);
@@ -422,17 +426,30 @@ int b200_qmm(const void* x, const uint32_t* wq, const void* scales, const void* 
              const void* bias, void* y, int M, int N, int K, int group_size, int dtype,
              void* workspace, size_t workspace_bytes, void* stream) {
     if (M < 1) return B200_EINVAL;
-    // Rows beyond 32 (prompt ingestion) are processed in passes of 32; each pass streams W again.
-    for (int m0 = 0; m0 < M; m0 += 32) {
-        const int mb = (M - m0 < 32) ? (M - m0) : 32;
-        const char* xp = static_cast<const char*>(x) + (size_t)m0 * K * 2;
-        char* yp = static_cast<char*>(y) + (size_t)m0 * N * 2;
-        int rc = b200::qmm_launch(xp, wq, scales, biases, nullptr, nullptr, nullptr, bias, nullptr, yp,
-                                  mb, N, K, group_size, dtype, B200_EPI_NONE, workspace,
-                                  workspace_bytes, static_cast<cudaStream_t>(stream));
-        if (rc != B200_OK) return rc;
+    if (M <= 32)
+        return b200::qmm_launch(x, wq, scales, biases, nullptr, nullptr, nullptr, bias, nullptr, y, M, N, K, group_size, dtype,
+                                B200_EPI_NONE, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+    // Beyond 32 rows one weight read serves all of them on the tensor cores (csrc/qmm_gemm.cu).
+    if (dtype != B200_DTYPE_F16 || group_size != 64) return B200_EUNSUPPORTED;
+    if (N < 8 || (N % 8) != 0 || K < b200::kChunkK || (K % b200::kChunkK) != 0) return B200_EINVAL;
+    if (!x || !wq || !scales || !biases || !y) return B200_EINVAL;
+    if (!b200::aligned16(x) || !b200::aligned16(wq) || !b200::aligned16(y) || !b200::aligned16(bias) || !b200::aligned16(workspace))
+        return B200_EALIGN;
+    if ((reinterpret_cast<uintptr_t>(scales) | reinterpret_cast<uintptr_t>(biases)) & 3u) {
+        // (its asynchronous copies take the two scales of a chunk together; odd addresses go 32 rows at a time)
+        for (int m0 = 0; m0 < M; m0 += 32) {
+            const int rc = b200::qmm_launch(static_cast<const char*>(x) + (size_t)m0 * K * 2, wq, scales, biases, nullptr, nullptr, nullptr,
+                                            bias, nullptr, static_cast<char*>(y) + (size_t)m0 * N * 2, M - m0 < 32 ? M - m0 : 32, N, K,
+                                            group_size, dtype, B200_EPI_NONE, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+            if (rc != B200_OK) return rc;
+        }
+        return B200_OK;
     }
-    return B200_OK;
+    b200::GemmArgs a{};
+    a.x = x; a.wq = wq; a.scales = scales; a.biases = biases; a.bias = bias; a.y = y;
+    a.M = M; a.N = N; a.K = K; a.epilogue = B200_EPI_NONE;
+    b200::gemm_workspace(a, workspace, workspace_bytes);
+    return b200::qmm_gemm(a, static_cast<cudaStream_t>(stream));
 }
 
 int b200_qmm_fused(const void* x, const uint32_t* wq, const void* scales, const void* biases,

@@ -1,0 +1,718 @@
+// 4-bit affine quantised matmul for many token rows (prompt ingestion, the operator beyond 32 rows) on the
+// fifth-generation tensor cores (tcgen05, TMEM).
+//
+//   y[M][N] = x[M][K] . dequant(W)[N][K]^T     (+ bias | + residual | silu(gate) * up), fp16 in, fp32 accumulate
+//
+// Item = (S x 128 weight rows, NT tokens, K range).  S = 2 puts two row tiles (or the gate and the up tile of the same
+// rows) behind one activation tile, so an activation byte brought into shared memory feeds 256 weight rows.
+//
+//   producer warp    per 128-k chunk: the weights (records of the streaming layout, or TMA boxes of the row-major layout
+//                    plus 4-byte asynchronous copies of its scales and biases) and the activations (two TMA boxes of
+//                    64 k x NT rows, 128-byte swizzle, straight from row-major x; rows past M read as zero);
+//   16 dequant warps in four groups that take the tiles (row tile, chunk) in turn, thread = weight row: exact q*s+b rounded
+//                    once to fp16, written with tcgen05.st into the group's own tensor-memory tile (lane = weight row,
+//                    column = two k values); the A operand never touches shared memory as fp16.  A group's chain (packs
+//                    landed, tile free, loads, expansion, stores complete, arrival) is ~1500 cycles; four of them in
+//                    flight hide it (all sixteen warps on one tile ran at 2100 cycles per chunk of two tiles);
+//   MMA warp         one thread issues 8 x S tcgen05.mma (128 x NT x 16) per chunk, A from tensor memory, B from shared;
+//   epilogue         the dequant warps read the accumulators (tcgen05.ld) after they have expanded the first chunks of
+//                    their next item, so the tensor cores find work the moment the accumulator is free.
+//
+// What bounds it (S 2, NT 128, one chunk): the 16 MMAs take 1024 cycles at the tensor cores' rate; shared memory moves
+// 51 KB in, 64 KB to the MMAs and 18 KB to the dequant warps, 1060 cycles at 128 bytes a cycle; the expansion issues
+// ~700 of 1024 slots per scheduler.  With few tokens the weight stream is the bound: 18.4 KB per chunk are ~800 cycles of
+// an SM's share of HBM.
+//
+// Where the tiles alone would leave SMs idle the K range is cut across CTAs; the last CTA of a tile adds the fp32 partial
+// products in split order (deterministic).  Every wait is bounded; one that gives up sets the error word and the CTA runs
+// to its end (tensor memory is always freed).  No copy uses cluster multicast.
+#include <cuda.h>
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+#include <type_traits>
+
+#include "b200_eagle.h"
+#include "common.cuh"
+#include "pipeline.cuh"
+#include "qmm_common.cuh"
+#include "qmm_gemm.cuh"
+#include "tensor_map.cuh"
+
+namespace b200 {
+namespace {
+
+constexpr int kRecBytes = 1152;
+constexpr int kRunBytes = 4 * kRecBytes;         // the four records of a 64-row block for one chunk
+constexpr int kTileRows = 128;                   // weight rows of one MMA
+constexpr int kTileW = 2 * kRunBytes;            // weight bytes of a row tile and chunk (both layouts: 8192 + 1024)
+constexpr int kDeqWarps = 16;
+constexpr int kGroups = 4;                       // groups of four dequant warps, each with a tensor-memory tile of its own
+constexpr int kTileCols = kChunkK / 2;           // columns of a tile: two k values per column
+constexpr int kGThreads = (kDeqWarps + 4) * 32;  // + two producer warps + two MMA warps
+constexpr uint32_t kGemmWaitPolls = 1u << 19;    // about a microsecond each
+constexpr size_t kUmmaPartialBytes = 16u << 20;  // room for the partial products of a K split behind b200_qmm_umma
+constexpr int kGemmTiles = 896;                  // tiles that a K split can hand tickets to
+
+// Layouts of the weights
+enum { W_TILED = 0, W_ROWS = 1 };
+
+template <int S, int NT>
+struct GGeo {
+    static constexpr int XBYTES = NT * kChunkK * 2;                   // two boxes of 64 k
+    static constexpr int STAGE = S * kTileW + XBYTES;                 // a multiple of 1024: the boxes stay swizzle-aligned
+    static constexpr int FIT = (232448 - 2048) / STAGE;
+    // Ring stages: an even number, so that a stage belongs to one of the two producers (and, with S = 1, to one of the two MMA
+    // warps).  Even and odd chunks may drift apart; with an odd ring a wait could then meet a phase two uses away.
+    static constexpr int NP = FIT < 8 ? (FIT & ~1) : 8;
+    static constexpr int ACC = 2 * NT;                                // tensor-memory columns of an accumulator set: one per MMA warp
+    static constexpr int NACC = ACC <= 128 ? 2 : 1;
+    static constexpr int ACC0 = kGroups * kTileCols;                  // first accumulator column
+    static constexpr int SMEM = NP * STAGE + 1024;                    // + alignment slack
+    static_assert(STAGE % 1024 == 0 && ACC0 + NACC * ACC <= 512 && NP >= 4, "tile does not fit");
+};
+
+struct GParams {
+    CUtensorMap xmap;            // x [M][K], boxes of 64 k x NT rows, 128-byte swizzle
+    CUtensorMap wmap;            // row-major weights [N][K/8] words, boxes of 16 words x 128 rows, 64-byte swizzle
+    const unsigned char* w[2];   // streaming layout (gate / up)
+    const __half* sc;            // row-major layout: scales, biases [N][K/64]
+    const __half* bi;
+    const __half* bias;
+    const __half* extra;         // residual [M][N] (may be y)
+    __half* y;
+    int* counter;                // split tickets, one per tile, zero between launches
+    int* err;                    // error word or NULL
+    float* partial;
+    int M, N, K;
+    int row_items, tok_items, splits, chunks_per_split;
+    int epilogue;
+};
+
+__device__ __forceinline__ bool gwait(uint32_t bar, uint32_t parity) { return mbar_wait(bar, parity, kGemmWaitPolls); }
+
+// K-major shared-memory matrix, 128-byte swizzle: rows of 128 bytes, groups of 8 rows 1024 bytes apart.
+__device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
+    return (uint64_t)((saddr & 0x3ffffu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
+           ((uint64_t)2 << 61);
+}
+
+__device__ __forceinline__ void tma_box(uint32_t dst, const void* tmap, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
+                 ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(src) : "memory");
+}
+
+__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&d)[4][4]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(addr),
+                 "r"(d[0][0]), "r"(d[0][1]), "r"(d[0][2]), "r"(d[0][3]), "r"(d[1][0]), "r"(d[1][1]), "r"(d[1][2]), "r"(d[1][3]),
+                 "r"(d[2][0]), "r"(d[2][1]), "r"(d[2][2]), "r"(d[2][3]), "r"(d[3][0]), "r"(d[3][1]), "r"(d[3][2]), "r"(d[3][3]) : "memory");
+}
+template <int C>
+__device__ __forceinline__ void tmem_ld(uint32_t (&r)[C], uint32_t addr) {
+    static_assert(C % 8 == 0 || C == 4, "columns");
+    if constexpr (C % 8 == 0) {
+#pragma unroll
+        for (int i = 0; i < C; i += 8)
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                         : "=r"(r[i]), "=r"(r[i + 1]), "=r"(r[i + 2]), "=r"(r[i + 3]), "=r"(r[i + 4]), "=r"(r[i + 5]),
+                           "=r"(r[i + 6]), "=r"(r[i + 7]) : "r"(addr + i) : "memory");
+    } else {
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];\n"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+    }
+}
+
+// True when the fp16 exponent field is in 1..10: the range of dequant_pack_fast.
+__device__ __forceinline__ bool fast_scale(uint32_t bits) { return ((bits >> 10) & 31u) - 1u < 10u; }
+
+__device__ __forceinline__ void g_error(const GParams& p, int code) {
+    if (p.err != nullptr) atomicCAS(p.err, 0, code);
+}
+
+struct GItem {
+    int row_item, tok0, split, c_begin, nc;
+};
+__device__ __forceinline__ GItem g_item(const GParams& p, int item, int NT) {
+    GItem g;
+    const int tok = item % p.tok_items;              // neighbouring CTAs share the weights of a row tile
+    const int rest = item / p.tok_items;
+    g.row_item = rest % p.row_items;
+    g.split = rest / p.row_items;
+    g.tok0 = tok * NT;
+    g.c_begin = g.split * p.chunks_per_split;
+    g.nc = min(p.chunks_per_split, p.K / kChunkK - g.c_begin);
+    return g;
+}
+
+// The epilogue of one item, by the dequant warps: warp w reads lanes 32 (w % 4) .. of column group w / 4.
+template <int S, int NT, bool DUAL>
+__device__ __forceinline__ void gemm_epilogue(const GParams& p, const GItem& g, uint32_t acc, uint32_t accempty, int warp,
+                                              int lane, int* s_last, bool ok) {
+    constexpr int CG = (DUAL ? NT : S * NT) / 4;         // columns (of each matrix) per warp
+    constexpr int CM = DUAL ? 8 : 16;
+    constexpr int CH = CG < CM ? CG : CM;                // columns per trip
+    const int q = warp & 3, cg = warp >> 2;
+    const int s = DUAL ? 0 : (cg * CG) / NT;
+    const int col0 = DUAL ? cg * CG : (cg * CG) % NT;    // first token column of the warp inside its row tile
+    const int row = (DUAL ? g.row_item : g.row_item * S + s) * kTileRows + q * 32 + lane;
+    const uint32_t lane_base = acc + ((uint32_t)(q * 32) << 16);
+    const bool split = p.splits > 1;
+    const bool both = S == 1 && g.nc > 1;                // even and odd chunks were summed apart
+    const int ncol = min(CG, p.M - g.tok0 - col0);       // of them tokens
+    constexpr int PR = S * kTileRows;                    // rows of a partial tile
+    const size_t pstride = (size_t)p.row_items * p.tok_items * NT * PR;          // floats per split
+    float* const ptile = p.partial + ((size_t)g.row_item * p.tok_items + g.tok0 / NT) * NT * PR;
+    const int prow = (DUAL ? 0 : s * kTileRows) + q * 32 + lane;
+
+    if (split) {
+        // ---- partial products out: for every token column 32 consecutive floats per warp
+        float* mine = ptile + (size_t)g.split * pstride + prow;
+#pragma unroll 1
+        for (int c0 = 0; c0 < ncol && ok; c0 += CH) {
+            uint32_t a[CH], b[CH];
+            tmem_ld<CH>(a, lane_base + (DUAL ? 0 : s * NT) + col0 + c0);
+            if (DUAL || both) tmem_ld<CH>(b, lane_base + NT + col0 + c0);
+            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+            if (both) {
+#pragma unroll
+                for (int i = 0; i < CH; i++) a[i] = __float_as_uint(__uint_as_float(a[i]) + __uint_as_float(b[i]));
+            }
+#pragma unroll
+            for (int i = 0; i < CH; i++) {
+                __stcg(mine + (size_t)(col0 + c0 + i) * PR, __uint_as_float(a[i]));
+                if (DUAL) __stcg(mine + (size_t)(col0 + c0 + i) * PR + kTileRows, __uint_as_float(b[i]));
+            }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(accempty);
+        __threadfence();
+        consumer_sync(kDeqWarps * 32);
+        if (threadIdx.x == 0) {
+            int* ctr = p.counter + g.row_item * p.tok_items + g.tok0 / NT;
+            const int old = atomicAdd(ctr, 1);
+            *s_last = old == p.splits - 1;
+            if (old == p.splits - 1) *ctr = 0;
+            __threadfence();
+        }
+        consumer_sync(kDeqWarps * 32);
+        const bool last = *s_last;
+        consumer_sync(kDeqWarps * 32);                  // read by all before the next item rewrites it
+        if (!last) return;
+    }
+    if (!ok) return;
+    const bool row_ok = row < p.N;
+    const __half bv = (p.bias != nullptr && row_ok) ? p.bias[row] : __ushort_as_half(0);
+    const bool resid = p.epilogue == B200_EPI_RESIDUAL;
+    auto release = [&]() {                               // accumulator read: the MMA warp may start the next item
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(accempty);
+    };
+    if (!split && ncol <= 0) release();
+#pragma unroll 1
+    for (int c0 = 0; c0 < ncol; c0 += CH) {
+        __syncwarp();                                    // (rows past N leave the trip early)
+        uint32_t a[CH], b[CH];
+        if (split) {
+            const float* src = ptile + prow + (size_t)(col0 + c0) * PR;
+#pragma unroll
+            for (int i = 0; i < CH; i++) {
+                a[i] = __float_as_uint(__ldcg(src + (size_t)i * PR));
+                if (DUAL) b[i] = __float_as_uint(__ldcg(src + (size_t)i * PR + kTileRows));
+            }
+            for (int sp = 1; sp < p.splits; sp++) {     // in split order, all loads of a trip in flight together
+                const float* ss = src + (size_t)sp * pstride;
+                float v[CH], w[DUAL ? CH : 1];
+#pragma unroll
+                for (int i = 0; i < CH; i++) {
+                    v[i] = __ldcg(ss + (size_t)i * PR);
+                    if (DUAL) w[i] = __ldcg(ss + (size_t)i * PR + kTileRows);
+                }
+#pragma unroll
+                for (int i = 0; i < CH; i++) {
+                    a[i] = __float_as_uint(__uint_as_float(a[i]) + v[i]);
+                    if (DUAL) b[i] = __float_as_uint(__uint_as_float(b[i]) + w[i]);
+                }
+            }
+        } else {
+            tmem_ld<CH>(a, lane_base + (DUAL ? 0 : s * NT) + col0 + c0);
+            if (DUAL || both) tmem_ld<CH>(b, lane_base + NT + col0 + c0);
+            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+            if (both) {
+#pragma unroll
+                for (int i = 0; i < CH; i++) a[i] = __float_as_uint(__uint_as_float(a[i]) + __uint_as_float(b[i]));
+            }
+            if (c0 + CH >= ncol) release();
+        }
+        const int tok = g.tok0 + col0 + c0;
+        if (!row_ok) continue;
+        __half* dst = p.y + (size_t)tok * p.N + row;
+        const int cnt = min(CH, p.M - tok);
+        if (resid) {
+            const __half* rs = p.extra + (size_t)tok * p.N + row;
+            unsigned short r[CH];
+#pragma unroll
+            for (int i = 0; i < CH; i++) r[i] = i < cnt ? __ldcg(reinterpret_cast<const unsigned short*>(rs) + (size_t)i * p.N) : 0;
+#pragma unroll
+            for (int i = 0; i < CH; i++)
+                if (i < cnt) dst[(size_t)i * p.N] = __hadd(__ushort_as_half(r[i]), __float2half_rn(__uint_as_float(a[i])));
+        } else if (DUAL) {
+#pragma unroll
+            for (int i = 0; i < CH; i++)
+                if (i < cnt) dst[(size_t)i * p.N] = __float2half_rn(silu_mul_f16(__uint_as_float(a[i]), __uint_as_float(b[i])));
+        } else {
+#pragma unroll
+            for (int i = 0; i < CH; i++)
+                if (i < cnt) {
+                    __half o = __float2half_rn(__uint_as_float(a[i]));
+                    if (p.bias != nullptr) o = __hadd(o, bv);
+                    dst[(size_t)i * p.N] = o;
+                }
+        }
+    }
+}
+
+template <int S, int NT, bool DUAL, int LAYOUT>
+__global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_constant__ GParams p) {
+    using G = GGeo<S, NT>;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    __shared__ uint64_t s_bars[2 * 8 + 2 * kGroups + 4];
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_abort, s_last;
+    uint64_t* pfull = s_bars;                        // stage landed            (producer -> dequant warps, MMA warp)
+    uint64_t* pempty = pfull + G::NP;                // stage read              (S groups of warps + the MMAs -> producer)
+    uint64_t* tready = pempty + G::NP;               // tile expanded           (a group's 4 warps -> MMA warp)
+    uint64_t* tfree = tready + kGroups;              // tile's MMAs complete    (tcgen05.commit -> the group)
+    uint64_t* accfull = tfree + kGroups;             // accumulators complete   (tcgen05.commit -> epilogue)
+    uint64_t* accempty = accfull + G::NACC;          // accumulators read       (16 warps -> MMA warp)
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nitems = p.row_items * p.tok_items * p.splits;
+
+    if (threadIdx.x == 0) {
+        s_abort = 0;
+        for (int s = 0; s < G::NP; s++) {
+            mbar_init(smem_u32(pfull + s), LAYOUT == W_TILED ? 1 : 33);      // + the producer lanes' 4-byte copies
+            mbar_init(smem_u32(pempty + s), 4 * S + S);
+        }
+        for (int s = 0; s < kGroups; s++) {
+            mbar_init(smem_u32(tready + s), 4);
+            mbar_init(smem_u32(tfree + s), 1);
+        }
+        for (int s = 0; s < G::NACC; s++) {
+            mbar_init(smem_u32(accfull + s), 2);
+            mbar_init(smem_u32(accempty + s), kDeqWarps);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == kDeqWarps + 2) {                     // the first MMA warp owns the tensor memory (all 512 columns)
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(smem_u32(&s_tmem)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem = s_tmem;
+    volatile int* abort_flag = &s_abort;
+    pdl_launch_dependents();
+
+    if (warp >= kDeqWarps && warp < kDeqWarps + 2) {
+        // ------------------------------------------------------------------ producers: warp i asks for the chunks with number % 2 == i
+        const uint32_t par = __shfl_sync(0xffffffffu, warp - kDeqWarps, 0);
+        const int nchunks = p.K / kChunkK;
+        const int nblocks = (p.N + 63) / 64;
+        bool waited = LAYOUT == W_ROWS;              // (row-major weights may come from the kernel before this one)
+        if (waited) pdl_wait();
+        uint32_t n = 0;                              // chunks of earlier items
+        uint32_t pend = 0;                           // stages of this warp whose activations are still to be asked for
+        bool ok = true;
+        auto load_x = [&](uint32_t s, int c, int tok0) {
+            const uint32_t dst = smem_u32(ring + s * G::STAGE + S * kTileW), bar = smem_u32(pfull + s);
+            tma_box(dst, &p.xmap, c * kChunkK, tok0, bar);
+            tma_box(dst + NT * 128, &p.xmap, c * kChunkK + 64, tok0, bar);
+        };
+        for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
+            const GItem g = g_item(p, item, NT);
+            int c = (int)((par - n) & 1u);
+            // the item's 64-row blocks, one run of 4608 bytes each per chunk (gate blocks, then up blocks)
+            const unsigned char* wsrc[2 * S];
+#pragma unroll
+            for (int i = 0; i < 2 * S; i++)
+                wsrc[i] = p.w[DUAL ? i >> 1 : 0] +
+                          ((size_t)min(DUAL ? g.row_item * 2 + (i & 1) : g.row_item * 2 * S + i, nblocks - 1) * nchunks + g.c_begin + c) * kRunBytes;
+            uint32_t srow[4 * S];                    // row-major: first scale pair of this lane's rows
+#pragma unroll
+            for (int i = 0; i < 4 * S; i++)
+                srow[i] = LAYOUT == W_ROWS ? (uint32_t)min(g.row_item * S * kTileRows + i * 32 + lane, p.N - 1) * (uint32_t)(p.K / 128) : 0u;
+            for (; c < g.nc; c += 2) {
+                const uint32_t slot = (n + c) % G::NP, use = (n + c) / G::NP;
+                if (*abort_flag) { ok = false; break; }
+                if (use > 0 && !__all_sync(0xffffffffu, gwait(smem_u32(pempty + slot), (use - 1) & 1u))) {
+                    if (lane == 0) { *abort_flag = 1; g_error(p, 1); }
+                    ok = false;
+                    break;
+                }
+                const uint32_t bar = smem_u32(pfull + slot);
+                unsigned char* stage = ring + slot * G::STAGE;
+                if (elect_one()) {
+                    mbar_expect_tx(bar, LAYOUT == W_TILED ? G::STAGE : S * 8192 + G::XBYTES);
+                    if (LAYOUT == W_TILED) {
+#pragma unroll
+                        for (int i = 0; i < 2 * S; i++) bulk_copy_g2s(smem_u32(stage + i * kRunBytes), wsrc[i], kRunBytes, bar);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < S; i++)
+                            tma_box(smem_u32(stage + i * kTileW), &p.wmap, (g.c_begin + c) * 16, (g.row_item * S + i) * kTileRows, bar);
+                    }
+                    if (waited) load_x(slot, g.c_begin + c, g.tok0);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 2 * S; i++) wsrc[i] += 2 * kRunBytes;
+                if (LAYOUT == W_ROWS) {
+                    // the chunk's two scales and two biases of every row, 4 bytes each
+                    const uint32_t d0 = smem_u32(stage) + 8192 + lane * 4;
+#pragma unroll
+                    for (int i = 0; i < 4 * S; i++) {
+                        const uint32_t d = d0 + (i >> 2) * kTileW + (i & 3) * 128;
+                        const uint32_t e = srow[i] + (uint32_t)(g.c_begin + c);
+                        cp_async4(d, reinterpret_cast<const uint32_t*>(p.sc) + e);
+                        cp_async4(d + 512, reinterpret_cast<const uint32_t*>(p.bi) + e);
+                    }
+                    cp_async_arrive_noinc(bar);
+                }
+                if (!waited) {
+                    // the first stages' weights do not depend on the kernel before this one, the activations do
+                    pend++;
+                    if (c + 2 >= min(g.nc, (int)G::NP)) {
+                        pdl_wait();
+                        waited = true;
+                        if (elect_one())
+                            for (uint32_t i = 0; i < pend; i++) load_x(par + 2 * i, g.c_begin + (int)(par + 2 * i), g.tok0);
+                        __syncwarp();
+                    }
+                }
+            }
+            n += g.nc;
+            if (!waited) { pdl_wait(); waited = true; }       // (a first item of one chunk leaves the second warp without)
+        }
+        if (!waited) pdl_wait();
+    } else if (warp >= kDeqWarps + 2) {
+        // ------------------------------------------------------------------ MMA issuers (an elected thread each): S = 2: one per row
+        // tile, S = 1: even and odd chunks, each into an accumulator of its own; while one stands at a barrier after its eight
+        // MMAs (~190 cycles) the other's run.
+        const uint32_t me = __shfl_sync(0xffffffffu, warp - (kDeqWarps + 2), 0);
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(kTileRows >> 4) << 24);
+        uint32_t n = 0, it = 0;                          // chunks of earlier items, items
+        bool ok = true;
+        for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x, it++) {
+            const GItem g = g_item(p, item, NT);
+            const uint32_t ab = it % G::NACC, ause = it / G::NACC;
+            if (ause > 0) ok = __all_sync(0xffffffffu, gwait(smem_u32(accempty + ab), (ause - 1) & 1u));
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            const uint32_t d0 = tmem + G::ACC0 + ab * G::ACC + me * NT;
+            bool first = true;
+            for (int c = S == 2 ? 0 : (int)me; c < g.nc && ok; c += S == 2 ? 1 : 2) {
+                const uint32_t tile = (n + c) * S + (S == 2 ? me : 0);            // tile number: group and use of its tensor-memory tile
+                const uint32_t ts = tile % kGroups, slot = (n + c) % G::NP;
+                // (the expanded tile is ready only after its group has seen the whole stage land, the activations included)
+                ok = __all_sync(0xffffffffu, !*abort_flag && gwait(smem_u32(tready + ts), (tile / kGroups) & 1u));
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const uint64_t b0 = sw128_desc(smem_u32(ring + slot * G::STAGE + S * kTileW));
+                const uint32_t a0 = tmem + ts * kTileCols;
+                if (elect_one()) {
+                    const uint32_t accumulate = first ? 0u : 1u;
+#pragma unroll
+                    for (int ks = 0; ks < kChunkK / 16; ks++)
+                        asm volatile(
+                            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d0),
+                            "r"(a0 + ks * 8), "l"(b0 + ((ks >> 2) * (NT * 128) + (ks & 3) * 32) / 16), "r"(idesc), "r"(ks == 0 ? accumulate : 1u)
+                            : "memory");
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(tfree + ts)) : "memory");
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(pempty + slot)) : "memory");
+                }
+                __syncwarp();
+                first = false;
+            }
+            if (ok && elect_one())
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(accfull + ab)) : "memory");
+            __syncwarp();
+            n += g.nc;
+        }
+        if (!ok && lane == 0 && !*abort_flag) { *abort_flag = 1; g_error(p, 2); }
+    } else {
+        // ------------------------------------------------------------------ dequant warps + epilogue
+        const int q = warp & 3;
+        const uint32_t grp = warp >> 2;                   // takes the tiles with number % 4 == grp, into tensor-memory tile grp
+        const int r = q * 32 + lane;                      // weight row inside the tile = tensor-memory lane
+        const int rr = r & 15;
+        const uint32_t rowoff = LAYOUT == W_TILED ? ((r >> 6) * kRunBytes + ((r >> 4) & 3) * kRecBytes + (rr >> 3) * 512 + (rr & 7) * 64) : r * 64;
+        const uint32_t scoff = LAYOUT == W_TILED ? ((r >> 6) * kRunBytes + ((r >> 4) & 3) * kRecBytes + 1024 + rr * 8) : 8192 + r * 4;
+        const uint32_t trow = tmem + grp * kTileCols + ((uint32_t)(q * 32) << 16);
+        uint32_t cbase = 0, tbase = 0, tuse = 0, it = 0;  // chunks and tiles of earlier items, tiles of this group so far, items
+        bool ok = true, pending = false;
+        GItem prev{};
+        auto epilogue = [&]() {
+            const uint32_t ab = (it - 1) % G::NACC;
+            ok = __all_sync(0xffffffffu, ok && !*abort_flag && gwait(smem_u32(accfull + ab), ((it - 1) / G::NACC) & 1u));
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            // (after a timeout too: the warps meet on the same named barriers whatever each of them has seen)
+            gemm_epilogue<S, NT, DUAL>(p, prev, tmem + G::ACC0 + ab * G::ACC, smem_u32(accempty + ab), warp, lane, &s_last, ok);
+            pending = false;
+        };
+        for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+            const GItem g = g_item(p, item, NT);
+            const uint32_t ntiles = g.nc * S;
+            for (uint32_t k = (grp - tbase) & (kGroups - 1); k < ntiles; k += kGroups, tuse++) {
+                const uint32_t n = cbase + k / S, s = k % S;
+                const uint32_t slot = n % G::NP;
+                ok = ok && !*abort_flag && gwait(smem_u32(pfull + slot), (n / G::NP) & 1u);
+                if (ok && tuse > 0) ok = gwait(smem_u32(tfree + grp), (tuse - 1) & 1u);
+                ok = __all_sync(0xffffffffu, ok);
+                if (ok) {
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    const unsigned char* tile = ring + slot * G::STAGE + s * kTileW;
+                    uint4 u[4];
+                    uint32_t sc2[2], bi2[2];              // scale, bias of the chunk's two k groups, low halves
+                    if (LAYOUT == W_TILED) {
+                        // rows are 64 bytes apart: every other pair of rows reads its 16-byte units in the other order, so that
+                        // eight lanes meet in the same banks in pairs only
+                        const int flip = (r >> 1) & 1;
+#pragma unroll
+                        for (int i = 0; i < 4; i += 2) {
+                            const uint4 a = *reinterpret_cast<const uint4*>(tile + rowoff + (i + flip) * 16);
+                            const uint4 b = *reinterpret_cast<const uint4*>(tile + rowoff + (i + 1 - flip) * 16);
+                            u[i] = flip ? b : a;
+                            u[i + 1] = flip ? a : b;
+                        }
+                        const uint2 sb = *reinterpret_cast<const uint2*>(tile + scoff);
+                        sc2[0] = sb.x; bi2[0] = sb.x >> 16;
+                        sc2[1] = sb.y; bi2[1] = sb.y >> 16;
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 4; i++)
+                            u[i] = *reinterpret_cast<const uint4*>(tile + rowoff + ((i ^ ((r >> 1) & 3)) << 4));
+                        const uint32_t sv = *reinterpret_cast<const uint32_t*>(tile + scoff);
+                        const uint32_t bv = *reinterpret_cast<const uint32_t*>(tile + scoff + 512);
+                        sc2[0] = sv; sc2[1] = sv >> 16;
+                        bi2[0] = bv; bi2[1] = bv >> 16;
+                    }
+                    const bool fast = __all_sync(0xffffffffu, fast_scale(sc2[0]) && fast_scale(sc2[1]));
+                    auto expand = [&](auto fast_tag) {
+                        constexpr bool FAST = decltype(fast_tag)::value;
+                        // sixteen columns (32 k values) at a time.  Streaming layout: pack j of unit t is k group 4 j + t;
+                        // row-major: pack t of unit j.
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            __half2 s2 = dup_half((unsigned short)sc2[j >> 1]);
+                            const __half2 b2 = dup_half((unsigned short)bi2[j >> 1]);
+                            if (FAST) s2 = scale_times_2_20(s2);
+                            uint32_t d[4][4];
+#pragma unroll
+                            for (int t = 0; t < 4; t++) {
+                                const uint32_t pack = LAYOUT == W_TILED ? comp(u[t], j) : comp(u[j], t);
+                                if (FAST) dequant_pack_fast(pack, s2, b2, d[t]);
+                                else dequant_pack(pack, s2, b2, d[t]);
+                                if (LAYOUT == W_ROWS) {   // {e0,e4} {e1,e5} {e2,e6} {e3,e7} -> adjacent k pairs
+                                    const uint32_t e01 = __byte_perm(d[t][0], d[t][1], 0x5410), e45 = __byte_perm(d[t][0], d[t][1], 0x7632);
+                                    const uint32_t e23 = __byte_perm(d[t][2], d[t][3], 0x5410), e67 = __byte_perm(d[t][2], d[t][3], 0x7632);
+                                    d[t][0] = e01; d[t][1] = e23; d[t][2] = e45; d[t][3] = e67;
+                                }
+                            }
+                            tmem_st16(trow + 16 * j, d);
+                        }
+                    };
+                    if (fast) expand(std::true_type{});
+                    else expand(std::false_type{});
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(pempty + slot));       // the packs are in registers
+                    asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(tready + grp));
+                }
+                // the item before this one: its epilogue runs once this warp's first tile of this item is expanded
+                if (pending) epilogue();
+            }
+            if (pending) epilogue();
+            cbase += g.nc;
+            tbase += ntiles;
+            prev = g;
+            pending = true;
+            it++;
+            if (it == 1) pdl_wait();                      // before this thread's first global access
+        }
+        if (pending) epilogue();
+        if (!ok && lane == 0 && !*abort_flag) { *abort_flag = 1; g_error(p, 3); }
+    }
+
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (warp == kDeqWarps + 2)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(tmem) : "memory");
+}
+
+// ---- work split: token columns per item, row tiles behind one activation tile, K ranges
+struct GPlan {
+    int S, NT, splits, cps, row_items, tok_items;
+};
+
+int gemm_sms() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    return n;
+}
+
+size_t gemm_partial_bytes(const GPlan& pl) {
+    return pl.splits > 1 ? (size_t)pl.splits * pl.row_items * pl.tok_items * pl.NT * pl.S * kTileRows * sizeof(float) : 0;
+}
+
+// Cost in SM cycles, fitted to measurements on B200 (M 16 .. 1024; N x K of a few thousand): a chunk of one / two row tiles
+// costs 480 / 900 + 5 per token column, an item its fill and epilogue, a K split the partial products out and in (38 bytes a
+// cycle) and the ticket, a launch ~9000.
+GPlan gemm_plan(int M, int N, int K, bool dual, int sms, size_t partial_room) {
+    GPlan best{};
+    double best_cost = 1e30;
+    const int nchunks = K / kChunkK;
+    for (int NT = 16; NT <= 128; NT *= 2) {
+        if (NT < 128 && NT / 2 >= M && NT > 16) break;               // half the columns would do
+        for (int S = dual ? 2 : 1; S <= 2; S++) {
+            const int rows = dual ? kTileRows : S * kTileRows;
+            GPlan pl{};
+            pl.S = S; pl.NT = NT;
+            pl.row_items = (N + rows - 1) / rows;
+            pl.tok_items = (M + NT - 1) / NT;
+            const long long tiles = (long long)pl.row_items * pl.tok_items;
+            const double chunk = (S == 2 ? 900.0 : 480.0) + 5.0 * NT;
+            for (int splits = 1; splits <= std::max(1, nchunks / 2); splits++) {
+                if (splits > 1 && (tiles > kGemmTiles || splits > 32)) break;
+                pl.cps = (nchunks + splits - 1) / splits;
+                pl.splits = (nchunks + pl.cps - 1) / pl.cps;
+                if (pl.splits != splits) continue;
+                if (splits > 1 && gemm_partial_bytes(pl) > partial_room) break;
+                const long long rounds = (tiles * splits + sms - 1) / sms;
+                const double out = std::min(NT, M) * S * 128 * 4.0 / 38.0;    // partial products of an item, cycles
+                const double cost = 9000 + rounds * (pl.cps * chunk + 700 + NT * S * 4.0) + (splits > 1 ? 3400 + rounds * out + out * splits : 0.0);
+                if (cost < best_cost) { best_cost = cost; best = pl; }
+                if (tiles * splits >= 3LL * sms) break;
+            }
+        }
+    }
+    return best;
+}
+
+template <int S, int NT, bool DUAL, int LAYOUT>
+int launch_gemm(const GParams& p, int sms, cudaStream_t stream) {
+    auto kern = qmm_gemm_kernel<S, NT, DUAL, LAYOUT>;
+    static std::atomic<uint64_t> done{0};
+    if (!allow_smem(kern, GGeo<S, NT>::SMEM, done)) return check_launch();
+    const int nitems = p.row_items * p.tok_items * p.splits;
+    launch_kernel(kern, dim3(nitems < sms ? nitems : sms), dim3(kGThreads), (size_t)GGeo<S, NT>::SMEM, stream, p);
+    return check_launch();
+}
+
+template <int S, bool DUAL, int LAYOUT>
+int launch_gemm_nt(const GParams& p, int nt, int sms, cudaStream_t stream) {
+    switch (nt) {
+        case 16: return launch_gemm<S, 16, DUAL, LAYOUT>(p, sms, stream);
+        case 32: return launch_gemm<S, 32, DUAL, LAYOUT>(p, sms, stream);
+        case 64: return launch_gemm<S, 64, DUAL, LAYOUT>(p, sms, stream);
+        default: return launch_gemm<S, 128, DUAL, LAYOUT>(p, sms, stream);
+    }
+}
+
+}  // namespace
+
+size_t qmm_gemm_partial_bytes(int M, int N, int K, bool dual) {
+    return gemm_partial_bytes(gemm_plan(M, N, K, dual, gemm_sms(), (size_t)1 << 40));
+}
+
+int qmm_gemm(const GemmArgs& a, cudaStream_t stream) {
+    const bool dual = a.epilogue == B200_EPI_SILU_MUL, tiled = a.w_tiled != nullptr;
+    const int sms = gemm_sms();
+    const GPlan pl = gemm_plan(a.M, a.N, a.K, dual, sms, a.partial_bytes);
+    GParams p{};
+    int rc = make_map_2d(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a.x, (uint64_t)a.K, (uint64_t)a.M, (uint64_t)a.K * 2, 64, (uint32_t)pl.NT,
+                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+    if (rc != B200_OK) return rc;
+    if (!tiled) {
+        rc = make_map_2d(&p.wmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, a.wq, (uint64_t)a.K / 8, (uint64_t)a.N, (uint64_t)a.K / 2, 16, kTileRows,
+                         CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+        if (rc != B200_OK) return rc;
+    }
+    p.w[0] = static_cast<const unsigned char*>(a.w_tiled);
+    p.w[1] = static_cast<const unsigned char*>(a.w2_tiled);
+    p.sc = static_cast<const __half*>(a.scales);
+    p.bi = static_cast<const __half*>(a.biases);
+    p.bias = static_cast<const __half*>(a.bias);
+    p.extra = static_cast<const __half*>(a.extra);
+    p.y = static_cast<__half*>(a.y);
+    p.counter = a.counters;
+    p.err = a.err;
+    p.partial = static_cast<float*>(a.partial);
+    p.M = a.M; p.N = a.N; p.K = a.K;
+    p.row_items = pl.row_items; p.tok_items = pl.tok_items; p.splits = pl.splits; p.chunks_per_split = pl.cps;
+    p.epilogue = a.epilogue;
+    if (dual) return launch_gemm_nt<2, true, W_TILED>(p, pl.NT, sms, stream);
+    if (tiled) return pl.S == 2 ? launch_gemm_nt<2, false, W_TILED>(p, pl.NT, sms, stream) : launch_gemm_nt<1, false, W_TILED>(p, pl.NT, sms, stream);
+    return pl.S == 2 ? launch_gemm_nt<2, false, W_ROWS>(p, pl.NT, sms, stream) : launch_gemm_nt<1, false, W_ROWS>(p, pl.NT, sms, stream);
+}
+
+}  // namespace b200
+
+extern "C" {
+
+using namespace b200;
+
+size_t b200_qmm_gemm_workspace_bytes(int M, int N, int K, int epilogue) {
+    if (M < 1 || N < 8 || (N % 8) != 0 || K < kChunkK || (K % kChunkK) != 0) return 0;
+    return kCounterBytes + qmm_gemm_partial_bytes(M, N, K, epilogue == B200_EPI_SILU_MUL);
+}
+
+int b200_qmm_gemm(const void* x, const void* wt, const void* wt2, const void* bias, const void* extra, void* y, int M, int N, int K,
+                  int epilogue, void* workspace, size_t workspace_bytes, void* stream) {
+    if (M < 1 || N < 8 || (N % 8) != 0 || K < kChunkK || (K % kChunkK) != 0) return B200_EINVAL;
+    if (epilogue < B200_EPI_NONE || epilogue > B200_EPI_SILU_MUL) return B200_EINVAL;
+    const bool dual = epilogue == B200_EPI_SILU_MUL;
+    if (!x || !wt || !y || !workspace || (dual && (!wt2 || bias)) || (epilogue == B200_EPI_RESIDUAL && (!extra || bias))) return B200_EINVAL;
+    if (!aligned16(x) || !aligned16(wt) || !aligned16(wt2) || !aligned16(y) || !aligned16(bias) || !aligned16(extra) || !aligned16(workspace))
+        return B200_EALIGN;
+    if (workspace_bytes < (size_t)kCounterBytes) return B200_EWORKSPACE;
+    GemmArgs a{};
+    a.x = x; a.w_tiled = wt; a.w2_tiled = wt2; a.bias = bias; a.extra = extra; a.y = y;
+    a.M = M; a.N = N; a.K = K; a.epilogue = epilogue;
+    gemm_workspace(a, workspace, workspace_bytes);
+    return qmm_gemm(a, static_cast<cudaStream_t>(stream));
+}
+
+// The fixed form of round row counts: up to 128 rows, whole 128-row tiles, the error word first in the workspace.
+size_t b200_qmm_umma_workspace_bytes(int M, int K) {
+    if (M < 1 || M > 128 || K < kChunkK || (K % kChunkK) != 0) return 0;
+    return kCounterBytes + kUmmaPartialBytes;
+}
+
+int b200_qmm_umma(const void* x, const void* w_tiled, const void* bias, void* y, int M, int N, int K, void* workspace,
+                  size_t workspace_bytes, void* stream) {
+    if (!x || !w_tiled || !y || !workspace || M < 1 || M > 128 || N < kTileRows || K < kChunkK) return B200_EINVAL;
+    if ((N % kTileRows) != 0 || (K % kChunkK) != 0) return B200_EUNSUPPORTED;
+    if (!aligned16(x) || !aligned16(w_tiled) || !aligned16(y) || !aligned16(workspace) || !aligned16(bias)) return B200_EALIGN;
+    if (workspace_bytes < b200_qmm_umma_workspace_bytes(M, K)) return B200_EWORKSPACE;
+    GemmArgs a{};
+    a.x = x; a.w_tiled = w_tiled; a.bias = bias; a.y = y;
+    a.M = M; a.N = N; a.K = K; a.epilogue = B200_EPI_NONE;
+    gemm_workspace(a, workspace, workspace_bytes);
+    a.err = static_cast<int*>(workspace);
+    a.counters = static_cast<int*>(workspace) + 64;
+    return qmm_gemm(a, static_cast<cudaStream_t>(stream));
+}
+
+}  // extern "C"

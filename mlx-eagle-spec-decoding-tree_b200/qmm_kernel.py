@@ -129,8 +129,8 @@ def matmul_umma(x, wt, n, *, bias=None, out=None):
         raise _lib.B200Error("b200_qmm_umma: need 1 <= M <= 128 and K a multiple of 128")
     key = (x.device, torch.cuda.current_stream(x.device).cuda_stream)
     ws = _umma_ws.get(key)
-    if ws is None or ws.numel() < need:
-        ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=x.device)
+    if ws is None:               # (one size for every shape: it never moves, captured graphs may keep its address)
+        ws = torch.zeros(need, dtype=torch.uint8, device=x.device)
         _umma_ws[key] = ws
     rc = _lib.lib().b200_qmm_umma(_lib.ptr(x), _lib.ptr(wt), _lib.ptr(bias), _lib.ptr(y), m, n, k, _lib.ptr(ws),
                                   ws.numel(), _lib.stream_ptr(x.device))
