@@ -820,7 +820,7 @@ def main():
     prompt_host = torch.randint(0, vocab, (PROMPT,), generator=g, dtype=torch.int32).pin_memory()
 
     # ---- time to the first token: pinned host prompt -> both models ingest it -> first greedy token on the host
-    dec.prefill(prompt_host)            # untimed: records the CUDA graphs of the 128-row prompt passes for these caches
+    dec.prefill(prompt_host)            # untimed: allocates the buffers of the prompt passes
     torch.cuda.synchronize()
     t0 = time.perf_counter()
     dec.prefill(prompt_host)

@@ -360,6 +360,38 @@ int b200_forward(const b200_forward_desc* desc, void* stream);
  * hint.  The same string is read once from the environment variable B200_FWD_PLAN.  No counterpart in the reference. */
 void b200_forward_plan_hint(const char* spec);
 
+/* One causal pass of n prompt tokens (any n >= 1) after `off` committed cache rows: embedding, every layer, and the vocabulary
+ * projection of all rows, of the last one or of none.  Host-side launch loop over b200_qmm_gemm and the element-wise and
+ * attention kernels between the matmuls; nothing is allocated, nothing is synchronised.  Replaces the prompt chunks of
+ * mlx_eagle.py:522-535 through mlx_llama.py:231-249,298-313.  Weights in the streaming layout, the embedding in MLX's.
+ * Sizes as b200_forward (hidden, intermediate, n_heads * head_dim multiples of 128, hidden <= 8192, head_dim 64 or 128,
+ * vocab % 8 == 0).  The descriptor and `layers` are HOST memory: n_layers entries of 8 device pointers in the order of
+ * b200_forward_desc.layer_table. */
+typedef struct b200_prefill_desc {
+    int n, off;
+    int hidden, intermediate, n_heads, n_kv_heads, head_dim, vocab, n_layers, cache_rows;
+    float rms_eps, rope_scaling, attn_scale;
+    int head_out;               /* 0: cache rows only, 1: logits of all n rows, 2: logits of the last row */
+    const int* tokens;          /* [n] */
+    const float* inv_freq;
+    const uint32_t* embed_wq;
+    const void* embed_scales;
+    const void* embed_biases;
+    const void* final_norm;
+    const void* lm_head_tiled;
+    const void* const* layers;
+    void* h;                    /* scratch, fp16: [n][hidden] */
+    void* xn;                   /* [n][hidden] */
+    void* qkv;                  /* [n][(n_heads + 2 n_kv_heads) * head_dim] */
+    void* attn;                 /* [n][n_heads * head_dim] */
+    void* act;                  /* [n][intermediate] */
+    void* logits;               /* [n or 1][vocab] */
+    void* kv_cache;             /* [n_layers][2][n_kv_heads][cache_rows][head_dim] */
+    void* workspace;            /* as b200_qmm_gemm's; what exceeds 4 KiB holds partial sums (16 MiB serve every size well) */
+    size_t workspace_bytes;
+} b200_prefill_desc;
+int b200_prefill(const b200_prefill_desc* desc, void* stream);
+
 /* ------------------------------------------------------------------------------------------
  * Draft tree, acceptance and compaction.  One request; k = 8 children per node.
  * ctl is int32[16]: [0] committed length of the target cache, [1] of the draft cache, [2] accept

@@ -132,6 +132,8 @@ def _declare(l: ctypes.CDLL) -> None:
     l.b200_tp_argmax_combine.argtypes = [vp, i32, ctypes.c_uint, i32, i32, ctypes.POINTER(ctypes.c_void_p), vp]
     l.b200_forward.restype = i32
     l.b200_forward.argtypes = [ctypes.POINTER(ForwardDesc), vp]
+    l.b200_prefill.restype = i32
+    l.b200_prefill.argtypes = [ctypes.POINTER(PrefillDesc), vp]
     l.b200_add_f16.restype = i32
     l.b200_add_f16.argtypes = [vp, vp, sz, vp]
     l.b200_silu_mul_f16.restype = i32
@@ -159,6 +161,18 @@ class ForwardDesc(ctypes.Structure):
            ("phase_mask", ctypes.c_int), ("tp_world", ctypes.c_int), ("tp_rank", ctypes.c_int),
            ("head_rows", ctypes.c_int), ("grid_ctas", ctypes.c_int), ("tp_peers", ctypes.c_void_p * 8),
            ("scales_in_fast_range", ctypes.c_int), ("tp_two_shot", ctypes.c_int), ("requests", ctypes.c_int)])
+
+
+class PrefillDesc(ctypes.Structure):
+    """Mirror of ``b200_prefill_desc``."""
+    _fields_ = ([(n, ctypes.c_int) for n in (
+        "n", "off", "hidden", "intermediate", "n_heads", "n_kv_heads", "head_dim", "vocab", "n_layers", "cache_rows")]
+        + [(n, ctypes.c_float) for n in ("rms_eps", "rope_scaling", "attn_scale")]
+        + [("head_out", ctypes.c_int)]
+        + [(n, ctypes.c_void_p) for n in (
+            "tokens", "inv_freq", "embed_wq", "embed_scales", "embed_biases", "final_norm", "lm_head_tiled", "layers", "h",
+            "xn", "qkv", "attn", "act", "logits", "kv_cache", "workspace")]
+        + [("workspace_bytes", ctypes.c_size_t)])
 
 
 def check(rc: int, what: str) -> None:

@@ -1,5 +1,5 @@
 """The large-M tensor-core matmul (b200_qmm_gemm, and b200_qmm beyond 32 rows) at the edges of its tiles, against the fp64
-gold of the CPU oracle."""
+gold of the CPU oracle; prompt passes that cut the key range against the 32-row passes."""
 import numpy as np
 import pytest
 import torch
@@ -74,3 +74,22 @@ def test_operator_beyond_32_rows_matches_gold(be, cuda, m, n, k):
     odd.copy_(packed[1])
     y2 = be.matmul(x.to(cuda), args[0], odd, args[2], 64, bias=bias.to(cuda))[0]
     assert torch.allclose(y.float(), y2.float(), rtol=2.0 ** -9, atol=2e-3)
+
+
+@pytest.mark.parametrize("name,cached,n", [("tiny-qwen2", 700, 33), ("tiny-llama", 1500, 100), ("tiny-llama", 0, 1100)])
+def test_prompt_chunk_on_a_filled_cache_matches_the_32_row_passes(be, cuda, name, cached, n):
+    """Key range cut across CTAs (few tokens, long cache), and more tokens than one pass takes."""
+    m = be.Model.random_init(be.shape_preset(name), 5, cuda, gen_device="cpu").relayout()
+    cache = m.make_cache(64 * ((cached + n + 127) // 64))
+    g = torch.Generator().manual_seed(3)
+    cache.data[:, :, :, :cached] = torch.randn(cache.data[:, :, :, :cached].shape, generator=g).half().to(cuda)
+    tokens = torch.randint(0, m.args.vocab_size, (1, n), generator=g)
+    cache.offset = cached
+    got = m(tokens, cache)[0].float()
+    kv = cache.data.clone()
+    m.prefill_large_m = False
+    cache.offset = cached
+    want = m(tokens, cache)[0].float()
+    m.check_fused_error()
+    assert torch.all((got - want).abs() <= 2.0 ** -6 * want.abs() + 2e-2)
+    assert torch.all((kv.float() - cache.data.float()).abs() <= 2.0 ** -6 * cache.data.float().abs() + 2e-2)
