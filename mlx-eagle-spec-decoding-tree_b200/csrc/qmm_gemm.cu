@@ -6,8 +6,8 @@
 // Item = (S x 128 weight rows, NT tokens, K range).  S = 2 puts two row tiles (or the gate and the up tile of the same
 // rows) behind one activation tile, so an activation byte brought into shared memory feeds 256 weight rows.
 //
-//   producer warp    per 128-k chunk: the weights (records of the streaming layout, or TMA boxes of the row-major layout
-//                    plus 4-byte asynchronous copies of its scales and biases) and the activations (two TMA boxes of
+//   2 producer warps per 128-k chunk: the weights (records of the streaming layout, or TMA boxes of the row-major layout,
+//                    whose scales and biases the dequant threads load themselves, ahead) and the activations (two TMA boxes of
 //                    64 k x NT rows, 128-byte swizzle, straight from row-major x; rows past M read as zero);
 //   16 dequant warps in four groups that take the tiles (row tile, chunk) in turn, thread = weight row: exact q*s+b rounded
 //                    once to fp16, written with tcgen05.st into the group's own tensor-memory tile (lane = weight row,
@@ -59,11 +59,13 @@ constexpr int kGemmTiles = 896;                  // tiles that a K split can han
 // Layouts of the weights
 enum { W_TILED = 0, W_ROWS = 1 };
 
-template <int S, int NT>
+template <int S, int NT, int LAYOUT>
 struct GGeo {
     static constexpr int XBYTES = NT * kChunkK * 2;                   // two boxes of 64 k
     static constexpr int STAGE = S * kTileW + XBYTES;                 // a multiple of 1024: the boxes stay swizzle-aligned
-    static constexpr int FIT = (232448 - 2048) / STAGE;
+    // Row-major scales are read through L1, a 32-byte sector of a row serving eight chunks if it survives until then: half of
+    // the SM's memory is left to it (64 x 4096 x 14336: 35 us with a full ring, 26 us so).
+    static constexpr int FIT = LAYOUT == W_ROWS ? std::max(4, 112 * 1024 / STAGE) : (232448 - 2048) / STAGE;
     // Ring stages: an even number, so that a stage belongs to one of the two producers (and, with S = 1, to one of the two MMA
     // warps).  Even and odd chunks may drift apart; with an odd ring a wait could then meet a phase two uses away.
     static constexpr int NP = FIT < 8 ? (FIT & ~1) : 8;
@@ -76,13 +78,14 @@ struct GGeo {
 
 struct GParams {
     CUtensorMap xmap;            // x [M][K], boxes of 64 k x NT rows, 128-byte swizzle
-    CUtensorMap wmap;            // row-major weights [N][K/8] words, boxes of 16 words x 128 rows, 64-byte swizzle
+    CUtensorMap wmap[2];         // row-major weights [N][K/8] words, boxes of 16 words x 128 rows, 64-byte swizzle (gate / up)
     const unsigned char* w[2];   // streaming layout (gate / up)
-    const __half* sc;            // row-major layout: scales, biases [N][K/64]
-    const __half* bi;
+    const __half* sc[2];         // row-major layout: scales, biases [N][K/64]
+    const __half* bi[2];
+    int sb_pairs;                // their addresses are multiples of four: the two of a chunk can be loaded together
     const __half* bias;
     const __half* extra;         // residual [M][N] (may be y)
-    __half* y;
+    __half* y;                   // [M][N]; float with B200_EPI_F32
     int* counter;                // split tickets, one per tile, zero between launches
     int* err;                    // error word or NULL
     float* partial;
@@ -103,10 +106,6 @@ __device__ __forceinline__ void tma_box(uint32_t dst, const void* tmap, int x, i
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
                  ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(src) : "memory");
-}
-
 __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&d)[4][4]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(addr),
                  "r"(d[0][0]), "r"(d[0][1]), "r"(d[0][2]), "r"(d[0][3]), "r"(d[1][0]), "r"(d[1][1]), "r"(d[1][2]), "r"(d[1][3]),
@@ -154,7 +153,7 @@ template <int S, int NT, bool DUAL>
 __device__ __forceinline__ void gemm_epilogue(const GParams& p, const GItem& g, uint32_t acc, uint32_t accempty, int warp,
                                               int lane, int* s_last, bool ok) {
     constexpr int CG = (DUAL ? NT : S * NT) / 4;         // columns (of each matrix) per warp
-    constexpr int CM = DUAL ? 8 : 16;
+    constexpr int CM = (DUAL || S == 1) ? 8 : 16;        // (two accumulators per column there)
     constexpr int CH = CG < CM ? CG : CM;                // columns per trip
     const int q = warp & 3, cg = warp >> 2;
     const int s = DUAL ? 0 : (cg * CG) / NT;
@@ -261,11 +260,20 @@ __device__ __forceinline__ void gemm_epilogue(const GParams& p, const GItem& g, 
             for (int i = 0; i < CH; i++) r[i] = i < cnt ? __ldcg(reinterpret_cast<const unsigned short*>(rs) + (size_t)i * p.N) : 0;
 #pragma unroll
             for (int i = 0; i < CH; i++)
-                if (i < cnt) dst[(size_t)i * p.N] = __hadd(__ushort_as_half(r[i]), __float2half_rn(__uint_as_float(a[i])));
+                if (i < cnt) {
+                    __half o = __float2half_rn(__uint_as_float(a[i]));
+                    if (p.bias != nullptr) o = __hadd(o, bv);
+                    dst[(size_t)i * p.N] = __hadd(__ushort_as_half(r[i]), o);
+                }
         } else if (DUAL) {
 #pragma unroll
             for (int i = 0; i < CH; i++)
                 if (i < cnt) dst[(size_t)i * p.N] = __float2half_rn(silu_mul_f16(__uint_as_float(a[i]), __uint_as_float(b[i])));
+        } else if (p.epilogue == B200_EPI_F32) {
+            float* out = reinterpret_cast<float*>(p.y) + (size_t)tok * p.N + row;
+#pragma unroll
+            for (int i = 0; i < CH; i++)
+                if (i < cnt) out[(size_t)i * p.N] = __uint_as_float(a[i]);
         } else {
 #pragma unroll
             for (int i = 0; i < CH; i++)
@@ -280,7 +288,7 @@ __device__ __forceinline__ void gemm_epilogue(const GParams& p, const GItem& g, 
 
 template <int S, int NT, bool DUAL, int LAYOUT>
 __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_constant__ GParams p) {
-    using G = GGeo<S, NT>;
+    using G = GGeo<S, NT, LAYOUT>;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ uint64_t s_bars[2 * 8 + 2 * kGroups + 4];
@@ -299,7 +307,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
     if (threadIdx.x == 0) {
         s_abort = 0;
         for (int s = 0; s < G::NP; s++) {
-            mbar_init(smem_u32(pfull + s), LAYOUT == W_TILED ? 1 : 33);      // + the producer lanes' 4-byte copies
+            mbar_init(smem_u32(pfull + s), 1);
             mbar_init(smem_u32(pempty + s), 4 * S + S);
         }
         for (int s = 0; s < kGroups; s++) {
@@ -347,10 +355,6 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
             for (int i = 0; i < 2 * S; i++)
                 wsrc[i] = p.w[DUAL ? i >> 1 : 0] +
                           ((size_t)min(DUAL ? g.row_item * 2 + (i & 1) : g.row_item * 2 * S + i, nblocks - 1) * nchunks + g.c_begin + c) * kRunBytes;
-            uint32_t srow[4 * S];                    // row-major: first scale pair of this lane's rows
-#pragma unroll
-            for (int i = 0; i < 4 * S; i++)
-                srow[i] = LAYOUT == W_ROWS ? (uint32_t)min(g.row_item * S * kTileRows + i * 32 + lane, p.N - 1) * (uint32_t)(p.K / 128) : 0u;
             for (; c < g.nc; c += 2) {
                 const uint32_t slot = (n + c) % G::NP, use = (n + c) / G::NP;
                 if (*abort_flag) { ok = false; break; }
@@ -369,25 +373,14 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
                     } else {
 #pragma unroll
                         for (int i = 0; i < S; i++)
-                            tma_box(smem_u32(stage + i * kTileW), &p.wmap, (g.c_begin + c) * 16, (g.row_item * S + i) * kTileRows, bar);
+                            tma_box(smem_u32(stage + i * kTileW), &p.wmap[DUAL ? i : 0], (g.c_begin + c) * 16,
+                                    (DUAL ? g.row_item : g.row_item * S + i) * kTileRows, bar);
                     }
                     if (waited) load_x(slot, g.c_begin + c, g.tok0);
                 }
                 __syncwarp();
 #pragma unroll
                 for (int i = 0; i < 2 * S; i++) wsrc[i] += 2 * kRunBytes;
-                if (LAYOUT == W_ROWS) {
-                    // the chunk's two scales and two biases of every row, 4 bytes each
-                    const uint32_t d0 = smem_u32(stage) + 8192 + lane * 4;
-#pragma unroll
-                    for (int i = 0; i < 4 * S; i++) {
-                        const uint32_t d = d0 + (i >> 2) * kTileW + (i & 3) * 128;
-                        const uint32_t e = srow[i] + (uint32_t)(g.c_begin + c);
-                        cp_async4(d, reinterpret_cast<const uint32_t*>(p.sc) + e);
-                        cp_async4(d + 512, reinterpret_cast<const uint32_t*>(p.bi) + e);
-                    }
-                    cp_async_arrive_noinc(bar);
-                }
                 if (!waited) {
                     // the first stages' weights do not depend on the kernel before this one, the activations do
                     pend++;
@@ -456,8 +449,25 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
         const int r = q * 32 + lane;                      // weight row inside the tile = tensor-memory lane
         const int rr = r & 15;
         const uint32_t rowoff = LAYOUT == W_TILED ? ((r >> 6) * kRunBytes + ((r >> 4) & 3) * kRecBytes + (rr >> 3) * 512 + (rr & 7) * 64) : r * 64;
-        const uint32_t scoff = LAYOUT == W_TILED ? ((r >> 6) * kRunBytes + ((r >> 4) & 3) * kRecBytes + 1024 + rr * 8) : 8192 + r * 4;
+        const uint32_t scoff = (r >> 6) * kRunBytes + ((r >> 4) & 3) * kRecBytes + 1024 + rr * 8;
         const uint32_t trow = tmem + grp * kTileCols + ((uint32_t)(q * 32) << 16);
+        // Row-major layout: this row's scales and biases of a chunk, loaded one tile ahead.
+        uint32_t sb_s = 0, sb_b = 0;
+        auto load_sb = [&](const GItem& g, uint32_t k) {
+            const uint32_t s = k % S;
+            const int tile_row = DUAL ? g.row_item : g.row_item * S + (int)s;
+            const size_t e = (size_t)min(tile_row * kTileRows + r, p.N - 1) * (p.K / 64) + (g.c_begin + k / S) * 2;
+            const __half *sp = p.sc[DUAL ? s : 0] + e, *bp = p.bi[DUAL ? s : 0] + e;
+            if (p.sb_pairs) {
+                sb_s = __ldg(reinterpret_cast<const uint32_t*>(sp));
+                sb_b = __ldg(reinterpret_cast<const uint32_t*>(bp));
+            } else {
+                const unsigned short *su = reinterpret_cast<const unsigned short*>(sp), *bu = reinterpret_cast<const unsigned short*>(bp);
+                sb_s = __ldg(su) | (uint32_t)__ldg(su + 1) << 16;
+                sb_b = __ldg(bu) | (uint32_t)__ldg(bu + 1) << 16;
+            }
+        };
+        if (LAYOUT == W_ROWS) pdl_wait();                 // (the kernel before this one may have written the weights)
         uint32_t cbase = 0, tbase = 0, tuse = 0, it = 0;  // chunks and tiles of earlier items, tiles of this group so far, items
         bool ok = true, pending = false;
         GItem prev{};
@@ -472,7 +482,9 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
         for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
             const GItem g = g_item(p, item, NT);
             const uint32_t ntiles = g.nc * S;
-            for (uint32_t k = (grp - tbase) & (kGroups - 1); k < ntiles; k += kGroups, tuse++) {
+            const uint32_t k0 = (grp - tbase) & (kGroups - 1);
+            if (LAYOUT == W_ROWS && k0 < ntiles) load_sb(g, k0);
+            for (uint32_t k = k0; k < ntiles; k += kGroups, tuse++) {
                 const uint32_t n = cbase + k / S, s = k % S;
                 const uint32_t slot = n % G::NP;
                 ok = ok && !*abort_flag && gwait(smem_u32(pfull + slot), (n / G::NP) & 1u);
@@ -501,8 +513,8 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
 #pragma unroll
                         for (int i = 0; i < 4; i++)
                             u[i] = *reinterpret_cast<const uint4*>(tile + rowoff + ((i ^ ((r >> 1) & 3)) << 4));
-                        const uint32_t sv = *reinterpret_cast<const uint32_t*>(tile + scoff);
-                        const uint32_t bv = *reinterpret_cast<const uint32_t*>(tile + scoff + 512);
+                        const uint32_t sv = sb_s, bv = sb_b;
+                        if (k + kGroups < ntiles) load_sb(g, k + kGroups);
                         sc2[0] = sv; sc2[1] = sv >> 16;
                         bi2[0] = bv; bi2[1] = bv >> 16;
                     }
@@ -566,12 +578,6 @@ struct GPlan {
     int S, NT, splits, cps, row_items, tok_items;
 };
 
-int gemm_sms() {
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    return n;
-}
-
 size_t gemm_partial_bytes(const GPlan& pl) {
     return pl.splits > 1 ? (size_t)pl.splits * pl.row_items * pl.tok_items * pl.NT * pl.S * kTileRows * sizeof(float) : 0;
 }
@@ -600,7 +606,7 @@ GPlan gemm_plan(int M, int N, int K, bool dual, int sms, size_t partial_room) {
                 if (pl.splits != splits) continue;
                 if (splits > 1 && gemm_partial_bytes(pl) > partial_room) break;
                 const long long rounds = (tiles * splits + sms - 1) / sms;
-                const double out = std::min(NT, M) * S * 128 * 4.0 / 38.0;    // partial products of an item, cycles
+                const double out = std::min(NT, (M + 15) & ~15) * S * 128 * 4.0 / 38.0;    // partial products of an item, cycles
                 const double cost = 9000 + rounds * (pl.cps * chunk + 700 + NT * S * 4.0) + (splits > 1 ? 3400 + rounds * out + out * splits : 0.0);
                 if (cost < best_cost) { best_cost = cost; best = pl; }
                 if (tiles * splits >= 3LL * sms) break;
@@ -614,9 +620,9 @@ template <int S, int NT, bool DUAL, int LAYOUT>
 int launch_gemm(const GParams& p, int sms, cudaStream_t stream) {
     auto kern = qmm_gemm_kernel<S, NT, DUAL, LAYOUT>;
     static std::atomic<uint64_t> done{0};
-    if (!allow_smem(kern, GGeo<S, NT>::SMEM, done)) return check_launch();
+    if (!allow_smem(kern, GGeo<S, NT, LAYOUT>::SMEM, done)) return check_launch();
     const int nitems = p.row_items * p.tok_items * p.splits;
-    launch_kernel(kern, dim3(nitems < sms ? nitems : sms), dim3(kGThreads), (size_t)GGeo<S, NT>::SMEM, stream, p);
+    launch_kernel(kern, dim3(nitems < sms ? nitems : sms), dim3(kGThreads), (size_t)GGeo<S, NT, LAYOUT>::SMEM, stream, p);
     return check_launch();
 }
 
@@ -632,6 +638,16 @@ int launch_gemm_nt(const GParams& p, int nt, int sms, cudaStream_t stream) {
 
 }  // namespace
 
+int gemm_sms() {
+    static std::atomic<int> known[64];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+    if ((n = known[dev & 63].load(std::memory_order_relaxed)) > 0) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    known[dev & 63].store(n, std::memory_order_relaxed);
+    return n;
+}
+
 size_t qmm_gemm_partial_bytes(int M, int N, int K, bool dual) {
     return gemm_partial_bytes(gemm_plan(M, N, K, dual, gemm_sms(), (size_t)1 << 40));
 }
@@ -644,15 +660,19 @@ int qmm_gemm(const GemmArgs& a, cudaStream_t stream) {
     int rc = make_map_2d(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a.x, (uint64_t)a.K, (uint64_t)a.M, (uint64_t)a.K * 2, 64, (uint32_t)pl.NT,
                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
     if (rc != B200_OK) return rc;
-    if (!tiled) {
-        rc = make_map_2d(&p.wmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, a.wq, (uint64_t)a.K / 8, (uint64_t)a.N, (uint64_t)a.K / 2, 16, kTileRows,
+    for (int i = 0; !tiled && i < (dual ? 2 : 1); i++) {
+        rc = make_map_2d(&p.wmap[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, a.wq[i], (uint64_t)a.K / 8, (uint64_t)a.N, (uint64_t)a.K / 2, 16, kTileRows,
                          CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
         if (rc != B200_OK) return rc;
     }
     p.w[0] = static_cast<const unsigned char*>(a.w_tiled);
     p.w[1] = static_cast<const unsigned char*>(a.w2_tiled);
-    p.sc = static_cast<const __half*>(a.scales);
-    p.bi = static_cast<const __half*>(a.biases);
+    p.sb_pairs = 1;
+    for (int i = 0; i < 2; i++) {
+        p.sc[i] = static_cast<const __half*>(a.scales[i]);
+        p.bi[i] = static_cast<const __half*>(a.biases[i]);
+        if ((reinterpret_cast<uintptr_t>(a.scales[i]) | reinterpret_cast<uintptr_t>(a.biases[i])) & 3u) p.sb_pairs = 0;
+    }
     p.bias = static_cast<const __half*>(a.bias);
     p.extra = static_cast<const __half*>(a.extra);
     p.y = static_cast<__half*>(a.y);
@@ -662,7 +682,7 @@ int qmm_gemm(const GemmArgs& a, cudaStream_t stream) {
     p.M = a.M; p.N = a.N; p.K = a.K;
     p.row_items = pl.row_items; p.tok_items = pl.tok_items; p.splits = pl.splits; p.chunks_per_split = pl.cps;
     p.epilogue = a.epilogue;
-    if (dual) return launch_gemm_nt<2, true, W_TILED>(p, pl.NT, sms, stream);
+    if (dual) return tiled ? launch_gemm_nt<2, true, W_TILED>(p, pl.NT, sms, stream) : launch_gemm_nt<2, true, W_ROWS>(p, pl.NT, sms, stream);
     if (tiled) return pl.S == 2 ? launch_gemm_nt<2, false, W_TILED>(p, pl.NT, sms, stream) : launch_gemm_nt<1, false, W_TILED>(p, pl.NT, sms, stream);
     return pl.S == 2 ? launch_gemm_nt<2, false, W_ROWS>(p, pl.NT, sms, stream) : launch_gemm_nt<1, false, W_ROWS>(p, pl.NT, sms, stream);
 }

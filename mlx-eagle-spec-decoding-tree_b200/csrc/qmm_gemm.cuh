@@ -10,12 +10,12 @@ struct GemmArgs {
     const void* x;               // [M][K] fp16, row-major
     const void* w_tiled;         // streaming layout, or NULL: row-major weights below
     const void* w2_tiled;        // up_proj (B200_EPI_SILU_MUL)
-    const uint32_t* wq;          // row-major packed weights, scales, biases
-    const void* scales;
-    const void* biases;
+    const uint32_t* wq[2];       // row-major packed weights, scales, biases (gate / up)
+    const void* scales[2];
+    const void* biases[2];
     const void* bias;            // [N] or NULL
     const void* extra;           // residual [M][N] (B200_EPI_RESIDUAL)
-    void* y;                     // [M][N]
+    void* y;                     // [M][N]; float with B200_EPI_F32
     int M, N, K;
     int epilogue;
     int* counters;               // 896 tickets of the K split, zero before first use, restored by every launch
@@ -26,13 +26,14 @@ struct GemmArgs {
 
 // The library's usual workspace: 4 KiB of counters (the last one the error word), then the partial products.
 inline void gemm_workspace(GemmArgs& a, void* workspace, size_t bytes) {
-    if (workspace == nullptr || bytes <= (size_t)kCounterBytes) return;
+    if (workspace == nullptr || bytes < (size_t)kCounterBytes) return;
     a.counters = static_cast<int*>(workspace);
     a.err = a.counters + kMaxCounters - 1;
     a.partial = static_cast<char*>(workspace) + kCounterBytes;
     a.partial_bytes = bytes - kCounterBytes;
 }
 
+int gemm_sms();                  // SMs of the current device
 size_t qmm_gemm_partial_bytes(int M, int N, int K, bool dual);
 
 
