@@ -8,12 +8,14 @@ torch; the library only sees raw device pointers and the current CUDA stream.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 
 import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libb200eagle.so")
+OPS_PATH = os.path.join(_HERE, "_b200ops.so")
 
 E_NAMES = {-1: "EINVAL (bad shape/size/flags)", -2: "EALIGN (pointer not 16-byte aligned)",
            -3: "EUNSUPPORTED (dtype/group size)", -4: "EWORKSPACE (workspace too small)",
@@ -38,6 +40,22 @@ def lib() -> ctypes.CDLL:
         if os.environ.get("B200_PDL", "1") == "0":
             _lib.b200_set_pdl(0)
     return _lib
+
+
+_ops = None
+
+
+def ops():
+    """The native operator module (``csrc/ops.cpp``); like the library, it has to have been built."""
+    global _ops
+    if _ops is None:
+        lib()
+        if not os.path.exists(OPS_PATH):
+            raise B200Error(f"{OPS_PATH} is missing: build it first (python {os.path.join(_HERE, 'build.py')}).")
+        spec = importlib.util.spec_from_file_location("_b200ops", OPS_PATH)
+        _ops = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(_ops)
+    return _ops
 
 
 def _declare(l: ctypes.CDLL) -> None:

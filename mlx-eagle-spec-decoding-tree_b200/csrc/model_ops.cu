@@ -1,6 +1,8 @@
 // Small per-token kernels of one decoder layer: quantised embedding gather, RMSNorm, and
 // tree-position RoPE fused with the KV-cache append.  All are tiny (<= 32 tokens), HBM/launch
 // bound; they exist so that a whole forward pass stays on the device with no host decisions.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace b200 {
@@ -174,6 +176,46 @@ __global__ void rope_positions_kernel(const __half* __restrict__ in, const int* 
     out[base + i + D / 2] = __float2half_rn(x1 * s + x2 * c);
 }
 
+// The same for D % 16 == 0 (16-byte vectors): one CTA per token and block of heads; the token's cos / sin are computed once per
+// CTA instead of once per head, a thread rotates one vector pair (i, i + D/2) of one head.  What bounds it: launch latency up to
+// a few MB, then HBM (a (4, 64, 512, 128) tensor: 67 MB in and out).
+constexpr int kRopeThreads = 256;
+__global__ void __launch_bounds__(kRopeThreads) rope_positions_vec_kernel(const __half* __restrict__ in, const int* __restrict__ offsets,
+                                                                          const float* __restrict__ inv_freq, float scaling,
+                                                                          __half* __restrict__ out, int H, int Lq, int D) {
+    pdl_wait();
+    pdl_launch_dependents();
+    extern __shared__ float2 cs[];
+    const int l = blockIdx.x, b = blockIdx.z;
+    const float pos = (float)offsets[(size_t)b * Lq + l];
+    for (int i = threadIdx.x; i < D / 2; i += kRopeThreads) {
+        float s, c;
+        sincosf((scaling * inv_freq[i]) * pos, &s, &c);
+        cs[i] = make_float2(c, s);
+    }
+    __syncthreads();
+    const int hv = D / 16, heads = max(1, kRopeThreads / hv);            // heads per CTA
+    const int h_end = min(H, ((int)blockIdx.y + 1) * heads);
+    for (int i = threadIdx.x; i < heads * hv; i += kRopeThreads) {
+        const int h = blockIdx.y * heads + i / hv, c0 = (i % hv) * 8;
+        if (h >= h_end) break;
+        const size_t at = (((size_t)b * H + h) * Lq + l) * D + c0;
+        const uint4 a = *reinterpret_cast<const uint4*>(in + at), d = *reinterpret_cast<const uint4*>(in + at + D / 2);
+        const __half* x1 = reinterpret_cast<const __half*>(&a);
+        const __half* x2 = reinterpret_cast<const __half*>(&d);
+        __align__(16) __half r1[8], r2[8];
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            const float2 t = cs[c0 + e];
+            const float f1 = __half2float(x1[e]), f2 = __half2float(x2[e]);
+            r1[e] = __float2half_rn(f1 * t.x - f2 * t.y);
+            r2[e] = __float2half_rn(f1 * t.y + f2 * t.x);
+        }
+        *reinterpret_cast<uint4*>(out + at) = *reinterpret_cast<const uint4*>(r1);
+        *reinterpret_cast<uint4*>(out + at + D / 2) = *reinterpret_cast<const uint4*>(r2);
+    }
+}
+
 }  // namespace
 }  // namespace b200
 
@@ -239,6 +281,13 @@ int b200_rope_positions(const void* in, const int* offsets, const float* inv_fre
                         void* out, int B, int H, int L, int D, void* stream) {
     if (!in || !offsets || !inv_freqs || !out) return B200_EINVAL;
     if (B < 1 || H < 1 || L < 1 || D < 2 || (D % 2) != 0 || D > 2048 || H > 65535 || B > 65535) return B200_EINVAL;
+    if (D % 16 == 0 && b200::aligned16(in) && b200::aligned16(out)) {
+        const int heads = std::max(1, b200::kRopeThreads / (D / 16));
+        b200::launch_kernel(b200::rope_positions_vec_kernel, dim3(L, (H + heads - 1) / heads, B), dim3(b200::kRopeThreads),
+                            (size_t)(D / 2) * sizeof(float2), static_cast<cudaStream_t>(stream), static_cast<const __half*>(in), offsets,
+                            inv_freqs, scaling_factor, static_cast<__half*>(out), H, L, D);
+        return b200::check_launch();
+    }
     dim3 grid(L, H, B);
     b200::launch_kernel(b200::rope_positions_kernel, dim3(grid), dim3(D / 2), 0, static_cast<cudaStream_t>(stream), static_cast<const __half*>(in), offsets, inv_freqs, scaling_factor, static_cast<__half*>(out), H, L, D);
     return b200::check_launch();

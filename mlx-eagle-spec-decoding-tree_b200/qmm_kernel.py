@@ -47,6 +47,12 @@ def _check_operands(x, w, s, b, group_size):
 
 def matmul(x, w, s, b, group_size=64, d_dtype=torch.float16, bias=None, **_ignored):
     """``[x @ dequant(w, s, b).T]`` with x ``(*B, K)`` fp16 and w ``(N, K/8)`` packed 4-bit."""
+    if d_dtype is torch.float16 and isinstance(x, torch.Tensor):
+        ws = _workspaces.get(x.device.index)
+        if ws is not None:
+            y = _lib.ops().qmm(x, w, s, b, group_size, bias, ws)
+            if y is not None:
+                return [y]
     _check_operands(x, w, s, b, group_size)
     if d_dtype != torch.float16:
         raise _lib.B200Error("only float16 output is implemented")
@@ -100,6 +106,12 @@ def relayout(w, s, b) -> torch.Tensor:
 
 def matmul_tiled(x, wt, n, *, epilogue=EPI_NONE, wt2=None, bias=None, extra=None, out=None):
     """``x (M<=32, K) @ W.T`` on re-laid-out weights ``wt`` (from ``relayout``) of ``n`` output rows."""
+    if epilogue == EPI_NONE and out is None and isinstance(x, torch.Tensor):
+        ws = _workspaces.get(x.device.index)
+        if ws is not None:
+            y = _lib.ops().qmm_tiled(x, wt, n, bias, ws)
+            if y is not None:
+                return y
     _lib.require_cuda(x, wt)
     m, k = x.shape
     y = out if out is not None else torch.empty((m, n), dtype=torch.float16, device=x.device)

@@ -16,6 +16,9 @@ from . import _lib
 
 def rope_positions(inp: torch.Tensor, offsets: torch.Tensor, inv_freqs: torch.Tensor, scaling_factor: float = 1.0,
                    verbose: bool = False) -> torch.Tensor:
+    out = _lib.ops().rope_positions(inp, offsets, inv_freqs, scaling_factor)
+    if out is not None:
+        return out
     _lib.require_cuda(inp, offsets, inv_freqs)
     if inp.dtype != torch.float16 or inp.dim() != 4:
         raise _lib.B200Error("rope_positions expects a float16 (B, H, L, D) tensor")

@@ -171,3 +171,30 @@ def test_tiled_rows_do_not_depend_on_batch_size(be, cuda):
     y8 = be.qmm_kernel.matmul_tiled(x.to(cuda), wt, 1152)
     y1 = be.qmm_kernel.matmul_tiled(x[3:4].to(cuda), wt, 1152)
     assert torch.equal(y8[3:4], y1)
+
+
+def test_native_call_and_python_path_agree(be, cuda):
+    """The native operator call takes the plain case; gaps in memory and other layouts go through Python: same results."""
+    w, x = _case(264, 256, 6, 31)
+    wq, s, b = (t.to(cuda) for t in be.quantize.quantize(w))
+    bias = torch.randn(264, generator=torch.Generator().manual_seed(1)).half().to(cuda)
+    xd = x.to(cuda).reshape(2, 3, 256)
+    want = be.matmul(xd, wq, s, b, 64, bias=bias)[0]
+    assert want.shape == (2, 3, 264)
+    gaps = torch.zeros(2, 3, 512, dtype=torch.float16, device=cuda)[:, :, ::2]
+    gaps.copy_(xd)
+    assert be._lib.ops().qmm(gaps, wq, s, b, 64, bias, be.qmm_kernel.workspace(cuda)) is None
+    assert torch.equal(be.matmul(gaps, wq, s, b, 64, bias=bias)[0], want)
+
+
+@pytest.mark.parametrize("b,h,l,d", [(1, 32, 31, 128), (2, 3, 5, 64), (1, 70, 2, 16), (1, 2, 3, 20), (1, 5, 1, 4096 // 2)])
+def test_rope_positions_vector_and_scalar_kernels(be, cuda, b, h, l, d):
+    g = torch.Generator().manual_seed(d)
+    x = torch.randn(b, h, l, d, generator=g).half()
+    pos = torch.randint(0, 4096, (b, l), generator=g, dtype=torch.int32)
+    inv = 1e4 ** (-torch.arange(0, d, 2).float() / d)
+    y = be.rope_positions(x.to(cuda), pos.to(cuda), inv.to(cuda), 0.5).cpu().float()
+    theta = (0.5 * inv.double()) * pos[:, None, :, None].double()
+    x1, x2 = x[..., : d // 2].double(), x[..., d // 2:].double()
+    want = torch.cat([x1 * theta.cos() - x2 * theta.sin(), x1 * theta.sin() + x2 * theta.cos()], -1)
+    assert torch.all((y.double() - want).abs() <= 2.0 ** -10 * want.abs() + 4e-3)
