@@ -319,8 +319,11 @@ typedef struct b200_forward_desc {
                                  * prefix[r], its own head-row offset row_index[r] (if row_index is given) and its own slab
                                  * of kv_cache, laid out [requests][layers][2][kv heads][cache_rows][head_dim]; write_off
                                  * and tail apply to each; attention never crosses requests; rows_out counts rows per
-                                 * request and logits is [requests * rows_out][vocab].  Needs cache_rows <= 2048 (single-
-                                 * phase attention) and tp_world <= 1. */
+                                 * request and logits is [requests * rows_out][vocab].  Needs cache_rows <= 2048 and
+                                 * tp_world <= 1. */
+    const void* const* layers_host;     /* HOST copy of layer_table (n_layers * 8 device pointers), read during the call.
+                                 * NULL: copied from layer_table by this call, which then synchronises with the device and
+                                 * must not run inside a stream capture.  Not needed with tp_world > 1. */
 } b200_forward_desc;
 
 size_t b200_forward_workspace_bytes(const b200_forward_desc* desc);

@@ -51,13 +51,15 @@ inline void launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t 
 
 // Lets `kern` use `bytes` of dynamic shared memory: a per-device attribute, set once per device (`done`: one bit each, a static
 // of the caller's).
+// `whole`: prefer the largest shared-memory carve-out, for kernels meant to have two CTAs on an SM.
 template <typename F>
-inline bool allow_smem(F kern, size_t bytes, std::atomic<uint64_t>& done) {
+inline bool allow_smem(F kern, size_t bytes, std::atomic<uint64_t>& done, bool whole = false) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return false;
     const uint64_t bit = 1ull << (dev & 63);
     if (done.load(std::memory_order_acquire) & bit) return true;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return false;
+    if (whole && cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess) return false;
     done.fetch_or(bit, std::memory_order_release);
     return true;
 }

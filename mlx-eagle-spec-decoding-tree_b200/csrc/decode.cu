@@ -1,0 +1,980 @@
+// One forward pass of the 4-bit decoder for up to 32 tokens as a chain of five kernels per layer (programmatic dependent
+// launch; the whole step is replayed from a CUDA graph):
+//
+//   embedding | per layer  A  q|k|v matmul (+ bias), RoPE, KV append      B  tree-masked attention
+//                          C  o_proj matmul + residual                    D  gate / up matmul, SiLU(gate) * up
+//                          E  down_proj matmul + residual                 | vocabulary projection
+//
+// Why a chain and not one persistent kernel: a kernel of such a chain whose every CTA reads what all CTAs of its predecessor
+// wrote costs 1.0 us, the load included; a device-wide barrier of 148 CTAs took 1.5 to 2.3 us and the first loads behind it
+// another 1.1.  A CTA here keeps to half of an SM (480 threads, 64 registers each, ~95 KB of shared memory, 256 columns of tensor memory), so
+// the next kernel's CTAs become resident beside it and stream and expand their first weights before its results are there.
+//
+// RMSNorm is folded into the matmuls around it: the producer of h (embedding, C, E) also writes h * w_norm (fp16, one
+// rounding) and sums of h^2 per 32 columns; the consumer multiplies its fp32 accumulator by rsqrt(mean(h^2) + eps).
+// All other rounding points are those of the per-op kernels.
+//
+// Replaces Model.__call__ (mlx_llama.py:298-313) for <= 32 tokens.  Every wait is bounded; one that gives up sets the error
+// word of the workspace and the kernel runs to its end.  No copy uses cluster multicast.
+#include <cuda.h>
+
+#include <algorithm>
+#include <atomic>
+#include <type_traits>
+
+#include "common.cuh"
+#include "decode.cuh"
+#include "pipeline.cuh"
+#include "qmm_common.cuh"
+#include "tensor_map.cuh"
+
+namespace b200 {
+namespace {
+
+constexpr float kLog2e = 1.4426950408889634f;
+constexpr int kRun = 4 * 1152;                   // the four records of a 64-row block for one chunk
+constexpr int kW = 2 * kRun;                     // weight bytes of a 128-row tile and chunk
+constexpr int kTile = 128;                       // weight rows of one MMA
+constexpr int kGroups = 3;                       // groups of four dequant warps, each with a tensor-memory tile of its own
+constexpr int kDeq = 4 * kGroups;                // dequant warps
+constexpr int kEpi = 8;                          // of which these run the epilogue
+constexpr int kDThreads = (kDeq + 3) * 32;       // + weight producer, activation producer, MMA issuer
+constexpr int kTCols = kChunkK / 2;              // tensor-memory columns of an expanded tile
+constexpr int kTmem = 256;                       // columns a CTA takes: two CTAs share an SM
+constexpr int kRedPitch = kTile + 4;             // floats per token row of the partial products in shared memory
+constexpr int kMaxCluster = 8;
+constexpr int kSsqPitch = 32, kCsPitch = 64, kKeyBlock = 64;
+constexpr uint32_t kDWaitPolls = 1u << 19;       // about a microsecond each
+
+enum { D_QKV = 0, D_RESID = 1, D_SILU = 2, D_HEAD = 3 };
+
+template <int NT>
+struct DGeo {
+    static constexpr int X = NT * kChunkK * 2;                  // activations of a chunk: two boxes of 64 k
+    static constexpr int ACC = kGroups * kTCols;                  // accumulator columns: two of NT
+    static constexpr int NW = 2 * kGroups;                       // weight stages (a multiple: a stage belongs to one of the groups)
+    static constexpr int NX = NT == 16 ? 6 : 4;                  // activation stages
+    static constexpr int XOFF = NW * kW;
+    static constexpr int INBOX = XOFF + NX * X;                  // partial products [source rank][token of this CTA][kRedPitch] fp32
+    static constexpr int SMEM = INBOX + (NT + kMaxCluster) * kRedPitch * 4 + 1024;
+    static_assert(XOFF % 1024 == 0 && 2 * (SMEM + 3072) <= 227 * 1024 && ACC + 2 * NT <= kTmem, "two CTAs per SM");
+};
+
+struct DenseParams {
+    CUtensorMap xmap;             // activations [M][K], boxes of 64 k x NT rows, 128-byte swizzle
+    const unsigned char* w[2];    // streaming layout (gate / up)
+    const __half* bias;
+    const __half* wn;             // norm weights applied to the new h (D_RESID)
+    __half* y;                    // q|k|v, activations or logits
+    __half* h;                    // residual stream (D_RESID)
+    __half* hw;
+    float* ssq;                   // [H / 32][32]
+    int H;
+    float eps;
+    int M, N, K;                  // N: output rows of each matrix
+    int tile_lo, tiles;           // 128-row tiles (64 + 64 rows of gate and up): first and end
+    int* err;
+    // D_QKV
+    const float2* cs;             // [token][hd / 2] (cos, sin)
+    __half* kc;                   // this layer's K and V of request 0
+    __half* vc;
+    const int* prefix;
+    int Hq, Hkv, hd, cap, write_off, mr;
+    size_t req_stride;            // halves between the caches of two requests
+    // D_HEAD
+    const int* row_index;
+    int rows_out;
+};
+
+// Bounded; once a wait of the CTA has given up (`abort`) the others do so at their next poll, and the kernel runs to its end on
+// whatever is there, in bounds, with the error word set.  No caller leaves its loop for it: the loops stay warp-uniform, so the
+// operands of copies and MMAs stay in uniform registers (eight MMAs and two commits: 290 cycles instead of 560).
+__device__ __forceinline__ void dwait(uint32_t bar, uint32_t parity, volatile int* abort, int* err, int code) {
+    bool ok = mbar_try_wait(bar, parity);
+    for (uint32_t i = 0; !ok && i < kDWaitPolls && !*abort; i++) ok = mbar_try_wait(bar, parity);
+    if (!ok && !*abort) {
+        *abort = 1;
+        atomicCAS(err, 0, code);
+    }
+}
+
+__device__ __forceinline__ uint64_t sw128(uint32_t saddr) {     // K-major, 128-byte swizzle: groups of 8 rows 1024 bytes apart
+    return (uint64_t)((saddr & 0x3ffffu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
+           ((uint64_t)2 << 61);
+}
+__device__ __forceinline__ void tma_box(uint32_t dst, const void* tmap, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
+                 ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void commit_to(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool fast_scale(uint32_t bits) { return ((bits >> 10) & 31u) - 1u < 10u; }   // range of dequant_pack_fast
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;\n" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ uint32_t peer_addr(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_async(uint32_t addr, uint32_t v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];\n" ::"r"(addr), "r"(v), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void arrive_peer(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool inbox_wait(uint32_t bar) {      // phase 0, with what the peers stored before they arrived
+    for (uint32_t i = 0; i < kDWaitPolls; i++) {
+        uint32_t ok;
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n selp.u32 %0, 1, 0, p;\n}\n"
+                     : "=r"(ok) : "r"(bar) : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void st_peer2(uint32_t addr, float x, float y) {
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};\n" ::"r"(addr), "f"(x), "f"(y) : "memory");
+}
+
+// ================================================================================ matmul kernel
+// Grid: 128-row tiles x cluster ranks; the cluster's CTAs share a tile's K range.  Each finishes its share of the token
+// columns: the others store their fp32 partial products for it straight into its shared memory and arrive at its barrier (a
+// cluster barrier and reading them from there took 1 us more).
+//
+// Three groups of four dequant warps (thread = weight row) take the chunks in turn, each with a tensor-memory tile; one MMA warp
+// follows in order.  Three chunks are expanded before the wait for the previous kernel: behind it
+// come the activation load (0.5 us), the MMAs (0.1 us a chunk) and the epilogue.  Code that runs once per kernel is kept short:
+// cold instructions cost 2 to 4 cycles each.
+template <int NT, int KIND>
+__global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_constant__ DenseParams p) {
+    using G = DGeo<NT>;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    float* inbox = reinterpret_cast<float*>(ring + G::INBOX);
+    __shared__ uint64_t wfull[G::NW], wempty[G::NW], xfull[G::NX], xempty[G::NX], tready[kGroups], tfree[kGroups], accfull[2], accempty[2], inboxfull;
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_abort;
+    __shared__ float s_part[kEpi][32];
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank(), cs = cluster_size();
+    const int tile0 = p.tile_lo + blockIdx.x / (int)cs, tstep = gridDim.x / (int)cs;
+    const int nit = cs > 1 ? 1 : (p.tiles - tile0 + tstep - 1) / tstep;                                   // this CTA's tiles: tile0, + tstep, ...
+    const int nchunks = p.K / kChunkK;
+    const int c_lo = nchunks * (int)rank / (int)cs, nc = nchunks * ((int)rank + 1) / (int)cs - c_lo;      // chunks of each
+    const int ntok = p.M > (int)rank ? (p.M - (int)rank + (int)cs - 1) / (int)cs : 0;                     // and tokens: rank, rank + cs, ...
+
+    if (threadIdx.x == 0) {
+        asm volatile("prefetch.tensormap [%0];\n" ::"l"(&p.xmap) : "memory");
+        s_abort = 0;
+        for (int s = 0; s < G::NW; s++) {
+            mbar_init(smem_u32(wfull + s), 1);
+            mbar_init(smem_u32(wempty + s), 4);                 // a group's warps
+        }
+        for (int s = 0; s < G::NX; s++) {
+            mbar_init(smem_u32(xfull + s), 1);
+            mbar_init(smem_u32(xempty + s), 1);
+        }
+        for (int s = 0; s < kGroups; s++) {
+            mbar_init(smem_u32(tready + s), 4);
+            mbar_init(smem_u32(tfree + s), 1);
+        }
+        for (int s = 0; s < 2; s++) {
+            mbar_init(smem_u32(accfull + s), 1);
+            mbar_init(smem_u32(accempty + s), kEpi);
+        }
+        mbar_init(smem_u32(&inboxfull), 1);
+        if (cs > 1) mbar_expect_tx(smem_u32(&inboxfull), cs * ntok * kTile * 4);     // what the cluster's CTAs will store here
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == kDeq + 2) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s_tmem)), "n"(kTmem) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem = s_tmem;
+    volatile int* abort_flag = &s_abort;
+    pdl_launch_dependents();
+    if (cs > 1) cluster_arrive();                                // (waited for before the first store to a peer)
+
+    if (warp == kDeq) {
+        // ------------------------------------------------------------------ weight producer: depends on nothing
+        const int nblocks = (p.N + 63) / 64;
+        uint32_t slot = 0, ph = 1;
+        bool lap = false;
+        for (int it = 0, tile = tile0; it < nit; it++, tile += tstep) {
+            const unsigned char* src0 = p.w[0] + ((size_t)(KIND == D_SILU ? tile : min(2 * tile, nblocks - 1)) * nchunks + c_lo) * kRun;
+            const unsigned char* src1 = KIND == D_SILU ? p.w[1] + ((size_t)tile * nchunks + c_lo) * kRun         // the same 64 rows of up
+                                                       : p.w[0] + ((size_t)min(2 * tile + 1, nblocks - 1) * nchunks + c_lo) * kRun;
+#pragma unroll 1
+            for (int c = 0; c < nc; c++) {
+                if (lap) dwait(smem_u32(wempty + slot), ph, abort_flag, p.err, 21);
+                __syncwarp();
+                if (elect_one()) {
+                    const uint32_t bar = smem_u32(wfull + slot), dst = smem_u32(ring + slot * kW);
+                    mbar_expect_tx(bar, kW);
+                    bulk_copy_g2s(dst, src0, kRun, bar);
+                    bulk_copy_g2s(dst + kRun, src1, kRun, bar);
+                }
+                __syncwarp();
+                src0 += kRun;
+                src1 += kRun;
+                if (++slot == (uint32_t)G::NW) { slot = 0; ph ^= 1; lap = true; }
+            }
+        }
+    } else if (warp == kDeq + 1) {
+        // ------------------------------------------------------------------ activation producer
+        pdl_wait();
+        uint32_t slot = 0, ph = 1;
+        bool lap = false;
+        for (int it = 0; it < nit; it++)
+#pragma unroll 1
+            for (int c = 0; c < nc; c++) {
+                if (lap) dwait(smem_u32(xempty + slot), ph, abort_flag, p.err, 26);
+                __syncwarp();
+                if (elect_one()) {
+                    const uint32_t bar = smem_u32(xfull + slot), dst = smem_u32(ring + G::XOFF + slot * G::X);
+                    mbar_expect_tx(bar, G::X);
+                    tma_box(dst, &p.xmap, (c_lo + c) * kChunkK, 0, bar);
+                    tma_box(dst + NT * 128, &p.xmap, (c_lo + c) * kChunkK + 64, 0, bar);
+                }
+                __syncwarp();
+                if (++slot == (uint32_t)G::NX) { slot = 0; ph ^= 1; lap = true; }
+            }
+    } else if (warp == kDeq + 2) {
+        // ------------------------------------------------------------------ MMA issuer (an elected thread)
+        constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(kTile >> 4) << 24);
+        const uint64_t xdesc = sw128(smem_u32(ring + G::XOFF));
+        uint32_t tl = 0, tph = 0, slot = 0, xph = 0;
+#pragma unroll 1
+        for (int it = 0; it < nit; it++) {
+            const uint32_t ab = it & 1, d0 = tmem + G::ACC + ab * NT;
+            if (it >= 2) dwait(smem_u32(accempty + ab), ((it >> 1) - 1) & 1, abort_flag, p.err, 27);
+#pragma unroll 1
+            for (int c = 0; c < nc; c++) {
+                dwait(smem_u32(xfull + slot), xph, abort_flag, p.err, 22);
+                dwait(smem_u32(tready + tl), tph, abort_flag, p.err, 22);
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                __syncwarp();
+                if (elect_one()) {                               // (~285 cycles a batch; of half the size, 280)
+                    const uint64_t b0 = xdesc + slot * (G::X / 16);
+                    const uint32_t a0 = tmem + tl * kTCols;
+                    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d0),
+                                 "r"(a0), "l"(b0), "r"(idesc), "r"(c) : "memory");
+#pragma unroll
+                    for (int ks = 1; ks < kChunkK / 16; ks++)
+                        asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.b32 p, 0, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d0),
+                                     "r"(a0 + ks * 8), "l"(b0 + ((ks >> 2) * (NT * 128) + (ks & 3) * 32) / 16), "r"(idesc) : "memory");
+                    commit_to(smem_u32(tfree + tl));
+                    commit_to(smem_u32(xempty + slot));
+                    if (c == nc - 1) commit_to(smem_u32(accfull + ab));
+                }
+                __syncwarp();
+                if (++tl == (uint32_t)kGroups) { tl = 0; tph ^= 1; }
+                if (++slot == (uint32_t)G::NX) { slot = 0; xph ^= 1; }
+            }
+        }
+        asm volatile("bar.sync 2, %0;\n" ::"n"((kEpi + 1) * 32) : "memory");         // accumulators read
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(kTmem) : "memory");
+    } else {
+        // ------------------------------------------------------------------ dequant warps
+        const uint32_t me = warp >> 2;                           // group (and, in the epilogue, which half of the tokens)
+        const int q = warp & 3, r = q * 32 + lane, rr = r & 15;
+        const uint32_t recoff = (r >> 6) * kRun + ((r >> 4) & 3) * 1152;
+        const uint32_t rowoff = recoff + (rr >> 3) * 512 + (rr & 7) * 64, scoff = recoff + 1024 + rr * 8;
+        const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
+        const int flip = (r >> 1) & 1;                           // (bank conflicts: see qmm_gemm.cu)
+        constexpr bool NORMED = KIND != D_RESID;                 // the input is h * w_norm: scale by 1 / rms
+        bool waited = false;
+        float rs_lane = 1.f;                                     // 1 / rms of token `lane`
+        auto dependent = [&]() {
+            // the tiles expanded so far wait for the activations: so does this thread, then takes its share of the sums of squares
+            pdl_wait();
+            waited = true;
+            if (NORMED && warp < kEpi) {
+                float ssum = 0.f;
+                if (lane < p.M) {
+#pragma unroll 4
+                    for (int part = warp; part < p.H / 32; part += kEpi) ssum += __ldcg(p.ssq + part * kSsqPitch + lane);
+                }
+                s_part[warp][lane] = ssum;
+            }
+        };
+        // ---- one finished tile: accumulators -> inbox of the CTA that finishes each token -> output
+        auto epilogue = [&](int it) {
+            const int tile = tile0 + it * tstep;
+            const uint32_t ab = it & 1;
+            const int r2 = KIND == D_SILU ? threadIdx.x & 63 : threadIdx.x & 127;     // row inside the tile that this thread finishes
+            const int j0 = KIND == D_SILU ? threadIdx.x >> 6 : threadIdx.x >> 7;      // its first token of this CTA's, and the step
+            constexpr int JS = KIND == D_SILU ? 4 : 2;
+            const int n = (KIND == D_SILU ? tile * 64 : tile * kTile) + r2;
+            const bool valid = n < p.N;
+            // what the output needs besides the product, asked for now: norm weight or bias, the first token's residual or rotation
+            const int half = p.hd >> 1, hi = r2 & (p.hd - 1), head = KIND == D_QKV ? n >> (p.hd == 128 ? 7 : 6) : 0;
+            const bool rotate = KIND == D_QKV && head < p.Hq + p.Hkv, first = hi < half;
+            const int pr = rotate ? (first ? r2 + half : r2 - half) : r2;      // the row it is rotated with, inside this tile
+            __half extra = __ushort_as_half(0), extra2 = __ushort_as_half(0);
+            auto ask_h = [&](int j) -> unsigned short {
+                return KIND == D_RESID && valid && j < ntok ? __ldcg(reinterpret_cast<const unsigned short*>(p.h) + (size_t)((int)rank + j * (int)cs) * p.N + n) : 0;
+            };
+            auto ask_r = [&](int j) -> float2 {
+                return KIND == D_QKV && rotate && j < ntok ? __ldcg(p.cs + ((int)rank + j * (int)cs) * kCsPitch + (first ? hi : hi - half)) : make_float2(0.f, 0.f);
+            };
+            if (KIND == D_RESID && valid) extra = p.wn[n];
+            if (KIND == D_QKV && valid && p.bias != nullptr) {
+                extra = p.bias[n];
+                extra2 = p.bias[tile * kTile + pr];
+            }
+            unsigned short h0 = ask_h(j0), h1 = ask_h(j0 + JS);
+            float2 t0 = ask_r(j0), t1 = ask_r(j0 + JS);
+
+            dwait(smem_u32(accfull + ab), (it >> 1) & 1, abort_flag, p.err, 23);
+            __syncwarp();
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            constexpr int C = NT / 2;                            // columns of this warp
+            uint32_t a[C];
+#pragma unroll
+            for (int i = 0; i < C; i += 8)
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                             : "=r"(a[i]), "=r"(a[i + 1]), "=r"(a[i + 2]), "=r"(a[i + 3]), "=r"(a[i + 4]), "=r"(a[i + 5]), "=r"(a[i + 6]), "=r"(a[i + 7])
+                             : "r"(tmem + G::ACC + ab * NT + me * C + i + ((uint32_t)(q * 32) << 16)) : "memory");
+            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            if (it == nit - 1) asm volatile("bar.arrive 2, %0;\n" ::"n"((kEpi + 1) * 32) : "memory");     // tensor memory may be given back
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(accempty + ab));
+            const int nslot = (p.M + (int)cs - 1) / (int)cs;     // tokens per source in an inbox
+            if (cs == 1) {
+                if (it > 0) consumer_sync(kEpi * 32);            // the tile before this one has been read
+#pragma unroll
+                for (int i = 0; i < C; i++)
+                    if ((int)me * C + i < p.M) inbox[((int)me * C + i) * kRedPitch + r] = __uint_as_float(a[i]);
+                consumer_sync(kEpi * 32);
+            } else {
+                // a store into a peer's memory counts its bytes at the peer's barrier by itself: no fence, no arrival behind it
+                cluster_wait();
+                const uint32_t in0 = smem_u32(inbox), inbar = smem_u32(&inboxfull);
+                uint32_t dst = (me * C) % cs, sl = (me * C) / cs;
+#pragma unroll
+                for (int i = 0; i < C; i++) {
+                    if ((int)me * C + i < p.M)
+                        st_async(peer_addr(in0 + ((rank * nslot + sl) * kRedPitch + r) * 4, dst), a[i], peer_addr(inbar, dst));
+                    if (++dst == cs) { dst = 0; sl++; }
+                }
+                if (NORMED) consumer_sync(kEpi * 32);            // s_part
+                if (!inbox_wait(inbar)) atomicCAS(p.err, 0, 28);     // (in full after a timeout too: a peer may still be storing here)
+                __syncwarp();
+            }
+            if (NORMED && it == 0) {
+                float t = 0.f;
+#pragma unroll
+                for (int i = 0; i < kEpi; i++) t += s_part[i][lane];
+                rs_lane = rsqrtf(t / (float)p.H + p.eps);
+            }
+            auto total = [&](int j, int row) {                   // the sources in rank order
+                const float* v = inbox + j * kRedPitch + row;
+                float t = v[0];
+#pragma unroll 1
+                for (int i = 1; i < (int)cs; i++) t += v[i * nslot * kRedPitch];
+                return t;
+            };
+#pragma unroll 1
+            for (int j = j0; j < ntok; j += JS) {                // (warp-uniform)
+                const int tok = (int)rank + j * (int)cs;
+                const float rs = NORMED ? __shfl_sync(0xffffffffu, rs_lane, tok) : 1.f;
+                const float v = total(j, r2) * rs;
+                const int rq = KIND == D_HEAD || KIND == D_QKV ? (p.mr == p.M ? 0 : tok / p.mr) : 0;
+                if (KIND == D_SILU) {
+                    const float up = total(j, r2 + 64) * rs;
+                    if (valid) p.y[(size_t)tok * p.N + n] = __float2half_rn(silu_mul_f16(v, up));
+                } else if (KIND == D_RESID) {
+                    float ss = 0.f;
+                    if (valid) {
+                        const size_t at = (size_t)tok * p.N + n;
+                        const __half o = __hadd(__ushort_as_half(h0), __float2half_rn(v));
+                        const float f = __half2float(o);
+                        ss = f * f;
+                        p.h[at] = o;
+                        p.hw[at] = __hmul(o, extra);
+                    }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                    if (lane == 0 && valid) p.ssq[(n >> 5) * kSsqPitch + tok] = ss;
+                    h0 = h1;
+                    h1 = ask_h(j + 2 * JS);
+                } else if (KIND == D_HEAD) {
+                    const int rel = tok - rq * p.mr - (p.row_index ? p.row_index[rq] : 0);
+                    if (valid && rel >= 0 && rel < p.rows_out) p.y[(size_t)(rq * p.rows_out + rel) * p.N + n] = __float2half_rn(v);
+                } else {
+                    __half x = __float2half_rn(v);
+                    if (p.bias != nullptr) x = __hadd(x, extra);
+                    if (rotate) {
+                        __half y = __float2half_rn(total(j, pr) * rs);
+                        if (p.bias != nullptr) y = __hadd(y, extra2);
+                        const float xs = __half2float(x), ys = __half2float(y);
+                        x = __float2half_rn(first ? xs * t0.x - ys * t0.y : ys * t0.y + xs * t0.x);
+                    }
+                    if (valid) {
+                        if (head < p.Hq) {
+                            p.y[(size_t)tok * p.N + n] = x;
+                        } else {
+                            const int row = p.prefix[rq] + p.write_off + (tok - rq * p.mr);
+                            const int kvh = head - p.Hq - (rotate ? 0 : p.Hkv);
+                            if (row < p.cap) ((rotate ? p.kc : p.vc) + (size_t)rq * p.req_stride)[((size_t)kvh * p.cap + row) * p.hd + hi] = x;
+                        }
+                    }
+                    t0 = t1;
+                    t1 = ask_r(j + 2 * JS);
+                }
+            }
+        };
+        uint32_t slot = me, wph = 0, tph = 1;
+        int done = me;                                           // number of this group's next chunk, over all tiles
+#pragma unroll 1
+        for (int it = 0; it <= nit; it++) {
+            const int end = it < nit ? (it + 1) * nc : 0;
+            bool pending = it > 0;                               // the tile before this one, once this one's first chunk is expanded
+#pragma unroll 1
+            do {
+                if (done < end) {
+                    if (done >= kGroups && !waited) dependent();
+                    dwait(smem_u32(wfull + slot), wph, abort_flag, p.err, 24);
+                    __syncwarp();
+                    const unsigned char* st = ring + slot * kW;
+                    uint4 u[4];
+#pragma unroll
+                    for (int i = 0; i < 4; i += 2) {
+                        const uint4 a = *reinterpret_cast<const uint4*>(st + rowoff + (i + flip) * 16);
+                        const uint4 b = *reinterpret_cast<const uint4*>(st + rowoff + (i + 1 - flip) * 16);
+                        u[i] = flip ? b : a;
+                        u[i + 1] = flip ? a : b;
+                    }
+                    const uint2 sb = *reinterpret_cast<const uint2*>(st + scoff);
+                    const bool fast = __all_sync(0xffffffffu, fast_scale(sb.x) && fast_scale(sb.y));
+                    if (lane == 0) mbar_arrive(smem_u32(wempty + slot));             // the packs are in registers
+                    if (done >= kGroups) dwait(smem_u32(tfree + me), tph, abort_flag, p.err, 24);
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    __syncwarp();
+                    auto expand = [&](auto fast_tag) {
+                        constexpr bool FAST = decltype(fast_tag)::value;
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {            // pack j of unit t = k group 4 j + t
+                            const uint32_t s = j < 2 ? sb.x : sb.y;
+                            __half2 s2 = dup_half((unsigned short)s);
+                            const __half2 b2 = dup_half((unsigned short)(s >> 16));
+                            if (FAST) s2 = scale_times_2_20(s2);
+                            uint32_t d[4][4];
+#pragma unroll
+                            for (int t = 0; t < 4; t++) {
+                                if (FAST) dequant_pack_fast(comp(u[t], j), s2, b2, d[t]);
+                                else dequant_pack(comp(u[t], j), s2, b2, d[t]);
+                            }
+                            asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(trow + me * kTCols + 16 * j),
+                                         "r"(d[0][0]), "r"(d[0][1]), "r"(d[0][2]), "r"(d[0][3]), "r"(d[1][0]), "r"(d[1][1]), "r"(d[1][2]), "r"(d[1][3]),
+                                         "r"(d[2][0]), "r"(d[2][1]), "r"(d[2][2]), "r"(d[2][3]), "r"(d[3][0]), "r"(d[3][1]), "r"(d[3][2]), "r"(d[3][3]) : "memory");
+                        }
+                    };
+                    if (fast) expand(std::true_type{});
+                    else expand(std::false_type{});
+                    asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(tready + me));
+                    done += kGroups;
+                    if ((slot += kGroups) >= (uint32_t)G::NW) { slot -= G::NW; wph ^= 1; }
+                    tph ^= 1;
+                }
+                if (pending) {
+                    if (!waited) dependent();
+                    if (warp < kEpi) epilogue(it - 1);
+                    pending = false;
+                }
+            } while (done < end);
+        }
+        return;
+    }
+    if (cs > 1) cluster_wait();
+}
+
+// ================================================================================ embedding
+// One CTA per token: dequantised embedding row -> h, h * w_norm, sums of squares per 32 columns, and the token's RoPE table.
+// The next kernel is let go only behind the wait: everything before the pass (tree kernels, KV compaction, other programs'
+// writes) is then complete before any kernel of the pass starts, which may so read committed K/V rows ahead of its own wait.
+__global__ void __launch_bounds__(256) embed_kernel(const int* __restrict__ tokens, const int* __restrict__ pos, const uint32_t* __restrict__ wq,
+                                                    const __half* __restrict__ sc, const __half* __restrict__ bi, const __half* __restrict__ wn,
+                                                    __half* __restrict__ h, __half* __restrict__ hw, float* __restrict__ ssq,
+                                                    float2* __restrict__ cs, const float* __restrict__ inv_freq, float scaling, int H, int V,
+                                                    int half_hd) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int m = blockIdx.x, units = H / 8;
+    const int tok = min(max(tokens[m], 0), V - 1);
+    for (int u = threadIdx.x; u < ((units + 31) & ~31); u += 256) {
+        float ss = 0.f;
+        if (u < units) {
+            const uint32_t w = wq[(size_t)tok * units + u];
+            const __half s = sc[(size_t)tok * (H / 64) + (u >> 3)], b = bi[(size_t)tok * (H / 64) + (u >> 3)];
+            const uint4 wv = *reinterpret_cast<const uint4*>(wn + u * 8);
+            const __half* wh = reinterpret_cast<const __half*>(&wv);
+            __align__(16) __half o[8], ow[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                o[j] = __hfma(__int2half_rn((int)((w >> (4 * j)) & 0xfu)), s, b);
+                const float f = __half2float(o[j]);
+                ss += f * f;
+                ow[j] = __hmul(o[j], wh[j]);
+            }
+            *reinterpret_cast<uint4*>(h + (size_t)m * H + u * 8) = *reinterpret_cast<const uint4*>(o);
+            *reinterpret_cast<uint4*>(hw + (size_t)m * H + u * 8) = *reinterpret_cast<const uint4*>(ow);
+        }
+        ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+        ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+        if (u < units && (u & 3) == 0) ssq[(u >> 2) * kSsqPitch + m] = ss;
+    }
+    if ((int)threadIdx.x < half_hd) {
+        float s, c;
+        sincosf((scaling * inv_freq[threadIdx.x]) * (float)pos[m], &s, &c);
+        cs[m * kCsPitch + threadIdx.x] = make_float2(c, s);
+    }
+}
+
+// ================================================================================ attention
+// CTA = (key range, kv head, request, set of 32, 64 or 128 query rows): a query row is (token, head of the group), a warp has 16
+// of them and all keys of a block or, where fewer rows leave warps over, a half or a quarter; all share the K/V blocks (TMA boxes, 128-byte
+// swizzle, three blocks of 64 keys in flight).  The CTAs of a cluster take
+// neighbouring key ranges; each finishes its share of the rows, whose partial softmax states the others store into its shared
+// memory, merged in range order.  Committed blocks are asked for before the wait for the kernel that appends this pass's rows.
+struct DAttn {
+    CUtensorMap kvmap;             // the cache as [rows][head_dim], 64 x 64 boxes
+    const __half* q;               // q|k|v buffer [M][pitch], q rotated
+    int pitch;
+    const unsigned long long* mask;
+    const int* prefix;
+    __half* out;                   // [M][Hq * HD]
+    int Hq, Hkv, mr, tail, nkb;
+    int set_rows, sets;                    // query rows of a CTA, and such sets per kv head
+    int row0, req_rows, cap, write_off;    // cache row of (this layer, K, head 0), rows of one request's cache
+    float scale_log2;
+    int* err;
+};
+
+__device__ __forceinline__ uint32_t kv_swz(int r, int v) {     // 16-byte vector v of row r of a block (boxes of 8 vectors side by side)
+    return (uint32_t)((v >> 3) * 8192 + r * 128 + (((v & 7) ^ (r & 7)) << 4));
+}
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+
+template <int HD>
+struct DAGeo {
+    static constexpr int BLOCK = 2 * 64 * HD * 2;                       // K and V of 64 keys
+    static constexpr int STAGES = 3;
+    static constexpr int OP = HD + 4;                                    // floats per row of a partial output
+    static constexpr int SLOTS = 128 + 4 * (kMaxCluster - 1);
+    static constexpr int INBOX = STAGES * BLOCK;                         // partial outputs [source][row of this CTA][OP]
+    static constexpr int INBOX_ML = INBOX + SLOTS * OP * 4;              // and their (max, sum)
+    static constexpr int SMEM = INBOX_ML + SLOTS * 8 + 1024;
+};
+
+template <int HD>
+__global__ void __launch_bounds__(256) attention_kernel(const __grid_constant__ DAttn p) {
+    using G = DAGeo<HD>;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    __shared__ uint64_t full[G::STAGES], inboxfull;
+    __shared__ int s_abort;
+    const uint32_t sbase = smem_u32(smem);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    const uint32_t rank = cluster_rank(), cs = cluster_size();
+    const int req = blockIdx.z, hk = (int)blockIdx.y / p.sets, set = (int)blockIdx.y - hk * p.sets;
+    if (threadIdx.x == 0) {
+        s_abort = 0;
+        for (int s = 0; s < G::STAGES; s++) mbar_init(smem_u32(full + s), 1);
+        mbar_init(smem_u32(&inboxfull), cs * 8);                         // every warp of the cluster
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    __syncthreads();
+    pdl_launch_dependents();
+    if (cs > 1) cluster_arrive();
+
+    const int prefix = p.prefix[req];
+    const int nact = min((prefix + p.tail + kKeyBlock - 1) / kKeyBlock, p.nkb);
+    const int b0 = nact * (int)rank / (int)cs, b1 = nact * ((int)rank + 1) / (int)cs;       // this CTA's key blocks
+    const int new0 = prefix + p.write_off;                              // first cache row this pass writes
+    const int krow = p.row0 + req * p.req_rows + hk * p.cap, vrow = krow + p.Hkv * p.cap;
+    auto load = [&](int b) {                                            // one thread
+        const uint32_t bar = smem_u32(full + (b - b0) % G::STAGES), dst = sbase + ((b - b0) % G::STAGES) * G::BLOCK;
+        mbar_expect_tx(bar, G::BLOCK);
+#pragma unroll
+        for (int x = 0; x < HD / 64; x++) {
+            tma_box(dst + x * 8192, &p.kvmap, x * 64, krow + b * kKeyBlock, bar);
+            tma_box(dst + (HD / 64 + x) * 8192, &p.kvmap, x * 64, vrow + b * kKeyBlock, bar);
+        }
+    };
+    const int committed = min(b1, new0 / kKeyBlock);                    // blocks below it hold no row of this pass
+    const int asked = max(b0, min(committed, b0 + G::STAGES));
+    constexpr int kLoader = 7;                                          // (the warp with the last rows, if it has any)
+    if (warp == kLoader) {
+        if (elect_one())
+            for (int b = b0; b < asked; b++) load(b);
+        __syncwarp();
+    }
+    pdl_wait();
+    if (warp == kLoader) {
+        if (elect_one()) {
+            asm volatile("fence.proxy.async;\n" ::: "memory");                 // rows appended by the previous kernel's ordinary stores
+            for (int b = asked; b < min(b1, b0 + G::STAGES); b++) load(b);
+        }
+        __syncwarp();
+    }
+
+    const int Gq = p.Hq / p.Hkv, QR = p.mr * Gq, rows = min(p.set_rows, QR - set * p.set_rows);
+    // warps: row tiles (rounded up to 2, 4 or 8) x parts of a key block
+    const int ntp = rows <= 32 ? 2 : (rows <= 64 ? 4 : 8), parts = 8 / ntp, units = 4 / parts;        // units of 16 keys per warp and block
+    const int lw = (warp & (ntp - 1)) * 16, part = warp / ntp;          // the warp's first row inside the set
+    const bool busy = lw < rows && b0 < b1;
+    const int r0 = set * p.set_rows + lw + g, r1 = r0 + 8;
+    const bool v0 = lw + g < rows, v1 = lw + g + 8 < rows;
+    const int q0r = v0 ? r0 / Gq : 0, q1r = v1 ? r1 / Gq : 0;
+    const int m0 = req * p.mr + q0r, m1 = req * p.mr + q1r;
+    uint32_t qa[HD / 16][4];
+    float mrun0 = -INFINITY, mrun1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+    float o[HD / 8][4];
+    unsigned long long mk0 = 0ull, mk1 = 0ull;
+    if (busy) {
+        const __half* q0 = p.q + (size_t)m0 * p.pitch + (size_t)(hk * Gq + (v0 ? r0 - q0r * Gq : 0)) * HD + 2 * t;
+        const __half* q1 = p.q + (size_t)m1 * p.pitch + (size_t)(hk * Gq + (v1 ? r1 - q1r * Gq : 0)) * HD + 2 * t;
+#pragma unroll
+        for (int ks = 0; ks < HD / 16; ks++) {
+            qa[ks][0] = __ldcg(reinterpret_cast<const uint32_t*>(q0 + ks * 16));
+            qa[ks][1] = __ldcg(reinterpret_cast<const uint32_t*>(q1 + ks * 16));
+            qa[ks][2] = __ldcg(reinterpret_cast<const uint32_t*>(q0 + ks * 16 + 8));
+            qa[ks][3] = __ldcg(reinterpret_cast<const uint32_t*>(q1 + ks * 16 + 8));
+        }
+        if (v0) mk0 = p.mask[m0];
+        if (v1) mk1 = p.mask[m1];
+#pragma unroll
+        for (int nd = 0; nd < HD / 8; nd++) o[nd][0] = o[nd][1] = o[nd][2] = o[nd][3] = 0.f;
+    }
+    const uint32_t krow_l = (uint32_t)(lane & 7), kvec_l = (uint32_t)(lane >> 3);                       // fragment rows and vectors of K
+    const uint32_t vrow_l = (uint32_t)(((lane >> 3) & 1) * 8 + (lane & 7)), vvec_l = (uint32_t)(lane >> 4);   // and of V
+
+#pragma unroll 1
+    for (int b = b0; b < b1; b++) {
+        const int st = (b - b0) % G::STAGES;
+        dwait(smem_u32(full + st), ((b - b0) / G::STAGES) & 1, &s_abort, p.err, 29);
+        __syncwarp();
+        if (busy) {
+            const uint32_t sk = sbase + st * G::BLOCK, sv = sk + (HD / 64) * 8192;
+#pragma unroll 1
+            for (int u = 0; u < units; u++) {
+                const int k0 = (part * units + u) * 16;                  // first key of the unit inside the block
+                float s[2][4];
+#pragma unroll
+                for (int nt = 0; nt < 2; nt++) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
+#pragma unroll
+                for (int ks = 0; ks < HD / 16; ks += 2)
+#pragma unroll
+                    for (int nt = 0; nt < 2; nt++) {
+                        uint32_t kf[4];
+                        ldsm4(kf, sk + kv_swz(k0 + nt * 8 + krow_l, ks * 2 + kvec_l));
+                        mma_m16n8k16(s[nt], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], kf[0], kf[1]);
+                        mma_m16n8k16(s[nt], qa[ks + 1][0], qa[ks + 1][1], qa[ks + 1][2], qa[ks + 1][3], kf[2], kf[3]);
+                    }
+                float mx0 = mrun0, mx1 = mrun1;
+                const int j0 = b * kKeyBlock + k0 + 2 * t - prefix;      // tail row of the thread's first key
+                const bool committed_unit = b * kKeyBlock + k0 + 16 <= prefix;
+#pragma unroll
+                for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        bool vis0 = v0, vis1 = v1;
+                        const int j = j0 + nt * 8 + e;
+                        if (!committed_unit && j >= 0) {
+                            vis0 = v0 && j < p.tail && ((mk0 >> (j & 63)) & 1ull);
+                            vis1 = v1 && j < p.tail && ((mk1 >> (j & 63)) & 1ull);
+                        }
+                        s[nt][e] = vis0 ? s[nt][e] * p.scale_log2 : -INFINITY;
+                        s[nt][2 + e] = vis1 ? s[nt][2 + e] * p.scale_log2 : -INFINITY;
+                        mx0 = fmaxf(mx0, s[nt][e]);
+                        mx1 = fmaxf(mx1, s[nt][2 + e]);
+                    }
+                mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
+                mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+                mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
+                mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+                const float base0 = (mx0 == -INFINITY) ? 0.f : mx0;
+                const float base1 = (mx1 == -INFINITY) ? 0.f : mx1;
+                if (__any_sync(0xffffffffu, mx0 != mrun0 || mx1 != mrun1)) {       // a running maximum moved: rescale sums and outputs
+                    const float al0 = (mrun0 == -INFINITY) ? 0.f : exp2f(mrun0 - base0);
+                    const float al1 = (mrun1 == -INFINITY) ? 0.f : exp2f(mrun1 - base1);
+                    l0 *= al0; l1 *= al1;
+#pragma unroll
+                    for (int nd = 0; nd < HD / 8; nd++) { o[nd][0] *= al0; o[nd][1] *= al0; o[nd][2] *= al1; o[nd][3] *= al1; }
+                    mrun0 = mx0; mrun1 = mx1;
+                }
+                uint32_t pa[2][2];
+#pragma unroll
+                for (int nt = 0; nt < 2; nt++) {
+                    const __half2 h0 = __floats2half2_rn(exp2f(s[nt][0] - base0), exp2f(s[nt][1] - base0));
+                    const __half2 h1 = __floats2half2_rn(exp2f(s[nt][2] - base1), exp2f(s[nt][3] - base1));
+                    // the sum uses the rounded probabilities so that numerator and denominator agree
+                    l0 += __low2float(h0) + __high2float(h0);
+                    l1 += __low2float(h1) + __high2float(h1);
+                    pa[nt][0] = h2_as_u32(h0);
+                    pa[nt][1] = h2_as_u32(h1);
+                }
+#pragma unroll
+                for (int nd = 0; nd < HD / 8; nd += 2) {
+                    uint32_t vb[4];
+                    ldsm4_t(vb, sv + kv_swz(k0 + vrow_l, nd + vvec_l));
+                    mma_m16n8k16(o[nd], pa[0][0], pa[0][1], pa[1][0], pa[1][1], vb[0], vb[1]);
+                    mma_m16n8k16(o[nd + 1], pa[0][0], pa[0][1], pa[1][0], pa[1][1], vb[2], vb[3]);
+                }
+            }
+        }
+        if (b + G::STAGES < b1) {                                        // the stage is asked for again
+            __syncthreads();
+            if (warp == kLoader) {
+                if (elect_one()) load(b + G::STAGES);
+                __syncwarp();
+            }
+        }
+    }
+    // ---- partial states -> the CTA that finishes each row
+    l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
+    l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+    const int nslot = (rows + (int)cs - 1) / (int)cs;
+    if (cs > 1) cluster_wait();
+#pragma unroll
+    for (int hrow = 0; hrow < 2; hrow++) {
+        const int lr = lw + g + 8 * hrow;
+        if (lr < rows) {
+            const uint32_t dst = lr / nslot, at = (rank * parts + part) * nslot + (lr - dst * nslot);      // (a warp's rows: mostly one CTA)
+            if (t == 0) st_peer2(peer_addr(sbase + G::INBOX_ML + at * 8, dst), hrow ? mrun1 : mrun0, hrow ? l1 : l0);
+            if (busy) {
+                const uint32_t row = peer_addr(sbase + G::INBOX + at * G::OP * 4, dst);
+#pragma unroll
+                for (int nd = 0; nd < HD / 8; nd++) st_peer2(row + (nd * 8 + 2 * t) * 4, o[nd][2 * hrow], o[nd][2 * hrow + 1]);
+            }
+        }
+    }
+    __syncwarp();
+    if (lane < (int)cs) arrive_peer(peer_addr(smem_u32(&inboxfull), lane));
+    if (!inbox_wait(smem_u32(&inboxfull))) atomicCAS(p.err, 0, 25);
+    __syncwarp();
+    // ---- merge: one warp per row, sources in key order
+    const int sources = (int)cs * parts;
+    const int row_lo = (int)rank * nslot, mine_rows = min(nslot, rows - row_lo);
+    for (int j = warp; j < mine_rows; j += 8) {
+        constexpr int C = HD / 32;
+        const float2* ml = reinterpret_cast<const float2*>(smem + G::INBOX_ML) + j;
+        const float2 mine = lane < sources ? ml[lane * nslot] : make_float2(-INFINITY, 0.f);          // (at most 32 sources)
+        float mstar = mine.x;
+#pragma unroll
+        for (int i = 16; i > 0; i >>= 1) mstar = fmaxf(mstar, __shfl_xor_sync(0xffffffffu, mstar, i));
+        const float w = mine.x == -INFINITY ? 0.f : exp2f(mine.x - mstar);
+        float den = w * mine.y;
+#pragma unroll
+        for (int i = 16; i > 0; i >>= 1) den += __shfl_xor_sync(0xffffffffu, den, i);
+        float acc[C];
+#pragma unroll
+        for (int c = 0; c < C; c++) acc[c] = 0.f;
+        const float* v = reinterpret_cast<const float*>(smem + G::INBOX) + j * G::OP + lane * C;
+#pragma unroll 4
+        for (int i = 0; i < sources; i++) {
+            const float wi = __shfl_sync(0xffffffffu, w, i);
+            if (wi != 0.f) {                                             // (an idle source has left no output)
+#pragma unroll
+                for (int c = 0; c < C; c++) acc[c] += wi * v[i * nslot * G::OP + c];
+            }
+        }
+        const float inv = den > 0.f ? 1.f / den : 0.f;
+        const int gr = set * p.set_rows + row_lo + j, m = req * p.mr + gr / Gq;
+        __half* dst = p.out + (size_t)m * p.Hq * HD + (size_t)(hk * Gq + gr % Gq) * HD + lane * C;
+        __align__(8) __half ov[C];
+#pragma unroll
+        for (int c = 0; c < C; c++) ov[c] = __float2half_rn(acc[c] * inv);
+        if (C == 4) *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(ov);
+        else *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(ov);
+    }
+}
+
+// ================================================================================ host
+// A kernel of the chain: programmatic dependent launch, clusters of `cluster` CTAs along x.
+template <typename P>
+int launch_chain(void (*kern)(P), dim3 grid, int threads, size_t smem, int cluster, cudaStream_t stream, const P& p) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (g_use_pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        n++;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    cudaLaunchKernelEx(&cfg, kern, p);
+    return check_launch();
+}
+
+// Cluster size along K for `tiles` row tiles of `nch` chunks, by a cost in microseconds fitted on B200 to passes of four model
+// shapes.  Three chunks are expanded before the wait and then cost 0.15 each, a further one 0.5 (on one CTA of an SM as on each
+// of two); a cluster's reduction 0.5; a token to finish 0.1.  CTAs beyond one per SM take the room of the next kernel's, which
+// then starts up to 1.5 later.  Clusters beyond what fits at once into eight GPCs of at least 16 SMs, two CTAs each, run as a
+// second wave (36 clusters of 7 or 48 of 6 added 2 to 8 us a kernel): not taken.
+int plan_cluster(int tiles, int nch, int tokens) {
+    int best = 1;
+    double best_cost = 1e30;
+    for (int cs = 1; cs <= kMaxCluster && cs <= nch && (cs == 1 || tiles <= 8 * (32 / cs)); cs++) {
+        const int ctas = tiles * cs, n = ((nch + cs - 1) / cs) * ((ctas + 295) / 296);
+        const double cost = n * 0.15 + std::max(0, n - 3) * 0.35 + (cs > 1 ? 0.5 + 0.03 * cs : 0.0) + 0.1 * ((tokens + cs - 1) / cs) +
+                            (ctas > 148 ? std::min(ctas - 148, 148) * 0.01 : 0.0);
+        if (cost < best_cost - 1e-9) { best_cost = cost; best = cs; }
+    }
+    return best;
+}
+
+template <int NT, int KIND>
+int launch_dense(DenseParams& p, int split, cudaStream_t stream) {
+    static std::atomic<uint64_t> done{0};
+    if (!allow_smem(dense_kernel<NT, KIND>, DGeo<NT>::SMEM, done, true)) return check_launch();
+    const int nch = p.K / kChunkK;
+    const int tiles = KIND == D_SILU ? p.N / 64 : (p.N + kTile - 1) / kTile;
+    const int cs = split > 0 && split <= std::min(kMaxCluster, nch) ? split : plan_cluster(tiles, nch, p.M);
+    constexpr int cap = 296;
+    auto launch = [&](int lo, int n, int cluster) {
+        p.tile_lo = lo;
+        p.tiles = lo + n;
+        return launch_chain(dense_kernel<NT, KIND>, dim3(cluster > 1 ? n * cluster : std::min(n, cap)), kDThreads, DGeo<NT>::SMEM, cluster, stream, p);
+    };
+    // Whole waves of tiles, then what is left over as a launch of its own with K split over clusters: alone it would take as long
+    // as a whole wave.
+    const int rest = cs == 1 && tiles > cap ? tiles % cap : 0, rest_cs = rest > 0 ? std::min({cap / rest, kMaxCluster, nch}) : 1;
+    if (rest_cs < 2) return launch(0, tiles, cs);
+    const int rc = launch(0, tiles - rest, 1);
+    return rc != B200_OK ? rc : launch(tiles - rest, rest, rest_cs);
+}
+
+template <int HD>
+int launch_attention(const DAttn& a, int nreq, cudaStream_t stream) {
+    static std::atomic<uint64_t> done{0};
+    if (!allow_smem(attention_kernel<HD>, DAGeo<HD>::SMEM, done, true)) return check_launch();
+    const int cs = std::min(a.nkb, kMaxCluster);
+    return launch_chain(attention_kernel<HD>, dim3(cs, a.Hkv * a.sets, nreq), 256, DAGeo<HD>::SMEM, cs, stream, a);
+}
+
+template <int NT>
+int run_chain(const ChainArgs& c, cudaStream_t st) {
+    const b200_forward_desc* d = c.d;
+    const int M = d->M, H = d->hidden, I = d->intermediate, hd = d->head_dim, nreq = d->requests > 1 ? d->requests : 1;
+    const int nq = d->n_heads * hd, nqkv = (d->n_heads + 2 * d->n_kv_heads) * hd;
+    auto on = [&](int kind) { return d->phase_mask == 0 || ((d->phase_mask >> kind) & 1); };
+    CUtensorMap hw_map, attn_map, act_map;
+    auto xmap = [&](CUtensorMap* m, const void* x, int width) {
+        return make_map_2d(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x, width, M, (uint64_t)width * 2, 64, NT, CU_TENSOR_MAP_SWIZZLE_128B,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+    };
+    int rc;
+    if ((rc = xmap(&hw_map, d->hw, H)) || (rc = xmap(&attn_map, d->attn, nq)) || (rc = xmap(&act_map, d->act, I))) return rc;
+
+    DenseParams p{};
+    p.ssq = c.ssq; p.H = H; p.eps = d->rms_eps; p.M = M; p.err = c.err;
+    p.h = static_cast<__half*>(d->h); p.hw = static_cast<__half*>(d->hw);
+    p.cs = c.cs; p.prefix = d->prefix; p.Hq = d->n_heads; p.Hkv = d->n_kv_heads; p.hd = hd; p.cap = d->cache_rows;
+    p.write_off = d->write_off; p.mr = M / nreq;
+    const size_t half_stride = (size_t)d->n_kv_heads * d->cache_rows * hd;
+    p.req_stride = (size_t)d->n_layers * 2 * half_stride;
+    p.row_index = d->row_index; p.rows_out = d->rows_out;
+    DAttn a{};
+    if ((rc = make_map_2d(&a.kvmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, d->kv_cache, hd, (uint64_t)nreq * d->n_layers * 2 * d->n_kv_heads * d->cache_rows,
+                          (uint64_t)hd * 2, 64, 64, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B)))
+        return rc;
+    a.q = static_cast<const __half*>(d->qkv); a.pitch = nqkv; a.mask = d->mask; a.prefix = d->prefix;
+    a.out = static_cast<__half*>(d->attn); a.Hq = d->n_heads; a.Hkv = d->n_kv_heads; a.mr = p.mr; a.tail = d->tail;
+    a.nkb = (d->cache_rows + kKeyBlock - 1) / kKeyBlock;
+    // Query rows of a CTA: as few as still make one wave (a cluster of 8 CTAs to one or two per GPC): a warp then has fewer of a
+    // block's keys, and a CTA fewer rows to merge.
+    const int qr = p.mr * (d->n_heads / d->n_kv_heads), clusters = d->n_kv_heads * nreq;
+    a.set_rows = qr <= 32 || clusters * ((qr + 31) / 32) <= 16 ? 32 : (qr <= 64 || clusters * ((qr + 63) / 64) <= 16 ? 64 : 128);
+    a.sets = (qr + a.set_rows - 1) / a.set_rows;
+    a.req_rows = d->n_layers * 2 * d->n_kv_heads * d->cache_rows;
+    a.cap = d->cache_rows; a.write_off = d->write_off; a.scale_log2 = d->attn_scale * kLog2e; a.err = c.err;
+
+    const void* const* layers = c.layers;
+    if (on(0)) {
+        launch_kernel(embed_kernel, dim3(M), dim3(256), 0, st, d->tokens, d->pos, d->embed_wq, static_cast<const __half*>(d->embed_scales),
+                      static_cast<const __half*>(d->embed_biases), static_cast<const __half*>(layers[6]), p.h, p.hw, p.ssq, c.cs, d->inv_freq,
+                      d->rope_scaling, H, d->vocab, hd / 2);
+        if ((rc = check_launch()) != B200_OK) return rc;
+    }
+    for (int l = 0; l < d->n_layers; l++) {
+        const void* const* L = layers + (size_t)l * 8;       // qkv, qkv bias, o, gate, up, down, input norm, post norm
+        auto w = [&](int i) { return static_cast<const unsigned char*>(L[i]); };
+        if (on(1)) {
+            p.xmap = hw_map; p.w[0] = w(0); p.bias = static_cast<const __half*>(L[1]); p.y = static_cast<__half*>(d->qkv);
+            p.N = nqkv; p.K = H;
+            p.kc = static_cast<__half*>(d->kv_cache) + (size_t)l * 2 * half_stride;
+            p.vc = p.kc + half_stride;
+            if ((rc = launch_dense<NT, D_QKV>(p, c.splits[0], st)) != B200_OK) return rc;
+        }
+        if (on(2)) {
+            a.row0 = l * 2 * d->n_kv_heads * d->cache_rows;
+            if ((rc = hd == 128 ? launch_attention<128>(a, nreq, st) : launch_attention<64>(a, nreq, st)) != B200_OK) return rc;
+        }
+        p.bias = nullptr;
+        if (on(4)) {
+            p.xmap = attn_map; p.w[0] = w(2); p.wn = static_cast<const __half*>(L[7]); p.N = H; p.K = nq;
+            if ((rc = launch_dense<NT, D_RESID>(p, c.splits[1], st)) != B200_OK) return rc;
+        }
+        if (on(5)) {
+            p.xmap = hw_map; p.w[0] = w(3); p.w[1] = w(4); p.y = static_cast<__half*>(d->act); p.N = I; p.K = H;
+            if ((rc = launch_dense<NT, D_SILU>(p, c.splits[2], st)) != B200_OK) return rc;
+        }
+        if (on(6)) {
+            p.xmap = act_map; p.w[0] = w(5); p.wn = static_cast<const __half*>(l + 1 < d->n_layers ? L[8 + 6] : d->final_norm); p.N = H; p.K = I;
+            if ((rc = launch_dense<NT, D_RESID>(p, c.splits[3], st)) != B200_OK) return rc;
+        }
+    }
+    if (on(7)) {
+        p.xmap = hw_map; p.w[0] = static_cast<const unsigned char*>(d->lm_head_tiled); p.y = static_cast<__half*>(d->logits);
+        p.N = d->head_rows > 0 ? d->head_rows : d->vocab; p.K = H;
+        if ((rc = launch_dense<NT, D_HEAD>(p, c.splits[4], st)) != B200_OK) return rc;
+    }
+    return B200_OK;
+}
+
+}  // namespace
+
+int forward_chain(const ChainArgs& a, cudaStream_t stream) { return a.d->M <= 16 ? run_chain<16>(a, stream) : run_chain<32>(a, stream); }
+
+}  // namespace b200

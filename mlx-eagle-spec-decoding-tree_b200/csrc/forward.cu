@@ -36,6 +36,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "decode.cuh"
 #include "pipeline.cuh"
 #include "tp_layout.cuh"
 #include "qmm_common.cuh"
@@ -2177,6 +2178,13 @@ bool fwd_shape_ok(const b200_forward_desc* d) {
     return true;
 }
 
+// Scratch of the kernel chain: error word, sums of squares and RoPE table, whatever the cache.
+struct ChainWs {
+    static constexpr size_t kSsq = 256 + kCounterBytes;
+    static constexpr size_t kCs = kSsq + (size_t)kMaxSsqParts * kSsqPitch * sizeof(float);
+    static constexpr size_t kTotal = kCs + (size_t)32 * kCsPitch * sizeof(float2);
+};
+
 WsLayout fwd_layout(const b200_forward_desc* d, PhasePlan (&plan)[5], int* grid_out = nullptr) {
     const int grid = fwd_grid(d);
     if (grid_out) *grid_out = grid;
@@ -2270,11 +2278,7 @@ int launch_forward(const FwdParams& p, int grid, cudaStream_t stream) {
 
 template <int MT>
 int launch_forward_hd(const FwdParams& p, int grid, cudaStream_t stream) {
-    if (p.tp_world > 1)         // a shard: the variant with the exchange phases
-        return p.HD == 128 ? launch_forward<MT, 128, true, false>(p, grid, stream) : launch_forward<MT, 64, true, false>(p, grid, stream);
-    if (p.nreq > 1)             // several requests in the pass
-        return p.HD == 128 ? launch_forward<MT, 128, false, true>(p, grid, stream) : launch_forward<MT, 64, false, true>(p, grid, stream);
-    return p.HD == 128 ? launch_forward<MT, 128, false, false>(p, grid, stream) : launch_forward<MT, 64, false, false>(p, grid, stream);
+    return p.HD == 128 ? launch_forward<MT, 128, true, false>(p, grid, stream) : launch_forward<MT, 64, true, false>(p, grid, stream);
 }
 
 }  // namespace
@@ -2294,6 +2298,7 @@ void b200_forward_plan_hint(const char* spec) { parse_plan_hint(spec); }
 
 size_t b200_forward_workspace_bytes(const b200_forward_desc* d) {
     if (!fwd_shape_ok(d)) return 0;
+    if (d->tp_world <= 1) return ChainWs::kTotal;
     PhasePlan plan[5];
     return fwd_layout(d, plan).total;
 }
@@ -2309,6 +2314,28 @@ int b200_forward(const b200_forward_desc* d, void* stream) {
                         d->final_norm};
     for (const void* q : al)
         if (!aligned16(q)) return B200_EALIGN;
+    if (d->tp_world <= 1) {
+        // one GPU: a chain of kernels (csrc/decode.cu)
+        if (d->workspace_bytes < ChainWs::kTotal) return B200_EWORKSPACE;
+        char* ws = static_cast<char*>(d->workspace);
+        ChainArgs a{};
+        a.d = d;
+        a.err = reinterpret_cast<int*>(ws) + kSyncErr;
+        a.ssq = reinterpret_cast<float*>(ws + ChainWs::kSsq);
+        a.cs = reinterpret_cast<float2*>(ws + ChainWs::kCs);
+        for (int i = 0; i < 5; i++)
+            if (const PlanOverride* o = plan_override(i)) a.splits[i] = (o->kw & (o->kw - 1)) == 0 && o->kw <= 8 ? o->splits : 0;
+        const void* table[kMaxLayers * 8];
+        a.layers = d->layers_host;
+        if (a.layers == nullptr) {
+            cudaStream_t st = static_cast<cudaStream_t>(stream);
+            if (cudaMemcpyAsync(table, d->layer_table, (size_t)d->n_layers * 8 * sizeof(void*), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+                cudaStreamSynchronize(st) != cudaSuccess)
+                return check_launch() == B200_OK ? B200_ECUDA : B200_ECUDA;
+            a.layers = table;
+        }
+        return forward_chain(a, static_cast<cudaStream_t>(stream));
+    }
     FwdParams p{};
     int grid = 0;
     const WsLayout w = fwd_layout(d, p.plan, &grid);

@@ -511,6 +511,8 @@ class Model:
                               lw["gate"].tiled.data_ptr(), lw["up"].tiled.data_ptr(), lw["down"].tiled.data_ptr(),
                               lw["input_norm"].data_ptr(), lw["post_norm"].data_ptr()])
             self._layer_table = torch.tensor(rows_, dtype=torch.int64).to(self.device)
+            flat = [v for row in rows_ for v in row]
+            self._layers_host = (ctypes.c_void_p * len(flat))(*flat)
         d = _lib.ForwardDesc()
         d.M, d.rows_out = M, rows
         d.hidden, d.intermediate, d.n_heads, d.n_kv_heads = a.hidden_size, a.intermediate_size, \
@@ -527,6 +529,7 @@ class Model:
             p(self.xt_act), p(self.logits)
         d.kv_cache = p(cache.data)
         d.requests = requests
+        d.layers_host = ctypes.cast(self._layers_host, ctypes.c_void_p)
         if self.tp is not None:
             d.head_rows = self.vocab_local
         d.grid_ctas = self.grid_ctas

@@ -1,0 +1,55 @@
+"""The kernel chain of a pass of up to 32 tokens (csrc/decode.cu) at the edges of its tiles, key blocks and clusters, against the
+per-op kernels."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [
+    # heads, kv heads, head dim, hidden, intermediate, vocab
+    (2, 1, 64, 128, 128, 1032),          # one chunk of K, a last row tile of 8 rows
+    (14, 2, 64, 896, 640, 520),          # groups of 7 heads, seven chunks
+    (16, 2, 128, 1024, 2176, 2048),      # groups of 8 heads of 128: up to 256 query rows per kv head
+]
+
+
+def _model(be, cuda, heads, kv, hd, hidden, inter, vocab):
+    args = be.ModelArgs(model_type="qwen2", hidden_size=hidden, num_hidden_layers=2, intermediate_size=inter, num_attention_heads=heads,
+                        num_key_value_heads=kv, rms_norm_eps=1e-6, vocab_size=vocab, tie_word_embeddings=True)
+    assert args.head_dim == hd
+    return be.Model.random_init(args, seed=3, device=cuda, gen_device="cpu").relayout()
+
+
+def _cache(m, cached, seed):
+    cache = m.make_cache(64 * ((cached + 32 + 63) // 64))
+    g = torch.Generator().manual_seed(seed)
+    cache.data[:, :, :, :cached] = (0.3 * torch.randn(cache.data[:, :, :, :cached].shape, generator=g)).half().to(cache.data.device)
+    cache.offset = cached
+    return cache
+
+
+def _tree(rows, rng):
+    tm = np.eye(rows, dtype=bool)
+    for i in range(1, rows):
+        tm[i] |= tm[int(rng.integers(0, i))]
+    return tm
+
+
+@pytest.mark.parametrize("rows,cached", [(1, 0), (1, 63), (2, 64), (16, 31), (16, 447), (17, 448), (31, 600), (32, 1500)])
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
+def test_chain_equals_per_op_kernels(be, cuda, shape, rows, cached):
+    m = _model(be, cuda, *shape)
+    rng = np.random.default_rng(rows + cached)
+    tokens = torch.from_numpy(rng.integers(0, shape[-1], rows))[None]
+    tm = torch.from_numpy(_tree(rows, rng))
+    out = []
+    for fused in (True, False):
+        m.fused = fused
+        assert m.can_fuse() == fused
+        cache = _cache(m, cached, 1)
+        logits = be.eagle.tree_decoding(tokens, tm, tm.sum(1) - 1, m, cache)[0].float()
+        out.append((logits, cache.data[:, :, :, :cached + rows].float()))
+    m.check_fused_error()
+    for got, want in zip(*out):
+        assert ((got - want).abs() <= 2.0 ** -6 * want.abs() + 1e-2).all()
