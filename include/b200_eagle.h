@@ -154,6 +154,14 @@ int b200_qmm_umma(const void* x, const void* w_tiled, const void* bias, void* y,
  * tree_attention, qmm(residual), rms_norm, qmm(silu-mul), qmm(residual)).
  * ------------------------------------------------------------------------------------------ */
 
+/* The device-side inputs of a pass of L <= 32 tokens (b200_forward's tokens / pos / mask / prefix) from a caller's tensors, in
+ * one launch.  tokens and pos: int32, or int64 where tok64 / pos64; position of token m = pos_base + m * pos_step, plus
+ * pos[m * pos_stride] if pos is given.  vis_type: 0 causal, 1 bool [L][L], 2 additive fp32 [L][L] (0 = visible), < 0 leave the
+ * mask words.  out_prefix gets `prefix` nprefix (<= 32) times, out_last L - 1.  (mlx_llama.py:121-196 builds these on the fly.) */
+int b200_pass_inputs(const void* tokens, int tok64, const void* pos, int pos64, int pos_stride, int pos_base, int pos_step, const void* vis,
+                     int vis_type, int L, int prefix, int* out_tokens, int* out_pos, unsigned long long* out_mask, int* out_prefix, int nprefix,
+                     int* out_last, void* stream);
+
 /* Quantised embedding lookup, h[m,:] = dequant(E[tokens[m],:]).  Replaces `self.embed_tokens(inputs)`
  * (mlx_llama.py:273) on a 4-bit nn.QuantizedEmbedding.  out [M,H] fp16; H % 64 == 0. */
 int b200_embed_gather(const int* tokens, const uint32_t* wq, const void* scales, const void* biases,

@@ -92,6 +92,8 @@ def _declare(l: ctypes.CDLL) -> None:
     l.b200_qmm_gemm_workspace_bytes.argtypes = [i32] * 4
     l.b200_qmm_gemm.restype = i32
     l.b200_qmm_gemm.argtypes = [vp] * 6 + [i32] * 4 + [vp, sz, vp]
+    l.b200_pass_inputs.restype = i32
+    l.b200_pass_inputs.argtypes = [vp, i32, vp] + [i32] * 4 + [vp] + [i32] * 3 + [vp] * 4 + [i32, vp, vp]
     l.b200_embed_gather.restype = i32
     l.b200_embed_gather.argtypes = [vp] * 5 + [i32] * 3 + [vp]
     l.b200_rms_norm.restype = i32

@@ -216,10 +216,51 @@ __global__ void __launch_bounds__(kRopeThreads) rope_positions_vec_kernel(const 
     }
 }
 
+// ---- inputs of a pass from what a caller of the model hands over: token ids, positions, visibility ----
+// One warp, a token per lane.  A pass of one token on a small model is under a millisecond; filling these from the host took
+// four copies and a read-back of the mask, ~100 us.
+__global__ void pass_inputs_kernel(const void* __restrict__ tokens, int tok64, const void* __restrict__ pos, int pos64, int pos_stride,
+                                   int pos_base, int pos_step, const void* __restrict__ vis, int vis_type, int L, int prefix,
+                                   int* __restrict__ out_tokens, int* __restrict__ out_pos, unsigned long long* __restrict__ out_mask,
+                                   int* __restrict__ out_prefix, int nprefix, int* __restrict__ out_last) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int m = threadIdx.x;
+    if (m < nprefix) out_prefix[m] = prefix;
+    if (m == 0) *out_last = L - 1;
+    if (m >= L) return;
+    out_tokens[m] = tok64 ? (int)static_cast<const long long*>(tokens)[m] : static_cast<const int*>(tokens)[m];
+    int p = pos_base + m * pos_step;
+    if (pos) p += pos64 ? (int)static_cast<const long long*>(pos)[m * pos_stride] : static_cast<const int*>(pos)[m * pos_stride];
+    out_pos[m] = p;
+    if (vis_type < 0) return;                                 // (the mask words are there already)
+    unsigned long long bits = (2ull << m) - 1;                // causal
+    if (vis_type > 0) {
+        bits = 0;
+        for (int j = 0; j < L; j++) {
+            bool v;
+            if (vis_type == 1) v = static_cast<const unsigned char*>(vis)[m * L + j] != 0;
+            else v = static_cast<const float*>(vis)[m * L + j] == 0.f;                  // additive: 0 or -inf
+            bits |= (unsigned long long)v << j;
+        }
+    }
+    out_mask[m] = bits;
+}
+
 }  // namespace
 }  // namespace b200
 
 extern "C" {
+
+int b200_pass_inputs(const void* tokens, int tok64, const void* pos, int pos64, int pos_stride, int pos_base, int pos_step, const void* vis,
+                     int vis_type, int L, int prefix, int* out_tokens, int* out_pos, unsigned long long* out_mask, int* out_prefix, int nprefix,
+                     int* out_last, void* stream) {
+    if (!tokens || !out_tokens || !out_pos || !out_mask || !out_prefix || !out_last) return B200_EINVAL;
+    if (L < 1 || L > 32 || nprefix < 1 || nprefix > 32 || vis_type > 2 || (vis_type > 0 && !vis)) return B200_EINVAL;
+    b200::launch_kernel(b200::pass_inputs_kernel, dim3(1), dim3(32), 0, static_cast<cudaStream_t>(stream), tokens, tok64, pos, pos64, pos_stride,
+                        pos_base, pos_step, vis, vis_type, L, prefix, out_tokens, out_pos, out_mask, out_prefix, nprefix, out_last);
+    return b200::check_launch();
+}
 
 int b200_embed_gather(const int* tokens, const uint32_t* wq, const void* scales, const void* biases,
                       void* out, int M, int H, int V, void* stream) {

@@ -528,6 +528,9 @@ def tree_decoding(token_ids: torch.Tensor, tree_mask: torch.Tensor, tree_positio
     or boolean ``(T+1, T+1)``."""
     offset = cache.offset
     tm = tree_mask
+    L = token_ids.numel()
+    if isinstance(base_model, Model) and L <= MAX_ROWS and tm.shape == (L, L) and tree_position_ids.numel() == L:
+        return base_model.tree_pass(token_ids, tm, tree_position_ids, offset, cache)
     if tm.dtype == torch.bool:
         tm = torch.where(tm, 0.0, float("-inf"))
     tm = tm.float().cpu()

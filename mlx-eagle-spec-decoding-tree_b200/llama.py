@@ -228,6 +228,7 @@ class FwdInputs:
         self.pos = torch.zeros(MAX_ROWS, dtype=torch.int32, device=device)
         self.mask = torch.zeros(MAX_ROWS, dtype=torch.int64, device=device)   # uint64 bit masks
         self.prefix = torch.zeros(MAX_REQUESTS, dtype=torch.int32, device=device)   # committed length per request
+        self.last = torch.zeros(1, dtype=torch.int32, device=device)                # index of the pass's last token
 
 
 class KVCache:
@@ -310,6 +311,7 @@ class Model:
         self.prefill_large_m = True                      # prompts: 128 rows per weight read through b200_prefill
         self._pf, self._pf_buf, self._pf_fits = None, None, False     # descriptor and buffers of that path, made on first use
         self._scales_fast = None
+        self._desc, self._fuse_fits = None, False
         self.fwd = FwdInputs(self.device)
 
     # ------------------------------------------------------------------ construction
@@ -492,19 +494,24 @@ class Model:
             return False
         if self.tp is not None and (self.tp.peers is None or self.tp.world > 8):
             return False                         # a shard fuses once open_exchange() has mapped the peers' buffers
+        if self._fuse_fits:                      # (relayout only adds: a yes stays a yes)
+            return True
         a = self.args
         if any(lw[k].tiled is None for lw in self.layers for k in ("qkv", "o", "gate", "up", "down")):
             return False
         if self.lm_head.tiled is None or self.embed.weight is None:
             return False
-        return (a.hidden_size % 128 == 0 and a.hidden_size <= 8192 and a.intermediate_size % 128 == 0
+        self._fuse_fits = (a.hidden_size % 128 == 0 and a.hidden_size <= 8192 and a.intermediate_size % 128 == 0
                 and self.nq % 128 == 0 and a.head_dim in (64, 128) and a.vocab_size % 8 == 0
-                and self.vocab_local % 8 == 0)
+                           and self.vocab_local % 8 == 0)
+        return self._fuse_fits
 
-    def _fused_desc(self, M, cache, write_off, tail, fwd, rows, row_index, requests=1):
-        a = self.args
+    def _fused_desc(self, M, cache, write_off, tail, fwd, rows, row_index, requests=1, logits=None):
+        """The descriptor of ``b200_forward``: what a model keeps is filled in once, the rest on each call."""
         p = lambda t: None if t is None else t.data_ptr()
-        if self._layer_table is None:
+        d = self._desc
+        if d is None:
+            a = self.args
             rows_ = []
             for lw in self.layers:
                 rows_.append([lw["qkv"].tiled.data_ptr(), p(lw["qkv"].bias) or 0, lw["o"].tiled.data_ptr(),
@@ -513,49 +520,41 @@ class Model:
             self._layer_table = torch.tensor(rows_, dtype=torch.int64).to(self.device)
             flat = [v for row in rows_ for v in row]
             self._layers_host = (ctypes.c_void_p * len(flat))(*flat)
-        d = _lib.ForwardDesc()
-        d.M, d.rows_out = M, rows
-        d.hidden, d.intermediate, d.n_heads, d.n_kv_heads = a.hidden_size, a.intermediate_size, \
-            a.num_attention_heads, a.num_key_value_heads
-        d.head_dim, d.vocab, d.n_layers = a.head_dim, a.vocab_size, a.num_hidden_layers
-        d.cache_rows, d.write_off, d.tail = cache.rows, write_off, tail
-        d.rms_eps, d.rope_scaling, d.attn_scale = float(a.rms_norm_eps), self.rope_scaling_factor, self.scale
-        d.tokens, d.pos, d.mask, d.prefix = p(fwd.tokens), p(fwd.pos), p(fwd.mask), p(fwd.prefix)
-        d.row_index = p(row_index)
-        d.inv_freq = p(self.inv_freqs)
-        d.embed_wq, d.embed_scales, d.embed_biases = p(self.embed.weight), p(self.embed.scales), p(self.embed.biases)
-        d.final_norm, d.lm_head_tiled, d.layer_table = p(self.norm), p(self.lm_head.tiled), p(self._layer_table)
-        d.h, d.hw, d.qkv, d.attn, d.act, d.logits = p(self.h), p(self.hw), p(self.qkv), p(self.xt_attn), \
-            p(self.xt_act), p(self.logits)
-        d.kv_cache = p(cache.data)
-        d.requests = requests
-        d.layers_host = ctypes.cast(self._layers_host, ctypes.c_void_p)
-        if self.tp is not None:
-            d.head_rows = self.vocab_local
-        d.grid_ctas = self.grid_ctas
-        if self._scales_fast is None:
             self._scales_fast = all(lw[k].scales_fast for lw in self.layers for k in ("qkv", "o", "gate", "up", "down")) \
                 and self.lm_head.scales_fast
+            d = _lib.ForwardDesc()
+            d.hidden, d.intermediate, d.n_heads, d.n_kv_heads = a.hidden_size, a.intermediate_size, \
+                a.num_attention_heads, a.num_key_value_heads
+            d.head_dim, d.vocab, d.n_layers = a.head_dim, a.vocab_size, a.num_hidden_layers
+            d.rms_eps, d.rope_scaling, d.attn_scale = float(a.rms_norm_eps), self.rope_scaling_factor, self.scale
+            d.inv_freq = p(self.inv_freqs)
+            d.embed_wq, d.embed_scales, d.embed_biases = p(self.embed.weight), p(self.embed.scales), p(self.embed.biases)
+            d.final_norm, d.lm_head_tiled, d.layer_table = p(self.norm), p(self.lm_head.tiled), p(self._layer_table)
+            d.h, d.hw, d.qkv, d.attn, d.act = p(self.h), p(self.hw), p(self.qkv), p(self.xt_attn), p(self.xt_act)
+            d.layers_host = ctypes.cast(self._layers_host, ctypes.c_void_p)
+            self._desc = d
+        d.M, d.rows_out, d.requests = M, rows, requests
+        d.cache_rows, d.write_off, d.tail = cache.rows, write_off, tail
+        d.tokens, d.pos, d.mask, d.prefix = p(fwd.tokens), p(fwd.pos), p(fwd.mask), p(fwd.prefix)
+        d.row_index, d.logits, d.kv_cache = p(row_index), p(self.logits if logits is None else logits), p(cache.data)
+        d.grid_ctas, d.phase_mask, d.attn_split_blocks = self.grid_ctas, self.phase_mask, self.attn_split_blocks
         d.scales_in_fast_range = 1 if (self._scales_fast and self.fast_dequant) else 0
-        key = (cache.rows, self.grid_ctas)
+        if self.tp is not None:
+            d.tp_world, d.tp_rank, d.head_rows = self.tp.world, self.tp.rank, self.vocab_local
+            d.tp_two_shot = self.tp_two_shot
+            for r, q in enumerate(self.tp.peers):
+                d.tp_peers[r] = q
+        key = (cache.rows, self.grid_ctas) if self.tp is not None else 0      # (only a shard's scratch depends on them)
         if self._fwd_ws is None or self._fwd_ws_key != key:
             d32 = _lib.ForwardDesc.from_buffer_copy(d)
-            d32.M, d32.rows_out, d32.write_off, d32.tail = MAX_ROWS, MAX_ROWS, 0, MAX_TAIL
+            d32.M, d32.rows_out, d32.write_off, d32.tail, d32.requests = MAX_ROWS, MAX_ROWS, 0, MAX_TAIL, 1
             nbytes = _lib.lib().b200_forward_workspace_bytes(ctypes.byref(d32))
             if nbytes == 0:
                 raise _lib.B200Error("b200_forward_workspace_bytes rejected the model shape")
             self._fwd_ws = torch.zeros(nbytes, dtype=torch.uint8, device=self.device)
             self._fwd_ws_key = key
         d.workspace, d.workspace_bytes = p(self._fwd_ws), self._fwd_ws.numel()
-        d.phase_mask = self.phase_mask
-        d.attn_split_blocks = self.attn_split_blocks
-        if self.tp is not None:
-            d.tp_world, d.tp_rank, d.head_rows = self.tp.world, self.tp.rank, self.vocab_local
-            d.tp_two_shot = self.tp_two_shot
-            for r, q in enumerate(self.tp.peers):
-                d.tp_peers[r] = q
-        if self.timeline is not None:
-            d.timeline, d.timeline_pitch = p(self.timeline), self.timeline.shape[1]
+        d.timeline, d.timeline_pitch = (p(self.timeline), self.timeline.shape[1]) if self.timeline is not None else (None, 0)
         return d
 
     def enable_timeline(self, on: bool = True):
@@ -614,6 +613,11 @@ class Model:
         rows ``< prefix`` and tail row j iff bit j of ``fwd.mask[m]``.  Returns fp16 logits
         ``(logits_rows or M, V)`` (a view of an internal buffer); with ``row_index`` (device int) only
         rows ``row_index .. row_index+logits_rows-1`` of the hidden state reach the head."""
+        return self._forward(M, cache, write_off, tail, fwd, logits_rows, row_index, requests)
+
+    def _forward(self, M, cache, write_off, tail, fwd=None, logits_rows=None, row_index=None, requests=1, out=None):
+        """``forward_device`` into ``out`` (contiguous fp16, its rows of this model's share of the vocabulary), or into the
+        model's own buffer."""
         if not (1 <= M <= MAX_ROWS and 1 <= tail <= MAX_TAIL and write_off + M // requests <= tail):
             raise _lib.B200Error("forward_device: need 1 <= M <= 32, tail <= 64, write_off + M <= tail")
         fwd = fwd or self.fwd
@@ -625,13 +629,15 @@ class Model:
                     and M % requests == 0 and self.tp is None):
                 raise _lib.B200Error("forward_device: several requests need relayouted weights and a BatchKVCache")
             rows = M // requests if logits_rows is None else logits_rows
-            desc = self._fused_desc(M, cache, write_off, tail, fwd, rows, row_index, requests)
+            desc = self._fused_desc(M, cache, write_off, tail, fwd, rows, row_index, requests, out)
             _lib.check(_lib.lib().b200_forward(ctypes.byref(desc), _lib.stream_ptr(self.device)), "b200_forward")
-            return self.logits[: requests * rows]
+            return self.logits[: requests * rows] if out is None else out
         if self.can_fuse():
             rows = M if logits_rows is None else logits_rows
-            desc = self._fused_desc(M, cache, write_off, tail, fwd, rows, row_index)
+            desc = self._fused_desc(M, cache, write_off, tail, fwd, rows, row_index, logits=out)
             _lib.check(_lib.lib().b200_forward(ctypes.byref(desc), _lib.stream_ptr(self.device)), "b200_forward")
+            if out is not None:
+                return out
             vl = self.vocab_local
             return self.logits[:rows] if vl == self.args.vocab_size else self.logits.view(-1)[: rows * vl].view(rows, vl)
         a, L, lib = self.args, _lib.lib(), _lib.lib()
@@ -660,7 +666,9 @@ class Model:
             self._row_parallel(self.act, lw["down"], M)
         rows = M if logits_rows is None else logits_rows
         ck(L.b200_rms_norm(p(self.h), p(self.norm), p(self.xn), p(row_index), rows, H, eps, st), "final norm")
-        self._linear(self.xn, self.lm_head, self.logits, rows, qk.EPI_NONE)
+        self._linear(self.xn, self.lm_head, self.logits if out is None else out, rows, qk.EPI_NONE)
+        if out is not None:
+            return out
         vl = self.vocab_local                      # a tensor-parallel shard produces its slice of the vocabulary
         return self.logits[:rows] if vl == a.vocab_size else self.logits.view(-1)[: rows * vl].view(rows, vl)
 
@@ -725,13 +733,14 @@ class Model:
         """
         if cache is None:
             raise _lib.B200Error("a KVCache is required (the reference's cache-less branch is not on this path)")
-        inputs = inputs.reshape(-1).to(torch.int32)
+        inputs = inputs.reshape(-1)
         Ltot = inputs.numel()
+        if Ltot == 0:
+            raise _lib.B200Error("no tokens")
         if Ltot > MAX_ROWS and (mask is not None or position_ids is not None):
             raise _lib.B200Error("explicit masks / positions are limited to 32 tokens per call")
-        outs = []
         if Ltot > MAX_ROWS and self.can_prefill_large_m():
-            inputs = inputs.to(self.device).contiguous()
+            inputs = inputs.to(self.device, torch.int32).contiguous()
             out = torch.empty(1 if logits_last_only else Ltot, self.args.vocab_size, dtype=torch.float16, device=self.device)
             for c0 in range(0, Ltot, PREFILL_ROWS):
                 chunk = inputs[c0:c0 + PREFILL_ROWS]
@@ -744,6 +753,8 @@ class Model:
                     self._prefill_large_m(chunk, cache, off, out[c0:c0 + n], n)
                 cache.offset = off + n
             return out.unsqueeze(0)
+        inputs = self._ids(inputs)
+        out = torch.empty(1 if logits_last_only else Ltot, self.vocab_local, dtype=torch.float16, device=self.device)
         for c0 in range(0, Ltot, MAX_ROWS):
             chunk = inputs[c0:c0 + MAX_ROWS]
             L = chunk.numel()
@@ -751,45 +762,69 @@ class Model:
             if off + L > cache.rows:
                 raise _lib.B200Error("KV cache is full")
             if position_ids is None:
-                pos = off + torch.arange(L, dtype=torch.int32)
+                pos, base, step = None, off, 1
             elif isinstance(position_ids, int):
-                pos = torch.full((L,), position_ids, dtype=torch.int32) if flat_rope else \
-                    position_ids + torch.arange(L, dtype=torch.int32)
+                pos, base, step = None, position_ids, 0 if flat_rope else 1
             else:
-                pos = position_ids.reshape(-1).to(torch.int32).cpu()
-            if mask is None:
-                prefix, write_off, tail = off, 0, L
-                bits = [(2 << m) - 1 for m in range(L)]
-            else:
-                vis = (mask.reshape(L, -1).float().cpu() == 0)
-                cols = vis.shape[1]
+                pos, base, step = position_ids, 0, 0
+            prefix, write_off, tail, vis = off, 0, L, None
+            if mask is not None:
+                shown = (mask.reshape(L, -1).float().cpu() == 0)
+                cols = shown.shape[1]
                 if cols != off + L:
                     raise _lib.B200Error("mask must have cache.offset + L columns")
-                all_vis = vis.all(dim=0)
-                first_hidden = int((~all_vis).nonzero()[0]) if (~all_vis).any() else cols
+                hidden = (~shown.all(dim=0)).nonzero()
+                first_hidden = int(hidden[0]) if hidden.numel() else cols
                 prefix = max(min(first_hidden, off), cols - MAX_TAIL)
-                if not bool(vis[:, :prefix].all()):
+                if not bool(shown[:, :prefix].all()):
                     raise _lib.B200Error("mask hides a column more than 64 rows before the end of the cache")
                 tail, write_off = cols - prefix, off - prefix
-                bits = []
-                for m in range(L):
-                    v = 0
-                    for j in range(tail):
-                        if vis[m, prefix + j]:
-                            v |= 1 << j
-                    bits.append(v)
-            f = self.fwd
-            f.tokens[:L].copy_(chunk)
-            f.pos[:L].copy_(pos.to(self.device) if isinstance(pos, torch.Tensor) else pos)
-            f.mask[:L].copy_(torch.tensor([b - (1 << 64) if b >= (1 << 63) else b for b in bits], dtype=torch.int64))
-            f.prefix.fill_(prefix)
-            logits = self.forward_device(L, cache, write_off, tail)
+                # bit j = tail row j (bit 63 is the sign: distinct powers of two add up without a carry)
+                vis = (shown[:, prefix:].to(torch.int64) << torch.arange(tail, dtype=torch.int64)).sum(dim=1)
+            self._pass(chunk, cache, prefix, write_off, tail, pos, base, step, vis, out if logits_last_only else out[c0:c0 + L])
             cache.offset = off + L
-            if logits_last_only:
-                outs = [logits[L - 1:L].clone()]
+        return out.unsqueeze(0)
+
+    def _ids(self, t: torch.Tensor) -> torch.Tensor:
+        """Token ids or positions as the device takes them: int32 or int64, flat, on the model's device."""
+        t = t.reshape(-1)
+        return t.to(self.device, t.dtype if t.dtype in (torch.int32, torch.int64) else torch.int32).contiguous()
+
+    def _pass(self, tokens, cache, prefix, write_off, tail, pos, pos_base, pos_step, vis, out):
+        """Inputs and launch of one pass of up to 32 tokens.  ``vis``: None = causal, int64 mask words, or the visibility of
+        the pass's own tokens to each other, bool or additive fp32 ``(L, L)``.  ``out``: the logits of all tokens, or of the
+        last (one row)."""
+        f, L = self.fwd, tokens.numel()
+        pp, pos64, stride, vp, kind = None, 0, 1, None, 0
+        if pos is not None:
+            pos = self._ids(pos)
+            if pos.numel() not in (1, L):
+                raise _lib.B200Error(f"{pos.numel()} positions for {L} tokens")
+            pp, pos64, stride = pos.data_ptr(), pos.dtype == torch.int64, 0 if pos.numel() == 1 else 1
+        if vis is not None:
+            if vis.dtype == torch.int64:
+                f.mask[:L].copy_(vis)
+                kind = -1
             else:
-                outs.append(logits.clone())
-        return torch.cat(outs, 0).unsqueeze(0)
+                vp, kind = vis.data_ptr(), 1 if vis.dtype == torch.bool else 2
+        _lib.check(_lib.lib().b200_pass_inputs(tokens.data_ptr(), tokens.dtype == torch.int64, pp, pos64, stride, pos_base, pos_step, vp,
+                                               kind, L, prefix, f.tokens.data_ptr(), f.pos.data_ptr(), f.mask.data_ptr(),
+                                               f.prefix.data_ptr(), MAX_REQUESTS, f.last.data_ptr(), _lib.stream_ptr(self.device)),
+                   "b200_pass_inputs")
+        rows = out.shape[0]
+        self._forward(L, cache, write_off, tail, f, rows, f.last if rows < L else None, out=out)
+
+    def tree_pass(self, tokens: torch.Tensor, visible: torch.Tensor, positions: torch.Tensor, offset: int, cache: KVCache):
+        """Logits ``(1, L, V)`` of a token tree behind ``cache.offset`` committed rows: token m sees those and the tokens that
+        row m of ``visible`` (bool, or additive 0 / -inf) shows it, at position ``positions[m] + offset``.  Nothing is read back."""
+        tokens, L = self._ids(tokens), tokens.numel()
+        if cache.offset + L > cache.rows:
+            raise _lib.B200Error("KV cache is full")
+        visible = visible.to(self.device, torch.bool if visible.dtype == torch.bool else torch.float32).contiguous()
+        out = torch.empty(L, self.vocab_local, dtype=torch.float16, device=self.device)
+        self._pass(tokens, cache, cache.offset, 0, L, positions, offset, 0, visible, out)
+        cache.offset += L
+        return out.unsqueeze(0)
 
 
 def shape_preset(name: str) -> ModelArgs:

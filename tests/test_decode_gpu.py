@@ -1,5 +1,5 @@
 """The kernel chain of a pass of up to 32 tokens (csrc/decode.cu) at the edges of its tiles, key blocks and clusters, against the
-per-op kernels."""
+per-op kernels; and the inputs of a pass from a caller's tensors."""
 import numpy as np
 import pytest
 import torch
@@ -53,3 +53,30 @@ def test_chain_equals_per_op_kernels(be, cuda, shape, rows, cached):
     m.check_fused_error()
     for got, want in zip(*out):
         assert ((got - want).abs() <= 2.0 ** -6 * want.abs() + 1e-2).all()
+
+
+@pytest.mark.parametrize("rows,cached", [(1, 5), (7, 0), (32, 90)])
+def test_pass_inputs_whatever_their_form(be, cuda, rows, cached):
+    m = _model(be, cuda, *SHAPES[1])
+    rng = np.random.default_rng(rows)
+    tokens = torch.from_numpy(rng.integers(0, SHAPES[1][-1], rows))[None]
+    tm = torch.from_numpy(_tree(rows, rng))
+    pos = tm.sum(1) - 1
+    additive = torch.where(tm, 0.0, float("-inf"))
+    full = torch.cat([torch.zeros(rows, cached), additive], dim=-1)[None, None]
+    cache = _cache(m, cached, 2)
+    outs = []
+    for call in (lambda c: be.eagle.tree_decoding(tokens, tm, pos, m, c),
+                 lambda c: be.eagle.tree_decoding(tokens.to(cuda, torch.int32), additive.half().to(cuda), pos.to(cuda, torch.int32), m, c),
+                 lambda c: m(tokens, c, mask=full, position_ids=pos + cached)):
+        cache.offset = cached
+        outs.append(call(cache))
+        assert cache.offset == cached + rows
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    cache.offset = cached
+    every = m(tokens, cache)
+    cache.offset = cached
+    last = m(tokens.to(cuda), cache, logits_last_only=True)
+    cache.offset = cached
+    explicit = m(tokens, cache, position_ids=cached + torch.arange(rows))
+    assert last.shape == (1, 1, SHAPES[1][-1]) and torch.equal(last, every[:, -1:]) and torch.equal(explicit, every)
