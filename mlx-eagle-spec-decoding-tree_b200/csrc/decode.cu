@@ -553,10 +553,11 @@ __global__ void __launch_bounds__(256) embed_kernel(const int* __restrict__ toke
 }
 
 // ================================================================================ attention
-// CTA = (key range, kv head, request, set of 32, 64 or 128 query rows): a query row is (token, head of the group), a warp has 16
-// of them and all keys of a block or, where fewer rows leave warps over, a half or a quarter; all share the K/V blocks (TMA boxes, 128-byte
-// swizzle, three blocks of 64 keys in flight).  The CTAs of a cluster take
-// neighbouring key ranges; each finishes its share of the rows, whose partial softmax states the others store into its shared
+// CTA = (key range, kv head, request, set of query rows); a query row is (token, head of the group).  PT warps share a tile of 16
+// rows: each takes 1 / PT of a block's keys for the scores and, the probabilities exchanged through shared memory, 1 / PT of the
+// dims for the output, so partial outputs leave the CTA once per row.  (Each warp all dims for its keys sent PT times as much to
+// the peers, which took longer than the matmuls.)  All share the K/V blocks (TMA boxes, 128-byte swizzle).  The CTAs of a cluster
+// take neighbouring key ranges; each finishes its share of the rows, whose partial softmax states the others store into its shared
 // memory, merged in range order.  Committed blocks are asked for before the wait for the kernel that appends this pass's rows.
 struct DAttn {
     CUtensorMap kvmap;             // the cache as [rows][head_dim], 64 x 64 boxes
@@ -566,7 +567,7 @@ struct DAttn {
     const int* prefix;
     __half* out;                   // [M][Hq * HD]
     int Hq, Hkv, mr, tail, nkb;
-    int set_rows, sets;                    // query rows of a CTA, and such sets per kv head
+    int sets;                              // sets of query rows per kv head
     int row0, req_rows, cap, write_off;    // cache row of (this layer, K, head 0), rows of one request's cache
     float scale_log2;
     int* err;
@@ -582,30 +583,35 @@ __device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
 
-template <int HD>
+template <int HD, int PT>
 struct DAGeo {
-    static constexpr int BLOCK = 2 * 64 * HD * 2;                       // K and V of 64 keys
-    static constexpr int STAGES = 3;
+    static constexpr int ROWS = 128 / PT;                                // query rows of a CTA: 8 / PT tiles of 16
+    static constexpr int BLOCK = 2 * 64 * HD * 2;                        // K and V of 64 keys
+    static constexpr int STAGES = HD == 128 ? 2 : 3;
+    static constexpr int Q = STAGES * BLOCK;                             // queries [row][HD], 16-byte units swizzled
+    static constexpr int P = Q + ROWS * HD * 2;                          // probabilities of a block [tile][16][64], swizzled
     static constexpr int OP = HD + 4;                                    // floats per row of a partial output
-    static constexpr int SLOTS = 128 + 4 * (kMaxCluster - 1);
-    static constexpr int INBOX = STAGES * BLOCK;                         // partial outputs [source][row of this CTA][OP]
-    static constexpr int INBOX_ML = INBOX + SLOTS * OP * 4;              // and their (max, sum)
-    static constexpr int SMEM = INBOX_ML + SLOTS * 8 + 1024;
+    static constexpr int INBOX = P + ROWS * 128;                         // partial outputs [source CTA][row of this CTA][OP]
+    static constexpr int INBOX_ML = INBOX + (ROWS + kMaxCluster) * OP * 4;       // and (max, sum) [source CTA][part][row]
+    static constexpr int SMEM = INBOX_ML + PT * (ROWS + kMaxCluster) * 8 + 1024;
+    static_assert(SMEM + DGeo<16>::SMEM + 4 * 1024 <= 228 * 1024, "a CTA of the next kernel (up to 16 tokens) fits beside");
 };
 
-template <int HD>
+template <int HD, int PT>
 __global__ void __launch_bounds__(256) attention_kernel(const __grid_constant__ DAttn p) {
-    using G = DAGeo<HD>;
+    using G = DAGeo<HD, PT>;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ uint64_t full[G::STAGES], inboxfull;
     __shared__ int s_abort;
+    __shared__ float s_max[8 / PT][PT][16];
     const uint32_t sbase = smem_u32(smem);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const uint32_t rank = cluster_rank(), cs = cluster_size();
     const int req = blockIdx.z, hk = (int)blockIdx.y / p.sets, set = (int)blockIdx.y - hk * p.sets;
     if (threadIdx.x == 0) {
+        asm volatile("prefetch.tensormap [%0];\n" ::"l"(&p.kvmap) : "memory");
         s_abort = 0;
         for (int s = 0; s < G::STAGES; s++) mbar_init(smem_u32(full + s), 1);
         mbar_init(smem_u32(&inboxfull), cs * 8);                         // every warp of the cluster
@@ -637,6 +643,10 @@ __global__ void __launch_bounds__(256) attention_kernel(const __grid_constant__ 
             for (int b = b0; b < asked; b++) load(b);
         __syncwarp();
     }
+    const int Gq = p.Hq / p.Hkv, QR = p.mr * Gq, row_base = set * G::ROWS, rows = min(G::ROWS, QR - row_base);
+    const int tile = warp / PT, part = warp % PT;
+    const int lr = tile * 16 + g;                                       // this thread's rows: lr, lr + 8
+    const bool v0 = lr < rows, v1 = lr + 8 < rows, busy = tile * 16 < rows && b0 < b1;
     pdl_wait();
     if (warp == kLoader) {
         if (elect_one()) {
@@ -645,37 +655,32 @@ __global__ void __launch_bounds__(256) attention_kernel(const __grid_constant__ 
         }
         __syncwarp();
     }
-
-    const int Gq = p.Hq / p.Hkv, QR = p.mr * Gq, rows = min(p.set_rows, QR - set * p.set_rows);
-    // warps: row tiles (rounded up to 2, 4 or 8) x parts of a key block
-    const int ntp = rows <= 32 ? 2 : (rows <= 64 ? 4 : 8), parts = 8 / ntp, units = 4 / parts;        // units of 16 keys per warp and block
-    const int lw = (warp & (ntp - 1)) * 16, part = warp / ntp;          // the warp's first row inside the set
-    const bool busy = lw < rows && b0 < b1;
-    const int r0 = set * p.set_rows + lw + g, r1 = r0 + 8;
-    const bool v0 = lw + g < rows, v1 = lw + g + 8 < rows;
-    const int q0r = v0 ? r0 / Gq : 0, q1r = v1 ? r1 / Gq : 0;
-    const int m0 = req * p.mr + q0r, m1 = req * p.mr + q1r;
-    uint32_t qa[HD / 16][4];
-    float mrun0 = -INFINITY, mrun1 = -INFINITY, l0 = 0.f, l1 = 0.f;
-    float o[HD / 8][4];
-    unsigned long long mk0 = 0ull, mk1 = 0ull;
-    if (busy) {
-        const __half* q0 = p.q + (size_t)m0 * p.pitch + (size_t)(hk * Gq + (v0 ? r0 - q0r * Gq : 0)) * HD + 2 * t;
-        const __half* q1 = p.q + (size_t)m1 * p.pitch + (size_t)(hk * Gq + (v1 ? r1 - q1r * Gq : 0)) * HD + 2 * t;
-#pragma unroll
-        for (int ks = 0; ks < HD / 16; ks++) {
-            qa[ks][0] = __ldcg(reinterpret_cast<const uint32_t*>(q0 + ks * 16));
-            qa[ks][1] = __ldcg(reinterpret_cast<const uint32_t*>(q1 + ks * 16));
-            qa[ks][2] = __ldcg(reinterpret_cast<const uint32_t*>(q0 + ks * 16 + 8));
-            qa[ks][3] = __ldcg(reinterpret_cast<const uint32_t*>(q1 + ks * 16 + 8));
+    // queries -> shared memory, 16 bytes a thread
+#pragma unroll 2
+    for (int i = threadIdx.x; i < G::ROWS * HD / 8; i += 256) {
+        const int r = i / (HD / 8), v = i % (HD / 8);
+        uint4 q = make_uint4(0, 0, 0, 0);
+        if (r < rows) {
+            const int tok = (row_base + r) / Gq;
+            q = __ldcg(reinterpret_cast<const uint4*>(p.q + (size_t)(req * p.mr + tok) * p.pitch + (size_t)(hk * Gq + row_base + r - tok * Gq) * HD) + v);
         }
-        if (v0) mk0 = p.mask[m0];
-        if (v1) mk1 = p.mask[m1];
-#pragma unroll
-        for (int nd = 0; nd < HD / 8; nd++) o[nd][0] = o[nd][1] = o[nd][2] = o[nd][3] = 0.f;
+        *reinterpret_cast<uint4*>(smem + G::Q + r * HD * 2 + ((v ^ (r & 7)) << 4)) = q;
     }
-    const uint32_t krow_l = (uint32_t)(lane & 7), kvec_l = (uint32_t)(lane >> 3);                       // fragment rows and vectors of K
-    const uint32_t vrow_l = (uint32_t)(((lane >> 3) & 1) * 8 + (lane & 7)), vvec_l = (uint32_t)(lane >> 4);   // and of V
+    const unsigned long long mk0 = v0 ? p.mask[req * p.mr + (row_base + lr) / Gq] : 0ull;
+    const unsigned long long mk1 = v1 ? p.mask[req * p.mr + (row_base + lr + 8) / Gq] : 0ull;
+    __syncthreads();
+
+    constexpr int KT = 8 / PT;                                          // 8-key columns of a warp in the first matmul
+    constexpr int ND = HD / PT / 8;                                     // 8-dim columns in the second
+    float mrun0 = -INFINITY, mrun1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+    float o[ND][4];
+#pragma unroll
+    for (int nd = 0; nd < ND; nd++) o[nd][0] = o[nd][1] = o[nd][2] = o[nd][3] = 0.f;
+    const uint32_t arow = (uint32_t)(lane & 15), avec = (uint32_t)(lane >> 4);                           // fragments of Q and P
+    const uint32_t krow_l = (uint32_t)(lane & 7), kvec_l = (uint32_t)(lane >> 3);                        // of K
+    const uint32_t vrow_l = (uint32_t)(((lane >> 3) & 1) * 8 + (lane & 7)), vvec_l = (uint32_t)(lane >> 4);    // and of V
+    const uint32_t qaddr = sbase + G::Q + (tile * 16 + arow) * (HD * 2), paddr = sbase + G::P + tile * 2048;
+    auto tile_sync = [&]() { asm volatile("bar.sync %0, %1;\n" ::"r"(tile + 1), "n"(PT * 32) : "memory"); };
 
 #pragma unroll 1
     for (int b = b0; b < b1; b++) {
@@ -684,70 +689,89 @@ __global__ void __launch_bounds__(256) attention_kernel(const __grid_constant__ 
         __syncwarp();
         if (busy) {
             const uint32_t sk = sbase + st * G::BLOCK, sv = sk + (HD / 64) * 8192;
-#pragma unroll 1
-            for (int u = 0; u < units; u++) {
-                const int k0 = (part * units + u) * 16;                  // first key of the unit inside the block
-                float s[2][4];
+            // scores of this warp's keys
+            const int k0 = part * KT * 8;
+            float s[KT][4];
 #pragma unroll
-                for (int nt = 0; nt < 2; nt++) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
+            for (int nt = 0; nt < KT; nt++) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
+#pragma unroll 2
+            for (int ks = 0; ks < HD / 16; ks += 2) {
+                uint32_t qa[4], qb[4];
+                ldsm4(qa, qaddr + (((ks * 2 + avec) ^ (arow & 7)) << 4));
+                ldsm4(qb, qaddr + (((ks * 2 + 2 + avec) ^ (arow & 7)) << 4));
 #pragma unroll
-                for (int ks = 0; ks < HD / 16; ks += 2)
-#pragma unroll
-                    for (int nt = 0; nt < 2; nt++) {
-                        uint32_t kf[4];
-                        ldsm4(kf, sk + kv_swz(k0 + nt * 8 + krow_l, ks * 2 + kvec_l));
-                        mma_m16n8k16(s[nt], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], kf[0], kf[1]);
-                        mma_m16n8k16(s[nt], qa[ks + 1][0], qa[ks + 1][1], qa[ks + 1][2], qa[ks + 1][3], kf[2], kf[3]);
-                    }
-                float mx0 = mrun0, mx1 = mrun1;
-                const int j0 = b * kKeyBlock + k0 + 2 * t - prefix;      // tail row of the thread's first key
-                const bool committed_unit = b * kKeyBlock + k0 + 16 <= prefix;
-#pragma unroll
-                for (int nt = 0; nt < 2; nt++)
-#pragma unroll
-                    for (int e = 0; e < 2; e++) {
-                        bool vis0 = v0, vis1 = v1;
-                        const int j = j0 + nt * 8 + e;
-                        if (!committed_unit && j >= 0) {
-                            vis0 = v0 && j < p.tail && ((mk0 >> (j & 63)) & 1ull);
-                            vis1 = v1 && j < p.tail && ((mk1 >> (j & 63)) & 1ull);
-                        }
-                        s[nt][e] = vis0 ? s[nt][e] * p.scale_log2 : -INFINITY;
-                        s[nt][2 + e] = vis1 ? s[nt][2 + e] * p.scale_log2 : -INFINITY;
-                        mx0 = fmaxf(mx0, s[nt][e]);
-                        mx1 = fmaxf(mx1, s[nt][2 + e]);
-                    }
-                mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-                mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-                mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-                mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-                const float base0 = (mx0 == -INFINITY) ? 0.f : mx0;
-                const float base1 = (mx1 == -INFINITY) ? 0.f : mx1;
-                if (__any_sync(0xffffffffu, mx0 != mrun0 || mx1 != mrun1)) {       // a running maximum moved: rescale sums and outputs
-                    const float al0 = (mrun0 == -INFINITY) ? 0.f : exp2f(mrun0 - base0);
-                    const float al1 = (mrun1 == -INFINITY) ? 0.f : exp2f(mrun1 - base1);
-                    l0 *= al0; l1 *= al1;
-#pragma unroll
-                    for (int nd = 0; nd < HD / 8; nd++) { o[nd][0] *= al0; o[nd][1] *= al0; o[nd][2] *= al1; o[nd][3] *= al1; }
-                    mrun0 = mx0; mrun1 = mx1;
+                for (int nt = 0; nt < KT; nt++) {
+                    uint32_t kf[4];
+                    ldsm4(kf, sk + kv_swz(k0 + nt * 8 + krow_l, ks * 2 + kvec_l));
+                    mma_m16n8k16(s[nt], qa[0], qa[1], qa[2], qa[3], kf[0], kf[1]);
+                    mma_m16n8k16(s[nt], qb[0], qb[1], qb[2], qb[3], kf[2], kf[3]);
                 }
-                uint32_t pa[2][2];
+            }
+            float mx0 = -INFINITY, mx1 = -INFINITY;
+            const int j0 = b * kKeyBlock + k0 + 2 * t - prefix;          // tail row of the thread's first key
+            const bool open = b * kKeyBlock + kKeyBlock <= prefix;       // committed rows only
 #pragma unroll
-                for (int nt = 0; nt < 2; nt++) {
-                    const __half2 h0 = __floats2half2_rn(exp2f(s[nt][0] - base0), exp2f(s[nt][1] - base0));
-                    const __half2 h1 = __floats2half2_rn(exp2f(s[nt][2] - base1), exp2f(s[nt][3] - base1));
-                    // the sum uses the rounded probabilities so that numerator and denominator agree
-                    l0 += __low2float(h0) + __high2float(h0);
-                    l1 += __low2float(h1) + __high2float(h1);
-                    pa[nt][0] = h2_as_u32(h0);
-                    pa[nt][1] = h2_as_u32(h1);
+            for (int nt = 0; nt < KT; nt++)
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    bool vis0 = v0, vis1 = v1;
+                    const int j = j0 + nt * 8 + e;
+                    if (!open && j >= 0) {
+                        vis0 = v0 && j < p.tail && ((mk0 >> (j & 63)) & 1ull);
+                        vis1 = v1 && j < p.tail && ((mk1 >> (j & 63)) & 1ull);
+                    }
+                    s[nt][e] = vis0 ? s[nt][e] * p.scale_log2 : -INFINITY;
+                    s[nt][2 + e] = vis1 ? s[nt][2 + e] * p.scale_log2 : -INFINITY;
+                    mx0 = fmaxf(mx0, s[nt][e]);
+                    mx1 = fmaxf(mx1, s[nt][2 + e]);
                 }
+            mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
+            mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+            mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
+            mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+            if (t == 0) {
+                s_max[tile][part][g] = mx0;
+                s_max[tile][part][g + 8] = mx1;
+            }
+            tile_sync();
+            mx0 = mrun0;
+            mx1 = mrun1;
 #pragma unroll
-                for (int nd = 0; nd < HD / 8; nd += 2) {
+            for (int i = 0; i < PT; i++) {
+                mx0 = fmaxf(mx0, s_max[tile][i][g]);
+                mx1 = fmaxf(mx1, s_max[tile][i][g + 8]);
+            }
+            const float base0 = (mx0 == -INFINITY) ? 0.f : mx0;
+            const float base1 = (mx1 == -INFINITY) ? 0.f : mx1;
+            const float al0 = (mrun0 == -INFINITY) ? 0.f : exp2f(mrun0 - base0);
+            const float al1 = (mrun1 == -INFINITY) ? 0.f : exp2f(mrun1 - base1);
+            l0 *= al0; l1 *= al1;
+            mrun0 = mx0; mrun1 = mx1;
+#pragma unroll
+            for (int nt = 0; nt < KT; nt++) {
+                const __half2 h0 = __floats2half2_rn(exp2f(s[nt][0] - base0), exp2f(s[nt][1] - base0));
+                const __half2 h1 = __floats2half2_rn(exp2f(s[nt][2] - base1), exp2f(s[nt][3] - base1));
+                // the sum uses the rounded probabilities so that numerator and denominator agree
+                l0 += __low2float(h0) + __high2float(h0);
+                l1 += __low2float(h1) + __high2float(h1);
+                unsigned char* d = smem + G::P + tile * 2048 + g * 128 + (((part * KT + nt) ^ g) << 4) + t * 4;      // (rows g and g + 8: the same swizzle)
+                *reinterpret_cast<__half2*>(d) = h0;
+                *reinterpret_cast<__half2*>(d + 1024) = h1;
+            }
+#pragma unroll
+            for (int nd = 0; nd < ND; nd++) { o[nd][0] *= al0; o[nd][1] *= al0; o[nd][2] *= al1; o[nd][3] *= al1; }
+            tile_sync();
+            // this warp's dims of the output, over all keys of the block
+#pragma unroll 2
+            for (int ks = 0; ks < 4; ks++) {
+                uint32_t pa[4];
+                ldsm4(pa, paddr + arow * 128 + (((ks * 2 + avec) ^ (arow & 7)) << 4));
+#pragma unroll
+                for (int nd = 0; nd < ND; nd += 2) {
                     uint32_t vb[4];
-                    ldsm4_t(vb, sv + kv_swz(k0 + vrow_l, nd + vvec_l));
-                    mma_m16n8k16(o[nd], pa[0][0], pa[0][1], pa[1][0], pa[1][1], vb[0], vb[1]);
-                    mma_m16n8k16(o[nd + 1], pa[0][0], pa[0][1], pa[1][0], pa[1][1], vb[2], vb[3]);
+                    ldsm4_t(vb, sv + kv_swz(ks * 16 + vrow_l, part * ND + nd + vvec_l));
+                    mma_m16n8k16(o[nd], pa[0], pa[1], pa[2], pa[3], vb[0], vb[1]);
+                    mma_m16n8k16(o[nd + 1], pa[0], pa[1], pa[2], pa[3], vb[2], vb[3]);
                 }
             }
         }
@@ -768,14 +792,14 @@ __global__ void __launch_bounds__(256) attention_kernel(const __grid_constant__ 
     if (cs > 1) cluster_wait();
 #pragma unroll
     for (int hrow = 0; hrow < 2; hrow++) {
-        const int lr = lw + g + 8 * hrow;
-        if (lr < rows) {
-            const uint32_t dst = lr / nslot, at = (rank * parts + part) * nslot + (lr - dst * nslot);      // (a warp's rows: mostly one CTA)
-            if (t == 0) st_peer2(peer_addr(sbase + G::INBOX_ML + at * 8, dst), hrow ? mrun1 : mrun0, hrow ? l1 : l0);
+        const int row = lr + 8 * hrow;
+        if (row < rows) {
+            const uint32_t dst = row / nslot, sl = row - dst * nslot;    // (a warp's rows: mostly one CTA)
+            if (t == 0) st_peer2(peer_addr(sbase + G::INBOX_ML + ((rank * PT + part) * nslot + sl) * 8, dst), hrow ? mrun1 : mrun0, hrow ? l1 : l0);
             if (busy) {
-                const uint32_t row = peer_addr(sbase + G::INBOX + at * G::OP * 4, dst);
+                const uint32_t at = peer_addr(sbase + G::INBOX + ((rank * nslot + sl) * G::OP + part * ND * 8 + 2 * t) * 4, dst);
 #pragma unroll
-                for (int nd = 0; nd < HD / 8; nd++) st_peer2(row + (nd * 8 + 2 * t) * 4, o[nd][2 * hrow], o[nd][2 * hrow + 1]);
+                for (int nd = 0; nd < ND; nd++) st_peer2(at + nd * 32, o[nd][2 * hrow], o[nd][2 * hrow + 1]);
             }
         }
     }
@@ -783,13 +807,13 @@ __global__ void __launch_bounds__(256) attention_kernel(const __grid_constant__ 
     if (lane < (int)cs) arrive_peer(peer_addr(smem_u32(&inboxfull), lane));
     if (!inbox_wait(smem_u32(&inboxfull))) atomicCAS(p.err, 0, 25);
     __syncwarp();
-    // ---- merge: one warp per row, sources in key order
-    const int sources = (int)cs * parts;
+    // ---- merge: one warp per row, CTAs in key order
     const int row_lo = (int)rank * nslot, mine_rows = min(nslot, rows - row_lo);
+#pragma unroll 1
     for (int j = warp; j < mine_rows; j += 8) {
         constexpr int C = HD / 32;
         const float2* ml = reinterpret_cast<const float2*>(smem + G::INBOX_ML) + j;
-        const float2 mine = lane < sources ? ml[lane * nslot] : make_float2(-INFINITY, 0.f);          // (at most 32 sources)
+        const float2 mine = lane < (int)cs * PT ? ml[lane * nslot] : make_float2(-INFINITY, 0.f);     // lane: (source, part); at most 32
         float mstar = mine.x;
 #pragma unroll
         for (int i = 16; i > 0; i >>= 1) mstar = fmaxf(mstar, __shfl_xor_sync(0xffffffffu, mstar, i));
@@ -801,17 +825,17 @@ __global__ void __launch_bounds__(256) attention_kernel(const __grid_constant__ 
 #pragma unroll
         for (int c = 0; c < C; c++) acc[c] = 0.f;
         const float* v = reinterpret_cast<const float*>(smem + G::INBOX) + j * G::OP + lane * C;
-#pragma unroll 4
-        for (int i = 0; i < sources; i++) {
-            const float wi = __shfl_sync(0xffffffffu, w, i);
+#pragma unroll 2
+        for (int i = 0; i < (int)cs; i++) {
+            const float wi = __shfl_sync(0xffffffffu, w, i * PT);
             if (wi != 0.f) {                                             // (an idle source has left no output)
 #pragma unroll
                 for (int c = 0; c < C; c++) acc[c] += wi * v[i * nslot * G::OP + c];
             }
         }
         const float inv = den > 0.f ? 1.f / den : 0.f;
-        const int gr = set * p.set_rows + row_lo + j, m = req * p.mr + gr / Gq;
-        __half* dst = p.out + (size_t)m * p.Hq * HD + (size_t)(hk * Gq + gr % Gq) * HD + lane * C;
+        const int gr = row_base + row_lo + j, tok = gr / Gq;
+        __half* dst = p.out + (size_t)(req * p.mr + tok) * p.Hq * HD + (size_t)(hk * Gq + gr - tok * Gq) * HD + lane * C;
         __align__(8) __half ov[C];
 #pragma unroll
         for (int c = 0; c < C; c++) ov[c] = __float2half_rn(acc[c] * inv);
@@ -885,12 +909,20 @@ int launch_dense(DenseParams& p, int split, cudaStream_t stream) {
     return rc != B200_OK ? rc : launch(tiles - rest, rest, rest_cs);
 }
 
-template <int HD>
-int launch_attention(const DAttn& a, int nreq, cudaStream_t stream) {
+template <int HD, int PT>
+int launch_attention_pt(DAttn& a, int nreq, cudaStream_t stream) {
+    using G = DAGeo<HD, PT>;
     static std::atomic<uint64_t> done{0};
-    if (!allow_smem(attention_kernel<HD>, DAGeo<HD>::SMEM, done, true)) return check_launch();
+    if (!allow_smem(attention_kernel<HD, PT>, G::SMEM, done, true)) return check_launch();
+    a.sets = (a.mr * (a.Hq / a.Hkv) + G::ROWS - 1) / G::ROWS;
     const int cs = std::min(a.nkb, kMaxCluster);
-    return launch_chain(attention_kernel<HD>, dim3(cs, a.Hkv * a.sets, nreq), 256, DAGeo<HD>::SMEM, cs, stream, a);
+    return launch_chain(attention_kernel<HD, PT>, dim3(cs, a.Hkv * a.sets, nreq), 256, G::SMEM, cs, stream, a);
+}
+// Sets of 32 query rows while that makes one wave (a cluster of 8 CTAs to one or two per GPC), of 64 beyond: fewer reads of K and V.
+template <int HD>
+int launch_attention(DAttn& a, int nreq, cudaStream_t stream) {
+    const int qr = a.mr * (a.Hq / a.Hkv);
+    return qr <= 32 || a.Hkv * nreq * ((qr + 31) / 32) <= 16 ? launch_attention_pt<HD, 4>(a, nreq, stream) : launch_attention_pt<HD, 2>(a, nreq, stream);
 }
 
 template <int NT>
@@ -922,11 +954,6 @@ int run_chain(const ChainArgs& c, cudaStream_t st) {
     a.q = static_cast<const __half*>(d->qkv); a.pitch = nqkv; a.mask = d->mask; a.prefix = d->prefix;
     a.out = static_cast<__half*>(d->attn); a.Hq = d->n_heads; a.Hkv = d->n_kv_heads; a.mr = p.mr; a.tail = d->tail;
     a.nkb = (d->cache_rows + kKeyBlock - 1) / kKeyBlock;
-    // Query rows of a CTA: as few as still make one wave (a cluster of 8 CTAs to one or two per GPC): a warp then has fewer of a
-    // block's keys, and a CTA fewer rows to merge.
-    const int qr = p.mr * (d->n_heads / d->n_kv_heads), clusters = d->n_kv_heads * nreq;
-    a.set_rows = qr <= 32 || clusters * ((qr + 31) / 32) <= 16 ? 32 : (qr <= 64 || clusters * ((qr + 63) / 64) <= 16 ? 64 : 128);
-    a.sets = (qr + a.set_rows - 1) / a.set_rows;
     a.req_rows = d->n_layers * 2 * d->n_kv_heads * d->cache_rows;
     a.cap = d->cache_rows; a.write_off = d->write_off; a.scale_log2 = d->attn_scale * kLog2e; a.err = c.err;
 

@@ -10,7 +10,7 @@ SHAPES = [
     # heads, kv heads, head dim, hidden, intermediate, vocab
     (2, 1, 64, 128, 128, 1032),          # one chunk of K, a last row tile of 8 rows
     (14, 2, 64, 896, 640, 520),          # groups of 7 heads, seven chunks
-    (16, 2, 128, 1024, 2176, 2048),      # groups of 8 heads of 128: up to 256 query rows per kv head
+    (16, 2, 128, 2048, 2176, 2048),      # groups of 8 heads of 128: up to 256 query rows per kv head
 ]
 
 
