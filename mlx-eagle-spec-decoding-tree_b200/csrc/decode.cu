@@ -7,7 +7,7 @@
 //
 // Why a chain and not one persistent kernel: a kernel of such a chain whose every CTA reads what all CTAs of its predecessor
 // wrote costs 1.0 us, the load included; a device-wide barrier of 148 CTAs took 1.5 to 2.3 us and the first loads behind it
-// another 1.1.  A CTA here keeps to half of an SM (480 threads, 64 registers each, ~95 KB of shared memory, 256 columns of tensor memory), so
+// another 1.1.  A CTA here keeps to half of an SM (512 threads, 64 registers each, ~95 KB of shared memory, 256 columns of tensor memory), so
 // the next kernel's CTAs become resident beside it and stream and expand their first weights before its results are there.
 //
 // RMSNorm is folded into the matmuls around it: the producer of h (embedding, C, E) also writes h * w_norm (fp16, one
@@ -38,7 +38,7 @@ constexpr int kTile = 128;                       // weight rows of one MMA
 constexpr int kGroups = 3;                       // groups of four dequant warps, each with a tensor-memory tile of its own
 constexpr int kDeq = 4 * kGroups;                // dequant warps
 constexpr int kEpi = 8;                          // of which these run the epilogue
-constexpr int kDThreads = (kDeq + 3) * 32;       // + weight producer, activation producer, MMA issuer
+constexpr int kDThreads = (kDeq + 4) * 32;       // + weight producer, activation producer, MMA issuer, sums of squares
 constexpr int kTCols = kChunkK / 2;              // tensor-memory columns of an expanded tile
 constexpr int kTmem = 256;                       // columns a CTA takes: two CTAs share an SM
 constexpr int kRedPitch = kTile + 4;             // floats per token row of the partial products in shared memory
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
     __shared__ uint64_t wfull[G::NW], wempty[G::NW], xfull[G::NX], xempty[G::NX], tready[kGroups], tfree[kGroups], accfull[2], accempty[2], inboxfull;
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
-    __shared__ float s_part[kEpi][32];
+    __shared__ float s_rs[32];                                   // 1 / rms per token
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank(), cs = cluster_size();
@@ -175,29 +175,53 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
     const int c_lo = nchunks * (int)rank / (int)cs, nc = nchunks * ((int)rank + 1) / (int)cs - c_lo;      // chunks of each
     const int ntok = p.M > (int)rank ? (p.M - (int)rank + (int)cs - 1) / (int)cs : 0;                     // and tokens: rank, rank + cs, ...
 
-    if (threadIdx.x == 0) {
-        asm volatile("prefetch.tensormap [%0];\n" ::"l"(&p.xmap) : "memory");
-        s_abort = 0;
-        for (int s = 0; s < G::NW; s++) {
-            mbar_init(smem_u32(wfull + s), 1);
-            mbar_init(smem_u32(wempty + s), 4);                 // a group's warps
+    if (threadIdx.x < 32) {                                      // (a thread a barrier: one thread for all took 400 cycles)
+        if (lane < G::NX) {
+            mbar_init(smem_u32(xfull + lane), 1);
+            mbar_init(smem_u32(xempty + lane), 1);
         }
-        for (int s = 0; s < G::NX; s++) {
-            mbar_init(smem_u32(xfull + s), 1);
-            mbar_init(smem_u32(xempty + s), 1);
+        if (lane < kGroups) {
+            mbar_init(smem_u32(tready + lane), 4);
+            mbar_init(smem_u32(tfree + lane), 1);
         }
-        for (int s = 0; s < kGroups; s++) {
-            mbar_init(smem_u32(tready + s), 4);
-            mbar_init(smem_u32(tfree + s), 1);
+        if (lane < 2) {
+            mbar_init(smem_u32(accfull + lane), 1);
+            mbar_init(smem_u32(accempty + lane), kEpi);
         }
-        for (int s = 0; s < 2; s++) {
-            mbar_init(smem_u32(accfull + s), 1);
-            mbar_init(smem_u32(accempty + s), kEpi);
+        if (lane == 31) {
+            s_abort = 0;
+            mbar_init(smem_u32(&inboxfull), 1);
+            if (cs > 1) mbar_expect_tx(smem_u32(&inboxfull), cs * ntok * kTile * 4); // what the cluster's CTAs will store here
         }
-        mbar_init(smem_u32(&inboxfull), 1);
-        if (cs > 1) mbar_expect_tx(smem_u32(&inboxfull), cs * ntok * kTile * 4);     // what the cluster's CTAs will store here
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
+    // The weight producer makes its own barriers and asks for the first stages before the block is set up.
+    const int nblocks = (p.N + 63) / 64;
+    auto wsrc = [&](int tile, int second) {                      // chunk c_lo of the tile's first or second 64 rows (gate / up: of the same rows of each)
+        return KIND == D_SILU ? p.w[second] + ((size_t)tile * nchunks + c_lo) * kRun
+                              : p.w[0] + ((size_t)min(2 * tile + second, nblocks - 1) * nchunks + c_lo) * kRun;
+    };
+    auto wload = [&](uint32_t slot, const unsigned char* src0, const unsigned char* src1) {
+        const uint32_t bar = smem_u32(wfull + slot), dst = smem_u32(ring + slot * kW);
+        mbar_expect_tx(bar, kW);
+        bulk_copy_g2s(dst, src0, kRun, bar);
+        bulk_copy_g2s(dst + kRun, src1, kRun, bar);
+    };
+    if (warp == kDeq) {
+        if (lane < G::NW) {
+            mbar_init(smem_u32(wfull + lane), 1);
+            mbar_init(smem_u32(wempty + lane), 4);               // a group's warps
+            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        }
+        __syncwarp();
+        if (elect_one()) {
+            const unsigned char *src0 = wsrc(tile0, 0), *src1 = wsrc(tile0, 1);
+#pragma unroll 1
+            for (int c = 0; c < min(nc, G::NW); c++) wload(c, src0 + c * kRun, src1 + c * kRun);
+        }
+        __syncwarp();
+    }
+    if (warp == kDeq + 1 && lane == 0) asm volatile("prefetch.tensormap [%0];\n" ::"l"(&p.xmap) : "memory");
     if (warp == kDeq + 2) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s_tmem)), "n"(kTmem) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
@@ -212,23 +236,19 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
 
     if (warp == kDeq) {
         // ------------------------------------------------------------------ weight producer: depends on nothing
-        const int nblocks = (p.N + 63) / 64;
-        uint32_t slot = 0, ph = 1;
-        bool lap = false;
-        for (int it = 0, tile = tile0; it < nit; it++, tile += tstep) {
-            const unsigned char* src0 = p.w[0] + ((size_t)(KIND == D_SILU ? tile : min(2 * tile, nblocks - 1)) * nchunks + c_lo) * kRun;
-            const unsigned char* src1 = KIND == D_SILU ? p.w[1] + ((size_t)tile * nchunks + c_lo) * kRun         // the same 64 rows of up
-                                                       : p.w[0] + ((size_t)min(2 * tile + 1, nblocks - 1) * nchunks + c_lo) * kRun;
+        const int first = min(nc, G::NW);                        // (asked for above)
+        uint32_t slot = first % G::NW, ph = 1;
+        bool lap = first == G::NW;
+        if (lap) ph = 0;
 #pragma unroll 1
-            for (int c = 0; c < nc; c++) {
+        for (int it = 0, tile = tile0; it < nit; it++, tile += tstep) {
+            const int c0 = it == 0 ? first : 0;
+            const unsigned char *src0 = wsrc(tile, 0) + c0 * kRun, *src1 = wsrc(tile, 1) + c0 * kRun;
+#pragma unroll 1
+            for (int c = c0; c < nc; c++) {
                 if (lap) dwait(smem_u32(wempty + slot), ph, abort_flag, p.err, 21);
                 __syncwarp();
-                if (elect_one()) {
-                    const uint32_t bar = smem_u32(wfull + slot), dst = smem_u32(ring + slot * kW);
-                    mbar_expect_tx(bar, kW);
-                    bulk_copy_g2s(dst, src0, kRun, bar);
-                    bulk_copy_g2s(dst + kRun, src1, kRun, bar);
-                }
+                if (elect_one()) wload(slot, src0, src1);
                 __syncwarp();
                 src0 += kRun;
                 src1 += kRun;
@@ -290,6 +310,34 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         asm volatile("bar.sync 2, %0;\n" ::"n"((kEpi + 1) * 32) : "memory");         // accumulators read
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(kTmem) : "memory");
+    } else if (warp == kDeq + 3) {
+        // ------------------------------------------------------------------ sums of squares -> 1 / rms of each token
+        // (by the dequant warps it held up every chunk behind the first three: 1.4 us at a hidden size of 3584)
+        if (KIND != D_RESID) {
+            pdl_wait();
+            // a lane: four tokens of every `step`-th part; as many parts at once as the tokens leave lanes for
+            const int quads = p.M <= 8 ? 2 : (p.M <= 16 ? 4 : 8), step = 32 / quads, quad = lane & (quads - 1);
+            float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 7
+            for (int part = lane / quads; part < p.H / 32; part += step) {
+                const float4 v = __ldcg(reinterpret_cast<const float4*>(p.ssq + part * kSsqPitch + quad * 4));
+                t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w;
+            }
+            for (int o = 16; o >= quads; o >>= 1) {
+                t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
+                t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
+                t.z += __shfl_xor_sync(0xffffffffu, t.z, o);
+                t.w += __shfl_xor_sync(0xffffffffu, t.w, o);
+            }
+            if (lane < quads) {
+                s_rs[quad * 4] = rsqrtf(t.x / (float)p.H + p.eps);
+                s_rs[quad * 4 + 1] = rsqrtf(t.y / (float)p.H + p.eps);
+                s_rs[quad * 4 + 2] = rsqrtf(t.z / (float)p.H + p.eps);
+                s_rs[quad * 4 + 3] = rsqrtf(t.w / (float)p.H + p.eps);
+            }
+            __syncwarp();
+            asm volatile("bar.arrive 3, %0;\n" ::"n"((kEpi + 1) * 32) : "memory");
+        }
     } else {
         // ------------------------------------------------------------------ dequant warps
         const uint32_t me = warp >> 2;                           // group (and, in the epilogue, which half of the tokens)
@@ -299,21 +347,6 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
         const int flip = (r >> 1) & 1;                           // (bank conflicts: see qmm_gemm.cu)
         constexpr bool NORMED = KIND != D_RESID;                 // the input is h * w_norm: scale by 1 / rms
-        bool waited = false;
-        float rs_lane = 1.f;                                     // 1 / rms of token `lane`
-        auto dependent = [&]() {
-            // the tiles expanded so far wait for the activations: so does this thread, then takes its share of the sums of squares
-            pdl_wait();
-            waited = true;
-            if (NORMED && warp < kEpi) {
-                float ssum = 0.f;
-                if (lane < p.M) {
-#pragma unroll 4
-                    for (int part = warp; part < p.H / 32; part += kEpi) ssum += __ldcg(p.ssq + part * kSsqPitch + lane);
-                }
-                s_part[warp][lane] = ssum;
-            }
-        };
         // ---- one finished tile: accumulators -> inbox of the CTA that finishes each token -> output
         auto epilogue = [&](int it) {
             const int tile = tile0 + it * tstep;
@@ -334,6 +367,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
             auto ask_r = [&](int j) -> float2 {
                 return KIND == D_QKV && rotate && j < ntok ? __ldcg(p.cs + ((int)rank + j * (int)cs) * kCsPitch + (first ? hi : hi - half)) : make_float2(0.f, 0.f);
             };
+            if (it == 0) pdl_wait();
             if (KIND == D_RESID && valid) extra = p.wn[n];
             if (KIND == D_QKV && valid && p.bias != nullptr) {
                 extra = p.bias[n];
@@ -375,16 +409,10 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                         st_async(peer_addr(in0 + ((rank * nslot + sl) * kRedPitch + r) * 4, dst), a[i], peer_addr(inbar, dst));
                     if (++dst == cs) { dst = 0; sl++; }
                 }
-                if (NORMED) consumer_sync(kEpi * 32);            // s_part
                 if (!inbox_wait(inbar)) atomicCAS(p.err, 0, 28);     // (in full after a timeout too: a peer may still be storing here)
                 __syncwarp();
             }
-            if (NORMED && it == 0) {
-                float t = 0.f;
-#pragma unroll
-                for (int i = 0; i < kEpi; i++) t += s_part[i][lane];
-                rs_lane = rsqrtf(t / (float)p.H + p.eps);
-            }
+            if (NORMED && it == 0) asm volatile("bar.sync 3, %0;\n" ::"n"((kEpi + 1) * 32) : "memory");      // s_rs
             auto total = [&](int j, int row) {                   // the sources in rank order
                 const float* v = inbox + j * kRedPitch + row;
                 float t = v[0];
@@ -395,7 +423,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
 #pragma unroll 1
             for (int j = j0; j < ntok; j += JS) {                // (warp-uniform)
                 const int tok = (int)rank + j * (int)cs;
-                const float rs = NORMED ? __shfl_sync(0xffffffffu, rs_lane, tok) : 1.f;
+                const float rs = NORMED ? s_rs[tok] : 1.f;
                 const float v = total(j, r2) * rs;
                 const int rq = KIND == D_HEAD || KIND == D_QKV ? (p.mr == p.M ? 0 : tok / p.mr) : 0;
                 if (KIND == D_SILU) {
@@ -447,11 +475,11 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
 #pragma unroll 1
         for (int it = 0; it <= nit; it++) {
             const int end = it < nit ? (it + 1) * nc : 0;
-            bool pending = it > 0;                               // the tile before this one, once this one's first chunk is expanded
+            bool pending = it > 0;                               // the tile before this one, once two chunks of this one are expanded:
+            int ahead = 0;                                       // its last MMA is done by then
 #pragma unroll 1
             do {
                 if (done < end) {
-                    if (done >= kGroups && !waited) dependent();
                     dwait(smem_u32(wfull + slot), wph, abort_flag, p.err, 24);
                     __syncwarp();
                     const unsigned char* st = ring + slot * kW;
@@ -495,11 +523,11 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(tready + me));
                     done += kGroups;
+                    ahead++;
                     if ((slot += kGroups) >= (uint32_t)G::NW) { slot -= G::NW; wph ^= 1; }
                     tph ^= 1;
                 }
-                if (pending) {
-                    if (!waited) dependent();
+                if (pending && (ahead == 2 || done >= end)) {
                     if (warp < kEpi) epilogue(it - 1);
                     pending = false;
                 }
