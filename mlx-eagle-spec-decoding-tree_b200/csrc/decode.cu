@@ -160,7 +160,7 @@ template <int NT, int KIND>
 __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_constant__ DenseParams p) {
     using G = DGeo<NT>;
     extern __shared__ unsigned char smem_raw[];
-    unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    unsigned char* ring = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);
     float* inbox = reinterpret_cast<float*>(ring + G::INBOX);
     __shared__ uint64_t wfull[G::NW], wempty[G::NW], xfull[G::NX], xempty[G::NX], tready[kGroups], tfree[kGroups], accfull[2], accempty[2], inboxfull;
     __shared__ uint32_t s_tmem;
@@ -345,7 +345,8 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         const uint32_t recoff = (r >> 6) * kRun + ((r >> 4) & 3) * 1152;
         const uint32_t rowoff = recoff + (rr >> 3) * 512 + (rr & 7) * 64, scoff = recoff + 1024 + rr * 8;
         const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
-        const int flip = (r >> 1) & 1;                           // (bank conflicts: see qmm_gemm.cu)
+        // (Four threads of a quarter-warp read the same banks: swapping units between threads to halve that took more issue slots, 16
+        // selects a chunk, than the reads took cycles.)
         constexpr bool NORMED = KIND != D_RESID;                 // the input is h * w_norm: scale by 1 / rms
         // ---- one finished tile: accumulators -> inbox of the CTA that finishes each token -> output
         auto epilogue = [&](int it) {
@@ -485,12 +486,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                     const unsigned char* st = ring + slot * kW;
                     uint4 u[4];
 #pragma unroll
-                    for (int i = 0; i < 4; i += 2) {
-                        const uint4 a = *reinterpret_cast<const uint4*>(st + rowoff + (i + flip) * 16);
-                        const uint4 b = *reinterpret_cast<const uint4*>(st + rowoff + (i + 1 - flip) * 16);
-                        u[i] = flip ? b : a;
-                        u[i + 1] = flip ? a : b;
-                    }
+                    for (int i = 0; i < 4; i++) u[i] = *reinterpret_cast<const uint4*>(st + rowoff + i * 16);
                     const uint2 sb = *reinterpret_cast<const uint2*>(st + scoff);
                     const bool fast = __all_sync(0xffffffffu, fast_scale(sb.x) && fast_scale(sb.y));
                     if (lane == 0) mbar_arrive(smem_u32(wempty + slot));             // the packs are in registers
@@ -581,8 +577,8 @@ __global__ void __launch_bounds__(256) embed_kernel(const int* __restrict__ toke
 }
 
 // ================================================================================ attention
-// CTA = (key range, kv head, request, set of query rows); a query row is (token, head of the group).  PT warps share a tile of 16
-// rows: each takes 1 / PT of a block's keys for the scores and, the probabilities exchanged through shared memory, 1 / PT of the
+// CTA = (key range, kv head, request, set of 32 query rows); a query row is (token, head of the group).  Four warps share a tile of 16
+// rows: each takes a quarter of a block's keys for the scores and, the probabilities exchanged through shared memory, 1 / PT of the
 // dims for the output, so partial outputs leave the CTA once per row.  (Each warp all dims for its keys sent PT times as much to
 // the peers, which took longer than the matmuls.)  All share the K/V blocks (TMA boxes, 128-byte swizzle).  The CTAs of a cluster
 // take neighbouring key ranges; each finishes its share of the rows, whose partial softmax states the others store into its shared
@@ -611,9 +607,10 @@ __device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
 
-template <int HD, int PT>
+constexpr int kAWarps = 8, kAParts = 4;            // warps of an attention CTA, warps that share a row tile
+template <int HD>
 struct DAGeo {
-    static constexpr int ROWS = 128 / PT;                                // query rows of a CTA: 8 / PT tiles of 16
+    static constexpr int ROWS = 16 * kAWarps / kAParts;                  // query rows of a CTA: tiles of 16
     static constexpr int BLOCK = 2 * 64 * HD * 2;                        // K and V of 64 keys
     static constexpr int STAGES = HD == 128 ? 2 : 3;
     static constexpr int Q = STAGES * BLOCK;                             // queries [row][HD], 16-byte units swizzled
@@ -621,18 +618,19 @@ struct DAGeo {
     static constexpr int OP = HD + 4;                                    // floats per row of a partial output
     static constexpr int INBOX = P + ROWS * 128;                         // partial outputs [source CTA][row of this CTA][OP]
     static constexpr int INBOX_ML = INBOX + (ROWS + kMaxCluster) * OP * 4;       // and (max, sum) [source CTA][part][row]
-    static constexpr int SMEM = INBOX_ML + PT * (ROWS + kMaxCluster) * 8 + 1024;
-    static_assert(SMEM + DGeo<16>::SMEM + 4 * 1024 <= 228 * 1024, "a CTA of the next kernel (up to 16 tokens) fits beside");
+    static constexpr int SMEM = INBOX_ML + kAParts * (ROWS + kMaxCluster) * 8 + 1024;
+    static_assert(2 * (SMEM + 2048) <= 227 * 1024 && SMEM + DGeo<32>::SMEM + 4 * 1024 <= 227 * 1024, "two CTAs per SM, or one beside a matmul CTA");
 };
 
-template <int HD, int PT>
-__global__ void __launch_bounds__(256) attention_kernel(const __grid_constant__ DAttn p) {
-    using G = DAGeo<HD, PT>;
+template <int HD>
+__global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_constant__ DAttn p) {
+    using G = DAGeo<HD>;
+    constexpr int PT = kAParts;
     extern __shared__ unsigned char smem_raw[];
-    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    unsigned char* smem = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);
     __shared__ uint64_t full[G::STAGES], inboxfull;
     __shared__ int s_abort;
-    __shared__ float s_max[8 / PT][PT][16];
+    __shared__ float s_max[kAWarps / PT][PT][16];
     const uint32_t sbase = smem_u32(smem);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
@@ -642,7 +640,7 @@ __global__ void __launch_bounds__(256) attention_kernel(const __grid_constant__ 
         asm volatile("prefetch.tensormap [%0];\n" ::"l"(&p.kvmap) : "memory");
         s_abort = 0;
         for (int s = 0; s < G::STAGES; s++) mbar_init(smem_u32(full + s), 1);
-        mbar_init(smem_u32(&inboxfull), cs * 8);                         // every warp of the cluster
+        mbar_init(smem_u32(&inboxfull), cs * kAWarps);                         // every warp of the cluster
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
@@ -665,7 +663,7 @@ __global__ void __launch_bounds__(256) attention_kernel(const __grid_constant__ 
     };
     const int committed = min(b1, new0 / kKeyBlock);                    // blocks below it hold no row of this pass
     const int asked = max(b0, min(committed, b0 + G::STAGES));
-    constexpr int kLoader = 7;                                          // (the warp with the last rows, if it has any)
+    constexpr int kLoader = kAWarps - 1;                                          // (the warp with the last rows, if it has any)
     if (warp == kLoader) {
         if (elect_one())
             for (int b = b0; b < asked; b++) load(b);
@@ -685,7 +683,7 @@ __global__ void __launch_bounds__(256) attention_kernel(const __grid_constant__ 
     }
     // queries -> shared memory, 16 bytes a thread
 #pragma unroll 2
-    for (int i = threadIdx.x; i < G::ROWS * HD / 8; i += 256) {
+    for (int i = threadIdx.x; i < G::ROWS * HD / 8; i += kAWarps * 32) {
         const int r = i / (HD / 8), v = i % (HD / 8);
         uint4 q = make_uint4(0, 0, 0, 0);
         if (r < rows) {
@@ -719,9 +717,11 @@ __global__ void __launch_bounds__(256) attention_kernel(const __grid_constant__ 
             const uint32_t sk = sbase + st * G::BLOCK, sv = sk + (HD / 64) * 8192;
             // scores of this warp's keys
             const int k0 = part * KT * 8;
-            float s[KT][4];
+            float s[KT][4], s1[KT][4];                                   // (even and odd steps apart: chains of half the length)
 #pragma unroll
-            for (int nt = 0; nt < KT; nt++) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
+            for (int nt = 0; nt < KT; nt++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) s[nt][e] = s1[nt][e] = 0.f;
 #pragma unroll 2
             for (int ks = 0; ks < HD / 16; ks += 2) {
                 uint32_t qa[4], qb[4];
@@ -732,9 +732,13 @@ __global__ void __launch_bounds__(256) attention_kernel(const __grid_constant__ 
                     uint32_t kf[4];
                     ldsm4(kf, sk + kv_swz(k0 + nt * 8 + krow_l, ks * 2 + kvec_l));
                     mma_m16n8k16(s[nt], qa[0], qa[1], qa[2], qa[3], kf[0], kf[1]);
-                    mma_m16n8k16(s[nt], qb[0], qb[1], qb[2], qb[3], kf[2], kf[3]);
+                    mma_m16n8k16(s1[nt], qb[0], qb[1], qb[2], qb[3], kf[2], kf[3]);
                 }
             }
+#pragma unroll
+            for (int nt = 0; nt < KT; nt++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) s[nt][e] += s1[nt][e];
             float mx0 = -INFINITY, mx1 = -INFINITY;
             const int j0 = b * kKeyBlock + k0 + 2 * t - prefix;          // tail row of the thread's first key
             const bool open = b * kKeyBlock + kKeyBlock <= prefix;       // committed rows only
@@ -838,7 +842,7 @@ __global__ void __launch_bounds__(256) attention_kernel(const __grid_constant__ 
     // ---- merge: one warp per row, CTAs in key order
     const int row_lo = (int)rank * nslot, mine_rows = min(nslot, rows - row_lo);
 #pragma unroll 1
-    for (int j = warp; j < mine_rows; j += 8) {
+    for (int j = warp; j < mine_rows; j += kAWarps) {
         constexpr int C = HD / 32;
         const float2* ml = reinterpret_cast<const float2*>(smem + G::INBOX_ML) + j;
         const float2 mine = lane < (int)cs * PT ? ml[lane * nslot] : make_float2(-INFINITY, 0.f);     // lane: (source, part); at most 32
@@ -937,20 +941,18 @@ int launch_dense(DenseParams& p, int split, cudaStream_t stream) {
     return rc != B200_OK ? rc : launch(tiles - rest, rest, rest_cs);
 }
 
-template <int HD, int PT>
-int launch_attention_pt(DAttn& a, int nreq, cudaStream_t stream) {
-    using G = DAGeo<HD, PT>;
-    static std::atomic<uint64_t> done{0};
-    if (!allow_smem(attention_kernel<HD, PT>, G::SMEM, done, true)) return check_launch();
-    a.sets = (a.mr * (a.Hq / a.Hkv) + G::ROWS - 1) / G::ROWS;
-    const int cs = std::min(a.nkb, kMaxCluster);
-    return launch_chain(attention_kernel<HD, PT>, dim3(cs, a.Hkv * a.sets, nreq), 256, G::SMEM, cs, stream, a);
-}
-// Sets of 32 query rows while that makes one wave (a cluster of 8 CTAs to one or two per GPC), of 64 beyond: fewer reads of K and V.
+// Clusters of as many key ranges as still run at once, two CTAs to an SM (33 clusters of 8 fit, 71 of 4; at one CTA to an SM, with
+// 64 query rows in a CTA, 15 of 8: the sixteenth ran alone and doubled the time).
 template <int HD>
 int launch_attention(DAttn& a, int nreq, cudaStream_t stream) {
-    const int qr = a.mr * (a.Hq / a.Hkv);
-    return qr <= 32 || a.Hkv * nreq * ((qr + 31) / 32) <= 16 ? launch_attention_pt<HD, 4>(a, nreq, stream) : launch_attention_pt<HD, 2>(a, nreq, stream);
+    using G = DAGeo<HD>;
+    static std::atomic<uint64_t> done{0};
+    if (!allow_smem(attention_kernel<HD>, G::SMEM, done, true)) return check_launch();
+    a.sets = (a.mr * (a.Hq / a.Hkv) + G::ROWS - 1) / G::ROWS;
+    const int clusters = a.Hkv * a.sets * nreq;
+    int cs = std::min(a.nkb, kMaxCluster);
+    while (cs > 1 && clusters > 8 * (32 / cs)) cs--;
+    return launch_chain(attention_kernel<HD>, dim3(cs, a.Hkv * a.sets, nreq), kAWarps * 32, G::SMEM, cs, stream, a);
 }
 
 template <int NT>

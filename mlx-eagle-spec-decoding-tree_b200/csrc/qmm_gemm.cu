@@ -290,7 +290,7 @@ template <int S, int NT, bool DUAL, int LAYOUT>
 __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_constant__ GParams p) {
     using G = GGeo<S, NT, LAYOUT>;
     extern __shared__ unsigned char smem_raw[];
-    unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    unsigned char* ring = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);
     __shared__ uint64_t s_bars[2 * 8 + 2 * kGroups + 4];
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort, s_last;
