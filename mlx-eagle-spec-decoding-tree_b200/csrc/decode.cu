@@ -41,22 +41,26 @@ constexpr int kEpi = 8;                          // of which these run the epilo
 constexpr int kDThreads = (kDeq + 4) * 32;       // + weight producer, activation producer, MMA issuer, sums of squares
 constexpr int kTCols = kChunkK / 2;              // tensor-memory columns of an expanded tile
 constexpr int kTmem = 256;                       // columns a CTA takes: two CTAs share an SM
-constexpr int kRedPitch = kTile + 4;             // floats per token row of the partial products in shared memory
 constexpr int kMaxCluster = 8;
 constexpr int kSsqPitch = 32, kCsPitch = 64, kKeyBlock = 64;
 constexpr uint32_t kDWaitPolls = 1u << 19;       // about a microsecond each
 
 enum { D_QKV = 0, D_RESID = 1, D_SILU = 2, D_HEAD = 3 };
 
-template <int NT>
+template <int TQ>
+struct __align__(TQ * 4) Vec { float v[TQ]; };      // a value per token of a group
+
+template <int NT, int TQ = 4>
 struct DGeo {
     static constexpr int X = NT * kChunkK * 2;                  // activations of a chunk: two boxes of 64 k
     static constexpr int ACC = kGroups * kTCols;                  // accumulator columns: two of NT
     static constexpr int NW = 2 * kGroups;                       // weight stages (a multiple: a stage belongs to one of the groups)
-    static constexpr int NX = NT == 16 ? 6 : 4;                  // activation stages
+    static constexpr int NX = NT == 16 ? 6 : 3;                  // activation stages
     static constexpr int XOFF = NW * kW;
-    static constexpr int INBOX = XOFF + NX * X;                  // partial products [source rank][token of this CTA][kRedPitch] fp32
-    static constexpr int SMEM = INBOX + (NT + kMaxCluster) * kRedPitch * 4 + 1024;
+    // Partial products [source rank][group of TQ tokens of this CTA][row][TQ] fp32.  The groups go to the CTAs in turn, so at most 8
+    // (of four tokens, up to 16), 14 (up to 32: 8 over 7 CTAs) or 8 (of two, up to 8) of them with their sources are here.
+    static constexpr int INBOX = XOFF + NX * X;
+    static constexpr int SMEM = INBOX + (NT == 16 ? 8 : 14) * kTile * TQ * 4 + 1024;
     static_assert(XOFF % 1024 == 0 && 2 * (SMEM + 3072) <= 227 * 1024 && ACC + 2 * NT <= kTmem, "two CTAs per SM");
 };
 
@@ -88,13 +92,22 @@ struct DenseParams {
 
 // Bounded; once a wait of the CTA has given up (`abort`) the others do so at their next poll, and the kernel runs to its end on
 // whatever is there, in bounds, with the error word set.  No caller leaves its loop for it: the loops stay warp-uniform, so the
-// operands of copies and MMAs stay in uniform registers (eight MMAs and two commits: 290 cycles instead of 560).
+// operands of copies and MMAs stay in uniform registers (eight MMAs and two commits: 290 cycles instead of 560).  Not unrolled:
+// a kernel of the chain mostly runs code for the first time, and every line of it costs.
+// After a wait that gave up: the CTA stays until the copies in flight have landed.
+__device__ __forceinline__ void settle() {
+#pragma unroll 1
+    for (int i = 0; i < 1000; i++) __nanosleep(1000);
+}
+template <bool SETTLE = false>
 __device__ __forceinline__ void dwait(uint32_t bar, uint32_t parity, volatile int* abort, int* err, int code) {
     bool ok = mbar_try_wait(bar, parity);
+#pragma unroll 1
     for (uint32_t i = 0; !ok && i < kDWaitPolls && !*abort; i++) ok = mbar_try_wait(bar, parity);
     if (!ok && !*abort) {
         *abort = 1;
         atomicCAS(err, 0, code);
+        if (SETTLE) settle();
     }
 }
 
@@ -128,14 +141,22 @@ __device__ __forceinline__ uint32_t peer_addr(uint32_t addr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
-__device__ __forceinline__ void st_async(uint32_t addr, uint32_t v, uint32_t bar) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];\n" ::"r"(addr), "r"(v), "r"(bar) : "memory");
+template <int TQ>
+__device__ __forceinline__ void st_async(uint32_t addr, const uint32_t* a, uint32_t bar) {
+    if (TQ == 4)
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];\n" ::"r"(addr), "r"(a[0]), "r"(a[1]),
+                     "r"(a[TQ - 2]), "r"(a[TQ - 1]), "r"(bar) : "memory");
+    else
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];\n" ::"r"(addr), "r"(a[0]), "r"(a[1]), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void arrive_peer(uint32_t bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ bool inbox_wait(uint32_t bar) {      // phase 0, with what the peers stored before they arrived
-    for (uint32_t i = 0; i < kDWaitPolls; i++) {
+// Phase 0, with what the peers stored before they arrived.  The limit is several times that of the other waits: a peer whose own
+// wait runs out still stores here, and must not find this CTA gone.
+__device__ __forceinline__ bool inbox_wait(uint32_t bar) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < 4 * kDWaitPolls; i++) {
         uint32_t ok;
         asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n selp.u32 %0, 1, 0, p;\n}\n"
                      : "=r"(ok) : "r"(bar) : "memory");
@@ -156,16 +177,17 @@ __device__ __forceinline__ void st_peer2(uint32_t addr, float x, float y) {
 // follows in order.  Three chunks are expanded before the wait for the previous kernel: behind it
 // come the activation load (0.5 us), the MMAs (0.1 us a chunk) and the epilogue.  Code that runs once per kernel is kept short:
 // cold instructions cost 2 to 4 cycles each.
-template <int NT, int KIND>
+template <int NT, int KIND, int TQ>
 __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_constant__ DenseParams p) {
-    using G = DGeo<NT>;
+    using G = DGeo<NT, TQ>;
+    using V = Vec<TQ>;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* ring = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);
-    float* inbox = reinterpret_cast<float*>(ring + G::INBOX);
+    V* inbox = reinterpret_cast<V*>(ring + G::INBOX);
     __shared__ uint64_t wfull[G::NW], wempty[G::NW], xfull[G::NX], xempty[G::NX], tready[kGroups], tfree[kGroups], accfull[2], accempty[2], inboxfull;
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
-    __shared__ float s_rs[32];                                   // 1 / rms per token
+    __shared__ __align__(16) float s_rs[32];                                   // 1 / rms per token
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank(), cs = cluster_size();
@@ -173,7 +195,8 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
     const int nit = cs > 1 ? 1 : (p.tiles - tile0 + tstep - 1) / tstep;                                   // this CTA's tiles: tile0, + tstep, ...
     const int nchunks = p.K / kChunkK;
     const int c_lo = nchunks * (int)rank / (int)cs, nc = nchunks * ((int)rank + 1) / (int)cs - c_lo;      // chunks of each
-    const int ntok = p.M > (int)rank ? (p.M - (int)rank + (int)cs - 1) / (int)cs : 0;                     // and tokens: rank, rank + cs, ...
+    const int quads = (p.M + TQ - 1) / TQ, qslots = (quads + (int)cs - 1) / (int)cs;                      // groups of tokens, most of a CTA's
+    const int nq = quads > (int)rank ? (quads - (int)rank + (int)cs - 1) / (int)cs : 0;                   // this CTA finishes rank, rank + cs, ...
 
     if (threadIdx.x < 32) {                                      // (a thread a barrier: one thread for all took 400 cycles)
         if (lane < G::NX) {
@@ -191,7 +214,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         if (lane == 31) {
             s_abort = 0;
             mbar_init(smem_u32(&inboxfull), 1);
-            if (cs > 1) mbar_expect_tx(smem_u32(&inboxfull), cs * ntok * kTile * 4); // what the cluster's CTAs will store here
+            if (cs > 1) mbar_expect_tx(smem_u32(&inboxfull), cs * nq * kTile * TQ * 4); // what the cluster's CTAs will store here
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -310,6 +333,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         asm volatile("bar.sync 2, %0;\n" ::"n"((kEpi + 1) * 32) : "memory");         // accumulators read
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(kTmem) : "memory");
+        if (*abort_flag) settle();                                      // (this warp has nothing else to do while the last epilogue runs)
     } else if (warp == kDeq + 3) {
         // ------------------------------------------------------------------ sums of squares -> 1 / rms of each token
         // (by the dequant warps it held up every chunk behind the first three: 1.4 us at a hidden size of 3584)
@@ -353,20 +377,25 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
             const int tile = tile0 + it * tstep;
             const uint32_t ab = it & 1;
             const int r2 = KIND == D_SILU ? threadIdx.x & 63 : threadIdx.x & 127;     // row inside the tile that this thread finishes
-            const int j0 = KIND == D_SILU ? threadIdx.x >> 6 : threadIdx.x >> 7;      // its first token of this CTA's, and the step
+            const int j0 = KIND == D_SILU ? threadIdx.x >> 6 : threadIdx.x >> 7;      // its first quad of this CTA's, and the step
             constexpr int JS = KIND == D_SILU ? 4 : 2;
             const int n = (KIND == D_SILU ? tile * 64 : tile * kTile) + r2;
             const bool valid = n < p.N;
-            // what the output needs besides the product, asked for now: norm weight or bias, the first token's residual or rotation
+            // what the output needs besides the product, asked for now: norm weight or bias, the first quad's residuals or rotations
             const int half = p.hd >> 1, hi = r2 & (p.hd - 1), head = KIND == D_QKV ? n >> (p.hd == 128 ? 7 : 6) : 0;
             const bool rotate = KIND == D_QKV && head < p.Hq + p.Hkv, first = hi < half;
             const int pr = rotate ? (first ? r2 + half : r2 - half) : r2;      // the row it is rotated with, inside this tile
             __half extra = __ushort_as_half(0), extra2 = __ushort_as_half(0);
-            auto ask_h = [&](int j) -> unsigned short {
-                return KIND == D_RESID && valid && j < ntok ? __ldcg(reinterpret_cast<const unsigned short*>(p.h) + (size_t)((int)rank + j * (int)cs) * p.N + n) : 0;
-            };
-            auto ask_r = [&](int j) -> float2 {
-                return KIND == D_QKV && rotate && j < ntok ? __ldcg(p.cs + ((int)rank + j * (int)cs) * kCsPitch + (first ? hi : hi - half)) : make_float2(0.f, 0.f);
+            unsigned short hres[TQ];
+            float2 rot[TQ];
+            auto ask = [&](int j) {                              // (warp-uniform j and token counts)
+                const int tok0 = TQ * ((int)rank + j * (int)cs);
+#pragma unroll
+                for (int k = 0; k < TQ; k++) {
+                    if (KIND == D_RESID && valid && tok0 + k < p.M)
+                        hres[k] = __ldcg(reinterpret_cast<const unsigned short*>(p.h) + (size_t)(tok0 + k) * p.N + n);
+                    if (KIND == D_QKV && rotate && tok0 + k < p.M) rot[k] = __ldcg(p.cs + (tok0 + k) * kCsPitch + (first ? hi : hi - half));
+                }
             };
             if (it == 0) pdl_wait();
             if (KIND == D_RESID && valid) extra = p.wn[n];
@@ -374,8 +403,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                 extra = p.bias[n];
                 extra2 = p.bias[tile * kTile + pr];
             }
-            unsigned short h0 = ask_h(j0), h1 = ask_h(j0 + JS);
-            float2 t0 = ask_r(j0), t1 = ask_r(j0 + JS);
+            if (j0 < nq) ask(j0);
 
             dwait(smem_u32(accfull + ab), (it >> 1) & 1, abort_flag, p.err, 23);
             __syncwarp();
@@ -392,82 +420,106 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
             if (it == nit - 1) asm volatile("bar.arrive 2, %0;\n" ::"n"((kEpi + 1) * 32) : "memory");     // tensor memory may be given back
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(accempty + ab));
-            const int nslot = (p.M + (int)cs - 1) / (int)cs;     // tokens per source in an inbox
             if (cs == 1) {
                 if (it > 0) consumer_sync(kEpi * 32);            // the tile before this one has been read
 #pragma unroll
-                for (int i = 0; i < C; i++)
-                    if ((int)me * C + i < p.M) inbox[((int)me * C + i) * kRedPitch + r] = __uint_as_float(a[i]);
+                for (int i = 0; i < C; i += TQ)
+                    if ((int)me * C + i < p.M) {
+                        V x;
+#pragma unroll
+                        for (int k = 0; k < TQ; k++) x.v[k] = __uint_as_float(a[i + k]);
+                        inbox[((int)me * C + i) / TQ * kTile + r] = x;
+                    }
                 consumer_sync(kEpi * 32);
             } else {
-                // a store into a peer's memory counts its bytes at the peer's barrier by itself: no fence, no arrival behind it
+                // A store into a peer's memory counts its bytes at the peer's barrier by itself: no fence, no arrival behind it.  TQ
+                // tokens a store: with one, the stores were what a pass of many tokens waited for (1.1 us for four more tokens).
                 cluster_wait();
                 const uint32_t in0 = smem_u32(inbox), inbar = smem_u32(&inboxfull);
-                uint32_t dst = (me * C) % cs, sl = (me * C) / cs;
+                uint32_t dst = (me * (C / TQ)) % cs, sl = (me * (C / TQ)) / cs;
 #pragma unroll
-                for (int i = 0; i < C; i++) {
+                for (int i = 0; i < C; i += TQ) {
                     if ((int)me * C + i < p.M)
-                        st_async(peer_addr(in0 + ((rank * nslot + sl) * kRedPitch + r) * 4, dst), a[i], peer_addr(inbar, dst));
+                        st_async<TQ>(peer_addr(in0 + ((rank * qslots + sl) * kTile + r) * (TQ * 4), dst), a + i, peer_addr(inbar, dst));
                     if (++dst == cs) { dst = 0; sl++; }
                 }
                 if (!inbox_wait(inbar)) atomicCAS(p.err, 0, 28);     // (in full after a timeout too: a peer may still be storing here)
                 __syncwarp();
             }
             if (NORMED && it == 0) asm volatile("bar.sync 3, %0;\n" ::"n"((kEpi + 1) * 32) : "memory");      // s_rs
-            auto total = [&](int j, int row) {                   // the sources in rank order
-                const float* v = inbox + j * kRedPitch + row;
-                float t = v[0];
 #pragma unroll 1
-                for (int i = 1; i < (int)cs; i++) t += v[i * nslot * kRedPitch];
-                return t;
-            };
+            for (int j = j0; j < nq; j += JS) {                  // (warp-uniform)
+                const int tok0 = TQ * ((int)rank + j * (int)cs);
+                if (j != j0) ask(j);
+                // the sources in rank order: this row, and the up row or the one it is rotated with
+                const int r3 = KIND == D_SILU ? r2 + 64 : pr;
+                V v = inbox[j * kTile + r2], w = v;
+                if (KIND == D_SILU || KIND == D_QKV) w = inbox[j * kTile + r3];
 #pragma unroll 1
-            for (int j = j0; j < ntok; j += JS) {                // (warp-uniform)
-                const int tok = (int)rank + j * (int)cs;
-                const float rs = NORMED ? s_rs[tok] : 1.f;
-                const float v = total(j, r2) * rs;
-                const int rq = KIND == D_HEAD || KIND == D_QKV ? (p.mr == p.M ? 0 : tok / p.mr) : 0;
-                if (KIND == D_SILU) {
-                    const float up = total(j, r2 + 64) * rs;
-                    if (valid) p.y[(size_t)tok * p.N + n] = __float2half_rn(silu_mul_f16(v, up));
-                } else if (KIND == D_RESID) {
-                    float ss = 0.f;
-                    if (valid) {
-                        const size_t at = (size_t)tok * p.N + n;
-                        const __half o = __hadd(__ushort_as_half(h0), __float2half_rn(v));
-                        const float f = __half2float(o);
-                        ss = f * f;
-                        p.h[at] = o;
-                        p.hw[at] = __hmul(o, extra);
-                    }
+                for (int i = 1; i < (int)cs; i++) {
+                    const V* src = inbox + (i * qslots + j) * kTile;
+                    const V x = src[r2];
 #pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-                    if (lane == 0 && valid) p.ssq[(n >> 5) * kSsqPitch + tok] = ss;
-                    h0 = h1;
-                    h1 = ask_h(j + 2 * JS);
-                } else if (KIND == D_HEAD) {
-                    const int rel = tok - rq * p.mr - (p.row_index ? p.row_index[rq] : 0);
-                    if (valid && rel >= 0 && rel < p.rows_out) p.y[(size_t)(rq * p.rows_out + rel) * p.N + n] = __float2half_rn(v);
-                } else {
-                    __half x = __float2half_rn(v);
-                    if (p.bias != nullptr) x = __hadd(x, extra);
-                    if (rotate) {
-                        __half y = __float2half_rn(total(j, pr) * rs);
-                        if (p.bias != nullptr) y = __hadd(y, extra2);
-                        const float xs = __half2float(x), ys = __half2float(y);
-                        x = __float2half_rn(first ? xs * t0.x - ys * t0.y : ys * t0.y + xs * t0.x);
+                    for (int k = 0; k < TQ; k++) v.v[k] += x.v[k];
+                    if (KIND == D_SILU || KIND == D_QKV) {
+                        const V y = src[r3];
+#pragma unroll
+                        for (int k = 0; k < TQ; k++) w.v[k] += y.v[k];
                     }
-                    if (valid) {
-                        if (head < p.Hq) {
-                            p.y[(size_t)tok * p.N + n] = x;
-                        } else {
-                            const int row = p.prefix[rq] + p.write_off + (tok - rq * p.mr);
-                            const int kvh = head - p.Hq - (rotate ? 0 : p.Hkv);
-                            if (row < p.cap) ((rotate ? p.kc : p.vc) + (size_t)rq * p.req_stride)[((size_t)kvh * p.cap + row) * p.hd + hi] = x;
+                }
+                if (NORMED) {
+                    const V rs = *reinterpret_cast<const V*>(s_rs + tok0);
+#pragma unroll
+                    for (int k = 0; k < TQ; k++) { v.v[k] *= rs.v[k]; w.v[k] *= rs.v[k]; }
+                }
+                float ss[TQ] = {};
+#pragma unroll
+                for (int k = 0; k < TQ; k++) {
+                    const int tok = tok0 + k;
+                    if (tok >= p.M) break;
+                    const int rq = KIND == D_HEAD || KIND == D_QKV ? (p.mr == p.M ? 0 : tok / p.mr) : 0;
+                    if (KIND == D_SILU) {
+                        if (valid) p.y[(size_t)tok * p.N + n] = __float2half_rn(silu_mul_f16(v.v[k], w.v[k]));
+                    } else if (KIND == D_RESID) {
+                        if (valid) {
+                            const size_t at = (size_t)tok * p.N + n;
+                            const __half o = __hadd(__ushort_as_half(hres[k]), __float2half_rn(v.v[k]));
+                            const float f = __half2float(o);
+                            ss[k] = f * f;
+                            p.h[at] = o;
+                            p.hw[at] = __hmul(o, extra);
+                        }
+                    } else if (KIND == D_HEAD) {
+                        const int rel = tok - rq * p.mr - (p.row_index ? p.row_index[rq] : 0);
+                        if (valid && rel >= 0 && rel < p.rows_out) p.y[(size_t)(rq * p.rows_out + rel) * p.N + n] = __float2half_rn(v.v[k]);
+                    } else {
+                        __half x = __float2half_rn(v.v[k]);
+                        if (p.bias != nullptr) x = __hadd(x, extra);
+                        if (rotate) {
+                            __half y = __float2half_rn(w.v[k]);
+                            if (p.bias != nullptr) y = __hadd(y, extra2);
+                            const float xs = __half2float(x), ys = __half2float(y);
+                            x = __float2half_rn(first ? xs * rot[k].x - ys * rot[k].y : ys * rot[k].y + xs * rot[k].x);
+                        }
+                        if (valid) {
+                            if (head < p.Hq) {
+                                p.y[(size_t)tok * p.N + n] = x;
+                            } else {
+                                const int row = p.prefix[rq] + p.write_off + (tok - rq * p.mr);
+                                const int kvh = head - p.Hq - (rotate ? 0 : p.Hkv);
+                                if (row < p.cap) ((rotate ? p.kc : p.vc) + (size_t)rq * p.req_stride)[((size_t)kvh * p.cap + row) * p.hd + hi] = x;
+                            }
                         }
                     }
-                    t0 = t1;
-                    t1 = ask_r(j + 2 * JS);
+                }
+                if (KIND == D_RESID) {
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                        for (int k = 0; k < TQ; k++) ss[k] += __shfl_xor_sync(0xffffffffu, ss[k], o);
+#pragma unroll
+                    for (int k = 0; k < TQ; k++)
+                        if (lane == k && valid && tok0 + k < p.M) p.ssq[(n >> 5) * kSsqPitch + tok0 + k] = ss[k];
                 }
             }
         };
@@ -711,7 +763,7 @@ __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_co
 #pragma unroll 1
     for (int b = b0; b < b1; b++) {
         const int st = (b - b0) % G::STAGES;
-        dwait(smem_u32(full + st), ((b - b0) / G::STAGES) & 1, &s_abort, p.err, 29);
+        dwait<true>(smem_u32(full + st), ((b - b0) / G::STAGES) & 1, &s_abort, p.err, 29);
         __syncwarp();
         if (busy) {
             const uint32_t sk = sbase + st * G::BLOCK, sv = sk + (HD / 64) * 8192;
@@ -904,34 +956,36 @@ int launch_chain(void (*kern)(P), dim3 grid, int threads, size_t smem, int clust
 }
 
 // Cluster size along K for `tiles` row tiles of `nch` chunks, by a cost in microseconds fitted on B200 to passes of four model
-// shapes.  Three chunks are expanded before the wait and then cost 0.15 each, a further one 0.5 (on one CTA of an SM as on each
-// of two); a cluster's reduction 0.5; a token to finish 0.1.  CTAs beyond one per SM take the room of the next kernel's, which
-// then starts up to 1.5 later.  Clusters beyond what fits at once into eight GPCs of at least 16 SMs, two CTAs each, run as a
-// second wave (36 clusters of 7 or 48 of 6 added 2 to 8 us a kernel): not taken.
-int plan_cluster(int tiles, int nch, int tokens) {
+// shapes with 1 to 32 tokens (the choices are on average 0.09 us a kernel behind the best).  A chunk costs 0.2, one behind the
+// three that are expanded before the wait 0.125 more; a source of the reduction 0.08 and 0.0105 a token; two groups of tokens to
+// finish 0.24; CTAs beyond one per SM take the room of the next kernel's, which then starts later.  Clusters beyond what fits at
+// once into eight GPCs of at least 16 SMs, two CTAs each, run as a second wave (36 clusters of 7 or 48 of 6 added 2 to 8 us a
+// kernel): not taken.
+int plan_cluster(int tiles, int nch, int tokens, int group) {
     int best = 1;
     double best_cost = 1e30;
+    const int groups = (tokens + group - 1) / group;
     for (int cs = 1; cs <= kMaxCluster && cs <= nch && (cs == 1 || tiles <= 8 * (32 / cs)); cs++) {
         const int ctas = tiles * cs, n = ((nch + cs - 1) / cs) * ((ctas + 295) / 296);
-        const double cost = n * 0.15 + std::max(0, n - 3) * 0.35 + (cs > 1 ? 0.5 + 0.03 * cs : 0.0) + 0.1 * ((tokens + cs - 1) / cs) +
-                            (ctas > 148 ? std::min(ctas - 148, 148) * 0.01 : 0.0);
+        const double cost = n * 0.2 + std::max(0, n - 3) * 0.125 + (cs > 1 ? 0.5 + (0.08 + 0.0105 * tokens) * cs : 0.0) +
+                            0.24 * (((groups + cs - 1) / cs + 1) / 2) + (ctas > 148 ? std::min(ctas - 148, 148) * 0.018 : 0.0);
         if (cost < best_cost - 1e-9) { best_cost = cost; best = cs; }
     }
     return best;
 }
 
-template <int NT, int KIND>
+template <int NT, int TQ, int KIND>
 int launch_dense(DenseParams& p, int split, cudaStream_t stream) {
     static std::atomic<uint64_t> done{0};
-    if (!allow_smem(dense_kernel<NT, KIND>, DGeo<NT>::SMEM, done, true)) return check_launch();
+    if (!allow_smem(dense_kernel<NT, KIND, TQ>, DGeo<NT, TQ>::SMEM, done, true)) return check_launch();
     const int nch = p.K / kChunkK;
     const int tiles = KIND == D_SILU ? p.N / 64 : (p.N + kTile - 1) / kTile;
-    const int cs = split > 0 && split <= std::min(kMaxCluster, nch) ? split : plan_cluster(tiles, nch, p.M);
+    const int cs = split > 0 && split <= std::min(kMaxCluster, nch) ? split : plan_cluster(tiles, nch, p.M, TQ);
     constexpr int cap = 296;
     auto launch = [&](int lo, int n, int cluster) {
         p.tile_lo = lo;
         p.tiles = lo + n;
-        return launch_chain(dense_kernel<NT, KIND>, dim3(cluster > 1 ? n * cluster : std::min(n, cap)), kDThreads, DGeo<NT>::SMEM, cluster, stream, p);
+        return launch_chain(dense_kernel<NT, KIND, TQ>, dim3(cluster > 1 ? n * cluster : std::min(n, cap)), kDThreads, DGeo<NT, TQ>::SMEM, cluster, stream, p);
     };
     // Whole waves of tiles, then what is left over as a launch of its own with K split over clusters: alone it would take as long
     // as a whole wave.
@@ -955,7 +1009,7 @@ int launch_attention(DAttn& a, int nreq, cudaStream_t stream) {
     return launch_chain(attention_kernel<HD>, dim3(cs, a.Hkv * a.sets, nreq), kAWarps * 32, G::SMEM, cs, stream, a);
 }
 
-template <int NT>
+template <int NT, int TQ>
 int run_chain(const ChainArgs& c, cudaStream_t st) {
     const b200_forward_desc* d = c.d;
     const int M = d->M, H = d->hidden, I = d->intermediate, hd = d->head_dim, nreq = d->requests > 1 ? d->requests : 1;
@@ -1002,7 +1056,7 @@ int run_chain(const ChainArgs& c, cudaStream_t st) {
             p.N = nqkv; p.K = H;
             p.kc = static_cast<__half*>(d->kv_cache) + (size_t)l * 2 * half_stride;
             p.vc = p.kc + half_stride;
-            if ((rc = launch_dense<NT, D_QKV>(p, c.splits[0], st)) != B200_OK) return rc;
+            if ((rc = launch_dense<NT, TQ, D_QKV>(p, c.splits[0], st)) != B200_OK) return rc;
         }
         if (on(2)) {
             a.row0 = l * 2 * d->n_kv_heads * d->cache_rows;
@@ -1011,27 +1065,27 @@ int run_chain(const ChainArgs& c, cudaStream_t st) {
         p.bias = nullptr;
         if (on(4)) {
             p.xmap = attn_map; p.w[0] = w(2); p.wn = static_cast<const __half*>(L[7]); p.N = H; p.K = nq;
-            if ((rc = launch_dense<NT, D_RESID>(p, c.splits[1], st)) != B200_OK) return rc;
+            if ((rc = launch_dense<NT, TQ, D_RESID>(p, c.splits[1], st)) != B200_OK) return rc;
         }
         if (on(5)) {
             p.xmap = hw_map; p.w[0] = w(3); p.w[1] = w(4); p.y = static_cast<__half*>(d->act); p.N = I; p.K = H;
-            if ((rc = launch_dense<NT, D_SILU>(p, c.splits[2], st)) != B200_OK) return rc;
+            if ((rc = launch_dense<NT, TQ, D_SILU>(p, c.splits[2], st)) != B200_OK) return rc;
         }
         if (on(6)) {
             p.xmap = act_map; p.w[0] = w(5); p.wn = static_cast<const __half*>(l + 1 < d->n_layers ? L[8 + 6] : d->final_norm); p.N = H; p.K = I;
-            if ((rc = launch_dense<NT, D_RESID>(p, c.splits[3], st)) != B200_OK) return rc;
+            if ((rc = launch_dense<NT, TQ, D_RESID>(p, c.splits[3], st)) != B200_OK) return rc;
         }
     }
     if (on(7)) {
         p.xmap = hw_map; p.w[0] = static_cast<const unsigned char*>(d->lm_head_tiled); p.y = static_cast<__half*>(d->logits);
         p.N = d->head_rows > 0 ? d->head_rows : d->vocab; p.K = H;
-        if ((rc = launch_dense<NT, D_HEAD>(p, c.splits[4], st)) != B200_OK) return rc;
+        if ((rc = launch_dense<NT, TQ, D_HEAD>(p, c.splits[4], st)) != B200_OK) return rc;
     }
     return B200_OK;
 }
 
 }  // namespace
 
-int forward_chain(const ChainArgs& a, cudaStream_t stream) { return a.d->M <= 16 ? run_chain<16>(a, stream) : run_chain<32>(a, stream); }
+int forward_chain(const ChainArgs& a, cudaStream_t stream) { return a.d->M <= 8 ? run_chain<16, 2>(a, stream) : (a.d->M <= 16 ? run_chain<16, 4>(a, stream) : run_chain<32, 4>(a, stream)); }
 
 }  // namespace b200
