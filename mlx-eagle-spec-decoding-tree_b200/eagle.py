@@ -272,9 +272,9 @@ class SpecDecoder:
         """Greedy tree-speculative generation for one prompt (host or device tensor of token ids).
 
         Runs at most ``N`` steps and stops at the first step boundary where ``max_tokens`` were generated
-        (``mlx_eagle.py:544-546``).  Steps are enqueued ahead of the host: the stop test reads a pinned
-        copy of the device counters that trails the device by two steps, so the device never waits for
-        the host; steps launched past the stop point are discarded from the result.
+        (``mlx_eagle.py:544-546``).  Steps are enqueued up to two ahead of the host, which reads a pinned
+        copy of the device counters, as long as the ones in flight cannot reach ``max_tokens``; steps launched
+        past an end token are discarded from the result.
 
         Two stop rules the reference lacks: with ``eos_token_id`` the request ends at the first generated
         token equal to it (found on the device by ``b200_tree_accept``; the token itself is kept, everything
@@ -299,18 +299,20 @@ class SpecDecoder:
             self._pinned = [torch.zeros(16, dtype=torch.int32).pin_memory() for _ in range(4)]
             self._events = [torch.cuda.Event() for _ in range(4)]
         pinned, events = self._pinned, self._events
-        i = 0
-        first_is_eos = eos_token_id is not None and first == int(eos_token_id)
-        while i < N and not first_is_eos:
+        i = seen = known = 0                              # steps launched, steps whose counters were read, tokens after those
+        stop = eos_token_id is not None and first == int(eos_token_id)
+        while i < N and not stop:
             self.replay()
             pinned[i % 4].copy_(self.ctl, non_blocking=True)
             events[i % 4].record()
             i += 1
-            j = i - 1 - lead
-            if j >= 0:
-                events[j % 4].synchronize()
-                if int(pinned[j % 4][CTL_NGEN]) >= max_tokens or int(pinned[j % 4][CTL_DONE]):
-                    break
+            # (a step gives at most depth + 2 tokens: none is launched that the ones in flight may make superfluous, which
+            # leaves the device idle for the ~50 us of a launch instead of busy with steps that are thrown away)
+            while not stop and (i - seen > lead or (seen < i and known + (i - seen) * (self.depth + 2) >= max_tokens)):
+                events[seen % 4].synchronize()
+                known = int(pinned[seen % 4][CTL_NGEN])
+                stop = known >= max_tokens or int(pinned[seen % 4][CTL_DONE]) != 0
+                seen += 1
         torch.cuda.synchronize(self.device)
         total = time.perf_counter() - tic
         self.base.check_fused_error()
@@ -477,18 +479,19 @@ class BatchSpecDecoder:
             self._pinned = [torch.zeros(self.requests, 16, dtype=torch.int32).pin_memory() for _ in range(4)]
             self._events = [torch.cuda.Event() for _ in range(4)]
         pinned, events = self._pinned, self._events
-        i = 0
-        while i < N:
+        i = seen = known = 0                              # (as in SpecDecoder.generate; known: tokens of the slowest request)
+        stop = False
+        while i < N and not stop:
             self.replay()
             pinned[i % 4].copy_(self.ctl, non_blocking=True)
             events[i % 4].record()
             i += 1
-            j = i - 1 - lead
-            if j >= 0:
-                events[j % 4].synchronize()
-                c = pinned[j % 4]
-                if all(int(c[r][CTL_NGEN]) >= max_tokens or int(c[r][CTL_DONE]) for r in range(self.requests)):
-                    break
+            while not stop and (i - seen > lead or (seen < i and known + (i - seen) * (self.depth + 2) >= max_tokens)):
+                events[seen % 4].synchronize()
+                c = pinned[seen % 4].tolist()
+                open_ = [c[r][CTL_NGEN] for r in range(self.requests) if c[r][CTL_NGEN] < max_tokens and not c[r][CTL_DONE]]
+                known, stop = min(open_, default=max_tokens), not open_
+                seen += 1
         torch.cuda.synchronize(self.device)
         total = time.perf_counter() - tic
         self.base.check_fused_error()
