@@ -48,17 +48,16 @@ __device__ __forceinline__ unsigned long long make_key(float v, uint32_t idx) {
 __device__ __forceinline__ uint32_t key_index(unsigned long long k) { return 0xffffffffu - (uint32_t)(k & 0xffffffffu); }
 __device__ __forceinline__ float key_value(unsigned long long k) { return unorder_bits((uint32_t)(k >> 32)); }
 
+// Two 32-bit reductions over the warp, values first, then the low words of those that share the maximum: five steps of 64-bit
+// shuffles took about four times as long, and selections here are chains of eight of them.
 __device__ __forceinline__ unsigned long long warp_max_key(unsigned long long k) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        unsigned long long other = __shfl_xor_sync(0xffffffffu, k, o);
-        k = other > k ? other : k;
-    }
-    return k;
+    const uint32_t hi = (uint32_t)(k >> 32), m = __reduce_max_sync(0xffffffffu, hi);
+    const uint32_t lo = __reduce_max_sync(0xffffffffu, hi == m ? (uint32_t)k : 0u);
+    return ((unsigned long long)m << 32) | lo;
 }
 
 // ---------------------------------------------------------------- deterministic exp / log
-__device__ __forceinline__ double exp_det(double d) {
+__device__ __forceinline__ double exp_det(double d, int shift = 0) {
     const double LOG2E = 1.4426950408889634;
     const double LN2_HI = 6.93147180369123816490e-01;
     const double LN2_LO = 1.90821492927058770002e-10;
@@ -71,10 +70,11 @@ __device__ __forceinline__ double exp_det(double d) {
     double p = c[13];
 #pragma unroll
     for (int i = 12; i >= 0; i--) p = __dadd_rn(__dmul_rn(p, r), c[i]);
-    const double out = scalbn(p, (int)kf);
+    // p * 2^(kf + shift): p is in [0.7, 1.5] and the exponent in [-58, 40], so the addition to its exponent field is exact
+    const double out = __longlong_as_double(__double_as_longlong(p) + ((long long)((int)kf + shift) << 52));
     return d < -40.0 ? 0.0 : out;
 }
-__device__ __forceinline__ long long exp_fixed(double d) { return __double2ll_rn(scalbn(exp_det(d), 40)); }
+__device__ __forceinline__ long long exp_fixed(double d) { return __double2ll_rn(exp_det(d, 40)); }
 
 __device__ __forceinline__ double log_det(unsigned long long total) {
     const double LN2_HI = 6.93147180369123816490e-01;
@@ -102,17 +102,39 @@ __device__ __forceinline__ float score_of(float logit, double lse) {
 }
 
 // ---------------------------------------------------------------- row kernels over logits [R, V]
+// fn(value) for the elements [begin, end) of a row, by a block: four a load where the rows are whole 8-byte vectors (begin is).
+template <typename Fn>
+__device__ __forceinline__ void for_row(const __half* __restrict__ row, int V, int begin, int end, Fn fn) {
+    if (((reinterpret_cast<uintptr_t>(row) & 7) | (V & 3)) == 0) {
+        for (int i = begin + threadIdx.x * 4; i < end; i += blockDim.x * 4) {
+            const uint2 u = *reinterpret_cast<const uint2*>(row + i);
+            fn(__half2float(__ushort_as_half((unsigned short)u.x)));
+            fn(__half2float(__ushort_as_half((unsigned short)(u.x >> 16))));
+            fn(__half2float(__ushort_as_half((unsigned short)u.y)));
+            fn(__half2float(__ushort_as_half((unsigned short)(u.y >> 16))));
+        }
+    } else {
+        for (int i = begin + threadIdx.x; i < end; i += blockDim.x) fn(__half2float(row[i]));
+    }
+}
+
+// (One atomic a block in both kernels: one a warp made them queue for the row's word.)
 __global__ void row_max_kernel(const __half* __restrict__ logits, int V, uint32_t* __restrict__ row_max) {
     pdl_wait();
     pdl_launch_dependents();
     const int r = blockIdx.y;
-    const int begin = blockIdx.x * kStatChunk, end = min(V, begin + kStatChunk);
+    __shared__ uint32_t part[8];
+    const int begin = blockIdx.x * kTopkChunk, end = min(V, begin + kTopkChunk);
     const __half* row = logits + (size_t)r * V;
     uint32_t best = 0;
-    for (int i = begin + threadIdx.x; i < end; i += blockDim.x) best = max(best, order_bits(__half2float(row[i])));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(row_max + r, best);
+    for_row(row, V, begin, end, [&](float v) { best = max(best, order_bits(v)); });
+    best = __reduce_max_sync(0xffffffffu, best);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = best;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        best = __reduce_max_sync(0xffffffffu, threadIdx.x < 8 ? part[threadIdx.x] : 0u);
+        if (threadIdx.x == 0) atomicMax(row_max + r, best);
+    }
 }
 
 // temp: temperature the logits are divided by before the exponential (1.0: the plain soft-max; dividing by 1.0 is exact,
@@ -126,25 +148,34 @@ __global__ void row_sumexp_kernel(const __half* __restrict__ logits, int V, cons
     const __half* row = logits + (size_t)r * V;
     const double mx = (double)unorder_bits(row_max[r]);
     unsigned long long acc = 0;
-    for (int i = begin + threadIdx.x; i < end; i += blockDim.x)
-        acc += (unsigned long long)exp_fixed(__ddiv_rn(__dsub_rn((double)__half2float(row[i]), mx), temp));
+    // Bound by fp64 arithmetic, ~35 operations an element: the division only where it does something.
+    if (temp == 1.0) for_row(row, V, begin, end, [&](float v) { acc += (unsigned long long)exp_fixed(__dsub_rn((double)v, mx)); });
+    else for_row(row, V, begin, end, [&](float v) { acc += (unsigned long long)exp_fixed(__ddiv_rn(__dsub_rn((double)v, mx), temp)); });
+    __shared__ unsigned long long part[8];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(row_sum + r, acc);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) acc += part[w];
+        atomicAdd(row_sum + r, acc);
+    }
 }
 
 // Local top-8 of one chunk of one row.  by_score == 0: order by the raw logit (root expansion,
 // mlx_eagle.py:411); by_score == 1: order by the fp32 log-probability (tree levels, :104-105).
-__global__ void __launch_bounds__(256) row_topk_kernel(const __half* __restrict__ logits, int V,
+constexpr int kTopkThreads = 256;
+__global__ void __launch_bounds__(kTopkThreads) row_topk_kernel(const __half* __restrict__ logits, int V,
                                                        const uint32_t* __restrict__ row_max,
                                                        const unsigned long long* __restrict__ row_sum,
                                                        int by_score, unsigned long long* __restrict__ cand) {
     pdl_wait();
     pdl_launch_dependents();
-    // Every thread keeps its 16 keys in registers; each warp selects the top 8 of its 512 keys with warp
-    // shuffles only, then one warp selects the top 8 of the 64 survivors: one block-wide barrier in all.
-    constexpr int PER = kTopkChunk / 256;
-    __shared__ unsigned long long wtop[8 * kK];
+    // Every thread keeps its 16 keys in registers; each warp selects the top 8 of its 512 keys with warp reductions only, then
+    // one warp selects the top 8 of the 64 survivors: one block-wide barrier in all.  Bound by the chains of eight dependent
+    // selections and, by score, the logarithm before them: 8 x 151936 takes 8.0 us, with 512 threads 10.3.
+    constexpr int PER = kTopkChunk / kTopkThreads, WARPS = kTopkThreads / 32;
+    __shared__ unsigned long long wtop[WARPS * kK];
     const int r = blockIdx.y;
     const int begin = blockIdx.x * kTopkChunk, end = min(V, begin + kTopkChunk);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -154,7 +185,7 @@ __global__ void __launch_bounds__(256) row_topk_kernel(const __half* __restrict_
     unsigned long long mine[PER];
 #pragma unroll
     for (int j = 0; j < PER; j++) {
-        const int i = begin + j * 256 + (int)threadIdx.x;
+        const int i = begin + j * kTopkThreads + (int)threadIdx.x;
         mine[j] = 0ull;                                        // past the end: never selected
         if (i < end) {
             const float l = __half2float(row[i]);
@@ -173,13 +204,16 @@ __global__ void __launch_bounds__(256) row_topk_kernel(const __half* __restrict_
     }
     __syncthreads();
     if (warp == 0) {
-        const unsigned long long k0 = wtop[lane], k1 = wtop[lane + 32];
+        unsigned long long k[WARPS * kK / 32];
+#pragma unroll
+        for (int j = 0; j < WARPS * kK / 32; j++) k[j] = wtop[j * 32 + lane];
         unsigned long long* out = cand + ((size_t)r * gridDim.x + blockIdx.x) * kK;
         bound = ~0ull;
         for (int round = 0; round < kK; round++) {
             unsigned long long best = 0;
-            if (k0 < bound && k0 > best) best = k0;
-            if (k1 < bound && k1 > best) best = k1;
+#pragma unroll
+            for (int j = 0; j < WARPS * kK / 32; j++)
+                if (k[j] < bound && k[j] > best) best = k[j];
             best = warp_max_key(best);
             if (lane == 0) out[round] = best;                  // 0 when the chunk has run out
             bound = best ? best : 0ull;
@@ -194,12 +228,28 @@ __global__ void row_argmax_kernel(const __half* __restrict__ logits, int V, unsi
     const int begin = blockIdx.x * kTopkChunk, end = min(V, begin + kTopkChunk);
     const __half* row = logits + (size_t)r * V;
     unsigned long long best = 0;
-    for (int i = begin + threadIdx.x; i < end; i += blockDim.x) {
-        const unsigned long long k = make_key(__half2float(row[i]), (uint32_t)i);
+    __shared__ unsigned long long part[8];
+    auto take = [&](unsigned short h, int i) {
+        const unsigned long long k = make_key(__half2float(__ushort_as_half(h)), (uint32_t)i);
         best = k > best ? k : best;
+    };
+    if (((reinterpret_cast<uintptr_t>(row) & 7) | (V & 3)) == 0) {
+#pragma unroll 4
+        for (int i = begin + threadIdx.x * 4; i < end; i += 1024) {
+            const uint2 u = *reinterpret_cast<const uint2*>(row + i);
+            take((unsigned short)u.x, i); take((unsigned short)(u.x >> 16), i + 1);
+            take((unsigned short)u.y, i + 2); take((unsigned short)(u.y >> 16), i + 3);
+        }
+    } else {
+        for (int i = begin + threadIdx.x; i < end; i += 256) take(__half_as_ushort(row[i]), i);
     }
     best = warp_max_key(best);
-    if ((threadIdx.x & 31) == 0) atomicMax(best_key + r, best);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = best;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        best = warp_max_key(threadIdx.x < 8 ? part[threadIdx.x] : 0ull);
+        if (threadIdx.x == 0) atomicMax(best_key + r, best);
+    }
 }
 
 __global__ void argmax_key_shift_kernel(unsigned long long* __restrict__ best_key, int R, unsigned int index_offset) {
@@ -789,7 +839,7 @@ int b200_logits_rowstats(const void* logits, int R, int V, uint32_t* row_max, un
     if (!logits || !row_max || !row_sum || R < 1 || R > 32 || V < 1) return B200_EINVAL;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     dim3 grid((V + b200::kStatChunk - 1) / b200::kStatChunk, R);
-    b200::launch_kernel(b200::row_max_kernel, dim3(grid), dim3(256), 0, st, static_cast<const __half*>(logits), V, row_max);
+    b200::launch_kernel(b200::row_max_kernel, dim3(b200::nblk_for(V), R), dim3(256), 0, st, static_cast<const __half*>(logits), V, row_max);
     b200::launch_kernel(b200::row_sumexp_kernel, dim3(grid), dim3(256), 0, st, static_cast<const __half*>(logits), V, row_max, row_sum, 1.0);
     return b200::check_launch();
 }
@@ -799,7 +849,7 @@ int b200_logits_rowstats_temp(const void* logits, int R, int V, uint32_t* row_ma
     if (!logits || !row_max || !row_sum || R < 1 || R > 32 || V < 1 || !(temperature > 0.0)) return B200_EINVAL;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     dim3 grid((V + b200::kStatChunk - 1) / b200::kStatChunk, R);
-    b200::launch_kernel(b200::row_max_kernel, dim3(grid), dim3(256), 0, st, static_cast<const __half*>(logits), V, row_max);
+    b200::launch_kernel(b200::row_max_kernel, dim3(b200::nblk_for(V), R), dim3(256), 0, st, static_cast<const __half*>(logits), V, row_max);
     b200::launch_kernel(b200::row_sumexp_kernel, dim3(grid), dim3(256), 0, st, static_cast<const __half*>(logits), V, row_max, row_sum,
                         temperature);
     return b200::check_launch();
@@ -811,7 +861,7 @@ int b200_logits_topk_candidates(const void* logits, int R, int V, const uint32_t
                                 unsigned long long* cand, void* stream) {
     if (!logits || !row_max || !row_sum || !cand || R < 1 || R > 32 || V < 1) return B200_EINVAL;
     dim3 grid(b200::nblk_for(V), R);
-    b200::launch_kernel(b200::row_topk_kernel, dim3(grid), dim3(256), 0, static_cast<cudaStream_t>(stream), static_cast<const __half*>(logits), V, row_max, row_sum, by_score, cand);
+    b200::launch_kernel(b200::row_topk_kernel, dim3(grid), dim3(b200::kTopkThreads), 0, static_cast<cudaStream_t>(stream), static_cast<const __half*>(logits), V, row_max, row_sum, by_score, cand);
     return b200::check_launch();
 }
 
