@@ -10,8 +10,8 @@ finalisation, one target pass on 16 tokens, acceptance, KV compaction).  Metric:
 state until at least two seconds have been timed; the median block gives ``value``, the spread is reported.
 
 The JSON line also carries: the end-to-end number through ``SpecDecoder.generate`` with a pinned host prompt
-(``e2e``), the roofline of the target pass (``roofline``: the persistent forward kernel at 16 rows) and of the
-draft pass (``roofline_draft``: the same kernel on the draft at 8 rows), the quantised-matmul operator sweep of
+(``e2e``), the roofline of the target pass (``roofline``: the kernel chain at 16 rows) and of the
+draft pass (``roofline_draft``: the same chain on the draft at 8 rows), the quantised-matmul operator sweep of
 the metric's second half (``qmm_sweep``: 8192 x 2048 at 1..32 rows, GB/s against the HBM peak), a lock-step
 parity check of the very models that are timed (``config.parity_checked``) and a CPU baseline (the CPU
 restatement of the reference's path on a bounded sample on this host's cores).  At N > 1 the ranks afterwards
@@ -153,8 +153,7 @@ def forward_algorithmic_bytes(model, rows, kv_rows):
 
 
 def forward_roofline(torch, model, cache, rows, prefix, reps):
-    """Time one forward pass alone (one launch of the persistent kernel = one pass of `rows` tokens over a
-    `prefix`-row cache) as a CUDA graph, with CUDA events on the launching stream."""
+    """Time one forward pass alone (`rows` tokens over a `prefix`-row cache) as a CUDA graph, with CUDA events on the launching stream."""
     f = model.fwd
     g = torch.Generator().manual_seed(99)
     f.tokens[:rows].copy_(torch.randint(0, model.args.vocab_size, (rows,), generator=g, dtype=torch.int32))
@@ -711,9 +710,8 @@ def batched_requests_numbers(torch, be, base, draft, depth, verify, prompt_len, 
     torch.cuda.synchronize()
     e2e_sec = time.perf_counter() - t0
     e2e_tokens = sum(r["produced"] for r in res)
-    mt = (R * (verify + 1) + 7) // 8
     target = roofline_block(torch, base, dec.slots[0].base_cache, min(32, R * (verify + 1)), prompt_len,
-                            f"forward_kernel<{mt},{base.args.head_dim}> at the rows of {R} requests (one cache: timing only)", reps=10)
+                            f"pass of {base.kernels_per_forward} kernels at the rows of {R} requests (one cache: timing only)", reps=10)
     out = {"requests_per_gpu": R, "tokens_per_second": produced / sec, "ms_per_step": 1e3 * sec / Kb, "steps": Kb,
            "blocks": len(secs), "tokens_per_step": produced / Kb,
            "e2e_tokens_per_second": e2e_tokens / e2e_sec,
@@ -813,7 +811,7 @@ def main():
                          max_steps=warmup + K + 64)
     if tname is None:
         dec.step = dec.draft_tree_step                     # the step (and its graph) is the tree build alone
-        dec.kernel_launches_per_step = (DEPTH + 1) * (draft.launches_per_forward + 4) + 2
+        dec.kernel_launches_per_step = (DEPTH + 1) * (draft.kernels_per_forward + 4) + 2
     dec.warmup(capture=True)
     g = torch.Generator().manual_seed(1234 + rank)
     vocab = min(draft.args.vocab_size, base.args.vocab_size)
@@ -905,11 +903,10 @@ def main():
             "gpu_launches": dec.kernel_launches_per_step * K * len(secs),
         }
         if tname is not None:
-            mt = (VERIFY + 1 + 7) // 8
             line["roofline"] = roofline_block(torch, base, dec.base_cache, VERIFY + 1, prefix_now,
-                                              f"forward_kernel<{mt},{base.args.head_dim}> (target pass)")
+                                              f"target pass of {base.kernels_per_forward} kernels")
         dblk = roofline_block(torch, draft, dec.draft_cache, 8, prefix_now,
-                              f"draft pass of {draft.launches_per_forward} launch(es), {dname} shape")
+                              f"draft pass of {draft.kernels_per_forward} kernels, {dname} shape")
         if tname is None:
             line["roofline"] = dblk
         else:

@@ -217,7 +217,8 @@ int b200_tree_attention(const void* q, int q_stride, const void* kcache, const v
                         void* workspace, size_t workspace_bytes, void* stream);
 
 /* ------------------------------------------------------------------------------------------
- * Whole forward pass as one persistent cooperative kernel.
+ * Whole forward pass: on one GPU a chain of five kernels per layer, for a tensor-parallel shard one persistent
+ * cooperative kernel.
  * Replaces one call of Model.__call__ (mlx_llama.py:298-313: embed_tokens, every TransformerBlock
  * :231-249 with Attention :121-196 and MLP :199-215, the final norm and lm_head / as_linear) for
  * M <= 32 tokens whose ids, rotary positions, tail masks and committed length are in device memory
@@ -229,8 +230,8 @@ int b200_tree_attention(const void* q, int q_stride, const void* kcache, const v
  *   { qkv weights (q|k|v rows concatenated), qkv bias [NQKV] fp16 or NULL, o_proj, gate_proj, up_proj,
  *     down_proj weights, input_layernorm weight [hidden] fp16, post_attention_layernorm weight }.
  * Buffers (all fp16): h [32][hidden]; qkv [32][(n_heads+2*n_kv_heads)*head_dim]; logits [rows_out][vocab];
- * hw, attn, act are scratch the kernel keeps in its own chunk-major padded layout and need
- * (width/128)*32*160 halves each, width = hidden, n_heads*head_dim, intermediate.  kv_cache is
+ * hw, attn, act are scratch in a layout of the kernels' own and need 32*width halves each, width = hidden,
+ * n_heads*head_dim, intermediate.  kv_cache is
  * [n_layers][2][n_kv_heads][cache_rows][head_dim] fp16; the K/V rows of the M new tokens are written
  * to cache row prefix[0]+write_off+m.  Output row r of logits belongs to token row_index[0]+r
  * (row_index may be NULL = 0).  RMSNorm is folded into the adjacent matmuls (h*w is rounded to fp16,
@@ -240,7 +241,7 @@ int b200_tree_attention(const void* q, int q_stride, const void* kcache, const v
  * workspace: b200_forward_workspace_bytes bytes, the first 4352 bytes zero before the first use (the
  * kernel restores that state).  Int word 2 of the workspace is an error flag: non-zero after a launch
  * means a bounded wait inside the kernel gave up; zero the first 4352 bytes before reusing it.
- * The launch is cooperative (one CTA per SM, all co-resident); launches sharing a workspace must be
+ * A shard's launch is cooperative (one CTA per SM, all co-resident).  Launches sharing a workspace must be
  * stream-ordered.  hidden, intermediate and n_heads*head_dim must be multiples of 128, hidden <= 8192,
  * head_dim 64 or 128, tail <= 64, write_off + M <= tail.
  * ------------------------------------------------------------------------------------------ */
@@ -249,7 +250,7 @@ typedef struct b200_forward_desc {
     int hidden, intermediate, n_heads, n_kv_heads, head_dim, vocab, n_layers;
     int cache_rows, write_off, tail;
     float rms_eps, rope_scaling, attn_scale;
-    int attn_split_blocks;  /* 0 = default (33): from this many 64-key blocks of cache on, attention splits the  */
+    int attn_split_blocks;  /* shards only.  0 = default (33): from this many 64-key blocks of cache on, attention splits the  */
                             /* keys across CTAs and merges in a second phase; below, one CTA per (kv head,      */
                             /* query tile) scores the key blocks on its warps side by side.  < 0 = always split  */
     const int* tokens;
@@ -273,7 +274,7 @@ typedef struct b200_forward_desc {
     void* kv_cache;
     void* workspace;
     size_t workspace_bytes;
-    void* timeline;         /* optional profiling hook, NULL = off: int64 [SMs][timeline_pitch][8]; CTA b  */
+    void* timeline;         /* shards only: optional profiling hook, NULL = off: int64 [SMs][timeline_pitch][8]; CTA b  */
     int timeline_pitch;     /* stores the nanosecond timer when it arrives at / leaves device barrier i   */
     int phase_mask;         /* (i = 0 after the embedding, then 6 per layer) and, arrive only, at its end */
                             /* phase_mask: profiling only, 0 = run everything; else bit k set = run phase  */
@@ -298,7 +299,7 @@ typedef struct b200_forward_desc {
      * be zeroed (with no launch in flight anywhere) before the next pass. */
     int tp_world, tp_rank;
     int head_rows;
-    int grid_ctas;          /* CTAs of the persistent kernel: 0 = one per SM.  A small model (a draft whose layer is
+    int grid_ctas;          /* shards only: CTAs of the persistent kernel, 0 = one per SM.  A small model (a draft whose layer is
                              * a few MB) is bound by the latency of its device-wide phase boundaries, not by
                              * bandwidth: fewer CTAs make every boundary cheaper and 16 to 64 SMs already pull 2 to
                              * 6.5 TB/s.  Size the workspace with the same value. */

@@ -1,10 +1,9 @@
-// One forward pass of the 4-bit decoder (<= 32 tokens) as ONE persistent cooperative kernel, sm_100a.
+// One forward pass of a tensor-parallel shard of the 4-bit decoder (<= 32 tokens) as ONE persistent cooperative kernel, sm_100a;
+// without tensor parallelism b200_forward runs the kernel chain of decode.cu.
 //
-// The per-op kernels of this library (rms_norm, qmm, rope_kv_append, tree_attention, ...) cost one
-// launch each: nine per decoder layer, ~250 per pass, and at <= 32 tokens every one of them is shorter
-// than its own launch/drain latency.  Here the whole pass of mlx_llama.py:298-313 (embedding ->
-// layers -> final norm -> vocabulary projection) is one kernel: one CTA per SM, eight consumer
-// warps plus one producer warp, and a device-wide barrier between the phases of a layer.
+// The whole pass of mlx_llama.py:298-313 (embedding -> layers -> final norm -> vocabulary projection) is one kernel, so that the
+// exchanges between the GPUs happen inside it: one CTA per SM, eight consumer warps plus one producer warp, and a device-wide
+// barrier between the phases of a layer.
 //
 //   phase 0   quantised embedding gather, h and h*w_norm, per-tile sums of squares, RoPE cos/sin table
 //   per layer A   q|k|v = rstd * ((h*w) . Wqkv^T) + bias            (RMSNorm folded, see below)
@@ -72,7 +71,7 @@ constexpr int kCsPitch = 64;                  // cos/sin table: cs[token][i], i 
 constexpr int kSyncExit = 1, kSyncErr = 2, kSyncBar = 8;   // exit count, error code, then kBarLanes arrival counters
 constexpr int kBarLanes = 8;
 
-enum { EPI_QKV = 0, EPI_SILU = 1, EPI_RESID = 2, EPI_HEAD = 3, EPI_TP = 4 };
+enum { EPI_QKV = 0, EPI_SILU = 1, EPI_HEAD = 3, EPI_TP = 4 };
 enum { K_EMBED = 0, K_A = 1, K_B1 = 2, K_B2 = 3, K_C = 4, K_D = 5, K_E = 6, K_HEAD = 7, K_R = 8 };
 constexpr uint32_t kTpWaitLimit = 1u << 22;   // polls of a peer's flag (a microsecond or so each) before giving up
 enum { PLAN_A = 0, PLAN_C = 1, PLAN_D = 2, PLAN_E = 3, PLAN_HEAD = 4 };
@@ -112,12 +111,6 @@ struct FwdParams {
     __half* kv;                    // [layers][2][Hkv][cap][HD]
     size_t kv_layer_stride, kv_half_stride;   // in halves
     int cap, write_off, tail;
-    // Several requests in one pass (nreq > 1): the M rows are nreq groups of mr rows; request r has its own
-    // committed length prefix[r], head-row offset row_index[r] and KV slab (kv + r * kv_req_stride); attention never
-    // crosses requests, every other phase just sees M rows.
-    int nreq, mr;
-    size_t kv_req_stride;          // in halves
-    int kv_req_rows;               // rows of the 2-D view of one request's slab (layers * 2 * Hkv * cap)
     int* sync;
     int* counter;
     float* ssq;
@@ -161,28 +154,18 @@ struct QDesc {
     const unsigned char* w0;
     const unsigned char* w1;    // up_proj in dual mode
     const __half* bias;
-    const __half* wn;           // norm weights applied to the new h (EPI_RESID)
+    const __half* wn;           // norm weights applied to the new h (by the exchange)
     __half* y;
     int N, K;
     PhasePlan pl;
     int xrows;                  // token rows of the pass
     int row_lo, row_cnt;        // token rows [row_lo, row_lo+row_cnt) are stored, as output rows 0.. (vocabulary projection)
-    int orow_sel;               // several requests per pass: which table of out_row_tab() maps token rows to output rows
                                 //   (1: the vocabulary projection keeps rows_out rows per request; 0: all rows kept)
     bool y_tiled;               // output goes to the chunk-major padded layout (it is a later phase's matmul input)
 };
 
 // Small per-launch tables in static shared memory, reached through functions so that no pointer to them has to
 // stay in a register across the matmul loops (the kernel sits at its register limit).
-__device__ __forceinline__ int* req_prefix_tab() {       // committed length of every request of the pass
-    __shared__ int s_prefix[kMaxReq];
-    return s_prefix;
-}
-__device__ __forceinline__ int* out_row_tab() {          // [2][32] output row of a token row, or -1 = not stored:
-    __shared__ int s_orow[2 * 32];                       //   [0] every row kept, [1] the vocabulary projection's selection
-    return s_orow;
-}
-
 struct Ctx {
     unsigned char* ring;
     uint64_t* full;
@@ -751,13 +734,11 @@ __device__ __forceinline__ void qmm_produce(const FwdParams& p, Ctx& c, const QD
 }
 
 // Output row of token row `tok` in a row-major result, or -1 if the row is not stored.
-template <bool BATCH>
 __device__ __forceinline__ int out_row(const QDesc& d, int tok) {
-    if (BATCH) return out_row_tab()[d.orow_sel * 32 + tok];
     return (tok >= d.row_lo && tok < d.row_lo + d.row_cnt) ? tok - d.row_lo : -1;
 }
 
-template <int MT, bool DUAL, bool TP, bool FAST, bool BATCH>
+template <int MT, bool DUAL, bool TP, bool FAST>
 __device__ __forceinline__ void qmm_consume(const FwdParams& p, Ctx& c, const QDesc& d, const int EPI) {
     using G = Geo<MT>;
     constexpr int S = DUAL ? 2 : 1;
@@ -777,7 +758,7 @@ __device__ __forceinline__ void qmm_consume(const FwdParams& p, Ctx& c, const QD
     const int rec_cstride = (TPI >= 4) ? 4 * kRec : chunk_bytes;
     const int nchunks_total = d.K / kChunkK;
     const int nitems = d.pl.row_items * d.pl.splits;
-    const bool need_rstd = (EPI != EPI_RESID && !(TP && EPI == EPI_TP));
+    const bool need_rstd = !(TP && EPI == EPI_TP);
     constexpr bool fast = FAST;                   // every scale of the model is in the range of dequant_pack_fast
     stamp(p, c, 2);
     bool rstd_done = !need_rstd;
@@ -930,13 +911,6 @@ __device__ __forceinline__ void qmm_consume(const FwdParams& p, Ctx& c, const QD
                     float a0[8], a1[8];
 #pragma unroll
                     for (int e = 0; e < 8; e++) a0[e] = a1[e] = 0.f;
-                    // residual and norm weights of the epilogue: issued now, so that their latency runs with the
-                    // partial sums' (h is read and written by this thread only)
-                    uint4 rv = make_uint4(0, 0, 0, 0), wv = make_uint4(0, 0, 0, 0);
-                    if (valid && EPI == EPI_RESID && !(TP && EPI == EPI_TP)) {
-                        rv = __ldcg(reinterpret_cast<const uint4*>(p.h + (size_t)tok * d.N + n0));
-                        wv = *reinterpret_cast<const uint4*>(d.wn + n0);
-                    }
                     if (valid) {
                         // four splits' loads in flight at a time (a load from L2 takes the better part of a
                         // microsecond); added in split order, so the result does not depend on the batching
@@ -983,24 +957,6 @@ __device__ __forceinline__ void qmm_consume(const FwdParams& p, Ctx& c, const QD
                             *reinterpret_cast<float4*>(dst) = make_float4(a0[0], a0[1], a0[2], a0[3]);
                             *reinterpret_cast<float4*>(dst + 4) = make_float4(a0[4], a0[5], a0[6], a0[7]);
                         }
-                    } else if (EPI == EPI_RESID) {
-                        float ss = 0.f;
-                        if (valid) {
-                            const __half* rh = reinterpret_cast<const __half*>(&rv);
-                            const __half* wh = reinterpret_cast<const __half*>(&wv);
-                            __align__(16) __half hw[8];
-#pragma unroll
-                            for (int e = 0; e < 8; e++) {
-                                out[e] = __hadd(rh[e], __float2half_rn(a0[e]));
-                                const float f = __half2float(out[e]);
-                                ss += f * f;
-                                hw[e] = __hmul(out[e], wh[e]);
-                            }
-                            *reinterpret_cast<uint4*>(p.h + (size_t)tok * d.N + n0) = *reinterpret_cast<const uint4*>(out);
-                            *reinterpret_cast<uint4*>(p.hw + xt_index(tok, n0, MP)) = *reinterpret_cast<const uint4*>(hw);
-                        }
-                        ss += __shfl_xor_sync(0xffffffffu, ss, 1);          // the two 8-column halves of a 16-row tile
-                        if (valid && (lane & 1) == 0) p.ssq[(n0 >> 4) * kSsqPitch + tok] = ss;
                     } else if (valid) {
                         const float rs = c.s_rstd[tok];
                         if (DUAL) {
@@ -1019,7 +975,7 @@ __device__ __forceinline__ void qmm_consume(const FwdParams& p, Ctx& c, const QD
                         if (d.y_tiled) {
                             *reinterpret_cast<uint4*>(d.y + xt_index(tok, n0, MP)) = *reinterpret_cast<const uint4*>(out);
                         } else {
-                            const int orow = out_row<BATCH>(d, tok);
+                            const int orow = out_row(d, tok);
                             if (orow >= 0) *reinterpret_cast<uint4*>(d.y + (size_t)orow * d.N + n0) = *reinterpret_cast<const uint4*>(out);
                         }
                     }
@@ -1044,47 +1000,6 @@ __device__ __forceinline__ void qmm_consume(const FwdParams& p, Ctx& c, const QD
                         }
                     }
                 }
-            } else if (EPI == EPI_RESID) {
-                // residuals and norm weights first, all loads in flight together (h is read and written here)
-                unsigned short res[MT][4];
-#pragma unroll
-                for (int mt = 0; mt < MT; mt++)
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const int tok = mt * 8 + 2 * t + (i & 1);
-                        const int nn = nbase + ((i >> 1) ? 8 : 0);
-                        res[mt][i] = (tok < d.xrows && nn < d.N)
-                                         ? __ldcg(reinterpret_cast<const unsigned short*>(p.h) + (size_t)tok * d.N + nn) : (unsigned short)0;
-                    }
-                const __half wn0 = nbase < d.N ? d.wn[nbase] : __ushort_as_half(0);
-                const __half wn8 = nbase + 8 < d.N ? d.wn[nbase + 8] : __ushort_as_half(0);
-#pragma unroll
-                for (int mt = 0; mt < MT; mt++) {
-                    float ss0 = 0.f, ss1 = 0.f;            // tokens 2t, 2t+1 of this token tile
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const int tok = mt * 8 + 2 * t + (i & 1);
-                        const int nn = nbase + ((i >> 1) ? 8 : 0);
-                        if (tok < d.xrows && nn < d.N) {
-                            const __half r = __ushort_as_half(res[mt][i]);
-                            const __half o = __hadd(r, __float2half_rn(acc[0][mt][i]));
-                            const float f = __half2float(o);
-                            if (i & 1) ss1 += f * f; else ss0 += f * f;
-                            p.h[(size_t)tok * d.N + nn] = o;
-                            p.hw[xt_index(tok, nn, MP)] = __hmul(o, (i >> 1) ? wn8 : wn0);
-                        }
-                    }
-#pragma unroll
-                    for (int o = 4; o < 32; o <<= 1) {
-                        ss0 += __shfl_xor_sync(0xffffffffu, ss0, o);
-                        ss1 += __shfl_xor_sync(0xffffffffu, ss1, o);
-                    }
-                    if (g == 0 && tile_global * 16 < d.N) {
-                        const int tok = mt * 8 + 2 * t;
-                        if (tok < d.xrows) p.ssq[tile_global * kSsqPitch + tok] = ss0;
-                        if (tok + 1 < d.xrows) p.ssq[tile_global * kSsqPitch + tok + 1] = ss1;
-                    }
-                }
             } else {
 #pragma unroll
                 for (int mt = 0; mt < MT; mt++) {
@@ -1104,7 +1019,7 @@ __device__ __forceinline__ void qmm_consume(const FwdParams& p, Ctx& c, const QD
                         if (d.y_tiled) {
                             d.y[xt_index(tok, nn, MP)] = o;
                         } else {
-                            const int orow = out_row<BATCH>(d, tok);
+                            const int orow = out_row(d, tok);
                             if (orow >= 0) d.y[(size_t)orow * d.N + nn] = o;
                         }
                     }
@@ -1461,23 +1376,21 @@ struct AGeo {
     static_assert(16 * OP * 4 + 16 * 8 <= SLOT, "a warp's partial state must fit its slot");
 };
 
-// BATCH: the pass holds several requests (compiled separately, so that the one-request kernel is unchanged by it).
-template <int MT, int HD, bool BATCH>
+template <int MT, int HD>
 __device__ __forceinline__ void attn_bp_produce(const FwdParams& p, Ctx& c, const ADesc& a, int layer) {
     using A = AGeo<MT, HD>;
     const int lane = c.lane;
     const int Gq = p.Hq / p.Hkv;
-    const int nreq = BATCH ? p.nreq : 1, mr = BATCH ? p.mr : p.M;
+    const int mr = p.M;
     const int ntiles = (mr * Gq + 15) / 16;
-    const int nitems = nreq * p.Hkv * ntiles;             // item = (request, kv head, query tile)
+    const int nitems = p.Hkv * ntiles;                    // item = (kv head, query tile)
     if ((int)blockIdx.x >= nitems) return;
     if (*c.abort_flag || !drain_stages<MT>(p, c)) return;
     for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
-        const int req = BATCH ? item / (p.Hkv * ntiles) : 0;
-        const int hk = BATCH ? (item / ntiles) % p.Hkv : item / ntiles;
-        const int nact = BATCH ? min((req_prefix_tab()[req] + p.tail + kKeyBlock - 1) / kKeyBlock, p.nkb) : a.nact;
-        const int krow0 = req * p.kv_req_rows + ((layer * 2 + 0) * p.Hkv + hk) * p.cap;   // row of the cache viewed as [rows][HD]
-        const int vrow0 = req * p.kv_req_rows + ((layer * 2 + 1) * p.Hkv + hk) * p.cap;
+        const int hk = item / ntiles;
+        const int nact = a.nact;
+        const int krow0 = ((layer * 2 + 0) * p.Hkv + hk) * p.cap;   // row of the cache viewed as [rows][HD]
+        const int vrow0 = ((layer * 2 + 1) * p.Hkv + hk) * p.cap;
         for (int kb = 0; kb < nact; kb++, c.apos++) {
             const uint32_t slot = c.apos % A::NS, use = c.apos / A::NS;
             if (*c.abort_flag) return;
@@ -1500,7 +1413,7 @@ __device__ __forceinline__ void attn_bp_produce(const FwdParams& p, Ctx& c, cons
     }
 }
 
-template <int MT, int HD, bool BATCH>
+template <int MT, int HD>
 __device__ __forceinline__ void attn_bp_consume(const FwdParams& p, Ctx& c, const ADesc& a) {
     using A = AGeo<MT, HD>;
     constexpr int NS = A::NS, NBX = A::NBX, OP = A::OP;
@@ -1510,25 +1423,22 @@ __device__ __forceinline__ void attn_bp_consume(const FwdParams& p, Ctx& c, cons
     const int lane = c.lane, warp = c.warp;
     const int g = lane >> 2, t = lane & 3;
     const int Gq = p.Hq / p.Hkv;
-    const int nreq = BATCH ? p.nreq : 1, mr = BATCH ? p.mr : p.M;
+    const int mr = p.M;
     const int QR = mr * Gq;                        // query rows (token, head of the group) of one request and kv head
     const int ntiles = (QR + 15) / 16;
-    const int nitems = nreq * p.Hkv * ntiles;
+    const int nitems = p.Hkv * ntiles;
     __half* sq = reinterpret_cast<__half*>(c.scratch);
     __half* nkv = sq + 16 * KS;                    // [2][M][HD]: rotated k rows, then v rows, of this pass
     static_assert(16 * KS * 2 + 2 * 32 * HD * 2 <= kScratch, "query tile and new K/V rows must fit the scratch area");
     unsigned char* myslot = c.ring + (warp < NS ? warp : 0) * A::SLOT;
 
     for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
-        const int req = BATCH ? item / (p.Hkv * ntiles) : 0;
-        const int hk = BATCH ? (item / ntiles) % p.Hkv : item / ntiles;
-        const int rt = item - (req * p.Hkv + hk) * ntiles;
-        const int prefix = BATCH ? req_prefix_tab()[req] : a.prefix;
-        const int nact = BATCH ? min((prefix + p.tail + kKeyBlock - 1) / kKeyBlock, p.nkb) : a.nact;
+        const int hk = item / ntiles;
+        const int rt = item - hk * ntiles;
+        const int prefix = a.prefix, nact = a.nact;
         const int new0 = prefix + p.write_off;
-        const int mbase = req * mr;                        // first token row of the request
-        __half* const kc = a.kc + (size_t)req * p.kv_req_stride;
-        __half* const vc = a.vc + (size_t)req * p.kv_req_stride;
+        __half* const kc = a.kc;
+        __half* const vc = a.vc;
         const uint32_t n0 = c.apos;                        // first block of this item in the phase's block sequence
         c.apos += nact;
         stamp(p, c, 2);
@@ -1541,7 +1451,7 @@ __device__ __forceinline__ void attn_bp_consume(const FwdParams& p, Ctx& c, cons
                 uint4 o1 = make_uint4(0, 0, 0, 0), o2 = make_uint4(0, 0, 0, 0);
                 if (r < QR) {
                     const int ml = r / Gq, hh = hk * Gq + (r - ml * Gq);
-                    const int m = mbase + ml;
+                    const int m = ml;
                     const __half* q = p.qkv + (size_t)m * p.NQKV + (size_t)hh * HD + cv * 8;
                     const uint4 x1v = __ldcg(reinterpret_cast<const uint4*>(q));
                     const uint4 x2v = __ldcg(reinterpret_cast<const uint4*>(q + HD / 2));
@@ -1573,7 +1483,7 @@ __device__ __forceinline__ void attn_bp_consume(const FwdParams& p, Ctx& c, cons
             for (int idx = threadIdx.x; idx < mr * VPR; idx += kNCons) {
                 const int m = idx / VPR, cv = idx - m * VPR;          // m: row inside the request
                 const int key = new0 + m;
-                const __half* src = p.qkv + (size_t)(mbase + m) * p.NQKV;
+                const __half* src = p.qkv + (size_t)(m) * p.NQKV;
                 const uint4 vv = __ldcg(reinterpret_cast<const uint4*>(src + (size_t)(p.Hq + p.Hkv) * HD + (size_t)hk * HD + cv * 8));
                 *reinterpret_cast<uint4*>(nkv + (mr + m) * HD + cv * 8) = vv;
                 if (writer && key < p.cap) *reinterpret_cast<uint4*>(vc + ((size_t)hk * p.cap + key) * HD + cv * 8) = vv;
@@ -1581,7 +1491,7 @@ __device__ __forceinline__ void attn_bp_consume(const FwdParams& p, Ctx& c, cons
                     const __half* ksrc = src + (size_t)p.Hq * HD + (size_t)hk * HD;
                     const uint4 x1v = __ldcg(reinterpret_cast<const uint4*>(ksrc + cv * 8));
                     const uint4 x2v = __ldcg(reinterpret_cast<const uint4*>(ksrc + HD / 2 + cv * 8));
-                    const float4* csp = reinterpret_cast<const float4*>(p.cs + (mbase + m) * kCsPitch + cv * 8);
+                    const float4* csp = reinterpret_cast<const float4*>(p.cs + (m) * kCsPitch + cv * 8);
                     float4 cs4[4];
 #pragma unroll
                     for (int e = 0; e < 4; e++) cs4[e] = __ldcg(csp + e);
@@ -1612,7 +1522,7 @@ __device__ __forceinline__ void attn_bp_consume(const FwdParams& p, Ctx& c, cons
 
         const int r0 = rt * 16 + g, r1 = r0 + 8;
         const bool v0 = r0 < QR, v1 = r1 < QR;
-        const int m0 = mbase + (v0 ? r0 / Gq : 0), m1 = mbase + (v1 ? r1 / Gq : 0);
+        const int m0 = (v0 ? r0 / Gq : 0), m1 = (v1 ? r1 / Gq : 0);
         const unsigned long long mk0 = v0 ? p.mask[m0] : 0ull, mk1 = v1 ? p.mask[m1] : 0ull;
 
         float mrun0 = -INFINITY, mrun1 = -INFINITY, l0 = 0.f, l1 = 0.f;
@@ -1798,7 +1708,7 @@ __device__ __forceinline__ void attn_bp_consume(const FwdParams& p, Ctx& c, cons
                 }
                 const float inv = denom > 0.f ? 1.f / denom : 0.f;
                 const int ml = r / Gq, hh = hk * Gq + (r - ml * Gq);
-                const int m = mbase + ml;
+                const int m = ml;
                 __align__(16) __half out[CPT];
 #pragma unroll
                 for (int e = 0; e < CPT; e++) out[e] = __float2half_rn(acc[e] * inv);
@@ -1858,7 +1768,7 @@ __device__ __forceinline__ void attn_merge(const FwdParams& p, Ctx& c, const ADe
 }
 
 // ================================================================================ the kernel
-template <int MT, int HD, bool TP, bool BATCH>
+template <int MT, int HD>
 __global__ void __launch_bounds__(kFwdThreads, 1) forward_kernel(const __grid_constant__ FwdParams p) {
     using G = Geo<MT>;
     extern __shared__ __align__(1024) unsigned char smem[];      // swizzled TMA boxes want 1024-byte aligned stages
@@ -1894,19 +1804,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1) forward_kernel(const __grid_co
     c.epoch = 0;
     c.lbar = 0;
     c.tpx = 0;
-    c.tp_seq0 = TP ? *reinterpret_cast<const volatile unsigned*>(p.tp_peers[p.tp_rank] + kTpFwdCount) : 0u;
+    c.tp_seq0 = *reinterpret_cast<const volatile unsigned*>(p.tp_peers[p.tp_rank] + kTpFwdCount);
     c.lane = threadIdx.x & 31;
     c.warp = threadIdx.x >> 5;
 
-    if (BATCH && (int)threadIdx.x < p.nreq) req_prefix_tab()[threadIdx.x] = p.prefix[threadIdx.x];
-    if (BATCH && threadIdx.x < 32) {
-        // the head keeps rows [row_index[q], +rows_out) of request q (of mr rows) as output rows q * rows_out ..
-        const int mr = BATCH ? p.mr : p.M;
-        const int tok = threadIdx.x, q = BATCH ? tok / mr : 0;
-        const int rel = tok - q * mr - ((p.row_index && tok < p.M) ? p.row_index[q] : 0);
-        out_row_tab()[tok] = tok < p.M ? tok : -1;
-        out_row_tab()[32 + tok] = (tok < p.M && rel >= 0 && rel < p.rows_out) ? q * p.rows_out + rel : -1;
-    }
     if (threadIdx.x == 0) {
         s_abort = 0;
         s_epoch = 0;
@@ -1955,8 +1856,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) forward_kernel(const __grid_co
             ad.kc = p.kv + (size_t)l * p.kv_layer_stride;
             ad.vc = ad.kc + p.kv_half_stride;
             if (attn_fused) {
-                if (producer) attn_bp_produce<MT, HD, BATCH>(p, c, ad, l);
-                else attn_bp_consume<MT, HD, BATCH>(p, c, ad);
+                if (producer) attn_bp_produce<MT, HD>(p, c, ad, l);
+                else attn_bp_consume<MT, HD>(p, c, ad);
             } else {
                 if (producer) attn_produce<MT, HD>(p, c, ad);
                 else attn_consume<MT, HD>(p, c, ad);
@@ -1969,10 +1870,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) forward_kernel(const __grid_co
             QDesc d;
             d.xrows = p.M;
             d.row_lo = 0; d.row_cnt = p.M;
-            d.orow_sel = 0;
             d.y_tiled = false;
             d.w1 = nullptr; d.bias = nullptr; d.wn = nullptr;
-            int epi = TP ? EPI_TP : EPI_RESID;
+            int epi = EPI_TP;
             if (kind == K_A) {
                 d.x = p.hw; d.w0 = lp.qkv_w; d.bias = lp.qkv_bias; d.y = p.qkv;
                 d.N = p.NQKV; d.K = p.H; d.pl = p.plan[PLAN_A]; epi = EPI_QKV;
@@ -1988,22 +1888,21 @@ __global__ void __launch_bounds__(kFwdThreads, 1) forward_kernel(const __grid_co
                 d.N = p.H; d.K = p.I; d.pl = p.plan[PLAN_E];
             } else {                                   // K_HEAD, on the selected rows
                 d.row_lo = row_off; d.row_cnt = p.rows_out;       // all rows are multiplied, the selected ones stored
-                d.orow_sel = 1;
                 d.x = p.hw; d.w0 = p.head_w; d.y = p.logits;
                 d.N = p.head_rows; d.K = p.H; d.pl = p.plan[PLAN_HEAD]; epi = EPI_HEAD;
             }
             tp_wn = d.wn;
             if (producer) {
-                qmm_produce<MT>(p, c, d, c.lbar, kind == K_D, epi != EPI_RESID && epi != EPI_TP);
+                qmm_produce<MT>(p, c, d, c.lbar, kind == K_D, epi != EPI_TP);
             } else if (p.fast_scales) {          // uniform: chosen once per launch by the host
-                if (kind == K_D) qmm_consume<MT, true, false, true, BATCH>(p, c, d, EPI_SILU);
-                else qmm_consume<MT, false, TP, true, BATCH>(p, c, d, epi);
+                if (kind == K_D) qmm_consume<MT, true, false, true>(p, c, d, EPI_SILU);
+                else qmm_consume<MT, false, true, true>(p, c, d, epi);
             } else {
-                if (kind == K_D) qmm_consume<MT, true, false, false, BATCH>(p, c, d, EPI_SILU);
-                else qmm_consume<MT, false, TP, false, BATCH>(p, c, d, epi);
+                if (kind == K_D) qmm_consume<MT, true, false, false>(p, c, d, EPI_SILU);
+                else qmm_consume<MT, false, true, false>(p, c, d, epi);
             }
         }
-        const bool exchange = TP && (kind == K_C || kind == K_E);
+        const bool exchange = kind == K_C || kind == K_E;
         if (kind != K_HEAD) {
             if (producer) { c.epoch++; if (!exchange) c.lbar++; }
             else if (exchange) tp_all_barrier(p, c, (c.tp_seq0 + c.tpx) * (p.tp_two_shot ? 2u : 1u));
@@ -2031,8 +1930,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) forward_kernel(const __grid_co
         if (old == (int)gridDim.x - 1) {
             for (int j = 0; j < kBarLanes; j++) p.sync[kSyncBar + j] = 0;
             p.sync[kSyncExit] = 0;
-            if (TP)                        // every CTA read the old count before its first barrier
-                *reinterpret_cast<volatile unsigned*>(p.tp_peers[p.tp_rank] + kTpFwdCount) = c.tp_seq0 + c.tpx;
+            // every CTA read the old count before its first barrier
+            *reinterpret_cast<volatile unsigned*>(p.tp_peers[p.tp_rank] + kTpFwdCount) = c.tp_seq0 + c.tpx;
         }
     }
 }
@@ -2253,9 +2152,9 @@ int make_kv_map(CUtensorMap* map, void* cache, int layers, int hkv, int cap, int
     return B200_OK;
 }
 
-template <int MT, int HD, bool TP, bool BATCH>
+template <int MT, int HD>
 int launch_forward(const FwdParams& p, int grid, cudaStream_t stream) {
-    auto kern = forward_kernel<MT, HD, TP, BATCH>;
+    auto kern = forward_kernel<MT, HD>;
     bool attr_set = false;
     if (!attr_set) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<MT>::SMEM) != cudaSuccess)
@@ -2278,7 +2177,7 @@ int launch_forward(const FwdParams& p, int grid, cudaStream_t stream) {
 
 template <int MT>
 int launch_forward_hd(const FwdParams& p, int grid, cudaStream_t stream) {
-    return p.HD == 128 ? launch_forward<MT, 128, true, false>(p, grid, stream) : launch_forward<MT, 64, true, false>(p, grid, stream);
+    return p.HD == 128 ? launch_forward<MT, 128>(p, grid, stream) : launch_forward<MT, 64>(p, grid, stream);
 }
 
 }  // namespace
@@ -2359,10 +2258,6 @@ int b200_forward(const b200_forward_desc* d, void* stream) {
     p.kv_half_stride = (size_t)d->n_kv_heads * d->cache_rows * d->head_dim;
     p.kv_layer_stride = 2 * p.kv_half_stride;
     p.cap = d->cache_rows; p.write_off = d->write_off; p.tail = d->tail;
-    p.nreq = d->requests > 1 ? d->requests : 1;
-    p.mr = d->M / p.nreq;
-    p.kv_req_stride = (size_t)d->n_layers * p.kv_layer_stride;
-    p.kv_req_rows = d->n_layers * 2 * d->n_kv_heads * d->cache_rows;
     char* ws = static_cast<char*>(d->workspace);
     p.sync = reinterpret_cast<int*>(ws + w.sync);
     p.counter = reinterpret_cast<int*>(ws + w.counter);
@@ -2373,7 +2268,7 @@ int b200_forward(const b200_forward_desc* d, void* stream) {
     p.partial = reinterpret_cast<float*>(ws + w.partial);
     p.nkb = w.nkb; p.qrp = w.qrp;
     {
-        const int rc = make_kv_map(&p.kvmap, d->kv_cache, d->n_layers * p.nreq, d->n_kv_heads, d->cache_rows, d->head_dim);
+        const int rc = make_kv_map(&p.kvmap, d->kv_cache, d->n_layers, d->n_kv_heads, d->cache_rows, d->head_dim);
         if (rc != B200_OK) return rc;
     }
     p.head_rows = d->head_rows > 0 ? d->head_rows : d->vocab;

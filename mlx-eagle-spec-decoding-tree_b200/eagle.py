@@ -90,7 +90,7 @@ class SpecDecoder:
         self.graph: Optional[torch.cuda.CUDAGraph] = None
         self.base_logits = None
         self.kernel_launches_per_step = (
-            (depth + 1) * draft_model.launches_per_forward + base_model.launches_per_forward
+            (depth + 1) * draft_model.kernels_per_forward + base_model.kernels_per_forward
             + 1 + (depth + 1) * 4 + 1 + 1 + 1 + 1)
         if base_model.tp is not None:                    # argmax combine over peer memory, or two key shifts around NCCL
             self.kernel_launches_per_step += 1 if base_model.tp.peers is not None else 2
@@ -397,7 +397,7 @@ class BatchSpecDecoder:
         # request's state: they go to one side stream per request, so that the captured graph has parallel branches
         self.side = [torch.cuda.Stream(device=self.device) for _ in range(R)]
         one = self.slots[0].kernel_launches_per_step
-        fwd = (depth + 1) * draft_model.launches_per_forward + base_model.launches_per_forward
+        fwd = (depth + 1) * draft_model.kernels_per_forward + base_model.kernels_per_forward
         self.kernel_launches_per_step = fwd + R * (one - fwd)
 
     def _per_request(self, fn):

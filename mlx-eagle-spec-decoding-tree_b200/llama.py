@@ -5,7 +5,8 @@
 positions, ``flat_rope`` giving every token of the call the same position.  All
 linear layers are 4-bit / group-64 quantised and run through ``libb200eagle.so``;
 q/k/v are stored as one fused matrix.  Once the weights are in the streaming layout
-(``Model.relayout``) a whole pass is ONE persistent kernel (``b200_forward``); before that, or
+(``Model.relayout``) a whole pass is one native call (``b200_forward``: a chain of five kernels per layer, or one
+persistent kernel for a tensor-parallel shard); before that, or
 with ``model.fused = False``, one layer is nine kernel launches:
 
     rms_norm -> qmm(+bias) -> rope_kv_append -> tree_attention (+ merge) -> qmm(+residual)
@@ -290,12 +291,12 @@ class Model:
         self.logits = torch.zeros(MAX_ROWS, args.vocab_size, **f16)
         self._attn_ws = None
         self._attn_ws_rows = 0
-        # matmul inputs of the fused forward, chunk-major padded: [width/128][rows <= 32][128], 16-byte units swizzled by the row parity
+        # matmul inputs of the fused forward, in a layout of its kernels: h * norm weight, attention output, MLP activations
         self.hw = torch.zeros(H // 128 * MAX_ROWS * 128 if H % 128 == 0 else 0, **f16)      # h * norm weight
         self.xt_attn = torch.zeros(self.nq // 128 * MAX_ROWS * 128 if self.nq % 128 == 0 else 0, **f16)
         self.xt_act = torch.zeros(args.intermediate_size // 128 * MAX_ROWS * 128
                                   if args.intermediate_size % 128 == 0 else 0, **f16)
-        self.fused = True                                # one persistent kernel per pass when possible
+        self.fused = True                                # b200_forward when possible
         self._fwd_ws = None
         self._fwd_ws_key = None
         self._layer_table = None
@@ -305,7 +306,7 @@ class Model:
         self.timeline = None
         self.attn_split_blocks = 0                       # 0 = library default; < 0 = always split the keys across CTAs
         self.phase_mask = 0                              # profiling: run only some phase kinds (0 = all)
-        self.grid_ctas = 0                               # CTAs of the persistent kernel (0 = one per SM)
+        self.grid_ctas = 0                               # CTAs of a shard's persistent kernel (0 = one per SM)
         self.fast_dequant = True                         # allow the short nibble expansion when every scale permits it
         self.tp_two_shot = 0                             # tensor-parallel exchange: 0 library's choice (push), 1 two-step, 2 pull behind a hierarchical barrier, 3 push, 4 pull
         self.prefill_large_m = True                      # prompts: 128 rows per weight read through b200_prefill
@@ -483,12 +484,18 @@ class Model:
 
     @property
     def launches_per_forward(self) -> int:
-        """Kernel launches of one pass: 1 (persistent kernel) or 9 per layer + embedding, final norm, head."""
+        """Launches of one pass from Python: 1 (``b200_forward``) or 9 per layer + embedding, final norm, head."""
         return 1 if self.can_fuse() else 9 * self.args.num_hidden_layers + 3
+
+    @property
+    def kernels_per_forward(self) -> int:
+        """Kernels of one pass: the five per layer of the chain, embedding and head (one more where the last row tiles of a wide
+        layer run as a launch of their own, not counted), the persistent kernel of a shard, or the per-op launches."""
+        return 5 * self.args.num_hidden_layers + 2 if self.can_fuse() and self.tp is None else self.launches_per_forward
 
     # ------------------------------------------------------------------ fused forward (one kernel)
     def can_fuse(self) -> bool:
-        """True when the pass can run as the single persistent kernel ``b200_forward``: every linear
+        """True when the pass can run as one call of ``b200_forward``: every linear
         layer in the streaming layout, the embedding still row-major, sizes in multiples of 128."""
         if not self.fused or os.environ.get("B200_FUSED_FORWARD", "1") == "0":
             return False
@@ -558,7 +565,7 @@ class Model:
         return d
 
     def enable_timeline(self, on: bool = True):
-        """Profiling hook of the persistent kernel: per SM, the device timer (ns) at arrival at and
+        """Profiling hook of a shard's persistent kernel: per SM, the device timer (ns) at arrival at and
         departure from every device-wide barrier of the next pass, plus six stamps inside the matmul phase
         that ends at the barrier: entry, rstd done, first stage landed, stages done, K-parts reduced, end
         (``self.timeline`` int64 ``[SMs, barriers + 1, 8]``; the last entry holds the end of the kernel)."""
@@ -571,7 +578,7 @@ class Model:
             self.timeline = None
 
     def check_fused_error(self):
-        """Raise if a bounded wait inside the persistent forward kernel ever gave up (synchronises)."""
+        """Raise if a bounded wait inside ``b200_forward`` ever gave up (synchronises)."""
         if self._fwd_ws is None:
             return
         code = int(self._fwd_ws[:16].view(torch.int32)[2])
