@@ -245,6 +245,7 @@ int b200_tree_attention(const void* q, int q_stride, const void* kcache, const v
  * stream-ordered.  hidden, intermediate and n_heads*head_dim must be multiples of 128, hidden <= 8192,
  * head_dim 64 or 128, tail <= 64, write_off + M <= tail.
  * ------------------------------------------------------------------------------------------ */
+#define B200_LAYERS_ON_HOST (-1)
 typedef struct b200_forward_desc {
     int M, rows_out;
     int hidden, intermediate, n_heads, n_kv_heads, head_dim, vocab, n_layers;
@@ -280,6 +281,10 @@ typedef struct b200_forward_desc {
                             /* phase_mask: profiling only, 0 = run everything; else bit k set = run phase  */
                             /* kind k (0 embedding, 1 qkv, 2 attention, 3 merge, 4 o_proj, 5 gate/up,      */
                             /* 6 down_proj, 7 vocabulary projection); results are then meaningless         */
+                            /* Without tensor parallelism timeline_pitch = B200_LAYERS_ON_HOST makes timeline  */
+                            /* a HOST copy of layer_table, read during the call.  Otherwise the call reads     */
+                            /* layer_table back first, which waits for the stream (inside a capture: for       */
+                            /* nothing, the table must be complete then)                                       */
     /* Tensor parallelism over the GPUs of one node (tp_world <= 1 = off, all fields below zero).  The call
      * then runs shard tp_rank of tp_world: n_heads, n_kv_heads and intermediate are this shard's counts
      * (heads and MLP rows cut evenly; o_proj / down_proj weights hold this shard's K columns), head_rows
@@ -330,9 +335,6 @@ typedef struct b200_forward_desc {
                                  * and tail apply to each; attention never crosses requests; rows_out counts rows per
                                  * request and logits is [requests * rows_out][vocab].  Needs cache_rows <= 2048 and
                                  * tp_world <= 1. */
-    const void* const* layers_host;     /* HOST copy of layer_table (n_layers * 8 device pointers), read during the call.
-                                 * NULL: copied from layer_table by this call, which then synchronises with the device and
-                                 * must not run inside a stream capture.  Not needed with tp_world > 1. */
 } b200_forward_desc;
 
 size_t b200_forward_workspace_bytes(const b200_forward_desc* desc);

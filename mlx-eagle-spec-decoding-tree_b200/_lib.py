@@ -166,6 +166,9 @@ def _declare(l: ctypes.CDLL) -> None:
     l.b200_kv_compact.argtypes = [vp, i32, i32, i32, i32, vp, vp, vp]
 
 
+LAYERS_ON_HOST = -1       # ForwardDesc.timeline_pitch: timeline is a host copy of the layer table
+
+
 class ForwardDesc(ctypes.Structure):
     """Mirror of ``b200_forward_desc`` (include/b200_eagle.h): host struct of sizes and device pointers."""
     _fields_ = ([(n, ctypes.c_int) for n in (
@@ -180,8 +183,7 @@ class ForwardDesc(ctypes.Structure):
         + [("workspace_bytes", ctypes.c_size_t), ("timeline", ctypes.c_void_p), ("timeline_pitch", ctypes.c_int),
            ("phase_mask", ctypes.c_int), ("tp_world", ctypes.c_int), ("tp_rank", ctypes.c_int),
            ("head_rows", ctypes.c_int), ("grid_ctas", ctypes.c_int), ("tp_peers", ctypes.c_void_p * 8),
-           ("scales_in_fast_range", ctypes.c_int), ("tp_two_shot", ctypes.c_int), ("requests", ctypes.c_int),
-           ("layers_host", ctypes.c_void_p)])
+           ("scales_in_fast_range", ctypes.c_int), ("tp_two_shot", ctypes.c_int), ("requests", ctypes.c_int)])
 
 
 class PrefillDesc(ctypes.Structure):

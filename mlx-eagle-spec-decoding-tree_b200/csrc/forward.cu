@@ -2180,6 +2180,24 @@ int launch_forward_hd(const FwdParams& p, int grid, cudaStream_t stream) {
     return p.HD == 128 ? launch_forward<MT, 128>(p, grid, stream) : launch_forward<MT, 64>(p, grid, stream);
 }
 
+// Copy of the device's layer table, for callers that have none on the host.  While `stream` is being captured it comes through a
+// stream of its own, which must not become part of the capture.
+bool read_table(const void** table, const b200_forward_desc* d, cudaStream_t stream) {
+    const size_t bytes = (size_t)d->n_layers * 8 * sizeof(void*);
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess) return false;
+    if (capturing == cudaStreamCaptureStatusNone)
+        return cudaMemcpyAsync(table, d->layer_table, bytes, cudaMemcpyDeviceToHost, stream) == cudaSuccess &&
+               cudaStreamSynchronize(stream) == cudaSuccess;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return false;
+    cudaStream_t own = nullptr;
+    bool ok = cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking) == cudaSuccess;
+    ok = ok && cudaMemcpyAsync(table, d->layer_table, bytes, cudaMemcpyDeviceToHost, own) == cudaSuccess && cudaStreamSynchronize(own) == cudaSuccess;
+    if (own != nullptr) cudaStreamDestroy(own);
+    return cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess && ok;
+}
+
 }  // namespace
 }  // namespace b200
 
@@ -2225,13 +2243,10 @@ int b200_forward(const b200_forward_desc* d, void* stream) {
         for (int i = 0; i < 5; i++)
             if (const PlanOverride* o = plan_override(i)) a.splits[i] = (o->kw & (o->kw - 1)) == 0 && o->kw <= 8 ? o->splits : 0;
         const void* table[kMaxLayers * 8];
-        a.layers = d->layers_host;
-        if (a.layers == nullptr) {
-            cudaStream_t st = static_cast<cudaStream_t>(stream);
-            if (cudaMemcpyAsync(table, d->layer_table, (size_t)d->n_layers * 8 * sizeof(void*), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-                cudaStreamSynchronize(st) != cudaSuccess)
-                return check_launch() == B200_OK ? B200_ECUDA : B200_ECUDA;
-            a.layers = table;
+        a.layers = d->timeline_pitch == B200_LAYERS_ON_HOST ? static_cast<const void* const*>(d->timeline) : table;
+        if (a.layers == table && !read_table(table, d, static_cast<cudaStream_t>(stream))) {
+            (void)check_launch();
+            return B200_ECUDA;
         }
         return forward_chain(a, static_cast<cudaStream_t>(stream));
     }
@@ -2290,8 +2305,8 @@ int b200_forward(const b200_forward_desc* d, void* stream) {
     p.tp_wait_limit = g_wait_limit ? g_wait_limit : kTpWaitLimit;
     p.fast_scales = d->scales_in_fast_range ? 1 : 0;
     p.attn_fused_max = d->attn_split_blocks > 0 ? d->attn_split_blocks - 1 : (d->attn_split_blocks < 0 ? 0 : 32);
-    p.timeline = static_cast<long long*>(d->timeline);
-    p.timeline_pitch = d->timeline ? d->timeline_pitch : 0;
+    p.timeline = d->timeline_pitch > 0 ? static_cast<long long*>(d->timeline) : nullptr;
+    p.timeline_pitch = p.timeline ? d->timeline_pitch : 0;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     switch ((d->M + 7) / 8) {
         case 1: return launch_forward_hd<1>(p, grid, st);

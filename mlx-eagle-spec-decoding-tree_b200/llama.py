@@ -538,7 +538,6 @@ class Model:
             d.embed_wq, d.embed_scales, d.embed_biases = p(self.embed.weight), p(self.embed.scales), p(self.embed.biases)
             d.final_norm, d.lm_head_tiled, d.layer_table = p(self.norm), p(self.lm_head.tiled), p(self._layer_table)
             d.h, d.hw, d.qkv, d.attn, d.act = p(self.h), p(self.hw), p(self.qkv), p(self.xt_attn), p(self.xt_act)
-            d.layers_host = ctypes.cast(self._layers_host, ctypes.c_void_p)
             self._desc = d
         d.M, d.rows_out, d.requests = M, rows, requests
         d.cache_rows, d.write_off, d.tail = cache.rows, write_off, tail
@@ -561,7 +560,10 @@ class Model:
             self._fwd_ws = torch.zeros(nbytes, dtype=torch.uint8, device=self.device)
             self._fwd_ws_key = key
         d.workspace, d.workspace_bytes = p(self._fwd_ws), self._fwd_ws.numel()
-        d.timeline, d.timeline_pitch = (p(self.timeline), self.timeline.shape[1]) if self.timeline is not None else (None, 0)
+        if self.tp is None:
+            d.timeline, d.timeline_pitch = ctypes.addressof(self._layers_host), _lib.LAYERS_ON_HOST
+        else:
+            d.timeline, d.timeline_pitch = (p(self.timeline), self.timeline.shape[1]) if self.timeline is not None else (None, 0)
         return d
 
     def enable_timeline(self, on: bool = True):

@@ -1,5 +1,7 @@
 """The kernel chain of a pass of up to 32 tokens (csrc/decode.cu) at the edges of its tiles, key blocks and clusters, against the
 per-op kernels; and the inputs of a pass from a caller's tensors."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -80,3 +82,25 @@ def test_pass_inputs_whatever_their_form(be, cuda, rows, cached):
     cache.offset = cached
     explicit = m(tokens, cache, position_ids=cached + torch.arange(rows))
     assert last.shape == (1, 1, SHAPES[1][-1]) and torch.equal(last, every[:, -1:]) and torch.equal(explicit, every)
+
+
+def test_layer_pointers_from_the_device_table(be, cuda):
+    """Without a host copy of the layer table the call reads it back: the same logits, and it stays capturable."""
+    m = _model(be, cuda, *SHAPES[1])
+    cache = _cache(m, 70, 4)
+    m.fwd.tokens.copy_(torch.arange(32))
+    m.fwd.pos.copy_(70 + torch.arange(32))
+    m.fwd.prefix.fill_(70)
+    m.fwd.mask.copy_(torch.tensor([(2 << i) - 1 for i in range(32)]))
+    want = m.forward_device(20, cache, 0, 20).clone()
+    desc = be._lib.ForwardDesc.from_buffer_copy(m._fused_desc(20, cache, 0, 20, m.fwd, 20, None))
+    assert desc.timeline_pitch == be._lib.LAYERS_ON_HOST
+    desc.timeline, desc.timeline_pitch = None, 0
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        be._lib.check(be._lib.lib().b200_forward(ctypes.byref(desc), be._lib.stream_ptr(m.device)), "b200_forward")
+    m.logits.zero_()
+    graph.replay()
+    m.check_fused_error()
+    assert torch.equal(m.logits[:20], want)
