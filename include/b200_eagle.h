@@ -366,6 +366,13 @@ int b200_tp_argmax_combine(unsigned long long* best_key, int R, unsigned int ind
                            int tp_rank, void* const* tp_peers, void* stream);
 int b200_forward(const b200_forward_desc* desc, void* stream);
 
+/* The same pass as an executable CUDA graph of the current device, for callers that repeat one descriptor (the data it points
+ * to may change, the descriptor and the layer table may not); not for tensor-parallel shards.  b200_graph_launch enqueues it
+ * on a stream, b200_graph_destroy releases it (NULL is allowed). */
+int b200_forward_graph(const b200_forward_desc* d, void** exec);
+int b200_graph_launch(void* exec, void* stream);
+int b200_graph_destroy(void* exec);
+
 /* Measurement aid, not part of the model interface: overrides the work split the planner would choose for the
  * matmul phases of later b200_forward calls.  spec = "A=kw:cps:splits,C=...,D=...,E=...,H=..." (A q|k|v, C o_proj,
  * D gate/up, E down_proj, H vocabulary projection; kw = K-parts inside a CTA, 1/2/4/8; cps = 128-column chunks of K

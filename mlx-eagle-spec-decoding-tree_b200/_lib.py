@@ -152,6 +152,12 @@ def _declare(l: ctypes.CDLL) -> None:
     l.b200_tp_argmax_combine.argtypes = [vp, i32, ctypes.c_uint, i32, i32, ctypes.POINTER(ctypes.c_void_p), vp]
     l.b200_forward.restype = i32
     l.b200_forward.argtypes = [ctypes.POINTER(ForwardDesc), vp]
+    l.b200_forward_graph.restype = i32
+    l.b200_forward_graph.argtypes = [ctypes.POINTER(ForwardDesc), ctypes.POINTER(ctypes.c_void_p)]
+    l.b200_graph_launch.restype = i32
+    l.b200_graph_launch.argtypes = [vp, vp]
+    l.b200_graph_destroy.restype = i32
+    l.b200_graph_destroy.argtypes = [vp]
     l.b200_prefill.restype = i32
     l.b200_prefill.argtypes = [ctypes.POINTER(PrefillDesc), vp]
     l.b200_add_f16.restype = i32

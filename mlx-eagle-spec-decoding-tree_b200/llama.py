@@ -18,6 +18,7 @@ device memory, so that a whole speculative step can be replayed as a CUDA graph.
 """
 from __future__ import annotations
 
+import collections
 import ctypes
 import math
 import os
@@ -266,6 +267,40 @@ class BatchKVCache:
         self.slabs = [KVCache(args, rows, device, data=self.data[r]) for r in range(self.requests)]
 
 
+class _Graphs:
+    """Graphs of the descriptors a model's passes repeat: at most ``KEEP``, the least recently used go first.  A descriptor holds
+    every address and size of its pass, so an equal one is the same pass; making its graph takes about as long as a pass of the
+    large models, so only one that has come up ``AFTER`` times while among the last ``KEEP`` gets one."""
+    KEEP, AFTER = 16, 4
+
+    def __init__(self):
+        self._seen = collections.OrderedDict()           # descriptor -> [times, graph]
+
+    def get(self, desc, device):
+        key = bytes(desc)
+        entry = self._seen.get(key)
+        if entry is None:
+            if len(self._seen) >= self.KEEP:
+                _lib.lib().b200_graph_destroy(self._seen.popitem(last=False)[1][1])
+            self._seen[key] = [1, None]
+            return None
+        self._seen.move_to_end(key)
+        entry[0] += 1
+        if entry[1] is None and entry[0] > self.AFTER:
+            exec_ = ctypes.c_void_p()
+            with torch.cuda.device(device):
+                _lib.check(_lib.lib().b200_forward_graph(ctypes.byref(desc), ctypes.byref(exec_)), "b200_forward_graph")
+            entry[1] = exec_.value
+        return entry[1]
+
+    def __del__(self):
+        try:
+            for entry in self._seen.values():
+                _lib.lib().b200_graph_destroy(entry[1])
+        except Exception:                                # (interpreter shutdown)
+            pass
+
+
 class Model:
     def __init__(self, args: ModelArgs, layers: List[dict], embed: QLinear, norm: torch.Tensor,
                  lm_head: Optional[QLinear], device):
@@ -313,6 +348,7 @@ class Model:
         self._pf, self._pf_buf, self._pf_fits = None, None, False     # descriptor and buffers of that path, made on first use
         self._scales_fast = None
         self._desc, self._fuse_fits = None, False
+        self._graphs = _Graphs()
         self.fwd = FwdInputs(self.device)
 
     # ------------------------------------------------------------------ construction
@@ -615,6 +651,17 @@ class Model:
             self._attn_ws_rows = cache.rows
         return self._attn_ws
 
+    def _run_fused(self, desc):
+        """``b200_forward``, or the graph of a descriptor that has come up ``_Graphs.AFTER`` times: a decode loop repeats one or two
+        (the result's address alternates), and a launch of the graph is 120 launches less."""
+        lib, stream = _lib.lib(), _lib.stream_ptr(self.device)
+        if self.tp is None and not torch.cuda.is_current_stream_capturing():
+            exec_ = self._graphs.get(desc, self.device)
+            if exec_ is not None:
+                _lib.check(lib.b200_graph_launch(exec_, stream), "b200_graph_launch")
+                return
+        _lib.check(lib.b200_forward(ctypes.byref(desc), stream), "b200_forward")
+
     def forward_device(self, M: int, cache: KVCache, write_off: int, tail: int, fwd: Optional[FwdInputs] = None,
                        logits_rows: Optional[int] = None, row_index: Optional[torch.Tensor] = None, requests: int = 1):
         """One forward pass of ``M`` tokens whose ids / positions / masks / committed length sit in
@@ -643,8 +690,7 @@ class Model:
             return self.logits[: requests * rows] if out is None else out
         if self.can_fuse():
             rows = M if logits_rows is None else logits_rows
-            desc = self._fused_desc(M, cache, write_off, tail, fwd, rows, row_index, logits=out)
-            _lib.check(_lib.lib().b200_forward(ctypes.byref(desc), _lib.stream_ptr(self.device)), "b200_forward")
+            self._run_fused(self._fused_desc(M, cache, write_off, tail, fwd, rows, row_index, logits=out))
             if out is not None:
                 return out
             vl = self.vocab_local

@@ -104,3 +104,25 @@ def test_layer_pointers_from_the_device_table(be, cuda):
     graph.replay()
     m.check_fused_error()
     assert torch.equal(m.logits[:20], want)
+
+
+def test_a_repeated_pass_runs_from_a_graph_on_the_data_of_the_call(be, cuda):
+    m = _model(be, cuda, *SHAPES[0])
+    keep = m._graphs.KEEP
+    cache = _cache(m, 10, 5)
+    for i in range(4 * m._graphs.AFTER):                 # (two result addresses in turn)
+        cache.offset = 10 + i % 3
+        tokens = torch.tensor([[i % 5, 7]])
+        got = m(tokens, cache)
+        cache.offset = 10 + i % 3
+        m.fused = False
+        assert ((got - m(tokens, cache)).abs() <= 2e-2).all()
+        m.fused = True
+    assert any(g for _, g in m._graphs._seen.values())
+    caches = [m.make_cache(64 * (1 + i)) for i in range(keep + 2)]       # more passes than graphs are kept for
+    for _ in range(m._graphs.AFTER + 2):
+        for c in caches:
+            c.offset = 0
+            m(tokens, c)
+    m.check_fused_error()
+    assert len(m._graphs._seen) <= keep
