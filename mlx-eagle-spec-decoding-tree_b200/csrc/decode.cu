@@ -45,7 +45,7 @@ constexpr int kMaxCluster = 8;
 constexpr int kSsqPitch = 32, kCsPitch = 64, kKeyBlock = 64;
 constexpr uint32_t kDWaitPolls = 1u << 19;       // about a microsecond each
 
-enum { D_QKV = 0, D_RESID = 1, D_SILU = 2, D_HEAD = 3 };
+enum { D_QKV = 0, D_RESID = 1, D_SILU = 2, D_HEAD = 3, D_PLAIN = 4 };      // D_PLAIN: y = x W^T (+ bias), a matmul on its own
 
 template <int TQ>
 struct __align__(TQ * 4) Vec { float v[TQ]; };      // a value per token of a group
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
     } else if (warp == kDeq + 3) {
         // ------------------------------------------------------------------ sums of squares -> 1 / rms of each token
         // (by the dequant warps it held up every chunk behind the first three: 1.4 us at a hidden size of 3584)
-        if (KIND != D_RESID) {
+        if (KIND != D_RESID && KIND != D_PLAIN) {
             pdl_wait();
             // a lane: four tokens of every `step`-th part; as many parts at once as the tokens leave lanes for
             const int quads = p.M <= 8 ? 2 : (p.M <= 16 ? 4 : 8), step = 32 / quads, quad = lane & (quads - 1);
@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
         // (Four threads of a quarter-warp read the same banks: swapping units between threads to halve that took more issue slots, 16
         // selects a chunk, than the reads took cycles.)
-        constexpr bool NORMED = KIND != D_RESID;                 // the input is h * w_norm: scale by 1 / rms
+        constexpr bool NORMED = KIND != D_RESID && KIND != D_PLAIN;                 // the input is h * w_norm: scale by 1 / rms
         // ---- one finished tile: accumulators -> inbox of the CTA that finishes each token -> output
         auto epilogue = [&](int it) {
             const int tile = tile0 + it * tstep;
@@ -399,9 +399,9 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
             };
             if (it == 0) pdl_wait();
             if (KIND == D_RESID && valid) extra = p.wn[n];
-            if (KIND == D_QKV && valid && p.bias != nullptr) {
+            if ((KIND == D_QKV || KIND == D_PLAIN) && valid && p.bias != nullptr) {
                 extra = p.bias[n];
-                extra2 = p.bias[tile * kTile + pr];
+                if (KIND == D_QKV) extra2 = p.bias[tile * kTile + pr];
             }
             if (j0 < nq) ask(j0);
 
@@ -489,6 +489,10 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                             p.h[at] = o;
                             p.hw[at] = __hmul(o, extra);
                         }
+                    } else if (KIND == D_PLAIN) {
+                        __half x = __float2half_rn(v.v[k]);
+                        if (p.bias != nullptr) x = __hadd(x, extra);
+                        if (valid) p.y[(size_t)tok * p.N + n] = x;
                     } else if (KIND == D_HEAD) {
                         const int rel = tok - rq * p.mr - (p.row_index ? p.row_index[rq] : 0);
                         if (valid && rel >= 0 && rel < p.rows_out) p.y[(size_t)(rq * p.rows_out + rel) * p.N + n] = __float2half_rn(v.v[k]);
@@ -1084,7 +1088,25 @@ int run_chain(const ChainArgs& c, cudaStream_t st) {
     return B200_OK;
 }
 
+template <int NT, int TQ>
+int run_matmul(const void* x, const void* w, const void* bias, void* y, int M, int N, int K, int* err, cudaStream_t st) {
+    DenseParams p{};
+    const int rc = make_map_2d(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x, K, M, (uint64_t)K * 2, 64, NT, CU_TENSOR_MAP_SWIZZLE_128B,
+                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+    if (rc != B200_OK) return rc;
+    p.w[0] = static_cast<const unsigned char*>(w);
+    p.bias = static_cast<const __half*>(bias);
+    p.y = static_cast<__half*>(y);
+    p.M = p.mr = M; p.N = N; p.K = K; p.hd = 64; p.err = err;
+    return launch_dense<NT, TQ, D_PLAIN>(p, 0, st);
+}
+
 }  // namespace
+
+int chain_matmul(const void* x, const void* w, const void* bias, void* y, int M, int N, int K, int* err, cudaStream_t st) {
+    return M <= 8 ? run_matmul<16, 2>(x, w, bias, y, M, N, K, err, st)
+                  : (M <= 16 ? run_matmul<16, 4>(x, w, bias, y, M, N, K, err, st) : run_matmul<32, 4>(x, w, bias, y, M, N, K, err, st));
+}
 
 int forward_chain(const ChainArgs& a, cudaStream_t stream) { return a.d->M <= 8 ? run_chain<16, 2>(a, stream) : (a.d->M <= 16 ? run_chain<16, 4>(a, stream) : run_chain<32, 4>(a, stream)); }
 

@@ -17,4 +17,7 @@ struct ChainArgs {
 
 int forward_chain(const ChainArgs& a, cudaStream_t stream);
 
+// y[M][N] = x[M][K] . W^T (+ bias), M <= 32, W in the streaming layout, by the chain's matmul kernel on its own.
+int chain_matmul(const void* x, const void* w, const void* bias, void* y, int M, int N, int K, int* err, cudaStream_t stream);
+
 }  // namespace b200
