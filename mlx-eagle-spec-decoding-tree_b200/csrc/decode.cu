@@ -45,7 +45,7 @@ constexpr int kMaxCluster = 8;
 constexpr int kSsqPitch = 32, kCsPitch = 64, kKeyBlock = 64;
 constexpr uint32_t kDWaitPolls = 1u << 19;       // about a microsecond each
 
-enum { D_QKV = 0, D_RESID = 1, D_SILU = 2, D_HEAD = 3, D_PLAIN = 4 };      // D_PLAIN: y = x W^T (+ bias), a matmul on its own
+enum { D_QKV = 0, D_RESID = 1, D_SILU = 2, D_HEAD = 3, D_PLAIN = 4, D_ROWS = 5 };      // the last two: y = x W^T (+ bias), a matmul on its own; D_ROWS: W as quantised
 
 template <int TQ>
 struct __align__(TQ * 4) Vec { float v[TQ]; };      // a value per token of a group
@@ -85,6 +85,10 @@ struct DenseParams {
     const int* prefix;
     int Hq, Hkv, hd, cap, write_off, mr;
     size_t req_stride;            // halves between the caches of two requests
+    // D_ROWS: packs [N][K / 8] as rows of bytes, boxes of 64 bytes x 128 rows, 64-byte swizzle; scales and biases [N][K / 64]
+    CUtensorMap wmap;
+    const __half* sc;
+    const __half* bi;
     // D_HEAD
     const int* row_index;
     int rows_out;
@@ -230,6 +234,11 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         bulk_copy_g2s(dst, src0, kRun, bar);
         bulk_copy_g2s(dst + kRun, src1, kRun, bar);
     };
+    auto wload_rows = [&](uint32_t slot, int tile, int c) {
+        const uint32_t bar = smem_u32(wfull + slot);
+        mbar_expect_tx(bar, kTile * 64);
+        tma_box(smem_u32(ring + slot * kW), &p.wmap, (c_lo + c) * 64, tile * kTile, bar);
+    };
     if (warp == kDeq) {
         if (lane < G::NW) {
             mbar_init(smem_u32(wfull + lane), 1);
@@ -237,10 +246,14 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
             asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         }
         __syncwarp();
+        if (KIND == D_ROWS) pdl_wait();                          // (the kernel before this one may have written the weights)
         if (elect_one()) {
             const unsigned char *src0 = wsrc(tile0, 0), *src1 = wsrc(tile0, 1);
 #pragma unroll 1
-            for (int c = 0; c < min(nc, G::NW); c++) wload(c, src0 + c * kRun, src1 + c * kRun);
+            for (int c = 0; c < min(nc, G::NW); c++) {
+                if (KIND == D_ROWS) wload_rows(c, tile0, c);
+                else wload(c, src0 + c * kRun, src1 + c * kRun);
+            }
         }
         __syncwarp();
     }
@@ -271,7 +284,10 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
             for (int c = c0; c < nc; c++) {
                 if (lap) dwait(smem_u32(wempty + slot), ph, abort_flag, p.err, 21);
                 __syncwarp();
-                if (elect_one()) wload(slot, src0, src1);
+                if (elect_one()) {
+                    if (KIND == D_ROWS) wload_rows(slot, tile, c);
+                    else wload(slot, src0, src1);
+                }
                 __syncwarp();
                 src0 += kRun;
                 src1 += kRun;
@@ -337,7 +353,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
     } else if (warp == kDeq + 3) {
         // ------------------------------------------------------------------ sums of squares -> 1 / rms of each token
         // (by the dequant warps it held up every chunk behind the first three: 1.4 us at a hidden size of 3584)
-        if (KIND != D_RESID && KIND != D_PLAIN) {
+        if (KIND != D_RESID && KIND != D_PLAIN && KIND != D_ROWS) {
             pdl_wait();
             // a lane: four tokens of every `step`-th part; as many parts at once as the tokens leave lanes for
             const int quads = p.M <= 8 ? 2 : (p.M <= 16 ? 4 : 8), step = 32 / quads, quad = lane & (quads - 1);
@@ -367,11 +383,11 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         const uint32_t me = warp >> 2;                           // group (and, in the epilogue, which half of the tokens)
         const int q = warp & 3, r = q * 32 + lane, rr = r & 15;
         const uint32_t recoff = (r >> 6) * kRun + ((r >> 4) & 3) * 1152;
-        const uint32_t rowoff = recoff + (rr >> 3) * 512 + (rr & 7) * 64, scoff = recoff + 1024 + rr * 8;
+        const uint32_t rowoff = KIND == D_ROWS ? r * 64 + (((r >> 1) & 3) << 4) : recoff + (rr >> 3) * 512 + (rr & 7) * 64, scoff = recoff + 1024 + rr * 8;
         const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
         // (Four threads of a quarter-warp read the same banks: swapping units between threads to halve that took more issue slots, 16
         // selects a chunk, than the reads took cycles.)
-        constexpr bool NORMED = KIND != D_RESID && KIND != D_PLAIN;                 // the input is h * w_norm: scale by 1 / rms
+        constexpr bool NORMED = KIND != D_RESID && KIND != D_PLAIN && KIND != D_ROWS;                 // the input is h * w_norm: scale by 1 / rms
         // ---- one finished tile: accumulators -> inbox of the CTA that finishes each token -> output
         auto epilogue = [&](int it) {
             const int tile = tile0 + it * tstep;
@@ -399,7 +415,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
             };
             if (it == 0) pdl_wait();
             if (KIND == D_RESID && valid) extra = p.wn[n];
-            if ((KIND == D_QKV || KIND == D_PLAIN) && valid && p.bias != nullptr) {
+            if ((KIND == D_QKV || KIND == D_PLAIN || KIND == D_ROWS) && valid && p.bias != nullptr) {
                 extra = p.bias[n];
                 if (KIND == D_QKV) extra2 = p.bias[tile * kTile + pr];
             }
@@ -489,7 +505,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                             p.h[at] = o;
                             p.hw[at] = __hmul(o, extra);
                         }
-                    } else if (KIND == D_PLAIN) {
+                    } else if (KIND == D_PLAIN || KIND == D_ROWS) {
                         __half x = __float2half_rn(v.v[k]);
                         if (p.bias != nullptr) x = __hadd(x, extra);
                         if (valid) p.y[(size_t)tok * p.N + n] = x;
@@ -529,6 +545,22 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         };
         uint32_t slot = me, wph = 0, tph = 1;
         int done = me;                                           // number of this group's next chunk, over all tiles
+        // D_ROWS: scales and biases of the group's next chunk (two groups of 64), asked for a chunk ahead
+        uint32_t next_s = 0, next_b = 0;
+        int ask_tile = tile0, ask_c = (int)me;
+        auto ask_scales = [&]() {
+            while (ask_c >= nc && ask_tile < p.tiles) { ask_c -= nc; ask_tile += tstep; }
+            if (ask_tile < p.tiles) {
+                const size_t at = (size_t)min(ask_tile * kTile + r, p.N - 1) * (p.K / 64) + 2 * (c_lo + ask_c);
+                next_s = __ldg(reinterpret_cast<const uint32_t*>(p.sc + at));
+                next_b = __ldg(reinterpret_cast<const uint32_t*>(p.bi + at));
+            }
+            ask_c += kGroups;
+        };
+        if (KIND == D_ROWS) {
+            pdl_wait();
+            ask_scales();
+        }
 #pragma unroll 1
         for (int it = 0; it <= nit; it++) {
             const int end = it < nit ? (it + 1) * nc : 0;
@@ -542,8 +574,14 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                     const unsigned char* st = ring + slot * kW;
                     uint4 u[4];
 #pragma unroll
-                    for (int i = 0; i < 4; i++) u[i] = *reinterpret_cast<const uint4*>(st + rowoff + i * 16);
-                    const uint2 sb = *reinterpret_cast<const uint2*>(st + scoff);
+                    for (int i = 0; i < 4; i++) u[i] = *reinterpret_cast<const uint4*>(st + (KIND == D_ROWS ? rowoff ^ (i * 16) : rowoff + i * 16));
+                    uint2 sb;                                    // (scale, bias) of the chunk's two groups
+                    if (KIND == D_ROWS) {
+                        sb = make_uint2(__byte_perm(next_s, next_b, 0x5410), __byte_perm(next_s, next_b, 0x7632));
+                        ask_scales();
+                    } else {
+                        sb = *reinterpret_cast<const uint2*>(st + scoff);
+                    }
                     const bool fast = __all_sync(0xffffffffu, fast_scale(sb.x) && fast_scale(sb.y));
                     if (lane == 0) mbar_arrive(smem_u32(wempty + slot));             // the packs are in registers
                     if (done >= kGroups) dwait(smem_u32(tfree + me), tph, abort_flag, p.err, 24);
@@ -552,7 +590,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                     auto expand = [&](auto fast_tag) {
                         constexpr bool FAST = decltype(fast_tag)::value;
 #pragma unroll
-                        for (int j = 0; j < 4; j++) {            // pack j of unit t = k group 4 j + t
+                        for (int j = 0; j < 4; j++) {            // pack j of unit t (D_ROWS: pack t of unit j) = k group 4 j + t
                             const uint32_t s = j < 2 ? sb.x : sb.y;
                             __half2 s2 = dup_half((unsigned short)s);
                             const __half2 b2 = dup_half((unsigned short)(s >> 16));
@@ -560,8 +598,14 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                             uint32_t d[4][4];
 #pragma unroll
                             for (int t = 0; t < 4; t++) {
-                                if (FAST) dequant_pack_fast(comp(u[t], j), s2, b2, d[t]);
-                                else dequant_pack(comp(u[t], j), s2, b2, d[t]);
+                                const uint32_t pack = KIND == D_ROWS ? comp(u[j], t) : comp(u[t], j);
+                                if (FAST) dequant_pack_fast(pack, s2, b2, d[t]);
+                                else dequant_pack(pack, s2, b2, d[t]);
+                                if (KIND == D_ROWS) {            // {e0,e4} {e1,e5} {e2,e6} {e3,e7} -> adjacent k pairs
+                                    const uint32_t e01 = __byte_perm(d[t][0], d[t][1], 0x5410), e45 = __byte_perm(d[t][0], d[t][1], 0x7632);
+                                    const uint32_t e23 = __byte_perm(d[t][2], d[t][3], 0x5410), e67 = __byte_perm(d[t][2], d[t][3], 0x7632);
+                                    d[t][0] = e01; d[t][1] = e23; d[t][2] = e45; d[t][3] = e67;
+                                }
                             }
                             asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(trow + me * kTCols + 16 * j),
                                          "r"(d[0][0]), "r"(d[0][1]), "r"(d[0][2]), "r"(d[0][3]), "r"(d[1][0]), "r"(d[1][1]), "r"(d[1][2]), "r"(d[1][3]),
@@ -981,7 +1025,7 @@ int plan_cluster(int tiles, int nch, int tokens, int group) {
 template <int NT, int TQ, int KIND>
 int launch_dense(DenseParams& p, int split, cudaStream_t stream) {
     static std::atomic<uint64_t> done{0};
-    if (!allow_smem(dense_kernel<NT, KIND, TQ>, DGeo<NT, TQ>::SMEM, done, true)) return check_launch();
+    if (!allow_smem(dense_kernel<NT, KIND, TQ>, DGeo<NT, TQ>::SMEM, done, KIND != D_ROWS)) return check_launch();
     const int nch = p.K / kChunkK;
     const int tiles = KIND == D_SILU ? p.N / 64 : (p.N + kTile - 1) / kTile;
     const int cs = split > 0 && split <= std::min(kMaxCluster, nch) ? split : plan_cluster(tiles, nch, p.M, TQ);
@@ -1089,23 +1133,29 @@ int run_chain(const ChainArgs& c, cudaStream_t st) {
 }
 
 template <int NT, int TQ>
-int run_matmul(const void* x, const void* w, const void* bias, void* y, int M, int N, int K, int* err, cudaStream_t st) {
+int run_matmul(const ChainMatmul& c, cudaStream_t st) {
     DenseParams p{};
-    const int rc = make_map_2d(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x, K, M, (uint64_t)K * 2, 64, NT, CU_TENSOR_MAP_SWIZZLE_128B,
-                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+    int rc = make_map_2d(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, c.x, c.K, c.M, (uint64_t)c.K * 2, 64, NT, CU_TENSOR_MAP_SWIZZLE_128B,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
     if (rc != B200_OK) return rc;
-    p.w[0] = static_cast<const unsigned char*>(w);
-    p.bias = static_cast<const __half*>(bias);
-    p.y = static_cast<__half*>(y);
-    p.M = p.mr = M; p.N = N; p.K = K; p.hd = 64; p.err = err;
-    return launch_dense<NT, TQ, D_PLAIN>(p, 0, st);
+    p.bias = static_cast<const __half*>(c.bias);
+    p.y = static_cast<__half*>(c.y);
+    p.M = p.mr = c.M; p.N = c.N; p.K = c.K; p.hd = 64; p.err = c.err;
+    if (c.scales == nullptr) {
+        p.w[0] = static_cast<const unsigned char*>(c.w);
+        return launch_dense<NT, TQ, D_PLAIN>(p, 0, st);
+    }
+    p.sc = static_cast<const __half*>(c.scales);
+    p.bi = static_cast<const __half*>(c.biases);
+    rc = make_map_2d(&p.wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, c.w, c.K / 2, c.N, c.K / 2, 64, kTile, CU_TENSOR_MAP_SWIZZLE_64B,
+                     CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+    return rc != B200_OK ? rc : launch_dense<NT, TQ, D_ROWS>(p, 0, st);
 }
 
 }  // namespace
 
-int chain_matmul(const void* x, const void* w, const void* bias, void* y, int M, int N, int K, int* err, cudaStream_t st) {
-    return M <= 8 ? run_matmul<16, 2>(x, w, bias, y, M, N, K, err, st)
-                  : (M <= 16 ? run_matmul<16, 4>(x, w, bias, y, M, N, K, err, st) : run_matmul<32, 4>(x, w, bias, y, M, N, K, err, st));
+int chain_matmul(const ChainMatmul& c, cudaStream_t st) {
+    return c.M <= 8 ? run_matmul<16, 2>(c, st) : (c.M <= 16 ? run_matmul<16, 4>(c, st) : run_matmul<32, 4>(c, st));
 }
 
 int forward_chain(const ChainArgs& a, cudaStream_t stream) { return a.d->M <= 8 ? run_chain<16, 2>(a, stream) : (a.d->M <= 16 ? run_chain<16, 4>(a, stream) : run_chain<32, 4>(a, stream)); }

@@ -5,6 +5,7 @@
 //
 // The kernel is csrc/qmm_gemm.cu.  (Up to 32 rows ran on mma.sync from registers before: 16 x 4096 x 14336 took 46 us there and
 // takes 18 us here, one row of 896 x 896 6.3 against 4.2 us; no size was left where it was ahead.)
+#include "decode.cuh"
 #include "qmm_common.cuh"
 #include "qmm_gemm.cuh"
 
@@ -73,6 +74,9 @@ int qmm_launch(const void* x, const uint32_t* wq, const void* scales, const void
     a.wq[1] = wq2; a.scales[1] = scales2; a.biases[1] = biases2;
     a.M = M; a.N = N; a.K = K; a.epilogue = epilogue;
     gemm_workspace(a, workspace, workspace_bytes);
+    if (epilogue == B200_EPI_NONE && a.err != nullptr && chain_matmul_wins(M, N, K, true) &&
+        ((reinterpret_cast<uintptr_t>(scales) | reinterpret_cast<uintptr_t>(biases)) & 3) == 0)
+        return chain_matmul({x, wq, scales, biases, bias, y, M, N, K, a.err}, stream);
     // (up to 32 rows no more than the built-in scratch holds, so that the allocation-free call cuts K the same way)
     if (M <= 32 && a.partial_bytes > kStaticScratchBytes - kCounterBytes) a.partial_bytes = kStaticScratchBytes - kCounterBytes;
     return qmm_gemm(a, stream);

@@ -91,12 +91,8 @@ int b200_qmm_tiled(const void* x, const void* wt, const void* wt2, const void* b
         !b200::aligned16(bias) || !b200::aligned16(extra) || !b200::aligned16(workspace))
         return B200_EALIGN;
     if (workspace_bytes < (size_t)b200::kCounterBytes) return B200_EWORKSPACE;
-    // Few chunks per SM: the kernel of the decode chain, whose clusters add up K without going through memory and whose CTAs are
-    // half as large.  (1024 x 4096: 6.2 -> 3.5 us, 8192 x 2048: 7.4 -> 5.1, 19200 x 256: 3.9 -> 3.6.)  Beyond ten or so its three
-    // groups of dequant warps stream less than the four of the other (2048 x 18944, 16 chunks: 9.8 against 10.9 us; 4096 x 14336,
-    // 24: the same; 19200 x 18944: 54 against 76).
-    if (epilogue == B200_EPI_NONE && (long long)((N + 127) / 128) * (K / b200::kChunkK) <= 1536)
-        return b200::chain_matmul(x, wt, bias, y, M, N, K, reinterpret_cast<int*>(static_cast<char*>(workspace) + b200::kCounterBytes - 4),
+    if (epilogue == B200_EPI_NONE && b200::chain_matmul_wins(M, N, K, false))
+        return b200::chain_matmul({x, wt, nullptr, nullptr, bias, y, M, N, K, static_cast<int*>(workspace) + b200::kMaxCounters - 1},
                                   static_cast<cudaStream_t>(stream));
     b200::GemmArgs a{};
     a.x = x; a.w_tiled = wt; a.w2_tiled = wt2; a.bias = bias; a.extra = extra; a.y = y;
