@@ -47,12 +47,17 @@ int b200_last_cuda_error(void);
  * predecessor drains and waits on the device before touching dependent data); 0 turns the launch
  * attribute off (plain stream order).  Process-wide; default on. */
 void b200_set_pdl(int enabled);
-/* Every device-side wait on another CTA or another GPU (grid barrier and all-GPU barrier of b200_forward,
- * the peer flags of b200_tp_argmax_combine) polls a bounded number of times, then sets an error word the host
- * can read and lets the kernel run to its end.  `polls` replaces the built-in limits (a few seconds) for
- * launches made after the call; 0 restores them.  Process-wide.  Meant for hosts that want a tighter
- * failure-detection time, and for testing the give-up path without a failing peer. */
+/* Every device-side wait polls a bounded number of times, then sets an error word the host can read.  `polls` (each up to
+ * about a microsecond) replaces the built-in limits, half a second to a few seconds, for launches made after the call; 0
+ * restores them.  It reaches the waits on another CTA or another GPU (grid barrier and all-GPU barrier of a shard's
+ * b200_forward, the peer flags of b200_tp_argmax_combine), after which the kernel runs to its end on what is there, and
+ * every wait of the kernels of an unsharded b200_forward and of the matmuls that share them, which go on waiting for some
+ * seconds before they end.  A graph keeps the limit it was made with.  Process-wide.  Meant for hosts that want a tighter
+ * failure-detection time, and for testing the error path without a failing peer. */
 void b200_set_wait_limit(unsigned int polls);
+/* A number that changes with every call of b200_set_pdl, b200_set_wait_limit and b200_forward_plan_hint: a host that keeps
+ * graphs of passes makes them anew when it has. */
+unsigned int b200_launch_settings(void);
 
 /* Bytes of scratch b200_qmm / b200_qmm_fused want for a given problem (split-K partial sums and
  * tile counters).  0 means the problem runs without scratch. */

@@ -66,6 +66,8 @@ def _declare(l: ctypes.CDLL) -> None:
     l.b200_set_pdl.argtypes = [i32]
     l.b200_set_wait_limit.restype = None
     l.b200_set_wait_limit.argtypes = [ctypes.c_uint]
+    l.b200_launch_settings.restype = ctypes.c_uint
+    l.b200_launch_settings.argtypes = []
     l.b200_qmm_workspace_bytes.restype = sz
     l.b200_qmm_workspace_bytes.argtypes = [i32, i32, i32]
     l.b200_qmm.restype = i32

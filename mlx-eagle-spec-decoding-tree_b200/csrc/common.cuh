@@ -29,9 +29,12 @@ inline int check_launch() {
 // kernel wrote and before its first global write.  0 disables the launch attribute.
 extern int g_use_pdl;
 
-// Poll limit of the device-side waits on other CTAs or other GPUs (grid barrier, all-GPU barrier, argmax
-// combine), set by b200_set_wait_limit; 0 = each kernel's built-in default (seconds).
+// Poll limit of the device-side waits, set by b200_set_wait_limit; 0 = each kernel's built-in default (seconds).
 extern unsigned g_wait_limit;
+extern std::atomic<unsigned> g_launch_settings;   // changes with each setting of the process
+
+// Of a kernel whose own limit is `built_in` and which takes no more than `most`.
+inline int wait_polls(uint32_t built_in, uint32_t most) { return (int)(g_wait_limit == 0 ? built_in : (g_wait_limit < most ? g_wait_limit : most)); }
 
 template <typename... KArgs, typename... Args>
 inline void launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,

@@ -14,7 +14,7 @@
 // rounding) and sums of h^2 per 32 columns; the consumer multiplies its fp32 accumulator by rsqrt(mean(h^2) + eps).
 // All other rounding points are those of the per-op kernels.
 //
-// Replaces Model.__call__ (mlx_llama.py:298-313) for <= 32 tokens.  Every wait is bounded; one that gives up sets the error
+// Replaces Model.__call__ (mlx_llama.py:298-313) for <= 32 tokens.  Every wait is bounded; one that runs out sets the error
 // word of the workspace and the kernel runs to its end.  No copy uses cluster multicast.
 #include <cuda.h>
 
@@ -44,6 +44,7 @@ constexpr int kTmem = 256;                       // columns a CTA takes: two CTA
 constexpr int kMaxCluster = 8;
 constexpr int kSsqPitch = 32, kCsPitch = 64, kKeyBlock = 64;
 constexpr uint32_t kDWaitPolls = 1u << 19;       // about a microsecond each
+constexpr uint32_t kDFirmPolls = 8 * kDWaitPolls;      // after which it is over all the same
 
 enum { D_QKV = 0, D_RESID = 1, D_SILU = 2, D_HEAD = 3, D_PLAIN = 4, D_ROWS = 5 };      // the last two: y = x W^T (+ bias), a matmul on its own; D_ROWS: W as quantised
 
@@ -78,6 +79,7 @@ struct DenseParams {
     int M, N, K;                  // N: output rows of each matrix
     int tile_lo, tiles;           // 128-row tiles (64 + 64 rows of gate and up): first and end
     int* err;
+    int polls;                    // of a wait before it gives up
     // D_QKV
     const float2* cs;             // [token][hd / 2] (cos, sin)
     __half* kc;                   // this layer's K and V of request 0
@@ -94,24 +96,19 @@ struct DenseParams {
     int rows_out;
 };
 
-// Bounded; once a wait of the CTA has given up (`abort`) the others do so at their next poll, and the kernel runs to its end on
-// whatever is there, in bounds, with the error word set.  No caller leaves its loop for it: the loops stay warp-uniform, so the
-// operands of copies and MMAs stay in uniform registers (eight MMAs and two commits: 290 cycles instead of 560).  Not unrolled:
-// a kernel of the chain mostly runs code for the first time, and every line of it costs.
-// After a wait that gave up: the CTA stays until the copies in flight have landed.
-__device__ __forceinline__ void settle() {
-#pragma unroll 1
-    for (int i = 0; i < 1000; i++) __nanosleep(1000);
-}
-template <bool SETTLE = false>
-__device__ __forceinline__ void dwait(uint32_t bar, uint32_t parity, volatile int* abort, int* err, int code) {
+// A wait that runs out of its polls sets the error word and goes on, for some seconds in all: what it waits for comes, since it
+// depends on nothing but copies, MMAs, kernels before this one and waits like it.  Nothing runs ahead of one: a ring whose one side
+// does not wait goes round twice, the other side then waits for a phase that has passed, and a CTA that left early would be stored
+// to by its cluster and written to by its copies.  So no caller looks at the outcome, and the loops stay warp-uniform, which keeps
+// the operands of copies and MMAs in uniform registers (eight MMAs and two commits: 290 cycles instead of 560).  Not unrolled: a
+// kernel of the chain mostly runs code for the first time, and every line of it costs (a flag in shared memory that let the CTA's
+// other waits give up too: 10 us of the 490 of a 0.5B-shape pass).
+__device__ __forceinline__ void dwait(uint32_t bar, uint32_t parity, int polls, int* err, int code) {
     bool ok = mbar_try_wait(bar, parity);
 #pragma unroll 1
-    for (uint32_t i = 0; !ok && i < kDWaitPolls && !*abort; i++) ok = mbar_try_wait(bar, parity);
-    if (!ok && !*abort) {
-        *abort = 1;
-        atomicCAS(err, 0, code);
-        if (SETTLE) settle();
+    for (int i = 0; !ok && i < (int)kDFirmPolls; i++) {
+        ok = mbar_try_wait(bar, parity);
+        if (i == polls) atomicCAS(err, 0, code);
     }
 }
 
@@ -156,17 +153,15 @@ __device__ __forceinline__ void st_async(uint32_t addr, const uint32_t* a, uint3
 __device__ __forceinline__ void arrive_peer(uint32_t bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
-// Phase 0, with what the peers stored before they arrived.  The limit is several times that of the other waits: a peer whose own
-// wait runs out still stores here, and must not find this CTA gone.
-__device__ __forceinline__ bool inbox_wait(uint32_t bar) {
+// Phase 0, with what the peers stored before they arrived; longer than their own waits take.
+__device__ __forceinline__ void inbox_wait(uint32_t bar, int polls, int* err, int code) {
+    uint32_t ok = 0;
 #pragma unroll 1
-    for (uint32_t i = 0; i < 4 * kDWaitPolls; i++) {
-        uint32_t ok;
+    for (int i = 0; !ok && i < 4 * (int)kDFirmPolls; i++) {
         asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n selp.u32 %0, 1, 0, p;\n}\n"
                      : "=r"(ok) : "r"(bar) : "memory");
-        if (ok) return true;
+        if (i == 4 * polls) atomicCAS(err, 0, code);
     }
-    return false;
 }
 __device__ __forceinline__ void st_peer2(uint32_t addr, float x, float y) {
     asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};\n" ::"r"(addr), "f"(x), "f"(y) : "memory");
@@ -190,7 +185,6 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
     V* inbox = reinterpret_cast<V*>(ring + G::INBOX);
     __shared__ uint64_t wfull[G::NW], wempty[G::NW], xfull[G::NX], xempty[G::NX], tready[kGroups], tfree[kGroups], accfull[2], accempty[2], inboxfull;
     __shared__ uint32_t s_tmem;
-    __shared__ int s_abort;
     __shared__ __align__(16) float s_rs[32];                                   // 1 / rms per token
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -216,7 +210,6 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
             mbar_init(smem_u32(accempty + lane), kEpi);
         }
         if (lane == 31) {
-            s_abort = 0;
             mbar_init(smem_u32(&inboxfull), 1);
             if (cs > 1) mbar_expect_tx(smem_u32(&inboxfull), cs * nq * kTile * TQ * 4); // what the cluster's CTAs will store here
         }
@@ -266,7 +259,6 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = s_tmem;
-    volatile int* abort_flag = &s_abort;
     pdl_launch_dependents();
     if (cs > 1) cluster_arrive();                                // (waited for before the first store to a peer)
 
@@ -282,7 +274,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
             const unsigned char *src0 = wsrc(tile, 0) + c0 * kRun, *src1 = wsrc(tile, 1) + c0 * kRun;
 #pragma unroll 1
             for (int c = c0; c < nc; c++) {
-                if (lap) dwait(smem_u32(wempty + slot), ph, abort_flag, p.err, 21);
+                if (lap) dwait(smem_u32(wempty + slot), ph, p.polls, p.err, 21);
                 __syncwarp();
                 if (elect_one()) {
                     if (KIND == D_ROWS) wload_rows(slot, tile, c);
@@ -302,7 +294,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         for (int it = 0; it < nit; it++)
 #pragma unroll 1
             for (int c = 0; c < nc; c++) {
-                if (lap) dwait(smem_u32(xempty + slot), ph, abort_flag, p.err, 26);
+                if (lap) dwait(smem_u32(xempty + slot), ph, p.polls, p.err, 26);
                 __syncwarp();
                 if (elect_one()) {
                     const uint32_t bar = smem_u32(xfull + slot), dst = smem_u32(ring + G::XOFF + slot * G::X);
@@ -321,11 +313,11 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
 #pragma unroll 1
         for (int it = 0; it < nit; it++) {
             const uint32_t ab = it & 1, d0 = tmem + G::ACC + ab * NT;
-            if (it >= 2) dwait(smem_u32(accempty + ab), ((it >> 1) - 1) & 1, abort_flag, p.err, 27);
+            if (it >= 2) dwait(smem_u32(accempty + ab), ((it >> 1) - 1) & 1, p.polls, p.err, 27);
 #pragma unroll 1
             for (int c = 0; c < nc; c++) {
-                dwait(smem_u32(xfull + slot), xph, abort_flag, p.err, 22);
-                dwait(smem_u32(tready + tl), tph, abort_flag, p.err, 22);
+                dwait(smem_u32(xfull + slot), xph, p.polls, p.err, 22);
+                dwait(smem_u32(tready + tl), tph, p.polls, p.err, 22);
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 __syncwarp();
                 if (elect_one()) {                               // (~285 cycles a batch; of half the size, 280)
@@ -349,7 +341,6 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         asm volatile("bar.sync 2, %0;\n" ::"n"((kEpi + 1) * 32) : "memory");         // accumulators read
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(kTmem) : "memory");
-        if (*abort_flag) settle();                                      // (this warp has nothing else to do while the last epilogue runs)
     } else if (warp == kDeq + 3) {
         // ------------------------------------------------------------------ sums of squares -> 1 / rms of each token
         // (by the dequant warps it held up every chunk behind the first three: 1.4 us at a hidden size of 3584)
@@ -421,7 +412,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
             }
             if (j0 < nq) ask(j0);
 
-            dwait(smem_u32(accfull + ab), (it >> 1) & 1, abort_flag, p.err, 23);
+            dwait(smem_u32(accfull + ab), (it >> 1) & 1, p.polls, p.err, 23);
             __syncwarp();
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             constexpr int C = NT / 2;                            // columns of this warp
@@ -459,7 +450,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                         st_async<TQ>(peer_addr(in0 + ((rank * qslots + sl) * kTile + r) * (TQ * 4), dst), a + i, peer_addr(inbar, dst));
                     if (++dst == cs) { dst = 0; sl++; }
                 }
-                if (!inbox_wait(inbar)) atomicCAS(p.err, 0, 28);     // (in full after a timeout too: a peer may still be storing here)
+                inbox_wait(inbar, p.polls, p.err, 28);
                 __syncwarp();
             }
             if (NORMED && it == 0) asm volatile("bar.sync 3, %0;\n" ::"n"((kEpi + 1) * 32) : "memory");      // s_rs
@@ -569,7 +560,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
 #pragma unroll 1
             do {
                 if (done < end) {
-                    dwait(smem_u32(wfull + slot), wph, abort_flag, p.err, 24);
+                    dwait(smem_u32(wfull + slot), wph, p.polls, p.err, 24);
                     __syncwarp();
                     const unsigned char* st = ring + slot * kW;
                     uint4 u[4];
@@ -584,7 +575,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                     }
                     const bool fast = __all_sync(0xffffffffu, fast_scale(sb.x) && fast_scale(sb.y));
                     if (lane == 0) mbar_arrive(smem_u32(wempty + slot));             // the packs are in registers
-                    if (done >= kGroups) dwait(smem_u32(tfree + me), tph, abort_flag, p.err, 24);
+                    if (done >= kGroups) dwait(smem_u32(tfree + me), tph, p.polls, p.err, 24);
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                     __syncwarp();
                     auto expand = [&](auto fast_tag) {
@@ -695,6 +686,7 @@ struct DAttn {
     int row0, req_rows, cap, write_off;    // cache row of (this layer, K, head 0), rows of one request's cache
     float scale_log2;
     int* err;
+    int polls;
 };
 
 __device__ __forceinline__ uint32_t kv_swz(int r, int v) {     // 16-byte vector v of row r of a block (boxes of 8 vectors side by side)
@@ -729,7 +721,6 @@ __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_co
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);
     __shared__ uint64_t full[G::STAGES], inboxfull;
-    __shared__ int s_abort;
     __shared__ float s_max[kAWarps / PT][PT][16];
     const uint32_t sbase = smem_u32(smem);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -738,7 +729,6 @@ __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_co
     const int req = blockIdx.z, hk = (int)blockIdx.y / p.sets, set = (int)blockIdx.y - hk * p.sets;
     if (threadIdx.x == 0) {
         asm volatile("prefetch.tensormap [%0];\n" ::"l"(&p.kvmap) : "memory");
-        s_abort = 0;
         for (int s = 0; s < G::STAGES; s++) mbar_init(smem_u32(full + s), 1);
         mbar_init(smem_u32(&inboxfull), cs * kAWarps);                         // every warp of the cluster
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -811,7 +801,7 @@ __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_co
 #pragma unroll 1
     for (int b = b0; b < b1; b++) {
         const int st = (b - b0) % G::STAGES;
-        dwait<true>(smem_u32(full + st), ((b - b0) / G::STAGES) & 1, &s_abort, p.err, 29);
+        dwait(smem_u32(full + st), ((b - b0) / G::STAGES) & 1, p.polls, p.err, 29);
         __syncwarp();
         if (busy) {
             const uint32_t sk = sbase + st * G::BLOCK, sv = sk + (HD / 64) * 8192;
@@ -937,7 +927,7 @@ __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_co
     }
     __syncwarp();
     if (lane < (int)cs) arrive_peer(peer_addr(smem_u32(&inboxfull), lane));
-    if (!inbox_wait(smem_u32(&inboxfull))) atomicCAS(p.err, 0, 25);
+    inbox_wait(smem_u32(&inboxfull), p.polls, p.err, 25);
     __syncwarp();
     // ---- merge: one warp per row, CTAs in key order
     const int row_lo = (int)rank * nslot, mine_rows = min(nslot, rows - row_lo);
@@ -1072,7 +1062,7 @@ int run_chain(const ChainArgs& c, cudaStream_t st) {
     if ((rc = xmap(&hw_map, d->hw, H)) || (rc = xmap(&attn_map, d->attn, nq)) || (rc = xmap(&act_map, d->act, I))) return rc;
 
     DenseParams p{};
-    p.ssq = c.ssq; p.H = H; p.eps = d->rms_eps; p.M = M; p.err = c.err;
+    p.ssq = c.ssq; p.H = H; p.eps = d->rms_eps; p.M = M; p.err = c.err; p.polls = wait_polls(kDWaitPolls, kDFirmPolls / 2);
     p.h = static_cast<__half*>(d->h); p.hw = static_cast<__half*>(d->hw);
     p.cs = c.cs; p.prefix = d->prefix; p.Hq = d->n_heads; p.Hkv = d->n_kv_heads; p.hd = hd; p.cap = d->cache_rows;
     p.write_off = d->write_off; p.mr = M / nreq;
@@ -1087,7 +1077,7 @@ int run_chain(const ChainArgs& c, cudaStream_t st) {
     a.out = static_cast<__half*>(d->attn); a.Hq = d->n_heads; a.Hkv = d->n_kv_heads; a.mr = p.mr; a.tail = d->tail;
     a.nkb = (d->cache_rows + kKeyBlock - 1) / kKeyBlock;
     a.req_rows = d->n_layers * 2 * d->n_kv_heads * d->cache_rows;
-    a.cap = d->cache_rows; a.write_off = d->write_off; a.scale_log2 = d->attn_scale * kLog2e; a.err = c.err;
+    a.cap = d->cache_rows; a.write_off = d->write_off; a.scale_log2 = d->attn_scale * kLog2e; a.err = c.err; a.polls = p.polls;
 
     const void* const* layers = c.layers;
     if (on(0)) {
@@ -1140,7 +1130,7 @@ int run_matmul(const ChainMatmul& c, cudaStream_t st) {
     if (rc != B200_OK) return rc;
     p.bias = static_cast<const __half*>(c.bias);
     p.y = static_cast<__half*>(c.y);
-    p.M = p.mr = c.M; p.N = c.N; p.K = c.K; p.hd = 64; p.err = c.err;
+    p.M = p.mr = c.M; p.N = c.N; p.K = c.K; p.hd = 64; p.err = c.err; p.polls = wait_polls(kDWaitPolls, kDFirmPolls / 2);
     if (c.scales == nullptr) {
         p.w[0] = static_cast<const unsigned char*>(c.w);
         return launch_dense<NT, TQ, D_PLAIN>(p, 0, st);

@@ -2211,7 +2211,10 @@ size_t b200_forward_tp_buffer_bytes(int hidden) {
            (size_t)2 * kMaxTp * 32 * hidden * sizeof(float);       // partial products, gather area, push slots
 }
 
-void b200_forward_plan_hint(const char* spec) { parse_plan_hint(spec); }
+void b200_forward_plan_hint(const char* spec) {
+    parse_plan_hint(spec);
+    g_launch_settings++;
+}
 
 size_t b200_forward_workspace_bytes(const b200_forward_desc* d) {
     if (!fwd_shape_ok(d)) return 0;

@@ -275,8 +275,17 @@ class _Graphs:
 
     def __init__(self):
         self._seen = collections.OrderedDict()           # descriptor -> [times, graph]
+        self._settings = 0                               # the process's, when they were made
+
+    def clear(self):
+        while self._seen:
+            _lib.lib().b200_graph_destroy(self._seen.popitem()[1][1])
 
     def get(self, desc, device):
+        settings = _lib.lib().b200_launch_settings()
+        if settings != self._settings:                   # (a graph keeps the poll limit, the plan and the launch attributes it was made with)
+            self.clear()
+            self._settings = settings
         key = bytes(desc)
         entry = self._seen.get(key)
         if entry is None:
@@ -295,8 +304,7 @@ class _Graphs:
 
     def __del__(self):
         try:
-            for entry in self._seen.values():
-                _lib.lib().b200_graph_destroy(entry[1])
+            self.clear()
         except Exception:                                # (interpreter shutdown)
             pass
 

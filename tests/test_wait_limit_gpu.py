@@ -73,3 +73,35 @@ def test_forward_all_gpu_barrier_gives_up_and_the_model_recovers(be, cuda, short
     again = whole(prompt[None], cache=whole.make_cache(128))
     whole.check_fused_error()
     assert torch.equal(again, want)
+
+
+@pytest.mark.parametrize("heads,kv,hd,inter", [(14, 2, 64, 4864), (16, 2, 128, 2176)])      # down_proj cut over clusters; 256 query rows per kv head
+def test_a_wait_of_the_kernel_chain_runs_out_is_reported_and_clears(be, cuda, heads, kv, hd, inter):
+    """A poll limit of one: the kernels of a pass start while the ones before them run, so waits for their activations run out.
+    The pass ends with its error word set (and, since what it waits for comes, with its result)."""
+    lib = be._lib.lib()
+    args = be.ModelArgs(model_type="qwen2", hidden_size=heads * hd, num_hidden_layers=3, intermediate_size=inter, num_attention_heads=heads,
+                        num_key_value_heads=kv, rms_norm_eps=1e-6, vocab_size=2048)
+    model = be.Model.random_init(args, seed=3, device=cuda, gen_device="cpu").relayout()
+    cache = model.make_cache(3584)
+    tokens = torch.arange(5, 37, dtype=torch.int32, device=cuda)[None]
+
+    def run(rows):
+        cache.offset = 3500
+        return model(tokens[:, :rows], cache)
+
+    for rows in (32, 8):
+        for _ in range(4 * model._graphs.AFTER):
+            want = run(rows)
+        assert any(g for _, g in model._graphs._seen.values())              # (replayed by now: the limit has to reach such passes too)
+        model.check_fused_error()
+        try:
+            lib.b200_set_wait_limit(1)
+            assert torch.equal(run(rows), want)
+            with pytest.raises(be._lib.B200Error, match="code 2[1-9]"):
+                model.check_fused_error()
+        finally:
+            lib.b200_set_wait_limit(0)
+        for _ in range(3):
+            assert torch.equal(run(rows), want)
+        model.check_fused_error()                                # clear again, and stays so
