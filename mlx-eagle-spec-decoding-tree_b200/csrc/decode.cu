@@ -43,8 +43,6 @@ constexpr int kTCols = kChunkK / 2;              // tensor-memory columns of an 
 constexpr int kTmem = 256;                       // columns a CTA takes: two CTAs share an SM
 constexpr int kMaxCluster = 8;
 constexpr int kSsqPitch = 32, kCsPitch = 64, kKeyBlock = 64;
-constexpr uint32_t kDWaitPolls = 1u << 19;       // about a microsecond each
-constexpr uint32_t kDFirmPolls = 8 * kDWaitPolls;      // after which it is over all the same
 
 enum { D_QKV = 0, D_RESID = 1, D_SILU = 2, D_HEAD = 3, D_PLAIN = 4, D_ROWS = 5 };      // the last two: y = x W^T (+ bias), a matmul on its own; D_ROWS: W as quantised
 
@@ -96,22 +94,6 @@ struct DenseParams {
     int rows_out;
 };
 
-// A wait that runs out of its polls sets the error word and goes on, for some seconds in all: what it waits for comes, since it
-// depends on nothing but copies, MMAs, kernels before this one and waits like it.  Nothing runs ahead of one: a ring whose one side
-// does not wait goes round twice, the other side then waits for a phase that has passed, and a CTA that left early would be stored
-// to by its cluster and written to by its copies.  So no caller looks at the outcome, and the loops stay warp-uniform, which keeps
-// the operands of copies and MMAs in uniform registers (eight MMAs and two commits: 290 cycles instead of 560).  Not unrolled: a
-// kernel of the chain mostly runs code for the first time, and every line of it costs (a flag in shared memory that let the CTA's
-// other waits give up too: 10 us of the 490 of a 0.5B-shape pass).
-__device__ __forceinline__ void dwait(uint32_t bar, uint32_t parity, int polls, int* err, int code) {
-    bool ok = mbar_try_wait(bar, parity);
-#pragma unroll 1
-    for (int i = 0; !ok && i < (int)kDFirmPolls; i++) {
-        ok = mbar_try_wait(bar, parity);
-        if (i == polls) atomicCAS(err, 0, code);
-    }
-}
-
 __device__ __forceinline__ uint64_t sw128(uint32_t saddr) {     // K-major, 128-byte swizzle: groups of 8 rows 1024 bytes apart
     return (uint64_t)((saddr & 0x3ffffu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
            ((uint64_t)2 << 61);
@@ -157,7 +139,7 @@ __device__ __forceinline__ void arrive_peer(uint32_t bar) {
 __device__ __forceinline__ void inbox_wait(uint32_t bar, int polls, int* err, int code) {
     uint32_t ok = 0;
 #pragma unroll 1
-    for (int i = 0; !ok && i < 4 * (int)kDFirmPolls; i++) {
+    for (int i = 0; !ok && i < 4 * kFirmPolls; i++) {
         asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n selp.u32 %0, 1, 0, p;\n}\n"
                      : "=r"(ok) : "r"(bar) : "memory");
         if (i == 4 * polls) atomicCAS(err, 0, code);
@@ -274,7 +256,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
             const unsigned char *src0 = wsrc(tile, 0) + c0 * kRun, *src1 = wsrc(tile, 1) + c0 * kRun;
 #pragma unroll 1
             for (int c = c0; c < nc; c++) {
-                if (lap) dwait(smem_u32(wempty + slot), ph, p.polls, p.err, 21);
+                if (lap) mbar_wait_reported(smem_u32(wempty + slot), ph, p.polls, p.err, 21);
                 __syncwarp();
                 if (elect_one()) {
                     if (KIND == D_ROWS) wload_rows(slot, tile, c);
@@ -294,7 +276,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         for (int it = 0; it < nit; it++)
 #pragma unroll 1
             for (int c = 0; c < nc; c++) {
-                if (lap) dwait(smem_u32(xempty + slot), ph, p.polls, p.err, 26);
+                if (lap) mbar_wait_reported(smem_u32(xempty + slot), ph, p.polls, p.err, 26);
                 __syncwarp();
                 if (elect_one()) {
                     const uint32_t bar = smem_u32(xfull + slot), dst = smem_u32(ring + G::XOFF + slot * G::X);
@@ -313,11 +295,11 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
 #pragma unroll 1
         for (int it = 0; it < nit; it++) {
             const uint32_t ab = it & 1, d0 = tmem + G::ACC + ab * NT;
-            if (it >= 2) dwait(smem_u32(accempty + ab), ((it >> 1) - 1) & 1, p.polls, p.err, 27);
+            if (it >= 2) mbar_wait_reported(smem_u32(accempty + ab), ((it >> 1) - 1) & 1, p.polls, p.err, 27);
 #pragma unroll 1
             for (int c = 0; c < nc; c++) {
-                dwait(smem_u32(xfull + slot), xph, p.polls, p.err, 22);
-                dwait(smem_u32(tready + tl), tph, p.polls, p.err, 22);
+                mbar_wait_reported(smem_u32(xfull + slot), xph, p.polls, p.err, 22);
+                mbar_wait_reported(smem_u32(tready + tl), tph, p.polls, p.err, 22);
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 __syncwarp();
                 if (elect_one()) {                               // (~285 cycles a batch; of half the size, 280)
@@ -412,7 +394,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
             }
             if (j0 < nq) ask(j0);
 
-            dwait(smem_u32(accfull + ab), (it >> 1) & 1, p.polls, p.err, 23);
+            mbar_wait_reported(smem_u32(accfull + ab), (it >> 1) & 1, p.polls, p.err, 23);
             __syncwarp();
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             constexpr int C = NT / 2;                            // columns of this warp
@@ -560,7 +542,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
 #pragma unroll 1
             do {
                 if (done < end) {
-                    dwait(smem_u32(wfull + slot), wph, p.polls, p.err, 24);
+                    mbar_wait_reported(smem_u32(wfull + slot), wph, p.polls, p.err, 24);
                     __syncwarp();
                     const unsigned char* st = ring + slot * kW;
                     uint4 u[4];
@@ -575,7 +557,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                     }
                     const bool fast = __all_sync(0xffffffffu, fast_scale(sb.x) && fast_scale(sb.y));
                     if (lane == 0) mbar_arrive(smem_u32(wempty + slot));             // the packs are in registers
-                    if (done >= kGroups) dwait(smem_u32(tfree + me), tph, p.polls, p.err, 24);
+                    if (done >= kGroups) mbar_wait_reported(smem_u32(tfree + me), tph, p.polls, p.err, 24);
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                     __syncwarp();
                     auto expand = [&](auto fast_tag) {
@@ -801,7 +783,7 @@ __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_co
 #pragma unroll 1
     for (int b = b0; b < b1; b++) {
         const int st = (b - b0) % G::STAGES;
-        dwait(smem_u32(full + st), ((b - b0) / G::STAGES) & 1, p.polls, p.err, 29);
+        mbar_wait_reported(smem_u32(full + st), ((b - b0) / G::STAGES) & 1, p.polls, p.err, 29);
         __syncwarp();
         if (busy) {
             const uint32_t sk = sbase + st * G::BLOCK, sv = sk + (HD / 64) * 8192;
@@ -1062,7 +1044,7 @@ int run_chain(const ChainArgs& c, cudaStream_t st) {
     if ((rc = xmap(&hw_map, d->hw, H)) || (rc = xmap(&attn_map, d->attn, nq)) || (rc = xmap(&act_map, d->act, I))) return rc;
 
     DenseParams p{};
-    p.ssq = c.ssq; p.H = H; p.eps = d->rms_eps; p.M = M; p.err = c.err; p.polls = wait_polls(kDWaitPolls, kDFirmPolls / 2);
+    p.ssq = c.ssq; p.H = H; p.eps = d->rms_eps; p.M = M; p.err = c.err; p.polls = wait_polls(kWaitPolls, kFirmPolls / 2);
     p.h = static_cast<__half*>(d->h); p.hw = static_cast<__half*>(d->hw);
     p.cs = c.cs; p.prefix = d->prefix; p.Hq = d->n_heads; p.Hkv = d->n_kv_heads; p.hd = hd; p.cap = d->cache_rows;
     p.write_off = d->write_off; p.mr = M / nreq;
@@ -1130,7 +1112,7 @@ int run_matmul(const ChainMatmul& c, cudaStream_t st) {
     if (rc != B200_OK) return rc;
     p.bias = static_cast<const __half*>(c.bias);
     p.y = static_cast<__half*>(c.y);
-    p.M = p.mr = c.M; p.N = c.N; p.K = c.K; p.hd = 64; p.err = c.err; p.polls = wait_polls(kDWaitPolls, kDFirmPolls / 2);
+    p.M = p.mr = c.M; p.N = c.N; p.K = c.K; p.hd = 64; p.err = c.err; p.polls = wait_polls(kWaitPolls, kFirmPolls / 2);
     if (c.scales == nullptr) {
         p.w[0] = static_cast<const unsigned char*>(c.w);
         return launch_dense<NT, TQ, D_PLAIN>(p, 0, st);

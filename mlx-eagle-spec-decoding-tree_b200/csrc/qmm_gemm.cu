@@ -24,8 +24,7 @@
 // an SM's share of HBM.
 //
 // Where the tiles alone would leave SMs idle the K range is cut across CTAs; the last CTA of a tile adds the fp32 partial
-// products in split order (deterministic).  Every wait is bounded; one that gives up sets the error word and the CTA runs
-// to its end (tensor memory is always freed).  No copy uses cluster multicast.
+// products in split order (deterministic).  Every wait is bounded; one that runs out sets the error word.  No copy uses cluster multicast.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -52,7 +51,6 @@ constexpr int kDeqWarps = 16;
 constexpr int kGroups = 4;                       // groups of four dequant warps, each with a tensor-memory tile of its own
 constexpr int kTileCols = kChunkK / 2;           // columns of a tile: two k values per column
 constexpr int kGThreads = (kDeqWarps + 4) * 32;  // + two producer warps + two MMA warps
-constexpr uint32_t kGemmWaitPolls = 1u << 19;    // about a microsecond each
 constexpr size_t kUmmaPartialBytes = 16u << 20;  // room for the partial products of a K split behind b200_qmm_umma
 constexpr int kGemmTiles = 896;                  // tiles that a K split can hand tickets to
 
@@ -88,13 +86,12 @@ struct GParams {
     __half* y;                   // [M][N]; float with B200_EPI_F32
     int* counter;                // split tickets, one per tile, zero between launches
     int* err;                    // error word or NULL
+    int polls;                   // of a wait before it sets that
     float* partial;
     int M, N, K;
     int row_items, tok_items, splits, chunks_per_split;
     int epilogue;
 };
-
-__device__ __forceinline__ bool gwait(uint32_t bar, uint32_t parity) { return mbar_wait(bar, parity, kGemmWaitPolls); }
 
 // K-major shared-memory matrix, 128-byte swizzle: rows of 128 bytes, groups of 8 rows 1024 bytes apart.
 __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
@@ -129,10 +126,6 @@ __device__ __forceinline__ void tmem_ld(uint32_t (&r)[C], uint32_t addr) {
 // True when the fp16 exponent field is in 1..10: the range of dequant_pack_fast.
 __device__ __forceinline__ bool fast_scale(uint32_t bits) { return ((bits >> 10) & 31u) - 1u < 10u; }
 
-__device__ __forceinline__ void g_error(const GParams& p, int code) {
-    if (p.err != nullptr) atomicCAS(p.err, 0, code);
-}
-
 struct GItem {
     int row_item, tok0, split, c_begin, nc;
 };
@@ -151,7 +144,7 @@ __device__ __forceinline__ GItem g_item(const GParams& p, int item, int NT) {
 // The epilogue of one item, by the dequant warps: warp w reads lanes 32 (w % 4) .. of column group w / 4.
 template <int S, int NT, bool DUAL>
 __device__ __forceinline__ void gemm_epilogue(const GParams& p, const GItem& g, uint32_t acc, uint32_t accempty, int warp,
-                                              int lane, int* s_last, bool ok) {
+                                              int lane, int* s_last) {
     constexpr int CG = (DUAL ? NT : S * NT) / 4;         // columns (of each matrix) per warp
     constexpr int CM = (DUAL || S == 1) ? 8 : 16;        // (two accumulators per column there)
     constexpr int CH = CG < CM ? CG : CM;                // columns per trip
@@ -172,7 +165,7 @@ __device__ __forceinline__ void gemm_epilogue(const GParams& p, const GItem& g, 
         // ---- partial products out: for every token column 32 consecutive floats per warp
         float* mine = ptile + (size_t)g.split * pstride + prow;
 #pragma unroll 1
-        for (int c0 = 0; c0 < ncol && ok; c0 += CH) {
+        for (int c0 = 0; c0 < ncol; c0 += CH) {
             uint32_t a[CH], b[CH];
             tmem_ld<CH>(a, lane_base + (DUAL ? 0 : s * NT) + col0 + c0);
             if (DUAL || both) tmem_ld<CH>(b, lane_base + NT + col0 + c0);
@@ -204,7 +197,6 @@ __device__ __forceinline__ void gemm_epilogue(const GParams& p, const GItem& g, 
         consumer_sync(kDeqWarps * 32);                  // read by all before the next item rewrites it
         if (!last) return;
     }
-    if (!ok) return;
     const bool row_ok = row < p.N;
     const __half bv = (p.bias != nullptr && row_ok) ? p.bias[row] : __ushort_as_half(0);
     const bool resid = p.epilogue == B200_EPI_RESIDUAL;
@@ -293,7 +285,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
     unsigned char* ring = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);
     __shared__ uint64_t s_bars[2 * 8 + 2 * kGroups + 4];
     __shared__ uint32_t s_tmem;
-    __shared__ int s_abort, s_last;
+    __shared__ int s_last;
     uint64_t* pfull = s_bars;                        // stage landed            (producer -> dequant warps, MMA warp)
     uint64_t* pempty = pfull + G::NP;                // stage read              (S groups of warps + the MMAs -> producer)
     uint64_t* tready = pempty + G::NP;               // tile expanded           (a group's 4 warps -> MMA warp)
@@ -305,7 +297,6 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
     const int nitems = p.row_items * p.tok_items * p.splits;
 
     if (threadIdx.x == 0) {
-        s_abort = 0;
         for (int s = 0; s < G::NP; s++) {
             mbar_init(smem_u32(pfull + s), 1);
             mbar_init(smem_u32(pempty + s), 4 * S + S);
@@ -328,7 +319,10 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = s_tmem;
-    volatile int* abort_flag = &s_abort;
+    auto gwait = [&](const uint64_t* bar, uint32_t parity, int code) {
+        mbar_wait_reported(smem_u32(bar), parity, p.polls, p.err, code);
+        __syncwarp();
+    };
     pdl_launch_dependents();
 
     if (warp >= kDeqWarps && warp < kDeqWarps + 2) {
@@ -340,13 +334,12 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
         if (waited) pdl_wait();
         uint32_t n = 0;                              // chunks of earlier items
         uint32_t pend = 0;                           // stages of this warp whose activations are still to be asked for
-        bool ok = true;
         auto load_x = [&](uint32_t s, int c, int tok0) {
             const uint32_t dst = smem_u32(ring + s * G::STAGE + S * kTileW), bar = smem_u32(pfull + s);
             tma_box(dst, &p.xmap, c * kChunkK, tok0, bar);
             tma_box(dst + NT * 128, &p.xmap, c * kChunkK + 64, tok0, bar);
         };
-        for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
+        for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
             const GItem g = g_item(p, item, NT);
             int c = (int)((par - n) & 1u);
             // the item's 64-row blocks, one run of 4608 bytes each per chunk (gate blocks, then up blocks)
@@ -357,12 +350,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
                           ((size_t)min(DUAL ? g.row_item * 2 + (i & 1) : g.row_item * 2 * S + i, nblocks - 1) * nchunks + g.c_begin + c) * kRunBytes;
             for (; c < g.nc; c += 2) {
                 const uint32_t slot = (n + c) % G::NP, use = (n + c) / G::NP;
-                if (*abort_flag) { ok = false; break; }
-                if (use > 0 && !__all_sync(0xffffffffu, gwait(smem_u32(pempty + slot), (use - 1) & 1u))) {
-                    if (lane == 0) { *abort_flag = 1; g_error(p, 1); }
-                    ok = false;
-                    break;
-                }
+                if (use > 0) gwait(pempty + slot, (use - 1) & 1u, 1);
                 const uint32_t bar = smem_u32(pfull + slot);
                 unsigned char* stage = ring + slot * G::STAGE;
                 if (elect_one()) {
@@ -404,20 +392,18 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
         const uint32_t me = __shfl_sync(0xffffffffu, warp - (kDeqWarps + 2), 0);
         const uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(kTileRows >> 4) << 24);
         uint32_t n = 0, it = 0;                          // chunks of earlier items, items
-        bool ok = true;
-        for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x, it++) {
+        for (int item = blockIdx.x; item < nitems; item += gridDim.x, it++) {
             const GItem g = g_item(p, item, NT);
             const uint32_t ab = it % G::NACC, ause = it / G::NACC;
-            if (ause > 0) ok = __all_sync(0xffffffffu, gwait(smem_u32(accempty + ab), (ause - 1) & 1u));
+            if (ause > 0) gwait(accempty + ab, (ause - 1) & 1u, 2);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t d0 = tmem + G::ACC0 + ab * G::ACC + me * NT;
             bool first = true;
-            for (int c = S == 2 ? 0 : (int)me; c < g.nc && ok; c += S == 2 ? 1 : 2) {
+            for (int c = S == 2 ? 0 : (int)me; c < g.nc; c += S == 2 ? 1 : 2) {
                 const uint32_t tile = (n + c) * S + (S == 2 ? me : 0);            // tile number: group and use of its tensor-memory tile
                 const uint32_t ts = tile % kGroups, slot = (n + c) % G::NP;
                 // (the expanded tile is ready only after its group has seen the whole stage land, the activations included)
-                ok = __all_sync(0xffffffffu, !*abort_flag && gwait(smem_u32(tready + ts), (tile / kGroups) & 1u));
-                if (!ok) break;
+                gwait(tready + ts, (tile / kGroups) & 1u, 2);
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 const uint64_t b0 = sw128_desc(smem_u32(ring + slot * G::STAGE + S * kTileW));
                 const uint32_t a0 = tmem + ts * kTileCols;
@@ -436,12 +422,11 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
                 __syncwarp();
                 first = false;
             }
-            if (ok && elect_one())
+            if (elect_one())
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(accfull + ab)) : "memory");
             __syncwarp();
             n += g.nc;
         }
-        if (!ok && lane == 0 && !*abort_flag) { *abort_flag = 1; g_error(p, 2); }
     } else {
         // ------------------------------------------------------------------ dequant warps + epilogue
         const int q = warp & 3;
@@ -469,14 +454,13 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
         };
         if (LAYOUT == W_ROWS) pdl_wait();                 // (the kernel before this one may have written the weights)
         uint32_t cbase = 0, tbase = 0, tuse = 0, it = 0;  // chunks and tiles of earlier items, tiles of this group so far, items
-        bool ok = true, pending = false;
+        bool pending = false;
         GItem prev{};
         auto epilogue = [&]() {
             const uint32_t ab = (it - 1) % G::NACC;
-            ok = __all_sync(0xffffffffu, ok && !*abort_flag && gwait(smem_u32(accfull + ab), ((it - 1) / G::NACC) & 1u));
+            gwait(accfull + ab, ((it - 1) / G::NACC) & 1u, 3);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            // (after a timeout too: the warps meet on the same named barriers whatever each of them has seen)
-            gemm_epilogue<S, NT, DUAL>(p, prev, tmem + G::ACC0 + ab * G::ACC, smem_u32(accempty + ab), warp, lane, &s_last, ok);
+            gemm_epilogue<S, NT, DUAL>(p, prev, tmem + G::ACC0 + ab * G::ACC, smem_u32(accempty + ab), warp, lane, &s_last);
             pending = false;
         };
         for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
@@ -487,71 +471,68 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
             for (uint32_t k = k0; k < ntiles; k += kGroups, tuse++) {
                 const uint32_t n = cbase + k / S, s = k % S;
                 const uint32_t slot = n % G::NP;
-                ok = ok && !*abort_flag && gwait(smem_u32(pfull + slot), (n / G::NP) & 1u);
-                if (ok && tuse > 0) ok = gwait(smem_u32(tfree + grp), (tuse - 1) & 1u);
-                ok = __all_sync(0xffffffffu, ok);
-                if (ok) {
-                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                    const unsigned char* tile = ring + slot * G::STAGE + s * kTileW;
-                    uint4 u[4];
-                    uint32_t sc2[2], bi2[2];              // scale, bias of the chunk's two k groups, low halves
-                    if (LAYOUT == W_TILED) {
-                        // rows are 64 bytes apart: every other pair of rows reads its 16-byte units in the other order, so that
-                        // eight lanes meet in the same banks in pairs only
-                        const int flip = (r >> 1) & 1;
+                gwait(pfull + slot, (n / G::NP) & 1u, 3);
+                if (tuse > 0) gwait(tfree + grp, (tuse - 1) & 1u, 3);
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const unsigned char* tile = ring + slot * G::STAGE + s * kTileW;
+                uint4 u[4];
+                uint32_t sc2[2], bi2[2];              // scale, bias of the chunk's two k groups, low halves
+                if (LAYOUT == W_TILED) {
+                    // rows are 64 bytes apart: every other pair of rows reads its 16-byte units in the other order, so that
+                    // eight lanes meet in the same banks in pairs only
+                    const int flip = (r >> 1) & 1;
 #pragma unroll
-                        for (int i = 0; i < 4; i += 2) {
-                            const uint4 a = *reinterpret_cast<const uint4*>(tile + rowoff + (i + flip) * 16);
-                            const uint4 b = *reinterpret_cast<const uint4*>(tile + rowoff + (i + 1 - flip) * 16);
-                            u[i] = flip ? b : a;
-                            u[i + 1] = flip ? a : b;
-                        }
-                        const uint2 sb = *reinterpret_cast<const uint2*>(tile + scoff);
-                        sc2[0] = sb.x; bi2[0] = sb.x >> 16;
-                        sc2[1] = sb.y; bi2[1] = sb.y >> 16;
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 4; i++)
-                            u[i] = *reinterpret_cast<const uint4*>(tile + rowoff + ((i ^ ((r >> 1) & 3)) << 4));
-                        const uint32_t sv = sb_s, bv = sb_b;
-                        if (k + kGroups < ntiles) load_sb(g, k + kGroups);
-                        sc2[0] = sv; sc2[1] = sv >> 16;
-                        bi2[0] = bv; bi2[1] = bv >> 16;
+                    for (int i = 0; i < 4; i += 2) {
+                        const uint4 a = *reinterpret_cast<const uint4*>(tile + rowoff + (i + flip) * 16);
+                        const uint4 b = *reinterpret_cast<const uint4*>(tile + rowoff + (i + 1 - flip) * 16);
+                        u[i] = flip ? b : a;
+                        u[i + 1] = flip ? a : b;
                     }
-                    const bool fast = __all_sync(0xffffffffu, fast_scale(sc2[0]) && fast_scale(sc2[1]));
-                    auto expand = [&](auto fast_tag) {
-                        constexpr bool FAST = decltype(fast_tag)::value;
-                        // sixteen columns (32 k values) at a time.  Streaming layout: pack j of unit t is k group 4 j + t;
-                        // row-major: pack t of unit j.
+                    const uint2 sb = *reinterpret_cast<const uint2*>(tile + scoff);
+                    sc2[0] = sb.x; bi2[0] = sb.x >> 16;
+                    sc2[1] = sb.y; bi2[1] = sb.y >> 16;
+                } else {
 #pragma unroll
-                        for (int j = 0; j < 4; j++) {
-                            __half2 s2 = dup_half((unsigned short)sc2[j >> 1]);
-                            const __half2 b2 = dup_half((unsigned short)bi2[j >> 1]);
-                            if (FAST) s2 = scale_times_2_20(s2);
-                            uint32_t d[4][4];
-#pragma unroll
-                            for (int t = 0; t < 4; t++) {
-                                const uint32_t pack = LAYOUT == W_TILED ? comp(u[t], j) : comp(u[j], t);
-                                if (FAST) dequant_pack_fast(pack, s2, b2, d[t]);
-                                else dequant_pack(pack, s2, b2, d[t]);
-                                if (LAYOUT == W_ROWS) {   // {e0,e4} {e1,e5} {e2,e6} {e3,e7} -> adjacent k pairs
-                                    const uint32_t e01 = __byte_perm(d[t][0], d[t][1], 0x5410), e45 = __byte_perm(d[t][0], d[t][1], 0x7632);
-                                    const uint32_t e23 = __byte_perm(d[t][2], d[t][3], 0x5410), e67 = __byte_perm(d[t][2], d[t][3], 0x7632);
-                                    d[t][0] = e01; d[t][1] = e23; d[t][2] = e45; d[t][3] = e67;
-                                }
-                            }
-                            tmem_st16(trow + 16 * j, d);
-                        }
-                    };
-                    if (fast) expand(std::true_type{});
-                    else expand(std::false_type{});
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(smem_u32(pempty + slot));       // the packs are in registers
-                    asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
-                    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(smem_u32(tready + grp));
+                    for (int i = 0; i < 4; i++)
+                        u[i] = *reinterpret_cast<const uint4*>(tile + rowoff + ((i ^ ((r >> 1) & 3)) << 4));
+                    const uint32_t sv = sb_s, bv = sb_b;
+                    if (k + kGroups < ntiles) load_sb(g, k + kGroups);
+                    sc2[0] = sv; sc2[1] = sv >> 16;
+                    bi2[0] = bv; bi2[1] = bv >> 16;
                 }
+                const bool fast = __all_sync(0xffffffffu, fast_scale(sc2[0]) && fast_scale(sc2[1]));
+                auto expand = [&](auto fast_tag) {
+                    constexpr bool FAST = decltype(fast_tag)::value;
+                    // sixteen columns (32 k values) at a time.  Streaming layout: pack j of unit t is k group 4 j + t;
+                    // row-major: pack t of unit j.
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        __half2 s2 = dup_half((unsigned short)sc2[j >> 1]);
+                        const __half2 b2 = dup_half((unsigned short)bi2[j >> 1]);
+                        if (FAST) s2 = scale_times_2_20(s2);
+                        uint32_t d[4][4];
+#pragma unroll
+                        for (int t = 0; t < 4; t++) {
+                            const uint32_t pack = LAYOUT == W_TILED ? comp(u[t], j) : comp(u[j], t);
+                            if (FAST) dequant_pack_fast(pack, s2, b2, d[t]);
+                            else dequant_pack(pack, s2, b2, d[t]);
+                            if (LAYOUT == W_ROWS) {   // {e0,e4} {e1,e5} {e2,e6} {e3,e7} -> adjacent k pairs
+                                const uint32_t e01 = __byte_perm(d[t][0], d[t][1], 0x5410), e45 = __byte_perm(d[t][0], d[t][1], 0x7632);
+                                const uint32_t e23 = __byte_perm(d[t][2], d[t][3], 0x5410), e67 = __byte_perm(d[t][2], d[t][3], 0x7632);
+                                d[t][0] = e01; d[t][1] = e23; d[t][2] = e45; d[t][3] = e67;
+                            }
+                        }
+                        tmem_st16(trow + 16 * j, d);
+                    }
+                };
+                if (fast) expand(std::true_type{});
+                else expand(std::false_type{});
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(pempty + slot));       // the packs are in registers
+                asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(tready + grp));
                 // the item before this one: its epilogue runs once this warp's first tile of this item is expanded
                 if (pending) epilogue();
             }
@@ -564,7 +545,6 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
             if (it == 1) pdl_wait();                      // before this thread's first global access
         }
         if (pending) epilogue();
-        if (!ok && lane == 0 && !*abort_flag) { *abort_flag = 1; g_error(p, 3); }
     }
 
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -678,6 +658,7 @@ int qmm_gemm(const GemmArgs& a, cudaStream_t stream) {
     p.y = static_cast<__half*>(a.y);
     p.counter = a.counters;
     p.err = a.err;
+    p.polls = wait_polls(kWaitPolls, kFirmPolls / 2);
     p.partial = static_cast<float*>(a.partial);
     p.M = a.M; p.N = a.N; p.K = a.K;
     p.row_items = pl.row_items; p.tok_items = pl.tok_items; p.splits = pl.splits; p.chunks_per_split = pl.cps;

@@ -1,4 +1,4 @@
-"""A device-side wait that runs out: the kernel gives up by itself, the host reads an error status, a reset
+"""A device-side wait that runs out: the kernel ends by itself, the host reads an error status, a reset
 restores service.  The waits are made to run out by giving them a short poll limit (``b200_set_wait_limit``) and
 a peer that never answers (a second buffer on the same GPU whose flags nobody raises): nothing faults, nothing
 hangs, no process dies."""
@@ -105,3 +105,37 @@ def test_a_wait_of_the_kernel_chain_runs_out_is_reported_and_clears(be, cuda, he
         for _ in range(3):
             assert torch.equal(run(rows), want)
         model.check_fused_error()                                # clear again, and stays so
+
+
+@pytest.mark.parametrize("m,n,k,epilogue", [(16, 4096, 512, 0), (100, 2048, 4096, 0), (40, 1024, 2048, 2)])
+def test_a_wait_of_a_matmul_runs_out_is_reported_and_clears(be, cuda, m, n, k, epilogue):
+    """The matmul starts on free SMs while one of a single long tile still runs, and waits for it before its activations."""
+    lib, p, st = be._lib.lib(), be._lib.ptr, be._lib.stream_ptr(cuda)
+    g = torch.Generator(device=cuda).manual_seed(m)
+
+    def operands(rows, outs, width):
+        w = be.quantize.quantize(torch.randn(outs, width, generator=g, device=cuda) * 0.02)
+        ws = torch.zeros(lib.b200_qmm_gemm_workspace_bytes(rows, outs, width, epilogue), dtype=torch.uint8, device=cuda)
+        return (torch.randn(rows, width, generator=g, device=cuda).half(), be.qmm_kernel.relayout(*w), be.qmm_kernel.relayout(*w),
+                torch.empty(rows, outs, dtype=torch.float16, device=cuda), ws)
+
+    def call(o, shape, epi, room):
+        assert lib.b200_qmm_gemm(p(o[0]), p(o[1]), p(o[2]) if epi == 2 else None, None, None, p(o[3]), *shape, epi, p(o[4]), room, st) == 0
+
+    long_, mine = operands(16, 128, 65536), operands(m, n, k)
+    call(mine, (m, n, k), epilogue, mine[4].numel())
+    want = mine[3].clone()
+    error = lambda: int(mine[4][4092:4096].view(torch.int32))
+    assert error() == 0
+    try:
+        lib.b200_set_wait_limit(1)
+        call(long_, (16, 128, 65536), 0, 4096)                   # (no cut of K: one CTA)
+        call(mine, (m, n, k), epilogue, mine[4].numel())
+        assert error() in (1, 2, 3)
+    finally:
+        lib.b200_set_wait_limit(0)
+    assert torch.equal(mine[3], want)
+    mine[4][4092:4096].zero_()
+    call(mine, (m, n, k), epilogue, mine[4].numel())
+    assert torch.equal(mine[3], want)
+    assert int(mine[4][:4096].view(torch.int32).abs().sum()) == 0            # tickets restored, no wait ran out
