@@ -624,13 +624,24 @@ class Model:
             self.timeline = None
 
     def check_fused_error(self):
-        """Raise if a bounded wait inside ``b200_forward`` ever gave up (synchronises)."""
-        if self._fwd_ws is None:
-            return
-        code = int(self._fwd_ws[:16].view(torch.int32)[2])
-        if code != 0:
-            self._fwd_ws[:4352].zero_()
-            raise _lib.B200Error(f"b200_forward: a bounded wait gave up inside the kernel (code {code})")
+        """Raise if a bounded wait inside ``b200_forward``, ``b200_prefill`` or a matmul of the per-op path ever ran out
+        (synchronises)."""
+        if self._fwd_ws is not None:
+            code = int(self._fwd_ws[:16].view(torch.int32)[2])
+            if code != 0:
+                self._fwd_ws[:4352].zero_()
+                raise _lib.B200Error(f"b200_forward: a bounded wait gave up inside the kernel (code {code})")
+        if self._pf_buf is not None:
+            word = self._pf_buf["ws"][4092:4096].view(torch.int32)
+            code = int(word)
+            if code != 0:
+                word.zero_()
+                raise _lib.B200Error(f"b200_prefill: a bounded wait ran out inside a matmul (code {code})")
+        if not self.can_fuse():
+            code = qk.stream_error(self.device)
+            if code != 0:
+                qk.workspace(self.device)[4092:4096].zero_()
+                raise _lib.B200Error(f"a bounded wait ran out inside a matmul (code {code})")
         if self.tp is not None:
             self.tp.check_error()
 

@@ -107,6 +107,33 @@ def test_a_wait_of_the_kernel_chain_runs_out_is_reported_and_clears(be, cuda, he
         model.check_fused_error()                                # clear again, and stays so
 
 
+def test_a_wait_of_a_prompt_pass_runs_out_is_reported_and_clears(be, cuda):
+    """The gate / up matmul of these sizes leaves twenty SMs free, on which the next one starts and waits for it."""
+    lib = be._lib.lib()
+    args = be.ModelArgs(model_type="llama", hidden_size=2048, num_hidden_layers=2, intermediate_size=2048, num_attention_heads=16,
+                        num_key_value_heads=2, rms_norm_eps=1e-5, vocab_size=2048)
+    model = be.Model.random_init(args, 5, cuda).relayout()
+    cache = model.make_cache(1024)
+    tokens = torch.randint(0, args.vocab_size, (1, 1000), generator=torch.Generator().manual_seed(1))
+
+    def run():
+        cache.offset = 0
+        return model(tokens, cache)
+
+    want = run()
+    model.check_fused_error()
+    try:
+        lib.b200_set_wait_limit(1)
+        torch.cuda._sleep(4_000_000)                             # (2 ms in which the host gets ahead: the kernels then follow at once)
+        assert torch.equal(run(), want)
+        with pytest.raises(be._lib.B200Error, match="b200_prefill"):
+            model.check_fused_error()
+    finally:
+        lib.b200_set_wait_limit(0)
+    assert torch.equal(run(), want)
+    model.check_fused_error()
+
+
 @pytest.mark.parametrize("m,n,k,epilogue", [(16, 4096, 512, 0), (100, 2048, 4096, 0), (40, 1024, 2048, 2)])
 def test_a_wait_of_a_matmul_runs_out_is_reported_and_clears(be, cuda, m, n, k, epilogue):
     """The matmul starts on free SMs while one of a single long tile still runs, and waits for it before its activations."""
