@@ -42,7 +42,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
 }
 constexpr int kWaitPolls = 1 << 19;             // of a wait before it reports: half a second
 constexpr int kFirmPolls = 8 * kWaitPolls;      // after which it is over all the same
-// A wait that runs out of its polls sets the error word (if there is one) and goes on, for some seconds in all: what it waits for
+constexpr int kNoReport = kFirmPolls;
+// A wait that runs out of its polls sets the error word (kNoReport: there is none) and goes on, for some seconds in all: what it waits for
 // comes, since it depends on nothing but copies, MMAs, kernels before this one and waits like it.  Nothing runs ahead of one: a ring
 // whose one side does not wait goes round twice, the other side then waits for a phase that has passed, and a CTA that left early
 // would be stored to by its cluster and written to by its copies.  So no caller looks at the outcome, and the loops stay
@@ -54,7 +55,7 @@ __device__ __forceinline__ void mbar_wait_reported(uint32_t bar, uint32_t parity
 #pragma unroll 1
     for (int i = 0; !ok && i < kFirmPolls; i++) {
         ok = mbar_try_wait(bar, parity);
-        if (i == polls && err != nullptr) atomicCAS(err, 0, code);
+        if (i == polls) atomicCAS(err, 0, code);
     }
 }
 // One lane of a converged warp.  A branch on this keeps the compiler's knowledge that everything else is warp-uniform, so the

@@ -86,7 +86,7 @@ struct GParams {
     __half* y;                   // [M][N]; float with B200_EPI_F32
     int* counter;                // split tickets, one per tile, zero between launches
     int* err;                    // error word or NULL
-    int polls;                   // of a wait before it sets that
+    int polls;                   // of a wait before it sets that (kNoReport without one)
     float* partial;
     int M, N, K;
     int row_items, tok_items, splits, chunks_per_split;
@@ -658,7 +658,7 @@ int qmm_gemm(const GemmArgs& a, cudaStream_t stream) {
     p.y = static_cast<__half*>(a.y);
     p.counter = a.counters;
     p.err = a.err;
-    p.polls = wait_polls(kWaitPolls, kFirmPolls / 2);
+    p.polls = a.err != nullptr ? wait_polls(kWaitPolls, kFirmPolls / 2) : kNoReport;
     p.partial = static_cast<float*>(a.partial);
     p.M = a.M; p.N = a.N; p.K = a.K;
     p.row_items = pl.row_items; p.tok_items = pl.tok_items; p.splits = pl.splits; p.chunks_per_split = pl.cps;
