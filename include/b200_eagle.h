@@ -287,9 +287,9 @@ typedef struct b200_forward_desc {
                             /* kind k (0 embedding, 1 qkv, 2 attention, 3 merge, 4 o_proj, 5 gate/up,      */
                             /* 6 down_proj, 7 vocabulary projection); results are then meaningless         */
                             /* Without tensor parallelism timeline_pitch = B200_LAYERS_ON_HOST makes timeline  */
-                            /* a HOST copy of layer_table, read during the call.  Otherwise the call reads     */
-                            /* layer_table back first, which waits for the stream (inside a capture: for       */
-                            /* nothing, the table must be complete then)                                       */
+                            /* a HOST copy of layer_table, read during the call (NULL is refused).  Otherwise  */
+                            /* the kernels read layer_table, which puts the load of a pointer ahead of their   */
+                            /* first weights                                                                   */
     /* Tensor parallelism over the GPUs of one node (tp_world <= 1 = off, all fields below zero).  The call
      * then runs shard tp_rank of tp_world: n_heads, n_kv_heads and intermediate are this shard's counts
      * (heads and MLP rows cut evenly; o_proj / down_proj weights hold this shard's K columns), head_rows

@@ -87,12 +87,22 @@ struct DenseParams {
     size_t req_stride;            // halves between the caches of two requests
     // D_ROWS: packs [N][K / 8] as rows of bytes, boxes of 64 bytes x 128 rows, 64-byte swizzle; scales and biases [N][K / 64]
     CUtensorMap wmap;
-    const __half* sc;
-    const __half* bi;
+    union {
+        const __half* sc;
+        const void* const* tw;    // TABLE: weights (gate, then up) in a layer table in device memory, for callers without a copy of it on the host
+    };
+    union {
+        const __half* bi;
+        const void* const* tv;    // TABLE: bias (D_QKV), norm weights (D_RESID) there; NULL: as given above
+    };
     // D_HEAD
     const int* row_index;
     int rows_out;
 };
+template <typename T>
+__device__ __forceinline__ const T* listed(const void* const* entry) {
+    return reinterpret_cast<const T*>(__ldcg(reinterpret_cast<const unsigned long long*>(entry)));
+}
 
 __device__ __forceinline__ uint64_t sw128(uint32_t saddr) {     // K-major, 128-byte swizzle: groups of 8 rows 1024 bytes apart
     return (uint64_t)((saddr & 0x3ffffu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
@@ -158,7 +168,7 @@ __device__ __forceinline__ void st_peer2(uint32_t addr, float x, float y) {
 // follows in order.  Three chunks are expanded before the wait for the previous kernel: behind it
 // come the activation load (0.5 us), the MMAs (0.1 us a chunk) and the epilogue.  Code that runs once per kernel is kept short:
 // cold instructions cost 2 to 4 cycles each.
-template <int NT, int KIND, int TQ>
+template <int NT, int KIND, int TQ, bool TABLE = false>
 __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_constant__ DenseParams p) {
     using G = DGeo<NT, TQ>;
     using V = Vec<TQ>;
@@ -200,8 +210,8 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
     // The weight producer makes its own barriers and asks for the first stages before the block is set up.
     const int nblocks = (p.N + 63) / 64;
     auto wsrc = [&](int tile, int second) {                      // chunk c_lo of the tile's first or second 64 rows (gate / up: of the same rows of each)
-        return KIND == D_SILU ? p.w[second] + ((size_t)tile * nchunks + c_lo) * kRun
-                              : p.w[0] + ((size_t)min(2 * tile + second, nblocks - 1) * nchunks + c_lo) * kRun;
+        const unsigned char* w = TABLE ? listed<unsigned char>(p.tw + (KIND == D_SILU ? second : 0)) : p.w[KIND == D_SILU ? second : 0];
+        return w + ((size_t)(KIND == D_SILU ? tile : min(2 * tile + second, nblocks - 1)) * nchunks + c_lo) * kRun;
     };
     auto wload = [&](uint32_t slot, const unsigned char* src0, const unsigned char* src1) {
         const uint32_t bar = smem_u32(wfull + slot), dst = smem_u32(ring + slot * kW);
@@ -361,6 +371,8 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         // (Four threads of a quarter-warp read the same banks: swapping units between threads to halve that took more issue slots, 16
         // selects a chunk, than the reads took cycles.)
         constexpr bool NORMED = KIND != D_RESID && KIND != D_PLAIN && KIND != D_ROWS;                 // the input is h * w_norm: scale by 1 / rms
+        const __half* const wn = TABLE && KIND == D_RESID && p.tv != nullptr ? listed<__half>(p.tv) : p.wn;
+        const __half* const bias = TABLE && KIND == D_QKV ? listed<__half>(p.tv) : p.bias;
         // ---- one finished tile: accumulators -> inbox of the CTA that finishes each token -> output
         auto epilogue = [&](int it) {
             const int tile = tile0 + it * tstep;
@@ -387,10 +399,10 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                 }
             };
             if (it == 0) pdl_wait();
-            if (KIND == D_RESID && valid) extra = p.wn[n];
-            if ((KIND == D_QKV || KIND == D_PLAIN || KIND == D_ROWS) && valid && p.bias != nullptr) {
-                extra = p.bias[n];
-                if (KIND == D_QKV) extra2 = p.bias[tile * kTile + pr];
+            if (KIND == D_RESID && valid) extra = wn[n];
+            if ((KIND == D_QKV || KIND == D_PLAIN || KIND == D_ROWS) && valid && bias != nullptr) {
+                extra = bias[n];
+                if (KIND == D_QKV) extra2 = bias[tile * kTile + pr];
             }
             if (j0 < nq) ask(j0);
 
@@ -480,17 +492,17 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                         }
                     } else if (KIND == D_PLAIN || KIND == D_ROWS) {
                         __half x = __float2half_rn(v.v[k]);
-                        if (p.bias != nullptr) x = __hadd(x, extra);
+                        if (bias != nullptr) x = __hadd(x, extra);
                         if (valid) p.y[(size_t)tok * p.N + n] = x;
                     } else if (KIND == D_HEAD) {
                         const int rel = tok - rq * p.mr - (p.row_index ? p.row_index[rq] : 0);
                         if (valid && rel >= 0 && rel < p.rows_out) p.y[(size_t)(rq * p.rows_out + rel) * p.N + n] = __float2half_rn(v.v[k]);
                     } else {
                         __half x = __float2half_rn(v.v[k]);
-                        if (p.bias != nullptr) x = __hadd(x, extra);
+                        if (bias != nullptr) x = __hadd(x, extra);
                         if (rotate) {
                             __half y = __float2half_rn(w.v[k]);
-                            if (p.bias != nullptr) y = __hadd(y, extra2);
+                            if (bias != nullptr) y = __hadd(y, extra2);
                             const float xs = __half2float(x), ys = __half2float(y);
                             x = __float2half_rn(first ? xs * rot[k].x - ys * rot[k].y : ys * rot[k].y + xs * rot[k].x);
                         }
@@ -608,16 +620,19 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
 }
 
 // ================================================================================ embedding
-// One CTA per token: dequantised embedding row -> h, h * w_norm, sums of squares per 32 columns, and the token's RoPE table.
+// One CTA per token: dequantised embedding row -> h, h * w_norm, sums of squares per 32 columns, and the token's RoPE table.  The norm
+// weights may come from the layer table (`wn_entry`).
 // The next kernel is let go only behind the wait: everything before the pass (tree kernels, KV compaction, other programs'
-// writes) is then complete before any kernel of the pass starts, which may so read committed K/V rows ahead of its own wait.
+// writes) is then complete before any kernel of the pass starts, which may so read committed K/V rows, and the layer table, ahead
+// of its own wait.
 __global__ void __launch_bounds__(256) embed_kernel(const int* __restrict__ tokens, const int* __restrict__ pos, const uint32_t* __restrict__ wq,
-                                                    const __half* __restrict__ sc, const __half* __restrict__ bi, const __half* __restrict__ wn,
+                                                    const __half* __restrict__ sc, const __half* __restrict__ bi, const __half* wn,
                                                     __half* __restrict__ h, __half* __restrict__ hw, float* __restrict__ ssq,
                                                     float2* __restrict__ cs, const float* __restrict__ inv_freq, float scaling, int H, int V,
-                                                    int half_hd) {
+                                                    int half_hd, const void* const* wn_entry) {
     pdl_wait();
     pdl_launch_dependents();
+    if (wn_entry != nullptr) wn = listed<__half>(wn_entry);
     const int m = blockIdx.x, units = H / 8;
     const int tok = min(max(tokens[m], 0), V - 1);
     for (int u = threadIdx.x; u < ((units + 31) & ~31); u += 256) {
@@ -994,10 +1009,10 @@ int plan_cluster(int tiles, int nch, int tokens, int group) {
     return best;
 }
 
-template <int NT, int TQ, int KIND>
+template <int NT, int TQ, int KIND, bool TABLE = false>
 int launch_dense(DenseParams& p, int split, cudaStream_t stream) {
     static std::atomic<uint64_t> done{0};
-    if (!allow_smem(dense_kernel<NT, KIND, TQ>, DGeo<NT, TQ>::SMEM, done, KIND != D_ROWS)) return check_launch();
+    if (!allow_smem(dense_kernel<NT, KIND, TQ, TABLE>, DGeo<NT, TQ>::SMEM, done, KIND != D_ROWS)) return check_launch();
     const int nch = p.K / kChunkK;
     const int tiles = KIND == D_SILU ? p.N / 64 : (p.N + kTile - 1) / kTile;
     const int cs = split > 0 && split <= std::min(kMaxCluster, nch) ? split : plan_cluster(tiles, nch, p.M, TQ);
@@ -1005,7 +1020,7 @@ int launch_dense(DenseParams& p, int split, cudaStream_t stream) {
     auto launch = [&](int lo, int n, int cluster) {
         p.tile_lo = lo;
         p.tiles = lo + n;
-        return launch_chain(dense_kernel<NT, KIND, TQ>, dim3(cluster > 1 ? n * cluster : std::min(n, cap)), kDThreads, DGeo<NT, TQ>::SMEM, cluster, stream, p);
+        return launch_chain(dense_kernel<NT, KIND, TQ, TABLE>, dim3(cluster > 1 ? n * cluster : std::min(n, cap)), kDThreads, DGeo<NT, TQ>::SMEM, cluster, stream, p);
     };
     // Whole waves of tiles, then what is left over as a launch of its own with K split over clusters: alone it would take as long
     // as a whole wave.
@@ -1029,7 +1044,9 @@ int launch_attention(DAttn& a, int nreq, cudaStream_t stream) {
     return launch_chain(attention_kernel<HD>, dim3(cs, a.Hkv * a.sets, nreq), kAWarps * 32, G::SMEM, cs, stream, a);
 }
 
-template <int NT, int TQ>
+// TABLE: the kernels take a layer's pointers from the table in device memory, in stream order like everything else.  (Variants of
+// their own: the load is ahead of a CTA's first weights.)
+template <int NT, int TQ, bool TABLE>
 int run_chain(const ChainArgs& c, cudaStream_t st) {
     const b200_forward_desc* d = c.d;
     const int M = d->M, H = d->hidden, I = d->intermediate, hd = d->head_dim, nreq = d->requests > 1 ? d->requests : 1;
@@ -1061,22 +1078,26 @@ int run_chain(const ChainArgs& c, cudaStream_t st) {
     a.req_rows = d->n_layers * 2 * d->n_kv_heads * d->cache_rows;
     a.cap = d->cache_rows; a.write_off = d->write_off; a.scale_log2 = d->attn_scale * kLog2e; a.err = c.err; a.polls = p.polls;
 
-    const void* const* layers = c.layers;
-    if (on(0)) {
+    const void* const* layers = TABLE ? static_cast<const void* const*>(d->layer_table) : c.layers;      // (not read here with TABLE)
+    auto given = [&](const void* const* L, int i) { return TABLE ? nullptr : L[i]; };
+    if (on(0) || TABLE) {                                       // (what makes the table safe to read ahead of a kernel's wait)
         launch_kernel(embed_kernel, dim3(M), dim3(256), 0, st, d->tokens, d->pos, d->embed_wq, static_cast<const __half*>(d->embed_scales),
-                      static_cast<const __half*>(d->embed_biases), static_cast<const __half*>(layers[6]), p.h, p.hw, p.ssq, c.cs, d->inv_freq,
-                      d->rope_scaling, H, d->vocab, hd / 2);
+                      static_cast<const __half*>(d->embed_biases), static_cast<const __half*>(given(layers, 6)), p.h, p.hw, p.ssq, c.cs, d->inv_freq,
+                      d->rope_scaling, H, d->vocab, hd / 2, TABLE ? layers + 6 : nullptr);
         if ((rc = check_launch()) != B200_OK) return rc;
     }
     for (int l = 0; l < d->n_layers; l++) {
         const void* const* L = layers + (size_t)l * 8;       // qkv, qkv bias, o, gate, up, down, input norm, post norm
-        auto w = [&](int i) { return static_cast<const unsigned char*>(L[i]); };
+        auto weights = [&](int i, int n) {
+            for (int j = 0; j < n; j++) p.w[j] = static_cast<const unsigned char*>(given(L, i + j));
+            p.tw = L + i;
+        };
         if (on(1)) {
-            p.xmap = hw_map; p.w[0] = w(0); p.bias = static_cast<const __half*>(L[1]); p.y = static_cast<__half*>(d->qkv);
+            p.xmap = hw_map; weights(0, 1); p.bias = static_cast<const __half*>(given(L, 1)); p.tv = L + 1; p.y = static_cast<__half*>(d->qkv);
             p.N = nqkv; p.K = H;
             p.kc = static_cast<__half*>(d->kv_cache) + (size_t)l * 2 * half_stride;
             p.vc = p.kc + half_stride;
-            if ((rc = launch_dense<NT, TQ, D_QKV>(p, c.splits[0], st)) != B200_OK) return rc;
+            if ((rc = launch_dense<NT, TQ, D_QKV, TABLE>(p, c.splits[0], st)) != B200_OK) return rc;
         }
         if (on(2)) {
             a.row0 = l * 2 * d->n_kv_heads * d->cache_rows;
@@ -1084,16 +1105,18 @@ int run_chain(const ChainArgs& c, cudaStream_t st) {
         }
         p.bias = nullptr;
         if (on(4)) {
-            p.xmap = attn_map; p.w[0] = w(2); p.wn = static_cast<const __half*>(L[7]); p.N = H; p.K = nq;
-            if ((rc = launch_dense<NT, TQ, D_RESID>(p, c.splits[1], st)) != B200_OK) return rc;
+            p.xmap = attn_map; weights(2, 1); p.wn = static_cast<const __half*>(given(L, 7)); p.tv = L + 7; p.N = H; p.K = nq;
+            if ((rc = launch_dense<NT, TQ, D_RESID, TABLE>(p, c.splits[1], st)) != B200_OK) return rc;
         }
         if (on(5)) {
-            p.xmap = hw_map; p.w[0] = w(3); p.w[1] = w(4); p.y = static_cast<__half*>(d->act); p.N = I; p.K = H;
-            if ((rc = launch_dense<NT, TQ, D_SILU>(p, c.splits[2], st)) != B200_OK) return rc;
+            p.xmap = hw_map; weights(3, 2); p.y = static_cast<__half*>(d->act); p.N = I; p.K = H;
+            if ((rc = launch_dense<NT, TQ, D_SILU, TABLE>(p, c.splits[2], st)) != B200_OK) return rc;
         }
         if (on(6)) {
-            p.xmap = act_map; p.w[0] = w(5); p.wn = static_cast<const __half*>(l + 1 < d->n_layers ? L[8 + 6] : d->final_norm); p.N = H; p.K = I;
-            if ((rc = launch_dense<NT, TQ, D_RESID>(p, c.splits[3], st)) != B200_OK) return rc;
+            const bool more = l + 1 < d->n_layers;
+            p.xmap = act_map; weights(5, 1); p.wn = static_cast<const __half*>(more ? given(L, 8 + 6) : d->final_norm); p.tv = more ? L + 8 + 6 : nullptr;
+            p.N = H; p.K = I;
+            if ((rc = launch_dense<NT, TQ, D_RESID, TABLE>(p, c.splits[3], st)) != B200_OK) return rc;
         }
     }
     if (on(7)) {
@@ -1130,6 +1153,13 @@ int chain_matmul(const ChainMatmul& c, cudaStream_t st) {
     return c.M <= 8 ? run_matmul<16, 2>(c, st) : (c.M <= 16 ? run_matmul<16, 4>(c, st) : run_matmul<32, 4>(c, st));
 }
 
-int forward_chain(const ChainArgs& a, cudaStream_t stream) { return a.d->M <= 8 ? run_chain<16, 2>(a, stream) : (a.d->M <= 16 ? run_chain<16, 4>(a, stream) : run_chain<32, 4>(a, stream)); }
+template <bool TABLE>
+static int forward_chain_rows(const ChainArgs& a, cudaStream_t stream) {
+    return a.d->M <= 8 ? run_chain<16, 2, TABLE>(a, stream) : (a.d->M <= 16 ? run_chain<16, 4, TABLE>(a, stream) : run_chain<32, 4, TABLE>(a, stream));
+}
+
+int forward_chain(const ChainArgs& a, cudaStream_t stream) {
+    return a.layers != nullptr ? forward_chain_rows<false>(a, stream) : forward_chain_rows<true>(a, stream);
+}
 
 }  // namespace b200

@@ -8,7 +8,7 @@ namespace b200 {
 // What b200_forward has checked and laid out of the descriptor: everything is valid, tp_world <= 1.
 struct ChainArgs {
     const b200_forward_desc* d;
-    const void* const* layers;   // host copy of the layer table
+    const void* const* layers;   // host copy of the layer table, or NULL: the kernels read the descriptor's
     int* err;             // error word
     float* ssq;           // [hidden / 32][32]
     float2* cs;           // [32][64]

@@ -2180,24 +2180,6 @@ int launch_forward_hd(const FwdParams& p, int grid, cudaStream_t stream) {
     return p.HD == 128 ? launch_forward<MT, 128>(p, grid, stream) : launch_forward<MT, 64>(p, grid, stream);
 }
 
-// Copy of the device's layer table, for callers that have none on the host.  While `stream` is being captured it comes through a
-// stream of its own, which must not become part of the capture.
-bool read_table(const void** table, const b200_forward_desc* d, cudaStream_t stream) {
-    const size_t bytes = (size_t)d->n_layers * 8 * sizeof(void*);
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess) return false;
-    if (capturing == cudaStreamCaptureStatusNone)
-        return cudaMemcpyAsync(table, d->layer_table, bytes, cudaMemcpyDeviceToHost, stream) == cudaSuccess &&
-               cudaStreamSynchronize(stream) == cudaSuccess;
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return false;
-    cudaStream_t own = nullptr;
-    bool ok = cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking) == cudaSuccess;
-    ok = ok && cudaMemcpyAsync(table, d->layer_table, bytes, cudaMemcpyDeviceToHost, own) == cudaSuccess && cudaStreamSynchronize(own) == cudaSuccess;
-    if (own != nullptr) cudaStreamDestroy(own);
-    return cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess && ok;
-}
-
 }  // namespace
 }  // namespace b200
 
@@ -2245,12 +2227,9 @@ int b200_forward(const b200_forward_desc* d, void* stream) {
         a.cs = reinterpret_cast<float2*>(ws + ChainWs::kCs);
         for (int i = 0; i < 5; i++)
             if (const PlanOverride* o = plan_override(i)) a.splits[i] = (o->kw & (o->kw - 1)) == 0 && o->kw <= 8 ? o->splits : 0;
-        const void* table[kMaxLayers * 8];
-        a.layers = d->timeline_pitch == B200_LAYERS_ON_HOST ? static_cast<const void* const*>(d->timeline) : table;
-        if (a.layers == table && !read_table(table, d, static_cast<cudaStream_t>(stream))) {
-            (void)check_launch();
-            return B200_ECUDA;
-        }
+        const bool on_host = d->timeline_pitch == B200_LAYERS_ON_HOST;
+        if (on_host && d->timeline == nullptr) return B200_EINVAL;
+        a.layers = on_host ? static_cast<const void* const*>(d->timeline) : nullptr;
         return forward_chain(a, static_cast<cudaStream_t>(stream));
     }
     FwdParams p{};

@@ -67,6 +67,13 @@ def test_forward_descriptor_validation_without_gpu(be):
     d.vocab, d.n_layers, d.cache_rows, d.write_off, d.tail = 152064, 28, 1024, 0, 16
     assert lib.b200_forward_workspace_bytes(ctypes.byref(d)) > 4352
     assert lib.b200_forward(ctypes.byref(d), None) == -1          # null pointers: refused before any CUDA call
+    buf = (ctypes.c_char * 64)()
+    base = ctypes.addressof(buf) + (-ctypes.addressof(buf)) % 16
+    for name, kind in d._fields_:
+        if kind is ctypes.c_void_p:
+            setattr(d, name, base)
+    d.workspace_bytes, d.timeline, d.timeline_pitch = lib.b200_forward_workspace_bytes(ctypes.byref(d)), None, be._lib.LAYERS_ON_HOST
+    assert lib.b200_forward(ctypes.byref(d), None) == -1          # a host table that is not there: refused, not read
     d.hidden = 3500                                               # not a multiple of 128
     assert lib.b200_forward_workspace_bytes(ctypes.byref(d)) == 0
     d.hidden, d.head_dim = 3584, 96

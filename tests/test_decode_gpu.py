@@ -85,7 +85,7 @@ def test_pass_inputs_whatever_their_form(be, cuda, rows, cached):
 
 
 def test_layer_pointers_from_the_device_table(be, cuda):
-    """Without a host copy of the layer table the call reads it back: the same logits, and it stays capturable."""
+    """Without a host copy of the layer table the kernels read it: the same logits, and it stays capturable."""
     m = _model(be, cuda, *SHAPES[1])
     cache = _cache(m, 70, 4)
     m.fwd.tokens.copy_(torch.arange(32))
@@ -104,6 +104,37 @@ def test_layer_pointers_from_the_device_table(be, cuda):
     graph.replay()
     m.check_fused_error()
     assert torch.equal(m.logits[:20], want)
+
+
+@pytest.mark.parametrize("rows", [8, 16, 20])
+def test_without_a_host_table_the_call_returns_at_once_and_takes_the_table_in_stream_order(be, cuda, rows):
+    m, other = _model(be, cuda, *SHAPES[1]), _model(be, cuda, *SHAPES[1])
+    for lw in other.layers:
+        lw["input_norm"].mul_(0.5)
+        lw["post_norm"].neg_()
+        lw["qkv"].bias.zero_()
+    cache = _cache(m, 70, 4)
+    m.fwd.tokens.copy_(torch.arange(32))
+    m.fwd.pos.copy_(70 + torch.arange(32))
+    m.fwd.prefix.fill_(70)
+    m.fwd.mask.copy_(torch.tensor([(2 << i) - 1 for i in range(32)]))
+    want = m.forward_device(rows, cache, 0, rows).clone()
+    wrong = other.forward_device(rows, cache, 0, rows, m.fwd).clone()
+    assert not torch.equal(want, wrong)
+    desc = be._lib.ForwardDesc.from_buffer_copy(m._fused_desc(rows, cache, 0, rows, m.fwd, rows, None))
+    table, right = other._layer_table.clone(), m._layer_table
+    desc.timeline, desc.timeline_pitch, desc.layer_table = None, 0, table.data_ptr()
+    m.logits.zero_()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(200_000_000)                       # (a tenth of a second, which the call must not wait for)
+    table.copy_(right)
+    done = torch.cuda.Event()
+    be._lib.check(be._lib.lib().b200_forward(ctypes.byref(desc), be._lib.stream_ptr(m.device)), "b200_forward")
+    done.record()
+    assert not done.query()
+    done.synchronize()
+    m.check_fused_error()
+    assert torch.equal(m.logits[:rows], want)
 
 
 def test_a_repeated_pass_runs_from_a_graph_on_the_data_of_the_call(be, cuda):
