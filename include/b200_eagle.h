@@ -256,9 +256,11 @@ typedef struct b200_forward_desc {
     int hidden, intermediate, n_heads, n_kv_heads, head_dim, vocab, n_layers;
     int cache_rows, write_off, tail;
     float rms_eps, rope_scaling, attn_scale;
-    int attn_split_blocks;  /* shards only.  0 = default (33): from this many 64-key blocks of cache on, attention splits the  */
-                            /* keys across CTAs and merges in a second phase; below, one CTA per (kv head,      */
-                            /* query tile) scores the key blocks on its warps side by side.  < 0 = always split  */
+    int attn_split_blocks;  /* from this many 64-key blocks on, attention splits the keys across CTAs.  Shards: blocks of     */
+                            /* committed cache; 0 = default (33); split keys are merged in a second phase, below, one CTA     */
+                            /* per (kv head, query tile) scores the key blocks on its warps side by side; < 0 = always split. */
+                            /* Otherwise: blocks of cache_rows; 0 = default (into as many ranges, up to 8, as run at once);  */
+                            /* < 0 = into 8 (or one a block), even if those then run in turn                                  */
     const int* tokens;
     const int* pos;
     const unsigned long long* mask;

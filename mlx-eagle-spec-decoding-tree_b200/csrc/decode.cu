@@ -1031,16 +1031,17 @@ int launch_dense(DenseParams& p, int split, cudaStream_t stream) {
 }
 
 // Clusters of as many key ranges as still run at once, two CTAs to an SM (33 clusters of 8 fit, 71 of 4; at one CTA to an SM, with
-// 64 query rows in a CTA, 15 of 8: the sixteenth ran alone and doubled the time).
+// 64 query rows in a CTA, 15 of 8: the sixteenth ran alone and doubled the time).  `split` as b200_forward_desc.attn_split_blocks.
 template <int HD>
-int launch_attention(DAttn& a, int nreq, cudaStream_t stream) {
+int launch_attention(DAttn& a, int nreq, int split, cudaStream_t stream) {
     using G = DAGeo<HD>;
     static std::atomic<uint64_t> done{0};
     if (!allow_smem(attention_kernel<HD>, G::SMEM, done, true)) return check_launch();
     a.sets = (a.mr * (a.Hq / a.Hkv) + G::ROWS - 1) / G::ROWS;
     const int clusters = a.Hkv * a.sets * nreq;
     int cs = std::min(a.nkb, kMaxCluster);
-    while (cs > 1 && clusters > 8 * (32 / cs)) cs--;
+    while (split >= 0 && cs > 1 && clusters > 8 * (32 / cs)) cs--;
+    if (split > 0 && a.nkb < split) cs = 1;
     return launch_chain(attention_kernel<HD>, dim3(cs, a.Hkv * a.sets, nreq), kAWarps * 32, G::SMEM, cs, stream, a);
 }
 
@@ -1101,7 +1102,7 @@ int run_chain(const ChainArgs& c, cudaStream_t st) {
         }
         if (on(2)) {
             a.row0 = l * 2 * d->n_kv_heads * d->cache_rows;
-            if ((rc = hd == 128 ? launch_attention<128>(a, nreq, st) : launch_attention<64>(a, nreq, st)) != B200_OK) return rc;
+            if ((rc = hd == 128 ? launch_attention<128>(a, nreq, d->attn_split_blocks, st) : launch_attention<64>(a, nreq, d->attn_split_blocks, st)) != B200_OK) return rc;
         }
         p.bias = nullptr;
         if (on(4)) {

@@ -347,7 +347,7 @@ class Model:
         self.vocab_offset = 0
         self.part32 = None
         self.timeline = None
-        self.attn_split_blocks = 0                       # 0 = library default; < 0 = always split the keys across CTAs
+        self.attn_split_blocks = 0                       # 0 = library default; n: split the keys from n blocks on; < 0 = always
         self.phase_mask = 0                              # profiling: run only some phase kinds (0 = all)
         self.grid_ctas = 0                               # CTAs of a shard's persistent kernel (0 = one per SM)
         self.fast_dequant = True                         # allow the short nibble expansion when every scale permits it
