@@ -616,10 +616,11 @@ class Model:
         that ends at the barrier: entry, rstd done, first stage landed, stages done, K-parts reduced, end
         (``self.timeline`` int64 ``[SMs, barriers + 1, 8]``; the last entry holds the end of the kernel)."""
         if on:
+            if self.tp is None:
+                raise _lib.B200Error("the timeline is of a shard's persistent kernel: without tensor parallelism a pass is a "
+                                     "chain of kernels (time them with a profiler or CUDA events)")
             sms = torch.cuda.get_device_properties(self.device).multi_processor_count
-            per_layer = 6 if self.tp is None else 10         # a shard has two to four more barriers per layer
-            self.timeline = torch.zeros(sms, per_layer * self.args.num_hidden_layers + 2, 8, dtype=torch.int64,
-                                        device=self.device)
+            self.timeline = torch.zeros(sms, 10 * self.args.num_hidden_layers + 2, 8, dtype=torch.int64, device=self.device)
         else:
             self.timeline = None
 

@@ -55,6 +55,13 @@ def test_shard_refuses_degrees_that_do_not_divide(be):
         full.shard(0, 3)
 
 
+def test_the_timeline_of_a_model_that_is_no_shard_is_refused(be):
+    full = be.Model.random_init(be.shape_preset("tiny-qwen2"), seed=3, device="cpu")
+    with pytest.raises(be._lib.B200Error, match="shard"):        # (its passes have no device-wide barriers to stamp)
+        full.enable_timeline()
+    full.enable_timeline(False)
+
+
 def _rank(rank, world, port, out):
     os.environ["MASTER_ADDR"] = "127.0.0.1"
     os.environ["MASTER_PORT"] = str(port)
