@@ -568,7 +568,6 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                         sb = *reinterpret_cast<const uint2*>(st + scoff);
                     }
                     const bool fast = __all_sync(0xffffffffu, fast_scale(sb.x) && fast_scale(sb.y));
-                    if (lane == 0) mbar_arrive(smem_u32(wempty + slot));             // the packs are in registers
                     if (done >= kGroups) mbar_wait_reported(smem_u32(tfree + me), tph, p.polls, p.err, 24);
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                     __syncwarp();
@@ -599,6 +598,10 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                     };
                     if (fast) expand(std::true_type{});
                     else expand(std::false_type{});
+                    // Only now that the packs have been used: an arrival right behind the loads does not wait for them, and the next tile's
+                    // weights were there before the last of them were through (some rows of one stage in 1e8; 46 wrong passes of 200000).
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(wempty + slot));
                     asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
                     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                     __syncwarp();

@@ -1,6 +1,7 @@
 """The kernel chain of a pass of up to 32 tokens (csrc/decode.cu) at the edges of its tiles, key blocks and clusters, against the
 per-op kernels; and the inputs of a pass from a caller's tensors."""
 import ctypes
+import dataclasses
 
 import numpy as np
 import pytest
@@ -157,6 +158,24 @@ def test_a_repeated_pass_runs_from_a_graph_on_the_data_of_the_call(be, cuda):
             m(tokens, c)
     m.check_fused_error()
     assert len(m._graphs._seen) <= keep
+
+
+def test_every_repetition_of_a_pass_gives_the_same_bits(be, cuda):
+    """Thirty thousand passes with a wide head, whose CTAs go round their ring of weight stages many times: a stage given back
+    before all of its loads are through shows as wrong logits of a few rows in some of them."""
+    args = dataclasses.replace(be.shape_preset("qwen2-0.5b"), num_hidden_layers=1)
+    m = be.Model.random_init(args, seed=3, device=cuda).relayout()
+    tokens = torch.arange(32, dtype=torch.int32, device=cuda)[None]
+    cache = m.make_cache(64)
+    want = m(tokens, cache)
+    wrong = torch.zeros((), dtype=torch.int64, device=cuda)
+    for i in range(30000):
+        cache.offset = 0
+        wrong += (m(tokens, cache) != want).any()
+        if i % 200 == 0:
+            torch.cuda.synchronize()                     # (the host stays near)
+    assert int(wrong) == 0
+    m.check_fused_error()
 
 
 @pytest.mark.parametrize("rows", [1, 8, 9, 16, 17, 32])
