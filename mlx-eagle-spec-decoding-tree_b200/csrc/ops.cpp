@@ -109,8 +109,52 @@ PyObject* rope_positions(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return THPVariable_Wrap(std::move(y));
 }
 
+// layer_pointers(layers, table) -> 0: `table` (address of [layers][8] pointers in the order of b200_forward_desc.layer_table) holds
+// the device pointers of the layers already, 1: it does now, -1: a layer is not as it should be (no re-laid-out weights, say).
+// Runs ahead of every pass, so that a pass never sees the address of a tensor that has been replaced: ~0.3 us a layer.
+PyObject* layer_pointers(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    static PyObject* const linears[] = {PyUnicode_InternFromString("qkv"), PyUnicode_InternFromString("o"), PyUnicode_InternFromString("gate"),
+                                        PyUnicode_InternFromString("up"), PyUnicode_InternFromString("down")};
+    static PyObject* const norms[] = {PyUnicode_InternFromString("input_norm"), PyUnicode_InternFromString("post_norm")};
+    static PyObject* const tiled = PyUnicode_InternFromString("tiled");
+    static PyObject* const bias = PyUnicode_InternFromString("bias");
+    void** table = n == 2 && PyList_Check(a[0]) ? static_cast<void**>(PyLong_AsVoidPtr(a[1])) : nullptr;
+    if (PyErr_Occurred()) return nullptr;
+    if (table == nullptr) return PyLong_FromLong(-1);
+    bool plain = true, same = true;
+    auto put = [&](PyObject* t, bool optional) {              // (borrowed, may be NULL)
+        void* q = nullptr;
+        if (t == nullptr || !THPVariable_Check(t)) plain = plain && optional && t == Py_None;
+        else q = THPVariable_Unpack(t).data_ptr();
+        same = same && *table == q;
+        *table++ = q;
+    };
+    auto put_attr = [&](PyObject* o, PyObject* name, bool optional) {
+        PyObject* t = o == nullptr ? nullptr : PyObject_GetAttr(o, name);
+        if (t == nullptr) PyErr_Clear();
+        put(t, optional);
+        Py_XDECREF(t);                                           // (the layer still holds it)
+    };
+    try {
+        const Py_ssize_t layers = PyList_GET_SIZE(a[0]);
+        for (Py_ssize_t l = 0; l < layers; l++) {
+            PyObject* layer = PyList_GET_ITEM(a[0], l);
+            if (!PyDict_Check(layer)) return PyLong_FromLong(-1);
+            for (int i = 0; i < 5; i++) {
+                PyObject* lin = PyDict_GetItem(layer, linears[i]);
+                put_attr(lin, tiled, false);
+                if (i == 0) put_attr(lin, bias, true);
+            }
+            for (PyObject* name : norms) put(PyDict_GetItem(layer, name), false);
+        }
+    } catch (const std::exception&) {                            // (a tensor without storage)
+        plain = false;
+    }
+    return PyLong_FromLong(!plain ? -1 : (same ? 0 : 1));
+}
+
 #define FAST(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {FAST(qmm), FAST(qmm_tiled), FAST(rope_positions), {nullptr, nullptr, 0, nullptr}};
+PyMethodDef methods[] = {FAST(qmm), FAST(qmm_tiled), FAST(rope_positions), FAST(layer_pointers), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_b200ops", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

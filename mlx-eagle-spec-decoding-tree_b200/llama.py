@@ -342,7 +342,7 @@ class Model:
         self.fused = True                                # b200_forward when possible
         self._fwd_ws = None
         self._fwd_ws_key = None
-        self._layer_table = None
+        self._layers_host = self._layer_table = None     # device pointers of the layers: kept up to date by _gather_layers()
         self.tp: Optional[TensorParallel] = None         # set by shard(): this model is one shard of a tensor-parallel model
         self.vocab_offset = 0
         self.part32 = None
@@ -353,9 +353,8 @@ class Model:
         self.fast_dequant = True                         # allow the short nibble expansion when every scale permits it
         self.tp_two_shot = 0                             # tensor-parallel exchange: 0 library's choice (push), 1 two-step, 2 pull behind a hierarchical barrier, 3 push, 4 pull
         self.prefill_large_m = True                      # prompts: 128 rows per weight read through b200_prefill
-        self._pf, self._pf_buf, self._pf_fits = None, None, False     # descriptor and buffers of that path, made on first use
-        self._scales_fast = None
-        self._desc, self._fuse_fits = None, False
+        self._pf_buf, self._pf_fits = None, False        # buffers of that path, made on first use
+        self._scales_fast, self._layers_fast, self._fuse_fits = None, None, False
         self._graphs = _Graphs()
         self.fwd = FwdInputs(self.device)
 
@@ -545,49 +544,50 @@ class Model:
             return False
         if self.tp is not None and (self.tp.peers is None or self.tp.world > 8):
             return False                         # a shard fuses once open_exchange() has mapped the peers' buffers
-        if self._fuse_fits:                      # (relayout only adds: a yes stays a yes)
+        if not self._fuse_fits:
+            a = self.args
+            if any(lw[k].tiled is None for lw in self.layers for k in ("qkv", "o", "gate", "up", "down")):
+                return False
+            self._fuse_fits = (a.hidden_size % 128 == 0 and a.hidden_size <= 8192 and a.intermediate_size % 128 == 0
+                               and self.nq % 128 == 0 and a.head_dim in (64, 128) and a.vocab_size % 8 == 0
+                               and self.vocab_local % 8 == 0)
+        return self._fuse_fits and self.lm_head.tiled is not None and self.embed.weight is not None and self._gather_layers()
+
+    def _gather_layers(self) -> bool:
+        """The layers' device pointers as they are now (ahead of every pass: any tensor may have been replaced since the last).
+        False if a layer has no re-laid-out weights."""
+        n = self.args.num_hidden_layers
+        if self._layers_host is None:
+            self._layers_host = (ctypes.c_void_p * (8 * n))()
+        state = _lib.ops().layer_pointers(self.layers, ctypes.addressof(self._layers_host)) if len(self.layers) == n else -1
+        if state == 0 and self._layer_table is not None:
             return True
-        a = self.args
-        if any(lw[k].tiled is None for lw in self.layers for k in ("qkv", "o", "gate", "up", "down")):
+        self._graphs.clear()                             # (a graph has the layers' pointers in it)
+        self._layer_table = None
+        if state < 0:
+            self._fuse_fits = self._pf_fits = False
             return False
-        if self.lm_head.tiled is None or self.embed.weight is None:
-            return False
-        self._fuse_fits = (a.hidden_size % 128 == 0 and a.hidden_size <= 8192 and a.intermediate_size % 128 == 0
-                and self.nq % 128 == 0 and a.head_dim in (64, 128) and a.vocab_size % 8 == 0
-                           and self.vocab_local % 8 == 0)
-        return self._fuse_fits
+        self._layer_table = torch.tensor([p or 0 for p in self._layers_host], dtype=torch.int64).to(self.device)
+        self._layers_fast = all(lw[k].scales_fast for lw in self.layers for k in ("qkv", "o", "gate", "up", "down"))
+        return True
 
     def _fused_desc(self, M, cache, write_off, tail, fwd, rows, row_index, requests=1, logits=None):
-        """The descriptor of ``b200_forward``: what a model keeps is filled in once, the rest on each call."""
+        """The descriptor of ``b200_forward`` (after ``can_fuse()``, which brings the layers' pointers up to date)."""
         p = lambda t: None if t is None else t.data_ptr()
-        d = self._desc
-        if d is None:
-            a = self.args
-            rows_ = []
-            for lw in self.layers:
-                rows_.append([lw["qkv"].tiled.data_ptr(), p(lw["qkv"].bias) or 0, lw["o"].tiled.data_ptr(),
-                              lw["gate"].tiled.data_ptr(), lw["up"].tiled.data_ptr(), lw["down"].tiled.data_ptr(),
-                              lw["input_norm"].data_ptr(), lw["post_norm"].data_ptr()])
-            self._layer_table = torch.tensor(rows_, dtype=torch.int64).to(self.device)
-            flat = [v for row in rows_ for v in row]
-            self._layers_host = (ctypes.c_void_p * len(flat))(*flat)
-            self._scales_fast = all(lw[k].scales_fast for lw in self.layers for k in ("qkv", "o", "gate", "up", "down")) \
-                and self.lm_head.scales_fast
-            d = _lib.ForwardDesc()
-            d.hidden, d.intermediate, d.n_heads, d.n_kv_heads = a.hidden_size, a.intermediate_size, \
-                a.num_attention_heads, a.num_key_value_heads
-            d.head_dim, d.vocab, d.n_layers = a.head_dim, a.vocab_size, a.num_hidden_layers
-            d.rms_eps, d.rope_scaling, d.attn_scale = float(a.rms_norm_eps), self.rope_scaling_factor, self.scale
-            d.inv_freq = p(self.inv_freqs)
-            d.embed_wq, d.embed_scales, d.embed_biases = p(self.embed.weight), p(self.embed.scales), p(self.embed.biases)
-            d.final_norm, d.lm_head_tiled, d.layer_table = p(self.norm), p(self.lm_head.tiled), p(self._layer_table)
-            d.h, d.hw, d.qkv, d.attn, d.act = p(self.h), p(self.hw), p(self.qkv), p(self.xt_attn), p(self.xt_act)
-            self._desc = d
-        d.M, d.rows_out, d.requests = M, rows, requests
-        d.cache_rows, d.write_off, d.tail = cache.rows, write_off, tail
+        a, d = self.args, _lib.ForwardDesc()
+        d.M, d.rows_out, d.hidden, d.intermediate, d.n_heads, d.n_kv_heads = M, rows, a.hidden_size, a.intermediate_size, \
+            a.num_attention_heads, a.num_key_value_heads
+        d.head_dim, d.vocab, d.n_layers = a.head_dim, a.vocab_size, a.num_hidden_layers
+        d.cache_rows, d.write_off, d.tail, d.requests = cache.rows, write_off, tail, requests
+        d.rms_eps, d.rope_scaling, d.attn_scale = float(a.rms_norm_eps), self.rope_scaling_factor, self.scale
         d.tokens, d.pos, d.mask, d.prefix = p(fwd.tokens), p(fwd.pos), p(fwd.mask), p(fwd.prefix)
         d.row_index, d.logits, d.kv_cache = p(row_index), p(self.logits if logits is None else logits), p(cache.data)
+        d.inv_freq = p(self.inv_freqs)
+        d.embed_wq, d.embed_scales, d.embed_biases = p(self.embed.weight), p(self.embed.scales), p(self.embed.biases)
+        d.final_norm, d.lm_head_tiled, d.layer_table = p(self.norm), p(self.lm_head.tiled), p(self._layer_table)
+        d.h, d.hw, d.qkv, d.attn, d.act = p(self.h), p(self.hw), p(self.qkv), p(self.xt_attn), p(self.xt_act)
         d.grid_ctas, d.phase_mask, d.attn_split_blocks = self.grid_ctas, self.phase_mask, self.attn_split_blocks
+        self._scales_fast = self._layers_fast and self.lm_head.scales_fast
         d.scales_in_fast_range = 1 if (self._scales_fast and self.fast_dequant) else 0
         if self.tp is not None:
             d.tp_world, d.tp_rank, d.head_rows = self.tp.world, self.tp.rank, self.vocab_local
@@ -606,8 +606,8 @@ class Model:
         d.workspace, d.workspace_bytes = p(self._fwd_ws), self._fwd_ws.numel()
         if self.tp is None:
             d.timeline, d.timeline_pitch = ctypes.addressof(self._layers_host), _lib.LAYERS_ON_HOST
-        else:
-            d.timeline, d.timeline_pitch = (p(self.timeline), self.timeline.shape[1]) if self.timeline is not None else (None, 0)
+        elif self.timeline is not None:
+            d.timeline, d.timeline_pitch = p(self.timeline), self.timeline.shape[1]
         return d
 
     def enable_timeline(self, on: bool = True):
@@ -753,43 +753,36 @@ class Model:
         tensor-parallel shard."""
         if not self.prefill_large_m or self.tp is not None or os.environ.get("B200_PREFILL_LARGE_M", "1") == "0":
             return False
-        if not self._pf_fits:                            # (relayout only adds: a yes stays a yes)
+        if not self._pf_fits:
             a = self.args
             lins = [lw[k] for lw in self.layers for k in ("qkv", "o", "gate", "up", "down")] + [self.lm_head]
             self._pf_fits = (all(q.tiled is not None for q in lins) and self.embed.weight is not None
                              and all(q.out_features % 8 == 0 and q.in_features % 128 == 0 for q in lins)
                              and a.hidden_size <= 8192 and a.head_dim in (64, 128))
-        return self._pf_fits
+        return self._pf_fits and self.lm_head.tiled is not None and self.embed.weight is not None and self._gather_layers()
 
     def _prefill_large_m(self, tokens: torch.Tensor, cache: KVCache, off: int, logits: Optional[torch.Tensor], rows: int):
         """One causal pass of up to ``PREFILL_ROWS`` prompt tokens (device int32) starting at cache row ``off``
         (``mlx_eagle.py:522-535`` ingests the prompt in chunks; ``mlx_llama.py:231-249`` is the layer), launched from native
         code (``b200_prefill``).  Writes the logits of all tokens (``rows`` = their count) or of the last (``rows`` = 1) to
         ``logits``; ``rows`` = 0: cache rows only."""
-        d = self._pf
         p = lambda t: t.data_ptr()
-        if d is None:
-            a, R = self.args, PREFILL_ROWS
-            H, I = a.hidden_size, a.intermediate_size
-            f16 = dict(dtype=torch.float16, device=self.device)
-            ptr = lambda t: 0 if t is None else t.data_ptr()
-            table = [ptr(t) for lw in self.layers
-                     for t in (lw["qkv"].tiled, lw["qkv"].bias, lw["o"].tiled, lw["gate"].tiled, lw["up"].tiled,
-                               lw["down"].tiled, lw["input_norm"], lw["post_norm"])]
+        a, d, buf = self.args, _lib.PrefillDesc(), self._pf_buf
+        H, I = a.hidden_size, a.intermediate_size
+        if buf is None:
+            R, f16 = PREFILL_ROWS, dict(dtype=torch.float16, device=self.device)
             buf = dict(h=torch.empty(R, H, **f16), xn=torch.empty(R, H, **f16),
                        qkv=torch.empty(R, self.nq + 2 * self.nkv, **f16), attn=torch.empty(R, self.nq, **f16),
-                       act=torch.empty(R, I, **f16), table=(ctypes.c_void_p * len(table))(*table),
-                       ws=torch.zeros(4096 + (16 << 20), dtype=torch.uint8, device=self.device))
-            d = _lib.PrefillDesc()
-            d.hidden, d.intermediate, d.n_heads, d.n_kv_heads = H, I, a.num_attention_heads, a.num_key_value_heads
-            d.head_dim, d.vocab, d.n_layers = a.head_dim, a.vocab_size, a.num_hidden_layers
-            d.rms_eps, d.rope_scaling, d.attn_scale = float(a.rms_norm_eps), self.rope_scaling_factor, self.scale
-            d.inv_freq, d.final_norm, d.lm_head_tiled = p(self.inv_freqs), p(self.norm), p(self.lm_head.tiled)
-            d.embed_wq, d.embed_scales, d.embed_biases = p(self.embed.weight), p(self.embed.scales), p(self.embed.biases)
-            d.layers = ctypes.cast(buf["table"], ctypes.c_void_p)
-            d.h, d.xn, d.qkv, d.attn, d.act = (p(buf[k]) for k in ("h", "xn", "qkv", "attn", "act"))
-            d.workspace, d.workspace_bytes = p(buf["ws"]), buf["ws"].numel()
-            self._pf, self._pf_buf = d, buf
+                       act=torch.empty(R, I, **f16), ws=torch.zeros(4096 + (16 << 20), dtype=torch.uint8, device=self.device))
+            self._pf_buf = buf
+        d.hidden, d.intermediate, d.n_heads, d.n_kv_heads = H, I, a.num_attention_heads, a.num_key_value_heads
+        d.head_dim, d.vocab, d.n_layers = a.head_dim, a.vocab_size, a.num_hidden_layers
+        d.rms_eps, d.rope_scaling, d.attn_scale = float(a.rms_norm_eps), self.rope_scaling_factor, self.scale
+        d.inv_freq, d.final_norm, d.lm_head_tiled = p(self.inv_freqs), p(self.norm), p(self.lm_head.tiled)
+        d.embed_wq, d.embed_scales, d.embed_biases = p(self.embed.weight), p(self.embed.scales), p(self.embed.biases)
+        d.layers = ctypes.addressof(self._layers_host)   # (brought up to date by can_prefill_large_m())
+        d.h, d.xn, d.qkv, d.attn, d.act = (p(buf[k]) for k in ("h", "xn", "qkv", "attn", "act"))
+        d.workspace, d.workspace_bytes = p(buf["ws"]), buf["ws"].numel()
         d.n, d.off, d.cache_rows, d.kv_cache, d.tokens = tokens.numel(), off, cache.rows, p(cache.data), p(tokens)
         d.head_out = 0 if rows == 0 else (1 if rows == d.n and rows > 1 else 2)
         d.logits = p(logits) if rows else None

@@ -178,6 +178,47 @@ def test_every_repetition_of_a_pass_gives_the_same_bits(be, cuda):
     m.check_fused_error()
 
 
+@pytest.mark.parametrize("count", [5, 50])              # kernel chain (replayed from a graph), prompt path
+def test_a_tensor_replaced_between_passes_is_seen_by_the_next(be, cuda, count):
+    m = _model(be, cuda, *SHAPES[0])
+    other, third = (be.Model.random_init(m.args, seed=seed, device=cuda, gen_device="cpu") for seed in (8, 9))
+    o = other.layers[1]["o"]
+    rows = be.llama.QLinear(o.weight, o.scales, o.biases)
+    other.relayout()
+    head = third.relayout().embed
+    cache = _cache(m, 10, 5)
+    tokens = torch.arange(count)[None]
+
+    def run(fused):
+        m.fused = m.prefill_large_m = fused
+        cache.offset = 10
+        return m(tokens, cache).float()
+
+    steps = [lambda: setattr(m, "norm", other.norm), lambda: setattr(m, "embed", other.embed), lambda: setattr(m, "lm_head", head),
+             lambda: m.layers[0].update(input_norm=other.layers[0]["input_norm"]), lambda: m.layers[1].update(post_norm=other.layers[1]["post_norm"]),
+             lambda: m.layers[1].update(down=other.layers[1]["down"]), lambda: setattr(m.layers[0]["gate"], "tiled", other.layers[0]["gate"].tiled),
+             lambda: setattr(m.layers[0]["qkv"], "bias", None), lambda: m.layers.reverse(),
+             lambda: m.layers[0].update(o=rows)]
+    before = None
+    for step in steps:
+        for _ in range(2 * m._graphs.AFTER):
+            run(True)
+        step()
+        junk = [torch.full((1 << 16,), 77.0, dtype=torch.float16, device=cuda) for _ in range(8)]      # (where freed weights were)
+        got, want = run(True), run(False)
+        assert ((got - want).abs() <= 2.0 ** -6 * want.abs() + 1e-2).all()
+        assert before is None or not torch.equal(got, before)
+        before = got
+        del junk
+    m.fused = True
+    assert not m.can_fuse()                              # (the last one has no re-laid-out weights: the per-op kernels ran it)
+    rows.relayout(keep_rowmajor=True)
+    assert m.can_fuse()
+    got, want = run(True), run(False)
+    assert ((got - want).abs() <= 2.0 ** -6 * want.abs() + 1e-2).all()
+    m.check_fused_error()
+
+
 @pytest.mark.parametrize("rows", [1, 8, 9, 16, 17, 32])
 @pytest.mark.parametrize("n,k", [(8, 128), (136, 256), (904, 1152), (2056, 2176), (18432, 1024), (2048, 12288), (2048, 12416)])
 def test_matmul_of_the_chain_on_its_own(be, cuda, rows, n, k):
