@@ -79,3 +79,31 @@ def test_forward_descriptor_validation_without_gpu(be):
     d.hidden, d.head_dim = 3584, 96
     assert lib.b200_forward(ctypes.byref(d), None) == -1
     assert ctypes.sizeof(be._lib.ForwardDesc) == 64 + 20 * 8 + 8 + 16 + 16 + 64 + 8 + 8  # layout of b200_forward_desc in the header
+
+
+FAKE = """
+import torch
+import b200_eagle as be
+from torch._subclasses.fake_tensor import FakeTensorMode
+
+with FakeTensorMode(allow_non_fake_inputs=True):
+    new = lambda *shape, dtype=torch.float16: torch.empty(shape, dtype=dtype, device="cuda:0")
+    be.qmm_kernel._workspaces[0] = new(4096, dtype=torch.uint8)
+    calls = [lambda: be.rope_positions(new(1, 2, 4, 64), new(1, 4, dtype=torch.int32), new(32, dtype=torch.float32), 1.0),
+             lambda: be.matmul(new(2, 128), new(8, 16, dtype=torch.int32), new(8, 2), new(8, 2)),
+             lambda: be.qmm_kernel.matmul_tiled(new(2, 128), new(4608, dtype=torch.uint8), 8)]
+    for call in calls:
+        try:
+            call()
+        except Exception as e:
+            print("raised", type(e).__name__)
+"""
+
+
+def test_operators_on_tensors_without_storage_raise_in_python():
+    """An exception of torch's C++ inside the native operator module must not end the process."""
+    import subprocess
+    import sys
+    res = subprocess.run([sys.executable, "-c", FAKE], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0, res.stderr[-2000:]
+    assert res.stdout.count("raised") == 3
