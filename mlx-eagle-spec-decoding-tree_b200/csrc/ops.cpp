@@ -7,6 +7,8 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
+#include <climits>
+
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
@@ -62,7 +64,7 @@ PyObject* qmm(PyObject* const* a, Py_ssize_t n) {
     const int64_t K = x->size(-1), N = w.size(0);
     if (K < 128 || K % 128 || w.size(1) * 8 != K || s->size(0) != N || s->size(1) * 64 != K || b->size(0) != N || b->size(1) * 64 != K) Py_RETURN_NONE;
     const int64_t M = x->numel() / K;
-    if (M < 1 || (bias && bias->numel() != N)) Py_RETURN_NONE;
+    if (M < 1 || M > INT_MAX || N > INT_MAX || (bias && bias->numel() != N)) Py_RETURN_NONE;
     c10::SmallVector<int64_t, 5> sizes(x->sizes().begin(), x->sizes().end());
     sizes.back() = N;
     at::Tensor y = result(sizes, *x);
@@ -82,7 +84,9 @@ PyObject* qmm_tiled(PyObject* const* a, Py_ssize_t n) {
     const int dev = on_current(*x);
     if (dev < 0 || !same_device(dev, wt) || !same_device(dev, bias) || !same_device(dev, ws)) Py_RETURN_NONE;
     const int64_t M = x->size(0), K = x->size(1);
-    if (M < 1 || M > 32 || N < 8) Py_RETURN_NONE;
+    if (M < 1 || M > 32 || N < 8 || N > INT_MAX || K > INT_MAX || (bias && bias->numel() != N)) Py_RETURN_NONE;
+    const size_t need = b200_qmm_tiled_bytes((int)N, (int)K);
+    if (need == 0 || (size_t)wt->numel() < need) Py_RETURN_NONE;
     at::Tensor y = result({M, (int64_t)N}, *x);
     const int rc = b200_qmm_tiled(x->data_ptr(), wt->data_ptr(), nullptr, bias ? bias->data_ptr() : nullptr, nullptr, y.data_ptr(), (int)M, (int)N,
                                   (int)K, B200_EPI_NONE, ws->data_ptr(), (size_t)ws->numel(), stream_of(dev));

@@ -45,6 +45,34 @@ def _check_operands(x, w, s, b, group_size):
         raise _lib.B200Error("weight / scale / bias shapes do not match x")
 
 
+def _check_size(what, t, dtype, count):
+    """An optional operand or result: on the GPU, of this type, without gaps, with room for ``count`` values."""
+    if t is None:
+        return
+    _lib.require_cuda(t)
+    if t.dtype != dtype or not t.is_contiguous() or t.numel() < count:
+        raise _lib.B200Error(f"{what} must be a contiguous {str(dtype).removeprefix('torch.')} tensor of {count} values, "
+                             f"not {str(t.dtype).removeprefix('torch.')} {tuple(t.shape)}")
+
+
+def _check_tiled(x, wt, n, epilogue=EPI_NONE, wt2=None, bias=None, extra=None, out=None):
+    """Operands of a matmul on re-laid-out weights against the ``n`` rows and the K that x gives them."""
+    _lib.require_cuda(x, wt)
+    if x.dim() != 2 or x.dtype != torch.float16:
+        raise _lib.B200Error("x must be a float16 (M, K) tensor")
+    m, k = x.shape
+    if not (0 < n < 1 << 31) or k >= 1 << 31:
+        raise _lib.B200Error(f"matrix of {n} x {k}: both must be positive and fit an int")
+    need = _lib.lib().b200_qmm_tiled_bytes(n, k)
+    if need == 0:
+        raise _lib.B200Error(f"K must be a multiple of 128, not {k}")
+    _check_size("the re-laid-out weights", wt, torch.uint8, need)
+    _check_size("the second matrix", wt2, torch.uint8, need)
+    _check_size("bias", bias, torch.float16, n)
+    _check_size("extra", extra, torch.float16, m * n)
+    _check_size("out", out, torch.float32 if epilogue == EPI_F32 else torch.float16, m * n)
+
+
 def matmul(x, w, s, b, group_size=64, d_dtype=torch.float16, bias=None, **_ignored):
     """``[x @ dequant(w, s, b).T]`` with x ``(*B, K)`` fp16 and w ``(N, K/8)`` packed 4-bit."""
     if d_dtype is torch.float16 and isinstance(x, torch.Tensor):
@@ -59,7 +87,8 @@ def matmul(x, w, s, b, group_size=64, d_dtype=torch.float16, bias=None, **_ignor
     *lead, k = x.shape
     m = reduce(lambda a, c: a * c, lead, 1)
     n = w.shape[0]
-    x2 = x.reshape(m, k).contiguous()
+    _check_size("bias", bias, torch.float16, n)
+    x2, w, s, b = x.reshape(m, k).contiguous(), w.contiguous(), s.contiguous(), b.contiguous()
     y = torch.empty((m, n), dtype=torch.float16, device=x.device)
     ws = workspace(x.device)
     rc = _lib.lib().b200_qmm(_lib.ptr(x2), _lib.ptr(w), _lib.ptr(s), _lib.ptr(b), _lib.ptr(bias),
@@ -76,6 +105,15 @@ def matmul_fused(x, w, s, b, *, epilogue=EPI_NONE, w2=None, s2=None, b2=None, bi
     _check_operands(x, w, s, b, group_size)
     m, k = x.shape
     n = w.shape[0]
+    if epilogue == EPI_SILU_MUL and w2 is not None:
+        _check_operands(x, w2, s2, b2, group_size)
+        if w2.shape != w.shape:
+            raise _lib.B200Error("gate and up must have the same shape")
+    _check_size("bias", bias, torch.float16, n)
+    _check_size("extra", extra, torch.float16, m * n)
+    _check_size("out", out, torch.float16, m * n)
+    x, w, s, b = x.contiguous(), w.contiguous(), s.contiguous(), b.contiguous()
+    w2, s2, b2 = (None if t is None else t.contiguous() for t in (w2, s2, b2))
     y = out if out is not None else torch.empty((m, n), dtype=torch.float16, device=x.device)
     ws = workspace(x.device)
     rc = _lib.lib().b200_qmm_fused(_lib.ptr(x), _lib.ptr(w), _lib.ptr(s), _lib.ptr(b), _lib.ptr(w2),
@@ -97,6 +135,9 @@ def relayout(w, s, b) -> torch.Tensor:
     tensor; ``matmul_tiled`` consumes it."""
     _lib.require_cuda(w, s, b)
     n, k = w.shape[0], w.shape[1] * 8
+    _check_size("scales", s, torch.float16, n * k // 64)
+    _check_size("biases", b, torch.float16, n * k // 64)
+    w = w.contiguous()
     out = torch.empty(_lib.lib().b200_qmm_tiled_bytes(n, k), dtype=torch.uint8, device=w.device)
     rc = _lib.lib().b200_qmm_relayout(_lib.ptr(w), _lib.ptr(s), _lib.ptr(b), _lib.ptr(out), n, k,
                                       _lib.stream_ptr(w.device))
@@ -112,9 +153,10 @@ def matmul_tiled(x, wt, n, *, epilogue=EPI_NONE, wt2=None, bias=None, extra=None
             y = _lib.ops().qmm_tiled(x, wt, n, bias, ws)
             if y is not None:
                 return y
-    _lib.require_cuda(x, wt)
+    _check_tiled(x, wt, n, epilogue, wt2, bias, extra, out)
+    x = x.contiguous()
     m, k = x.shape
-    y = out if out is not None else torch.empty((m, n), dtype=torch.float16, device=x.device)
+    y = out if out is not None else torch.empty((m, n), dtype=torch.float32 if epilogue == EPI_F32 else torch.float16, device=x.device)
     ws = workspace(x.device)
     rc = _lib.lib().b200_qmm_tiled(_lib.ptr(x), _lib.ptr(wt), _lib.ptr(wt2), _lib.ptr(bias), _lib.ptr(extra),
                                    _lib.ptr(y), m, n, k, epilogue, _lib.ptr(ws), ws.numel(), _lib.stream_ptr(x.device))
@@ -133,7 +175,8 @@ _umma_ws = {}
 def matmul_umma(x, wt, n, *, bias=None, out=None):
     """``x (M<=128, K) @ W.T`` on re-laid-out weights ``wt`` through the tcgen05 tensor cores
     (``b200_qmm_umma``; ``n`` and K multiples of 128, plain epilogue)."""
-    _lib.require_cuda(x, wt)
+    _check_tiled(x, wt, n, bias=bias, out=out)
+    x = x.contiguous()
     m, k = x.shape
     y = out if out is not None else torch.empty((m, n), dtype=torch.float16, device=x.device)
     need = _lib.lib().b200_qmm_umma_workspace_bytes(m, k)

@@ -198,3 +198,35 @@ def test_rope_positions_vector_and_scalar_kernels(be, cuda, b, h, l, d):
     x1, x2 = x[..., : d // 2].double(), x[..., d // 2:].double()
     want = torch.cat([x1 * theta.cos() - x2 * theta.sin(), x1 * theta.sin() + x2 * theta.cos()], -1)
     assert torch.all((y.double() - want).abs() <= 2.0 ** -10 * want.abs() + 4e-3)
+
+
+def test_operands_that_do_not_fit_the_matrix_are_refused(be, cuda):
+    """Every size that the kernels take from a shape or an argument, against the tensor it would be read from or written to."""
+    qk, E = be.qmm_kernel, be._lib.B200Error
+    g = torch.Generator(device=cuda).manual_seed(0)
+    w, s, b = be.quantize.quantize(torch.randn(136, 256, generator=g, device=cuda) * 0.02)
+    wt = qk.relayout(w, s, b)
+    x = torch.randn(5, 256, generator=g, device=cuda).half()
+    half = lambda *shape: torch.zeros(*shape, dtype=torch.float16, device=cuda)
+    want = qk.matmul_tiled(x, wt, 136)
+    for bad in (lambda: qk.matmul_tiled(x, wt, 200), lambda: qk.matmul_tiled(x, wt, 136 + (1 << 32)), lambda: qk.matmul_tiled(x, wt[:-16], 136),
+                lambda: qk.matmul_tiled(half(5, 384), wt, 136), lambda: qk.matmul_tiled(x, wt, 136, bias=half(128)),
+                lambda: qk.matmul_tiled(x, wt, 136, bias=torch.zeros(136, device=cuda)), lambda: qk.matmul_tiled(x.float(), wt, 136),
+                lambda: qk.matmul_tiled(x, wt, 136, epilogue=qk.EPI_SILU_MUL, wt2=wt[:-16]), lambda: qk.matmul_tiled(x, wt, 136, out=half(4, 136)),
+                lambda: qk.matmul_tiled(x, wt, 136, epilogue=qk.EPI_RESIDUAL, extra=half(4, 136)),
+                lambda: qk.matmul_tiled(x, wt, 136, epilogue=qk.EPI_F32, out=half(5, 136)),
+                lambda: qk.matmul_umma(half(5, 256), wt, 256), lambda: qk.matmul(x, w, s, b, 64, bias=half(128)),
+                lambda: qk.matmul_fused(x, w, s, b, epilogue=qk.EPI_RESIDUAL, extra=half(5, 128)),
+                lambda: qk.matmul_fused(x, w, s, b, epilogue=qk.EPI_SILU_MUL, w2=w[:128], s2=s[:128], b2=b[:128])):
+        with pytest.raises(E):
+            bad()
+    # ... and what is laid out otherwise gives the same result
+    gaps = torch.zeros(5, 512, dtype=torch.float16, device=cuda)
+    gaps[:, ::2] = x
+    assert torch.equal(qk.matmul_tiled(gaps[:, ::2], wt, 136), want)
+    assert torch.equal(qk.matmul_tiled(x, torch.cat([wt, wt[:64]]), 136), want)
+    f32 = qk.matmul_tiled(x, wt, 136, epilogue=qk.EPI_F32)
+    assert f32.dtype == torch.float32 and torch.equal(f32.half(), want)
+    rows = qk.matmul(x, w, s, b, 64)[0]
+    columns = s.t().contiguous().t()
+    assert not columns.is_contiguous() and torch.equal(qk.matmul(x, w, columns, b, 64)[0], rows)
