@@ -14,19 +14,13 @@
 // token and query head) merges the key blocks in block order and writes fp16.  Key blocks past the current length exit at once, so
 // one launch shape serves a growing cache (CUDA-graph friendly: the length is read on the device).
 #include "common.cuh"
+#include "pipeline.cuh"
 
 namespace b200 {
 namespace {
 
 constexpr int kKeyBlock = 64;
 constexpr float kLog2e = 1.4426950408889634f;
-
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* smem_ptr) {
-    uint32_t addr = (uint32_t)__cvta_generic_to_shared(smem_ptr);
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr));
-}
 
 struct AttnParams {
     const __half* q;       // rotated queries inside the qkv activation buffer
@@ -166,7 +160,7 @@ __global__ void __launch_bounds__(128) tree_attention_kernel(const AttnParams p)
             for (int nd = 0; nd < HD / 8; nd += 2) {
                 uint32_t vb[4];
                 const __half* vp = sv + (kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * KS + (nd + (lane >> 4)) * 8;
-                ldmatrix_x4_trans(vb, vp);
+                ldsm4_t(vb, smem_u32(vp));
                 mma_m16n8k16(o[nd], pa[2 * kk][0], pa[2 * kk][1], pa[2 * kk + 1][0], pa[2 * kk + 1][1], vb[0], vb[1]);
                 mma_m16n8k16(o[nd + 1], pa[2 * kk][0], pa[2 * kk][1], pa[2 * kk + 1][0], pa[2 * kk + 1][1], vb[2], vb[3]);
             }

@@ -20,26 +20,22 @@
 
 #include <algorithm>
 #include <atomic>
-#include <type_traits>
 
 #include "common.cuh"
 #include "decode.cuh"
 #include "pipeline.cuh"
 #include "qmm_common.cuh"
 #include "tensor_map.cuh"
+#include "umma.cuh"
 
 namespace b200 {
 namespace {
 
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr int kRun = 4 * 1152;                   // the four records of a 64-row block for one chunk
-constexpr int kW = 2 * kRun;                     // weight bytes of a 128-row tile and chunk
-constexpr int kTile = 128;                       // weight rows of one MMA
 constexpr int kGroups = 3;                       // groups of four dequant warps, each with a tensor-memory tile of its own
 constexpr int kDeq = 4 * kGroups;                // dequant warps
 constexpr int kEpi = 8;                          // of which these run the epilogue
 constexpr int kDThreads = (kDeq + 4) * 32;       // + weight producer, activation producer, MMA issuer, sums of squares
-constexpr int kTCols = kChunkK / 2;              // tensor-memory columns of an expanded tile
 constexpr int kTmem = 256;                       // columns a CTA takes: two CTAs share an SM
 constexpr int kMaxCluster = 8;
 constexpr int kSsqPitch = 32, kCsPitch = 64, kKeyBlock = 64;
@@ -52,14 +48,14 @@ struct __align__(TQ * 4) Vec { float v[TQ]; };      // a value per token of a gr
 template <int NT, int TQ = 4>
 struct DGeo {
     static constexpr int X = NT * kChunkK * 2;                  // activations of a chunk: two boxes of 64 k
-    static constexpr int ACC = kGroups * kTCols;                  // accumulator columns: two of NT
+    static constexpr int ACC = kGroups * kTileCols;                  // accumulator columns: two of NT
     static constexpr int NW = 2 * kGroups;                       // weight stages (a multiple: a stage belongs to one of the groups)
     static constexpr int NX = NT == 16 ? 6 : 3;                  // activation stages
-    static constexpr int XOFF = NW * kW;
+    static constexpr int XOFF = NW * kTileW;
     // Partial products [source rank][group of TQ tokens of this CTA][row][TQ] fp32.  The groups go to the CTAs in turn, so at most 8
     // (of four tokens, up to 16), 14 (up to 32: 8 over 7 CTAs) or 8 (of two, up to 8) of them with their sources are here.
     static constexpr int INBOX = XOFF + NX * X;
-    static constexpr int SMEM = INBOX + (NT == 16 ? 8 : 14) * kTile * TQ * 4 + 1024;
+    static constexpr int SMEM = INBOX + (NT == 16 ? 8 : 14) * kTileRows * TQ * 4 + 1024;
     static_assert(XOFF % 1024 == 0 && 2 * (SMEM + 3072) <= 227 * 1024 && ACC + 2 * NT <= kTmem, "two CTAs per SM");
 };
 
@@ -103,19 +99,6 @@ template <typename T>
 __device__ __forceinline__ const T* listed(const void* const* entry) {
     return reinterpret_cast<const T*>(__ldcg(reinterpret_cast<const unsigned long long*>(entry)));
 }
-
-__device__ __forceinline__ uint64_t sw128(uint32_t saddr) {     // K-major, 128-byte swizzle: groups of 8 rows 1024 bytes apart
-    return (uint64_t)((saddr & 0x3ffffu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
-           ((uint64_t)2 << 61);
-}
-__device__ __forceinline__ void tma_box(uint32_t dst, const void* tmap, int x, int y, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
-                 ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void commit_to(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool fast_scale(uint32_t bits) { return ((bits >> 10) & 31u) - 1u < 10u; }   // range of dequant_pack_fast
 
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
@@ -203,7 +186,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         }
         if (lane == 31) {
             mbar_init(smem_u32(&inboxfull), 1);
-            if (cs > 1) mbar_expect_tx(smem_u32(&inboxfull), cs * nq * kTile * TQ * 4); // what the cluster's CTAs will store here
+            if (cs > 1) mbar_expect_tx(smem_u32(&inboxfull), cs * nq * kTileRows * TQ * 4); // what the cluster's CTAs will store here
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -211,18 +194,18 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
     const int nblocks = (p.N + 63) / 64;
     auto wsrc = [&](int tile, int second) {                      // chunk c_lo of the tile's first or second 64 rows (gate / up: of the same rows of each)
         const unsigned char* w = TABLE ? listed<unsigned char>(p.tw + (KIND == D_SILU ? second : 0)) : p.w[KIND == D_SILU ? second : 0];
-        return w + ((size_t)(KIND == D_SILU ? tile : min(2 * tile + second, nblocks - 1)) * nchunks + c_lo) * kRun;
+        return w + ((size_t)(KIND == D_SILU ? tile : min(2 * tile + second, nblocks - 1)) * nchunks + c_lo) * kRunBytes;
     };
     auto wload = [&](uint32_t slot, const unsigned char* src0, const unsigned char* src1) {
-        const uint32_t bar = smem_u32(wfull + slot), dst = smem_u32(ring + slot * kW);
-        mbar_expect_tx(bar, kW);
-        bulk_copy_g2s(dst, src0, kRun, bar);
-        bulk_copy_g2s(dst + kRun, src1, kRun, bar);
+        const uint32_t bar = smem_u32(wfull + slot), dst = smem_u32(ring + slot * kTileW);
+        mbar_expect_tx(bar, kTileW);
+        bulk_copy_g2s(dst, src0, kRunBytes, bar);
+        bulk_copy_g2s(dst + kRunBytes, src1, kRunBytes, bar);
     };
     auto wload_rows = [&](uint32_t slot, int tile, int c) {
         const uint32_t bar = smem_u32(wfull + slot);
-        mbar_expect_tx(bar, kTile * 64);
-        tma_box(smem_u32(ring + slot * kW), &p.wmap, (c_lo + c) * 64, tile * kTile, bar);
+        mbar_expect_tx(bar, kTileRows * 64);
+        tma_box(smem_u32(ring + slot * kTileW), &p.wmap, (c_lo + c) * 64, tile * kTileRows, bar);
     };
     if (warp == kDeq) {
         if (lane < G::NW) {
@@ -237,7 +220,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
 #pragma unroll 1
             for (int c = 0; c < min(nc, G::NW); c++) {
                 if (KIND == D_ROWS) wload_rows(c, tile0, c);
-                else wload(c, src0 + c * kRun, src1 + c * kRun);
+                else wload(c, src0 + c * kRunBytes, src1 + c * kRunBytes);
             }
         }
         __syncwarp();
@@ -263,7 +246,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
 #pragma unroll 1
         for (int it = 0, tile = tile0; it < nit; it++, tile += tstep) {
             const int c0 = it == 0 ? first : 0;
-            const unsigned char *src0 = wsrc(tile, 0) + c0 * kRun, *src1 = wsrc(tile, 1) + c0 * kRun;
+            const unsigned char *src0 = wsrc(tile, 0) + c0 * kRunBytes, *src1 = wsrc(tile, 1) + c0 * kRunBytes;
 #pragma unroll 1
             for (int c = c0; c < nc; c++) {
                 if (lap) mbar_wait_reported(smem_u32(wempty + slot), ph, p.polls, p.err, 21);
@@ -273,8 +256,8 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                     else wload(slot, src0, src1);
                 }
                 __syncwarp();
-                src0 += kRun;
-                src1 += kRun;
+                src0 += kRunBytes;
+                src1 += kRunBytes;
                 if (++slot == (uint32_t)G::NW) { slot = 0; ph ^= 1; lap = true; }
             }
         }
@@ -299,8 +282,8 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
             }
     } else if (warp == kDeq + 2) {
         // ------------------------------------------------------------------ MMA issuer (an elected thread)
-        constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(kTile >> 4) << 24);
-        const uint64_t xdesc = sw128(smem_u32(ring + G::XOFF));
+        constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(kTileRows >> 4) << 24);
+        const uint64_t xdesc = sw128_desc(smem_u32(ring + G::XOFF));
         uint32_t tl = 0, tph = 0, slot = 0, xph = 0;
 #pragma unroll 1
         for (int it = 0; it < nit; it++) {
@@ -314,7 +297,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                 __syncwarp();
                 if (elect_one()) {                               // (~285 cycles a batch; of half the size, 280)
                     const uint64_t b0 = xdesc + slot * (G::X / 16);
-                    const uint32_t a0 = tmem + tl * kTCols;
+                    const uint32_t a0 = tmem + tl * kTileCols;
                     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d0),
                                  "r"(a0), "l"(b0), "r"(idesc), "r"(c) : "memory");
 #pragma unroll
@@ -365,7 +348,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         // ------------------------------------------------------------------ dequant warps
         const uint32_t me = warp >> 2;                           // group (and, in the epilogue, which half of the tokens)
         const int q = warp & 3, r = q * 32 + lane, rr = r & 15;
-        const uint32_t recoff = (r >> 6) * kRun + ((r >> 4) & 3) * 1152;
+        const uint32_t recoff = (r >> 6) * kRunBytes + ((r >> 4) & 3) * kRecBytes;
         const uint32_t rowoff = KIND == D_ROWS ? r * 64 + (((r >> 1) & 3) << 4) : recoff + (rr >> 3) * 512 + (rr & 7) * 64, scoff = recoff + 1024 + rr * 8;
         const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
         // (Four threads of a quarter-warp read the same banks: swapping units between threads to halve that took more issue slots, 16
@@ -380,7 +363,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
             const int r2 = KIND == D_SILU ? threadIdx.x & 63 : threadIdx.x & 127;     // row inside the tile that this thread finishes
             const int j0 = KIND == D_SILU ? threadIdx.x >> 6 : threadIdx.x >> 7;      // its first quad of this CTA's, and the step
             constexpr int JS = KIND == D_SILU ? 4 : 2;
-            const int n = (KIND == D_SILU ? tile * 64 : tile * kTile) + r2;
+            const int n = (KIND == D_SILU ? tile * 64 : tile * kTileRows) + r2;
             const bool valid = n < p.N;
             // what the output needs besides the product, asked for now: norm weight or bias, the first quad's residuals or rotations
             const int half = p.hd >> 1, hi = r2 & (p.hd - 1), head = KIND == D_QKV ? n >> (p.hd == 128 ? 7 : 6) : 0;
@@ -402,7 +385,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
             if (KIND == D_RESID && valid) extra = wn[n];
             if ((KIND == D_QKV || KIND == D_PLAIN || KIND == D_ROWS) && valid && bias != nullptr) {
                 extra = bias[n];
-                if (KIND == D_QKV) extra2 = bias[tile * kTile + pr];
+                if (KIND == D_QKV) extra2 = bias[tile * kTileRows + pr];
             }
             if (j0 < nq) ask(j0);
 
@@ -429,7 +412,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                         V x;
 #pragma unroll
                         for (int k = 0; k < TQ; k++) x.v[k] = __uint_as_float(a[i + k]);
-                        inbox[((int)me * C + i) / TQ * kTile + r] = x;
+                        inbox[((int)me * C + i) / TQ * kTileRows + r] = x;
                     }
                 consumer_sync(kEpi * 32);
             } else {
@@ -441,7 +424,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
 #pragma unroll
                 for (int i = 0; i < C; i += TQ) {
                     if ((int)me * C + i < p.M)
-                        st_async<TQ>(peer_addr(in0 + ((rank * qslots + sl) * kTile + r) * (TQ * 4), dst), a + i, peer_addr(inbar, dst));
+                        st_async<TQ>(peer_addr(in0 + ((rank * qslots + sl) * kTileRows + r) * (TQ * 4), dst), a + i, peer_addr(inbar, dst));
                     if (++dst == cs) { dst = 0; sl++; }
                 }
                 inbox_wait(inbar, p.polls, p.err, 28);
@@ -454,11 +437,11 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                 if (j != j0) ask(j);
                 // the sources in rank order: this row, and the up row or the one it is rotated with
                 const int r3 = KIND == D_SILU ? r2 + 64 : pr;
-                V v = inbox[j * kTile + r2], w = v;
-                if (KIND == D_SILU || KIND == D_QKV) w = inbox[j * kTile + r3];
+                V v = inbox[j * kTileRows + r2], w = v;
+                if (KIND == D_SILU || KIND == D_QKV) w = inbox[j * kTileRows + r3];
 #pragma unroll 1
                 for (int i = 1; i < (int)cs; i++) {
-                    const V* src = inbox + (i * qslots + j) * kTile;
+                    const V* src = inbox + (i * qslots + j) * kTileRows;
                     const V x = src[r2];
 #pragma unroll
                     for (int k = 0; k < TQ; k++) v.v[k] += x.v[k];
@@ -536,7 +519,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         auto ask_scales = [&]() {
             while (ask_c >= nc && ask_tile < p.tiles) { ask_c -= nc; ask_tile += tstep; }
             if (ask_tile < p.tiles) {
-                const size_t at = (size_t)min(ask_tile * kTile + r, p.N - 1) * (p.K / 64) + 2 * (c_lo + ask_c);
+                const size_t at = (size_t)min(ask_tile * kTileRows + r, p.N - 1) * (p.K / 64) + 2 * (c_lo + ask_c);
                 next_s = __ldg(reinterpret_cast<const uint32_t*>(p.sc + at));
                 next_b = __ldg(reinterpret_cast<const uint32_t*>(p.bi + at));
             }
@@ -556,48 +539,25 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                 if (done < end) {
                     mbar_wait_reported(smem_u32(wfull + slot), wph, p.polls, p.err, 24);
                     __syncwarp();
-                    const unsigned char* st = ring + slot * kW;
+                    const unsigned char* st = ring + slot * kTileW;
                     uint4 u[4];
 #pragma unroll
                     for (int i = 0; i < 4; i++) u[i] = *reinterpret_cast<const uint4*>(st + (KIND == D_ROWS ? rowoff ^ (i * 16) : rowoff + i * 16));
-                    uint2 sb;                                    // (scale, bias) of the chunk's two groups
+                    uint32_t sc[2], bi[2];                       // scale and bias of the chunk's two groups, low halves
                     if (KIND == D_ROWS) {
-                        sb = make_uint2(__byte_perm(next_s, next_b, 0x5410), __byte_perm(next_s, next_b, 0x7632));
+                        sc[0] = next_s; sc[1] = next_s >> 16;
+                        bi[0] = next_b; bi[1] = next_b >> 16;
                         ask_scales();
                     } else {
-                        sb = *reinterpret_cast<const uint2*>(st + scoff);
+                        const uint2 sb = *reinterpret_cast<const uint2*>(st + scoff);
+                        sc[0] = sb.x; bi[0] = sb.x >> 16;
+                        sc[1] = sb.y; bi[1] = sb.y >> 16;
                     }
-                    const bool fast = __all_sync(0xffffffffu, fast_scale(sb.x) && fast_scale(sb.y));
+                    const bool fast = __all_sync(0xffffffffu, fast_scale(sc[0]) && fast_scale(sc[1]));
                     if (done >= kGroups) mbar_wait_reported(smem_u32(tfree + me), tph, p.polls, p.err, 24);
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                     __syncwarp();
-                    auto expand = [&](auto fast_tag) {
-                        constexpr bool FAST = decltype(fast_tag)::value;
-#pragma unroll
-                        for (int j = 0; j < 4; j++) {            // pack j of unit t (D_ROWS: pack t of unit j) = k group 4 j + t
-                            const uint32_t s = j < 2 ? sb.x : sb.y;
-                            __half2 s2 = dup_half((unsigned short)s);
-                            const __half2 b2 = dup_half((unsigned short)(s >> 16));
-                            if (FAST) s2 = scale_times_2_20(s2);
-                            uint32_t d[4][4];
-#pragma unroll
-                            for (int t = 0; t < 4; t++) {
-                                const uint32_t pack = KIND == D_ROWS ? comp(u[j], t) : comp(u[t], j);
-                                if (FAST) dequant_pack_fast(pack, s2, b2, d[t]);
-                                else dequant_pack(pack, s2, b2, d[t]);
-                                if (KIND == D_ROWS) {            // {e0,e4} {e1,e5} {e2,e6} {e3,e7} -> adjacent k pairs
-                                    const uint32_t e01 = __byte_perm(d[t][0], d[t][1], 0x5410), e45 = __byte_perm(d[t][0], d[t][1], 0x7632);
-                                    const uint32_t e23 = __byte_perm(d[t][2], d[t][3], 0x5410), e67 = __byte_perm(d[t][2], d[t][3], 0x7632);
-                                    d[t][0] = e01; d[t][1] = e23; d[t][2] = e45; d[t][3] = e67;
-                                }
-                            }
-                            asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(trow + me * kTCols + 16 * j),
-                                         "r"(d[0][0]), "r"(d[0][1]), "r"(d[0][2]), "r"(d[0][3]), "r"(d[1][0]), "r"(d[1][1]), "r"(d[1][2]), "r"(d[1][3]),
-                                         "r"(d[2][0]), "r"(d[2][1]), "r"(d[2][2]), "r"(d[2][3]), "r"(d[3][0]), "r"(d[3][1]), "r"(d[3][2]), "r"(d[3][3]) : "memory");
-                        }
-                    };
-                    if (fast) expand(std::true_type{});
-                    else expand(std::false_type{});
+                    expand_row<KIND == D_ROWS>(u, sc, bi, fast, trow + me * kTileCols);
                     // Only now that the packs have been used: an arrival right behind the loads does not wait for them, and the next tile's
                     // weights were there before the last of them were through (some rows of one stage in 1e8; 46 wrong passes of 200000).
                     __syncwarp();
@@ -692,13 +652,6 @@ struct DAttn {
 __device__ __forceinline__ uint32_t kv_swz(int r, int v) {     // 16-byte vector v of row r of a block (boxes of 8 vectors side by side)
     return (uint32_t)((v >> 3) * 8192 + r * 128 + (((v & 7) ^ (r & 7)) << 4));
 }
-__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-
 constexpr int kAWarps = 8, kAParts = 4;            // warps of an attention CTA, warps that share a row tile
 template <int HD>
 struct DAGeo {
@@ -1017,7 +970,7 @@ int launch_dense(DenseParams& p, int split, cudaStream_t stream) {
     static std::atomic<uint64_t> done{0};
     if (!allow_smem(dense_kernel<NT, KIND, TQ, TABLE>, DGeo<NT, TQ>::SMEM, done, KIND != D_ROWS)) return check_launch();
     const int nch = p.K / kChunkK;
-    const int tiles = KIND == D_SILU ? p.N / 64 : (p.N + kTile - 1) / kTile;
+    const int tiles = KIND == D_SILU ? p.N / 64 : (p.N + kTileRows - 1) / kTileRows;
     const int cs = split > 0 && split <= std::min(kMaxCluster, nch) ? split : plan_cluster(tiles, nch, p.M, TQ);
     constexpr int cap = 296;
     auto launch = [&](int lo, int n, int cluster) {
@@ -1146,7 +1099,7 @@ int run_matmul(const ChainMatmul& c, cudaStream_t st) {
     }
     p.sc = static_cast<const __half*>(c.scales);
     p.bi = static_cast<const __half*>(c.biases);
-    rc = make_map_2d(&p.wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, c.w, c.K / 2, c.N, c.K / 2, 64, kTile, CU_TENSOR_MAP_SWIZZLE_64B,
+    rc = make_map_2d(&p.wmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, c.w, c.K / 2, c.N, c.K / 2, 64, kTileRows, CU_TENSOR_MAP_SWIZZLE_64B,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
     return rc != B200_OK ? rc : launch_dense<NT, TQ, D_ROWS>(p, 0, st);
 }

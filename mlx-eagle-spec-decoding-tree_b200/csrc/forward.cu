@@ -37,8 +37,9 @@
 
 #include "decode.cuh"
 #include "pipeline.cuh"
-#include "tp_layout.cuh"
 #include "qmm_common.cuh"
+#include "tensor_map.cuh"
+#include "tp_layout.cuh"
 
 namespace b200 {
 namespace {
@@ -219,13 +220,6 @@ __device__ __forceinline__ long long global_ns() {
 __device__ __forceinline__ void stamp(const FwdParams& p, const Ctx& c, int k) {
     if (p.timeline != nullptr && threadIdx.x == 0 && (int)c.epoch < p.timeline_pitch)
         p.timeline[((size_t)blockIdx.x * p.timeline_pitch + c.epoch) * 8 + k] = clock64();   // SM cycles
-}
-
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* smem_ptr) {
-    uint32_t addr = (uint32_t)__cvta_generic_to_shared(smem_ptr);
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr));
 }
 
 __device__ __forceinline__ int atom_add_acq_rel_gpu(int* addr, int v) {
@@ -1311,7 +1305,7 @@ __device__ __forceinline__ void attn_consume(const FwdParams& p, Ctx& c, const A
                     for (int nd = 0; nd < HD / 8; nd += 2) {
                         uint32_t vb[4];
                         const __half* vp = sv + (kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * KS + (nd + (lane >> 4)) * 8;
-                        ldmatrix_x4_trans(vb, vp);
+                        ldsm4_t(vb, smem_u32(vp));
                         mma_m16n8k16(o[nd], pa[2 * kk][0], pa[2 * kk][1], pa[2 * kk + 1][0], pa[2 * kk + 1][1], vb[0], vb[1]);
                         mma_m16n8k16(o[nd + 1], pa[2 * kk][0], pa[2 * kk][1], pa[2 * kk + 1][0], pa[2 * kk + 1][1], vb[2], vb[3]);
                     }
@@ -1346,21 +1340,6 @@ __device__ __forceinline__ void attn_consume(const FwdParams& p, Ctx& c, const A
 constexpr int kASlotsMax = 8;
 constexpr int kBox = 64 * 128;                // bytes of one 64-row x 128-byte TMA box
 
-__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr));
-}
-__device__ __forceinline__ void ldmatrix_x4_trans_u(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr));
-}
-// 2-D tiled TMA load: box at (x = column in halves, y = row) of the tensor map -> shared memory.
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, int x, int y, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
-                 ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(bar) : "memory");
-}
 // Byte offset of 16-byte vector v (of HD/8) of row r inside a swizzled K or V block (boxes of 8 vectors side by side).
 __device__ __forceinline__ uint32_t swz(int r, int v) {
     return (uint32_t)((v >> 3) * kBox + r * 128 + (((v & 7) ^ (r & 7)) << 4));
@@ -1407,7 +1386,7 @@ __device__ __forceinline__ void attn_bp_produce(const FwdParams& p, Ctx& c, cons
             __syncwarp();
             if (lane < 2 * A::NBX) {                  // K boxes, then V boxes
                 const int isv = lane / A::NBX, bx = lane - isv * A::NBX;
-                tma_load_2d(sk + lane * kBox, &p.kvmap, bx * 64, (isv ? vrow0 : krow0) + kb * kKeyBlock, fbar);
+                tma_box(sk + lane * kBox, &p.kvmap, bx * 64, (isv ? vrow0 : krow0) + kb * kKeyBlock, fbar);
             }
         }
     }
@@ -1571,13 +1550,13 @@ __device__ __forceinline__ void attn_bp_consume(const FwdParams& p, Ctx& c, cons
 #pragma unroll
                     for (int ks = 0; ks < HD / 16; ks += 2) {
                         uint32_t qa0[4], qa1[4];
-                        ldmatrix_x4(qa0, sq_frag + ks * 32);
-                        ldmatrix_x4(qa1, sq_frag + ks * 32 + 32);
+                        ldsm4(qa0, sq_frag + ks * 32);
+                        ldsm4(qa1, sq_frag + ks * 32 + 32);
 #pragma unroll
                         for (int nt = 0; nt < 4; nt++) {
                             uint32_t kf[4];
                             // matrices: (keys, hd ks*16..+8), (keys, +8), (keys, (ks+1)*16..+8), (keys, +8)
-                            ldmatrix_x4(kf, sk + swz(half * 32 + nt * 8 + (lane & 7), ks * 2 + (lane >> 3)));
+                            ldsm4(kf, sk + swz(half * 32 + nt * 8 + (lane & 7), ks * 2 + (lane >> 3)));
                             mma_m16n8k16(s[nt], qa0[0], qa0[1], qa0[2], qa0[3], kf[0], kf[1]);
                             mma_m16n8k16(s[nt], qa1[0], qa1[1], qa1[2], qa1[3], kf[2], kf[3]);
                         }
@@ -1648,7 +1627,7 @@ __device__ __forceinline__ void attn_bp_consume(const FwdParams& p, Ctx& c, cons
 #pragma unroll
                         for (int nd = 0; nd < HD / 8; nd += 2) {
                             uint32_t vb[4];
-                            ldmatrix_x4_trans_u(vb, sv + swz(half * 32 + kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), nd + (lane >> 4)));
+                            ldsm4_t(vb, sv + swz(half * 32 + kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), nd + (lane >> 4)));
                             mma_m16n8k16(o[nd], pa[2 * kk][0], pa[2 * kk][1], pa[2 * kk + 1][0], pa[2 * kk + 1][1], vb[0], vb[1]);
                             mma_m16n8k16(o[nd + 1], pa[2 * kk][0], pa[2 * kk][1], pa[2 * kk + 1][0], pa[2 * kk + 1][1], vb[2], vb[3]);
                         }
@@ -2124,43 +2103,11 @@ WsLayout fwd_layout(const b200_forward_desc* d, PhasePlan (&plan)[5], int* grid_
     return w;
 }
 
-// cuTensorMapEncodeTiled through the runtime's driver entry point lookup (no link against libcuda).
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn g_encode_tiled = nullptr;
-
-int make_kv_map(CUtensorMap* map, void* cache, int layers, int hkv, int cap, int hd) {
-    if (g_encode_tiled == nullptr) {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess || fn == nullptr)
-            return check_launch() == B200_OK ? B200_ECUDA : B200_ECUDA;
-        g_encode_tiled = reinterpret_cast<EncodeTiledFn>(fn);
-    }
-    const cuuint64_t dims[2] = {(cuuint64_t)hd, (cuuint64_t)layers * 2 * hkv * cap};
-    const cuuint64_t strides[1] = {(cuuint64_t)hd * 2};
-    const cuuint32_t box[2] = {64, 64};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = g_encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, cache, dims, strides, box, estr,
-                                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        g_last_cuda_error = (int)r;
-        return B200_ECUDA;
-    }
-    return B200_OK;
-}
-
 template <int MT, int HD>
 int launch_forward(const FwdParams& p, int grid, cudaStream_t stream) {
     auto kern = forward_kernel<MT, HD>;
-    bool attr_set = false;
-    if (!attr_set) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<MT>::SMEM) != cudaSuccess)
-            return check_launch();
-        attr_set = true;
-    }
+    static std::atomic<uint64_t> done{0};
+    if (!allow_smem(kern, Geo<MT>::SMEM, done)) return check_launch();
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kFwdThreads);
@@ -2265,7 +2212,9 @@ int b200_forward(const b200_forward_desc* d, void* stream) {
     p.partial = reinterpret_cast<float*>(ws + w.partial);
     p.nkb = w.nkb; p.qrp = w.qrp;
     {
-        const int rc = make_kv_map(&p.kvmap, d->kv_cache, d->n_layers, d->n_kv_heads, d->cache_rows, d->head_dim);
+        const int rc = make_map_2d(&p.kvmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, d->kv_cache, d->head_dim,
+                                   (uint64_t)d->n_layers * 2 * d->n_kv_heads * d->cache_rows, (uint64_t)d->head_dim * 2, 64, 64,
+                                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
         if (rc != B200_OK) return rc;
     }
     p.head_rows = d->head_rows > 0 ? d->head_rows : d->vocab;

@@ -7,8 +7,6 @@
 
 namespace b200 {
 
-constexpr uint32_t kWaitLimit = 1u << 18;   // polls before a bounded mbarrier wait gives up
-
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -26,13 +24,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait: returns false if the barrier did not complete within the iteration limit.
-__device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity) {
-    for (uint32_t i = 0; i < kWaitLimit; i++)
-        if (mbar_try_wait(bar, parity)) return true;
-    return false;
-}
-// Same, with the iteration limit given: a poll that does not find the phase complete suspends the thread for up to about a
+// Bounded wait: false if the phase did not complete within `polls`.  A poll that does not find the phase complete suspends the thread for up to about a
 // microsecond, so the limit is a time limit.  (Without a suspend-time hint a complete phase is seen in 14 cycles and a
 // suspended thread is back ~60 cycles after the arrival; with a hint the same two took 100 and 75 to 100 cycles.)
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t polls) {
@@ -88,16 +80,23 @@ __device__ __forceinline__ void bulk_copy_g2s_hint(uint32_t dst, const void* src
                  "l"(src), "r"(bytes), "r"(bar), "l"(policy)
                  : "memory");
 }
+// 2-D tiled TMA load: box at (x, y) of the tensor map -> shared memory.
+__device__ __forceinline__ void tma_box(uint32_t dst, const void* tmap, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
+                 ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
-}
-// Arrive on `bar` once all cp.async issued so far by this thread have landed (count pre-charged at init).
-__device__ __forceinline__ void cp_async_arrive_noinc(uint32_t bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void consumer_sync(int nthreads) {       // named barrier 1: consumer warps only
     asm volatile("bar.sync 1, %0;\n" ::"r"(nthreads) : "memory");

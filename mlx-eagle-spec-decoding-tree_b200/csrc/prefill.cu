@@ -21,15 +21,6 @@ namespace {
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr int kKeyBlock = 64;
 
-__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-
 __device__ __forceinline__ float block_sum(float v) {
     __shared__ float red[32];
 #pragma unroll
@@ -239,7 +230,7 @@ __global__ void __launch_bounds__(256) prefill_attention_kernel(const PAttn p) {
 #pragma unroll
                 for (int nt = 0; nt < 8; nt++) {
                     uint32_t kf[4];
-                    ldsm_x4(kf, sk + pswz(nt * 8 + (lane & 7), ks * 2 + (lane >> 3), HD));
+                    ldsm4(kf, sk + pswz(nt * 8 + (lane & 7), ks * 2 + (lane >> 3), HD));
                     mma_m16n8k16(s[nt], qa[ks][0], qa[ks][1], qa[ks][2], qa[ks][3], kf[0], kf[1]);
                     mma_m16n8k16(s[nt], qa[ks + 1][0], qa[ks + 1][1], qa[ks + 1][2], qa[ks + 1][3], kf[2], kf[3]);
                 }
@@ -297,7 +288,7 @@ __global__ void __launch_bounds__(256) prefill_attention_kernel(const PAttn p) {
 #pragma unroll
                 for (int nd = 0; nd < HD / 8; nd += 2) {
                     uint32_t vb[4];
-                    ldsm_x4_t(vb, sv + pswz(kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), nd + (lane >> 4), HD));
+                    ldsm4_t(vb, sv + pswz(kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), nd + (lane >> 4), HD));
                     mma_m16n8k16(o[nd], pa[2 * kk][0], pa[2 * kk][1], pa[2 * kk + 1][0], pa[2 * kk + 1][1], vb[0], vb[1]);
                     mma_m16n8k16(o[nd + 1], pa[2 * kk][0], pa[2 * kk][1], pa[2 * kk + 1][0], pa[2 * kk + 1][1], vb[2], vb[3]);
                 }

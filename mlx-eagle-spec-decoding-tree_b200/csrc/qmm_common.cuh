@@ -1,5 +1,4 @@
-// Pieces shared by the two quantised-matmul kernels (row-major weights / tiled weights): problem
-// description, nibble expansion, and the rounding points of the fused epilogues.
+// Pieces shared by all quantised-matmul kernels: sizes, nibble expansion, and the rounding points of the fused epilogues.
 #pragma once
 
 #include "common.cuh"
@@ -9,22 +8,6 @@ namespace b200 {
 constexpr int kChunkK = 128;          // k values one warp iteration covers
 constexpr int kCounterBytes = 4096;   // head of the workspace: one int per row tile
 constexpr int kMaxCounters = kCounterBytes / 4;
-
-struct QmmParams {
-    const __half* x;
-    const uint32_t* wq[2];
-    const __half* sc[2];
-    const __half* bi[2];
-    const __half* bias;
-    const __half* extra;
-    __half* y;
-    float* partial;
-    int* counter;
-    int M, N, K;
-    int chunks_per_split;
-    int splits;
-    int epilogue;
-};
 
 __device__ __forceinline__ __half2 dup_half(unsigned short bits) {
     uint32_t u = (uint32_t)bits | ((uint32_t)bits << 16);
@@ -64,6 +47,7 @@ __device__ __forceinline__ void dequant_pack_fast(uint32_t w, __half2 s20, __hal
     d[2] = h2_as_u32(__hfma2(__hmul2(u32_as_h2(w8 & kLow), k16), s20, b2));
     d[3] = h2_as_u32(__hfma2(u32_as_h2(w8 & kNib), s20, b2));
 }
+__device__ __forceinline__ bool fast_scale(uint32_t bits) { return ((bits >> 10) & 31u) - 1u < 10u; }   // (of the low half)
 __device__ __forceinline__ __half2 scale_times_2_20(__half2 s2) { return u32_as_h2(h2_as_u32(s2) + 0x50005000u); }
 
 __device__ __forceinline__ uint32_t comp(const uint4& v, int j) {

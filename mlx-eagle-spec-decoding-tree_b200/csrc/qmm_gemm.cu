@@ -31,7 +31,6 @@
 
 #include <algorithm>
 #include <cstdint>
-#include <type_traits>
 
 #include "b200_eagle.h"
 #include "common.cuh"
@@ -39,17 +38,13 @@
 #include "qmm_common.cuh"
 #include "qmm_gemm.cuh"
 #include "tensor_map.cuh"
+#include "umma.cuh"
 
 namespace b200 {
 namespace {
 
-constexpr int kRecBytes = 1152;
-constexpr int kRunBytes = 4 * kRecBytes;         // the four records of a 64-row block for one chunk
-constexpr int kTileRows = 128;                   // weight rows of one MMA
-constexpr int kTileW = 2 * kRunBytes;            // weight bytes of a row tile and chunk (both layouts: 8192 + 1024)
 constexpr int kDeqWarps = 16;
 constexpr int kGroups = 4;                       // groups of four dequant warps, each with a tensor-memory tile of its own
-constexpr int kTileCols = kChunkK / 2;           // columns of a tile: two k values per column
 constexpr int kGThreads = (kDeqWarps + 4) * 32;  // + two producer warps + two MMA warps
 constexpr size_t kUmmaPartialBytes = 16u << 20;  // room for the partial products of a K split behind b200_qmm_umma
 constexpr int kGemmTiles = 896;                  // tiles that a K split can hand tickets to
@@ -93,21 +88,6 @@ struct GParams {
     int epilogue;
 };
 
-// K-major shared-memory matrix, 128-byte swizzle: rows of 128 bytes, groups of 8 rows 1024 bytes apart.
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
-    return (uint64_t)((saddr & 0x3ffffu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
-           ((uint64_t)2 << 61);
-}
-
-__device__ __forceinline__ void tma_box(uint32_t dst, const void* tmap, int x, int y, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
-                 ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&d)[4][4]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(addr),
-                 "r"(d[0][0]), "r"(d[0][1]), "r"(d[0][2]), "r"(d[0][3]), "r"(d[1][0]), "r"(d[1][1]), "r"(d[1][2]), "r"(d[1][3]),
-                 "r"(d[2][0]), "r"(d[2][1]), "r"(d[2][2]), "r"(d[2][3]), "r"(d[3][0]), "r"(d[3][1]), "r"(d[3][2]), "r"(d[3][3]) : "memory");
-}
 template <int C>
 __device__ __forceinline__ void tmem_ld(uint32_t (&r)[C], uint32_t addr) {
     static_assert(C % 8 == 0 || C == 4, "columns");
@@ -122,9 +102,6 @@ __device__ __forceinline__ void tmem_ld(uint32_t (&r)[C], uint32_t addr) {
                      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
     }
 }
-
-// True when the fp16 exponent field is in 1..10: the range of dequant_pack_fast.
-__device__ __forceinline__ bool fast_scale(uint32_t bits) { return ((bits >> 10) & 31u) - 1u < 10u; }
 
 struct GItem {
     int row_item, tok0, split, c_begin, nc;
@@ -416,14 +393,13 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
                             "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d0),
                             "r"(a0 + ks * 8), "l"(b0 + ((ks >> 2) * (NT * 128) + (ks & 3) * 32) / 16), "r"(idesc), "r"(ks == 0 ? accumulate : 1u)
                             : "memory");
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(tfree + ts)) : "memory");
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(pempty + slot)) : "memory");
+                    commit_to(smem_u32(tfree + ts));
+                    commit_to(smem_u32(pempty + slot));
                 }
                 __syncwarp();
                 first = false;
             }
-            if (elect_one())
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(accfull + ab)) : "memory");
+            if (elect_one()) commit_to(smem_u32(accfull + ab));
             __syncwarp();
             n += g.nc;
         }
@@ -501,32 +477,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
                     bi2[0] = bv; bi2[1] = bv >> 16;
                 }
                 const bool fast = __all_sync(0xffffffffu, fast_scale(sc2[0]) && fast_scale(sc2[1]));
-                auto expand = [&](auto fast_tag) {
-                    constexpr bool FAST = decltype(fast_tag)::value;
-                    // sixteen columns (32 k values) at a time.  Streaming layout: pack j of unit t is k group 4 j + t;
-                    // row-major: pack t of unit j.
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        __half2 s2 = dup_half((unsigned short)sc2[j >> 1]);
-                        const __half2 b2 = dup_half((unsigned short)bi2[j >> 1]);
-                        if (FAST) s2 = scale_times_2_20(s2);
-                        uint32_t d[4][4];
-#pragma unroll
-                        for (int t = 0; t < 4; t++) {
-                            const uint32_t pack = LAYOUT == W_TILED ? comp(u[t], j) : comp(u[j], t);
-                            if (FAST) dequant_pack_fast(pack, s2, b2, d[t]);
-                            else dequant_pack(pack, s2, b2, d[t]);
-                            if (LAYOUT == W_ROWS) {   // {e0,e4} {e1,e5} {e2,e6} {e3,e7} -> adjacent k pairs
-                                const uint32_t e01 = __byte_perm(d[t][0], d[t][1], 0x5410), e45 = __byte_perm(d[t][0], d[t][1], 0x7632);
-                                const uint32_t e23 = __byte_perm(d[t][2], d[t][3], 0x5410), e67 = __byte_perm(d[t][2], d[t][3], 0x7632);
-                                d[t][0] = e01; d[t][1] = e23; d[t][2] = e45; d[t][3] = e67;
-                            }
-                        }
-                        tmem_st16(trow + 16 * j, d);
-                    }
-                };
-                if (fast) expand(std::true_type{});
-                else expand(std::false_type{});
+                expand_row<LAYOUT == W_ROWS>(u, sc2, bi2, fast, trow);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(pempty + slot));       // the packs are in registers
                 asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
