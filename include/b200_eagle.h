@@ -59,8 +59,9 @@ void b200_set_wait_limit(unsigned int polls);
  * graphs of passes makes them anew when it has. */
 unsigned int b200_launch_settings(void);
 
-/* Bytes of scratch b200_qmm / b200_qmm_fused want for a given problem (split-K partial sums and
- * tile counters).  0 means the problem runs without scratch. */
+/* Bytes of scratch for b200_qmm / b200_qmm_fused (split-K partial sums and tile counters).  Up to 32 rows these are the sizes
+ * of an earlier split, kept so that buffers and refusals (b200_qmm_noalloc) stay as they are; the split in use fits itself
+ * to the room it gets (b200_qmm_gemm_workspace_bytes says how much it can use).  0 means the problem needs no scratch. */
 size_t b200_qmm_workspace_bytes(int M, int N, int K);
 
 /*
@@ -104,10 +105,10 @@ int b200_qmm_fused(const void* x, const uint32_t* wq, const void* scales, const 
  * the split-K scratch is a fixed 4 MiB array inside the library image instead of a caller buffer:
  * nothing is allocated or freed, by this call or by anything it calls.  Every GPU that loads the
  * library carries those 4 MiB until the process exits.
- *   - Problems whose split-K scratch for the plain product (what b200_qmm itself would use; the
- *     gate/up pair counted by b200_qmm_workspace_bytes does not run here) exceeds
- *     b200_qmm_noalloc_max_scratch_bytes() are refused with B200_ELIMIT; nothing is launched
- *     (e.g. 32 rows x 3584 x 18944 wants 5.3 MiB: use b200_qmm with a caller buffer for those).
+ *   - Problems for which the rule of b200_qmm_workspace_bytes, for the plain product alone (the gate/up
+ *     pair counted there does not run here), gives more than b200_qmm_noalloc_max_scratch_bytes() are
+ *     refused with B200_ELIMIT; nothing is launched (e.g. 32 rows x 3584 x 18944, 5.3 MiB: use b200_qmm
+ *     with a caller buffer for those).
  *   - The first call on each device looks up the array's device address (with that device
  *     current); make that first call outside any stream capture, and do not let two host threads
  *     make their first call on the same device at the same time (the cached address is written
@@ -179,11 +180,10 @@ int b200_embed_gather(const int* tokens, const uint32_t* wq, const void* scales,
 int b200_rms_norm(const void* x, const void* w, void* y, const int* row_index, int M, int H, float eps,
                   void* stream);
 
-/* Element-wise halves of the fused matmul epilogues, for prompt ingestion (mlx_eagle.py:522-535), whose matmuls run
- * 128 token rows at a time through b200_qmm_umma (plain epilogue): h = fp16(h + y) (the residual add of
- * mlx_llama.py:246,248) and out = silu(gate) * up with every op result rounded to fp16 (mlx_llama.py:215), the same
- * rounding points as B200_EPI_RESIDUAL / B200_EPI_SILU_MUL.  n = element count, a multiple of 8; fp16 device arrays,
- * 16-byte aligned. */
+/* Element-wise halves of the fused matmul epilogues, for hosts that string a layer together from plain products
+ * (b200_qmm, b200_qmm_umma); b200_prefill fuses them.  h = fp16(h + y) (the residual add of mlx_llama.py:246,248) and
+ * out = silu(gate) * up with every op result rounded to fp16 (mlx_llama.py:215), the same rounding points as
+ * B200_EPI_RESIDUAL / B200_EPI_SILU_MUL.  n = element count, a multiple of 8; fp16 device arrays, 16-byte aligned. */
 int b200_add_f16(void* h, const void* y, size_t n, void* stream);
 int b200_silu_mul_f16(const void* gate, const void* up, void* out, size_t n, void* stream);
 

@@ -122,8 +122,8 @@ __global__ void residual_add_f32_kernel(__half* __restrict__ h, const float* __r
     hp[1] = __hadd2(hp[1], __floats2half2_rn(s.z, s.w));
 }
 
-// ---- element-wise halves of the fused matmul epilogues, for prompt ingestion through the large-M matmul (whose own
-// epilogue is plain): the same rounding points as B200_EPI_RESIDUAL and B200_EPI_SILU_MUL.
+// ---- element-wise halves of the fused matmul epilogues, for callers that string a layer together from plain products: the same
+// rounding points as B200_EPI_RESIDUAL and B200_EPI_SILU_MUL.
 __global__ void add_f16_kernel(__half* __restrict__ h, const __half* __restrict__ y, size_t n) {
     pdl_wait();
     pdl_launch_dependents();

@@ -42,8 +42,10 @@ int static_scratch_address(void** out) {
     return B200_OK;
 }
 
-// Scratch these entry points ask for: partial products of a split along K that fills the GPU twice over with 64- or 128-row
-// tiles, two matrices of them for the gate / up pair.  The split in use needs less and takes what it is given.
+// Scratch these entry points ask for up to 32 rows, and by which the allocation-free one refuses: partial products of a split along
+// K that fills the GPU twice over with 64- or 128-row tiles, two matrices of them for the gate / up pair.  It is the split of a kernel
+// that is gone; the rule stays because callers' buffers and refusals follow it.  The split in use fits itself to the room it gets
+// (32 x 3584 x 18944 would take 2.3 MiB of these 5.3).
 size_t scratch_bytes(int M, int N, int K, bool dual) {
     const int mt = (M + 7) / 8, rw = (dual || mt < 3) ? 16 : 32, target = 2 * gemm_sms(), nchunks = K / kChunkK;
     const int wn = (N + 8 * rw - 1) / (8 * rw) >= target ? 8 : 4;
@@ -120,8 +122,7 @@ size_t b200_qmm_noalloc_max_scratch_bytes(void) { return b200::kStaticScratchByt
 int b200_qmm_noalloc(const void* x, const uint32_t* wq, const void* scales, const void* biases,
                      const void* bias, void* y, int M, int N, int K, int group_size, int dtype, void* stream) {
     if (M < 1 || M > 32) return B200_EINVAL;
-    // The problem must fit the fixed scratch with the split it would normally use; no silent downgrade.
-    // (Only the plain epilogue runs here, so only its plan counts, not the gate/up pair's.)
+    // (Only the plain epilogue runs here, so only its scratch counts, not the gate/up pair's.)
     if (N < 8 || K < b200::kChunkK || (K % b200::kChunkK) != 0) return B200_EINVAL;
     if (b200::scratch_bytes(M, N, K, false) > b200::kStaticScratchBytes) return B200_ELIMIT;
     void* scratch = nullptr;

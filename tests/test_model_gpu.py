@@ -134,3 +134,15 @@ def test_call_rejects_what_it_cannot_do(be, pair):
         m(torch.zeros(1, 4, dtype=torch.int64))                       # no cache
     with pytest.raises(be._lib.B200Error):
         m(torch.zeros(1, 80, dtype=torch.int64), cache=cache)         # cache too small
+
+
+@pytest.mark.parametrize("n", [8, 2048, 40 * 4864 + 8])
+def test_element_wise_halves_of_the_epilogues(be, cuda, n):
+    lib, p, st = be._lib.lib(), be._lib.ptr, be._lib.stream_ptr(cuda)
+    g = torch.Generator(device=cuda).manual_seed(n)
+    a, b = (torch.randn(n, generator=g, device=cuda).half() for _ in range(2))
+    h, out = a.clone(), torch.empty_like(a)
+    assert lib.b200_add_f16(p(h), p(b), n, st) == 0 and lib.b200_silu_mul_f16(p(a), p(b), p(out), n, st) == 0
+    assert torch.equal(h, a + b)
+    want = a * torch.sigmoid(a.float()).half() * b
+    assert torch.allclose(out.float(), want.float(), rtol=2.0 ** -9, atol=1e-6)      # (an ulp of the exponential, rounded three times)
