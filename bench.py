@@ -197,7 +197,7 @@ def roofline_block(torch, model, cache, rows, prefix, name, reps=20):
     return {"bound": "hbm", "achieved": alg / sec / 1e9, "peak": peak, "unit": "GB/s", "frac": alg / sec / 1e9 / peak,
             "traffic": (FORWARD_KERNEL_DRAM_OVER_ALGORITHMIC if a.hidden_size >= 2048
                         else FORWARD_KERNEL_DRAM_OVER_ALGORITHMIC_SMALL) * alg,
-            "traffic_source": "dram bytes of an ncu capture of a 4-layer model of the same layer shape, scaled by the "
+            "traffic_source": "dram bytes of an ncu capture of a layer of the same shape, scaled by the "
                               "algorithmic bytes (traffic grows with the layers streamed)",
             "peak_source": peak_src,
             "kernel": f"{name}: one pass of {rows} rows over a {prefix}-row cache (embedding, {a.num_hidden_layers} layers, "

@@ -127,9 +127,9 @@ int b200_qmm_noalloc(const void* x, const uint32_t* wq, const void* scales, cons
  * kernels/swizzle.metal): records of 16 rows x 128 k = 1152 contiguous bytes, packs in the order the
  * lanes of a warp consume them followed by the {scale, bias} pairs; `out` needs b200_qmm_tiled_bytes.
  * b200_qmm_tiled computes the same product and epilogues as b200_qmm_fused (same arithmetic, same
- * rounding points) from that layout with persistent CTAs and bulk-copy rings; M <= 32, and a
- * workspace of at least b200_qmm_tiled_workspace_bytes is required (first 4 KiB zero before first use;
- * the last int of that block is an error flag set if a bounded wait on a bulk copy ever gives up).
+ * rounding points) from that layout; M <= 32, and a workspace of b200_qmm_tiled_workspace_bytes lets K be
+ * cut as the planner likes (4096 is enough for no cut; first 4 KiB zero before first use; the last int of
+ * that block is an error flag set if a bounded wait ever runs out).
  */
 size_t b200_qmm_tiled_bytes(int N, int K);
 int b200_qmm_relayout(const uint32_t* wq, const void* scales, const void* biases, void* out, int N, int K,

@@ -34,7 +34,7 @@ from .quantize import quantize
 MAX_ROWS = 32          # tokens per forward pass (tree size + 1 <= 32)
 MAX_TAIL = 64          # uncommitted cache rows a query can address through its bit mask
 MAX_REQUESTS = 4       # requests that can share one forward pass
-PREFILL_ROWS = 1024    # prompt tokens per pass of the large-M (tcgen05) matmul path
+PREFILL_ROWS = 1024    # prompt tokens per pass of b200_prefill
 
 
 @dataclass
@@ -203,7 +203,7 @@ class QLinear:
     def relayout(self, keep_rowmajor: bool = False):
         """Build the streaming layout of this layer's weights; drop the row-major tensors unless asked."""
         self._nbytes = self.nbytes()
-        # the persistent kernel expands nibbles with a shorter, bit-identical sequence when every scale's fp16
+        # a shard's persistent kernel expands nibbles with a shorter, bit-identical sequence when every scale's fp16
         # exponent field is in 1..10 (2^-14 <= |s| < 2^-4); recorded here, while the scales are still at hand
         e = (self.scales.view(torch.int16).to(torch.int32) >> 10) & 31
         self.scales_fast = bool(((e >= 1) & (e <= 10)).all())
@@ -352,7 +352,7 @@ class Model:
         self.grid_ctas = 0                               # CTAs of a shard's persistent kernel (0 = one per SM)
         self.fast_dequant = True                         # allow the short nibble expansion when every scale permits it
         self.tp_two_shot = 0                             # tensor-parallel exchange: 0 library's choice (push), 1 two-step, 2 pull behind a hierarchical barrier, 3 push, 4 pull
-        self.prefill_large_m = True                      # prompts: 128 rows per weight read through b200_prefill
+        self.prefill_large_m = True                      # prompts beyond 32 tokens through b200_prefill
         self._pf_buf, self._pf_fits = None, False        # buffers of that path, made on first use
         self._scales_fast, self._layers_fast, self._fuse_fits = None, None, False
         self._graphs = _Graphs()
@@ -536,7 +536,7 @@ class Model:
         layer run as a launch of their own, not counted), the persistent kernel of a shard, or the per-op launches."""
         return 5 * self.args.num_hidden_layers + 2 if self.can_fuse() and self.tp is None else self.launches_per_forward
 
-    # ------------------------------------------------------------------ fused forward (one kernel)
+    # ------------------------------------------------------------------ fused forward (one native call)
     def can_fuse(self) -> bool:
         """True when the pass can run as one call of ``b200_forward``: every linear
         layer in the streaming layout, the embedding still row-major, sizes in multiples of 128."""
@@ -795,8 +795,8 @@ class Model:
         """``logits (1, L, V)``; the argument meanings follow ``mlx_llama.py:298-313`` / ``:121-196``.
 
         ``mask`` is the additive matrix ``(1,1,L,cache.offset+L)`` of 0 / -inf the reference passes
-        (``mlx_eagle.py:177,338``); ``None`` means causal.  Calls longer than 32 tokens (prompt
-        ingestion) are split into passes of 32, which is only possible with the causal mask.
+        (``mlx_eagle.py:177,338``); ``None`` means causal.  Calls longer than 32 tokens (prompt ingestion) are split
+        into passes of 1024 (``b200_prefill``) or, where that does not apply, 32, which is only possible with the causal mask.
         ``logits_last_only`` (an addition) returns only the last token's logits ``(1, 1, V)``.
         """
         if cache is None:

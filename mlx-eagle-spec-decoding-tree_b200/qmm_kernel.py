@@ -3,8 +3,7 @@
 ``matmul(x, w, s, b, group_size)`` (``qmm_kernel.py:84-98``) returns a list with
 one array, which ``mlx_eagle.py:704-705`` unwraps as ``qmm(*args)[0]``; the same
 convention is kept so a maintainer can swap the import.  Unlike the Metal
-kernel this one takes any row count (1..32 in one pass, more in passes of 32),
-not just 8/16/24/32.
+kernel this one takes any row count, not just 8/16/24/32.
 """
 from __future__ import annotations
 
@@ -165,7 +164,10 @@ def matmul_tiled(x, wt, n, *, epilogue=EPI_NONE, wt2=None, bias=None, extra=None
 
 
 def stream_error(device) -> int:
-    """Non-zero if a bounded wait inside the tiled kernel ever gave up on this device (reads the flag)."""
+    """Non-zero if a bounded wait inside a matmul that used this device's workspace ever ran out (reads the flag)."""
+    device = torch.device(device)
+    if device.type != "cuda" or not _workspaces:
+        return 0
     return int(workspace(device)[4092:4096].view(torch.int32).item())
 
 

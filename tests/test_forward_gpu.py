@@ -1,4 +1,5 @@
-"""The whole-pass persistent kernel (b200_forward) against the CPU oracle and against the per-op kernels."""
+"""Whole passes in one native call (b200_forward: the kernel chain; b200_prefill) against the CPU oracle and against the per-op
+kernels."""
 import dataclasses
 
 import numpy as np
@@ -27,12 +28,17 @@ def pair(request, be, cuda):
     return args, m, om
 
 
-def test_causal_prompt_matches_oracle_logits_and_cache(pair):
+@pytest.mark.parametrize("large", [False, True])        # passes of 32 and 13 rows, one prompt pass
+def test_causal_prompt_matches_oracle_logits_and_cache(pair, large):
     args, m, om = pair
     rng = np.random.default_rng(1)
-    prompt = rng.integers(0, args.vocab_size, 45)          # passes of 32 and 13 rows
+    prompt = rng.integers(0, args.vocab_size, 45)
     cache = m.make_cache(128)
-    logits = m(torch.from_numpy(prompt)[None], cache=cache)[0].cpu().numpy()
+    m.prefill_large_m = large
+    try:
+        logits = m(torch.from_numpy(prompt)[None], cache=cache)[0].cpu().numpy()
+    finally:
+        m.prefill_large_m = True
     m.check_fused_error()
     oc = model_ref.make_prompt_cache(om, 128)
     want = om(prompt, oc)
@@ -107,14 +113,15 @@ SHAPES = [
 ]
 
 
-@pytest.mark.parametrize("plen", [300, 620])            # 5 key blocks (single-phase attention) / 10 (split keys)
+@pytest.mark.parametrize("plen", [300, 620])            # 5 key blocks / 10
 @pytest.mark.parametrize("name,layers", SHAPES)
 def test_fused_pass_equals_per_op_kernels_at_benchmark_shapes(be, cuda, name, layers, plen):
-    """Full-width layers of the benchmark shapes (few of them): the persistent kernel against the nine
+    """Full-width layers of the benchmark shapes (few of them): the kernel chain against the nine
     launches per layer, same weights, same inputs; prompt passes of 32 rows, then a 16-row tree pass
     over a 300- or 620-row prefix, then a one-row pass."""
     args = dataclasses.replace(be.shape_preset(name), num_hidden_layers=layers)
     m = be.Model.random_init(args, seed=21, device=cuda).relayout()
+    m.prefill_large_m = False
     assert m.can_fuse()
     g = torch.Generator().manual_seed(3)
     prompt = torch.randint(0, args.vocab_size, (plen,), generator=g)
@@ -168,7 +175,7 @@ def test_short_nibble_expansion_gives_the_same_bits_and_is_refused_for_out_of_ra
     for bit whenever it is allowed, and must not be chosen when a scale is zero, subnormal or >= 2^-4."""
     args = be.shape_preset("tiny-qwen2")
     rng = np.random.default_rng(8)
-    prompt = torch.from_numpy(rng.integers(0, args.vocab_size, 29))          # one pass of the persistent kernel
+    prompt = torch.from_numpy(rng.integers(0, args.vocab_size, 29))          # one pass of the kernel chain
     m = be.Model.random_init(args, seed=5, device=cuda, gen_device="cpu").relayout()
     outs = []
     for fast in (True, False):
@@ -190,7 +197,7 @@ def test_short_nibble_expansion_gives_the_same_bits_and_is_refused_for_out_of_ra
 
 
 def test_prompt_through_the_large_m_path_matches_the_oracle_and_the_32_row_passes(pair):
-    """A 300-token prompt goes through b200_qmm_umma 128 rows at a time (mlx_eagle.py:522-535): logits and every
+    """A 300-token prompt goes through b200_prefill in one pass (mlx_eagle.py:522-535): logits and every
     K/V row against the CPU oracle, and against the same prompt ingested 32 rows at a time."""
     args, m, om = pair
     rng = np.random.default_rng(11)
@@ -218,7 +225,7 @@ def test_prompt_through_the_large_m_path_matches_the_oracle_and_the_32_row_passe
 
 
 def test_plan_hint_changes_the_work_split_not_the_result(be, pair):
-    """``b200_forward_plan_hint`` (a measurement aid) moves work between K-parts, stages and split-K; the logits stay
+    """``b200_forward_plan_hint`` (a measurement aid) changes how K is split over the CTAs of a cluster; the logits stay
     within the summation-order tolerance, hints that do not fit the shape are ignored, and "" restores the planner."""
     args, m, _ = pair
     lib = be._lib.lib()
@@ -254,6 +261,7 @@ def test_fused_pass_equals_per_op_kernels_at_tensor_parallel_shard_shapes(be, cu
                                intermediate_size=full.intermediate_size // world,
                                vocab_size=full.vocab_size // world)
     m = be.Model.random_init(args, seed=33, device=cuda).relayout()
+    m.prefill_large_m = False
     assert m.can_fuse()
     g = torch.Generator().manual_seed(4)
     prompt = torch.randint(0, args.vocab_size, (140,), generator=g)
