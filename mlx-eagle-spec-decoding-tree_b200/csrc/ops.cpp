@@ -123,7 +123,7 @@ PyObject* layer_pointers(PyObject*, PyObject* const* a, Py_ssize_t n) {
     static PyObject* const norms[] = {PyUnicode_InternFromString("input_norm"), PyUnicode_InternFromString("post_norm")};
     static PyObject* const tiled = PyUnicode_InternFromString("tiled");
     static PyObject* const bias = PyUnicode_InternFromString("bias");
-    void** table = n == 2 && PyList_Check(a[0]) ? static_cast<void**>(PyLong_AsVoidPtr(a[1])) : nullptr;
+    void** table = n == 2 && (PyList_Check(a[0]) || PyTuple_Check(a[0])) ? static_cast<void**>(PyLong_AsVoidPtr(a[1])) : nullptr;
     if (PyErr_Occurred()) return nullptr;
     if (table == nullptr) return PyLong_FromLong(-1);
     bool plain = true, same = true;
@@ -141,9 +141,9 @@ PyObject* layer_pointers(PyObject*, PyObject* const* a, Py_ssize_t n) {
         Py_XDECREF(t);                                           // (the layer still holds it)
     };
     try {
-        const Py_ssize_t layers = PyList_GET_SIZE(a[0]);
+        const Py_ssize_t layers = PySequence_Fast_GET_SIZE(a[0]);
         for (Py_ssize_t l = 0; l < layers; l++) {
-            PyObject* layer = PyList_GET_ITEM(a[0], l);
+            PyObject* layer = PySequence_Fast_GET_ITEM(a[0], l);
             if (!PyDict_Check(layer)) return PyLong_FromLong(-1);
             for (int i = 0; i < 5; i++) {
                 PyObject* lin = PyDict_GetItem(layer, linears[i]);

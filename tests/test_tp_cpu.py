@@ -55,6 +55,32 @@ def test_shard_refuses_degrees_that_do_not_divide(be):
         full.shard(0, 3)
 
 
+def test_layer_pointers_follow_the_layers(be):
+    """The native walk over the layers: every pointer, whether any has changed, and what is no layer of re-laid-out weights."""
+    import ctypes
+    model = be.Model.random_init(be.shape_preset("tiny-qwen2"), seed=3, device="cpu")
+    walk, n = be._lib.ops().layer_pointers, len(model.layers)
+    table = (ctypes.c_void_p * (8 * (n + 1)))()
+    at = ctypes.addressof(table)
+    assert walk(model.layers, at) == -1                          # (not re-laid-out)
+    for lw in model.layers:
+        for k in ("qkv", "o", "gate", "up", "down"):
+            lw[k].tiled = torch.zeros(16)
+    assert walk(model.layers, at) == 1 and walk(model.layers, at) == 0 and walk(tuple(model.layers), at) == 0
+    assert [p or 0 for p in table[:8 * n]] == [0 if t is None else t.data_ptr() for lw in model.layers for t in (
+        lw["qkv"].tiled, lw["qkv"].bias, lw["o"].tiled, lw["gate"].tiled, lw["up"].tiled, lw["down"].tiled, lw["input_norm"], lw["post_norm"])]
+    model.layers[1]["post_norm"].set_(torch.zeros(8, dtype=torch.float16))      # (the same object, other storage)
+    assert walk(model.layers, at) == 1 and walk(model.layers, at) == 0
+    model.layers[0]["qkv"].bias = None
+    assert walk(model.layers, at) == 1 and table[1] is None
+    assert walk(model.layers + [None], at) == -1
+    without = [dict(lw) for lw in model.layers]
+    del without[1]["down"]
+    assert walk(without, at) == -1
+    model.layers[0]["up"].tiled = None
+    assert walk(model.layers, at) == -1
+
+
 def test_the_timeline_of_a_model_that_is_no_shard_is_refused(be):
     full = be.Model.random_init(be.shape_preset("tiny-qwen2"), seed=3, device="cpu")
     with pytest.raises(be._lib.B200Error, match="shard"):        # (its passes have no device-wide barriers to stamp)
