@@ -33,6 +33,18 @@ CTL_BASE_LEN, CTL_DRAFT_LEN, CTL_ACCEPT, CTL_NGEN, CTL_STEP, CTL_DRAFT_OFF, CTL_
 CTL_LOG_CAP, CTL_EOS, CTL_DONE, CTL_STOP_N, CTL_SEED, CTL_DRAW = 8, 9, 10, 11, 12, 13
 
 
+def _weights(decoder) -> bytes:
+    return decoder.base.weight_addresses() + decoder.draft.weight_addresses()
+
+
+def _recapture_if_replaced(decoder):
+    """A step graph holds the addresses of the weights: a tensor of either model replaced since it was captured has it made
+    anew (looked at once per request)."""
+    if decoder.graph is not None and decoder._captured != _weights(decoder):
+        decoder.graph = None
+        decoder.warmup()
+
+
 class SpecDecoder:
     """Device-resident state and launch sequence of the speculative decoding loop."""
 
@@ -99,6 +111,7 @@ class SpecDecoder:
     def prefill(self, prompt: torch.Tensor, prefill_step_size: int = 512, eos_token_id: Optional[int] = None) -> int:
         """Feed the prompt to both models (``mlx_eagle.py:522-535``) and take the first token greedily.
         ``eos_token_id`` arms the device-side stop test of ``b200_tree_accept`` for this request."""
+        _recapture_if_replaced(self)
         prompt = prompt.reshape(-1).to(torch.int32).to(self.device)
         n = prompt.numel()
         need = n + 8 * (self.depth + 1) + 40
@@ -245,7 +258,7 @@ class SpecDecoder:
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g):
             self.step()
-        self.graph = g
+        self.graph, self._captured = g, _weights(self)
         return g
 
     def replay(self):
@@ -434,7 +447,7 @@ class BatchSpecDecoder:
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g):
             self.step()
-        self.graph = g
+        self.graph, self._captured = g, _weights(self)
         return g
 
     def replay(self):
@@ -448,6 +461,7 @@ class BatchSpecDecoder:
         their first tokens."""
         if len(prompts) != self.requests:
             raise _lib.B200Error(f"need {self.requests} prompts")
+        _recapture_if_replaced(self)
         return [s.prefill(pr, prefill_step_size, eos_token_id) for s, pr in zip(self.slots, prompts)]
 
     def warmup(self, capture: bool = True):

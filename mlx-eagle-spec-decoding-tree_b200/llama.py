@@ -571,6 +571,18 @@ class Model:
         self._layers_fast = all(lw[k].scales_fast for lw in self.layers for k in ("qkv", "o", "gate", "up", "down"))
         return True
 
+    def weight_addresses(self) -> bytes:
+        """Where this model's weights are now, for whoever keeps graphs of its passes."""
+        linears, others = [self.embed, self.lm_head], [self.norm, self.inv_freqs]
+        layers = b""
+        if self.can_fuse():
+            layers = bytes(self._layers_host)
+        else:
+            linears += [lw[k] for lw in self.layers for k in ("qkv", "o", "gate", "up", "down")]
+            others += [lw[k] for lw in self.layers for k in ("input_norm", "post_norm")]
+        others += [t for q in linears for t in (q.weight, q.scales, q.biases, q.bias, q.tiled)]
+        return layers + repr([None if t is None else t.data_ptr() for t in others]).encode()
+
     def _fused_desc(self, M, cache, write_off, tail, fwd, rows, row_index, requests=1, logits=None):
         """The descriptor of ``b200_forward`` (after ``can_fuse()``, which brings the layers' pointers up to date)."""
         p = lambda t: None if t is None else t.data_ptr()

@@ -145,3 +145,27 @@ def test_tree_sizes_outside_the_reference_s_four_match_the_oracle(be, models, de
     ob, od = model_ref.OracleModel(args, states[0]), model_ref.OracleModel(args, states[1])
     ref = eagle_ref.generate_step(prompt, ob, od, depth=depth, verify_num_tokens=T, max_tokens=24, N=24)
     assert res["tokens"] == ref["tokens"] and res["accept_lengths"] == ref["accept_lengths"]
+
+
+def test_a_step_graph_is_made_anew_when_a_weight_has_been_replaced(be, cuda):
+    args = be.shape_preset("tiny-qwen2")
+    new = lambda seed: be.Model.random_init(args, seed=seed, device=cuda, gen_device="cpu").relayout()
+    base, draft, other = new(11), new(12), new(13)
+    prompt = torch.arange(5, 17, dtype=torch.int32)
+    run = lambda d: d.generate(prompt, max_tokens=16, N=16, clip=True)["tokens"]
+    decoder = be.SpecDecoder(base, draft, 3, 15, 320)
+    decoder.warmup()
+    graph = decoder.graph
+    before = run(decoder)
+    assert run(decoder) == before and decoder.graph is graph
+    base.lm_head, base.layers[1]["down"], draft.layers[0]["input_norm"] = other.lm_head, other.layers[1]["down"], other.layers[0]["input_norm"].neg()
+    after = run(decoder)
+    assert decoder.graph is not graph and after != before
+    fresh = be.SpecDecoder(base, draft, 3, 15, 320)
+    fresh.warmup()
+    assert run(fresh) == after and run(decoder) == after
+    batch = be.BatchSpecDecoder(base, draft, 3, 15, 320, 2)
+    batch.warmup()
+    graph = batch.graph
+    base.norm = other.norm.clone().mul_(0.5)
+    assert len(batch.generate([prompt, prompt], max_tokens=8, N=8)) == 2 and batch.graph is not graph
