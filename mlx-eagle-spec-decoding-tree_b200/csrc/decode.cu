@@ -38,7 +38,7 @@ constexpr int kEpi = 8;                          // of which these run the epilo
 constexpr int kDThreads = (kDeq + 4) * 32;       // + weight producer, activation producer, MMA issuer, sums of squares
 constexpr int kTmem = 256;                       // columns a CTA takes: two CTAs share an SM
 constexpr int kMaxCluster = 8;
-constexpr int kSsqPitch = 32, kCsPitch = 64, kKeyBlock = 64;
+constexpr int kSsqPitch = 32, kSsqCols = 32, kCsPitch = 64, kKeyBlock = 64;
 
 enum { D_QKV = 0, D_RESID = 1, D_SILU = 2, D_HEAD = 3, D_PLAIN = 4, D_ROWS = 5 };      // the last two: y = x W^T (+ bias), a matmul on its own; D_ROWS: W as quantised
 
@@ -161,6 +161,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
     __shared__ uint64_t wfull[G::NW], wempty[G::NW], xfull[G::NX], xempty[G::NX], tready[kGroups], tfree[kGroups], accfull[2], accempty[2], inboxfull;
     __shared__ uint32_t s_tmem;
     __shared__ __align__(16) float s_rs[32];                                   // 1 / rms per token
+    __shared__ int s_base[32];                                                 // per request: committed rows (D_QKV), first row of logits (D_HEAD)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank(), cs = cluster_size();
@@ -320,15 +321,27 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         // ------------------------------------------------------------------ sums of squares -> 1 / rms of each token
         // (by the dequant warps it held up every chunk behind the first three: 1.4 us at a hidden size of 3584)
         if (KIND != D_RESID && KIND != D_PLAIN && KIND != D_ROWS) {
+            // (both were there before the pass; read in the epilogue they were 0.5 us of every q|k|v kernel)
+            if (KIND == D_QKV && lane < p.M / p.mr) s_base[lane] = __ldcg(p.prefix + lane);
+            if (KIND == D_HEAD && lane < p.M / p.mr) s_base[lane] = p.row_index != nullptr ? __ldcg(p.row_index + lane) : 0;
             pdl_wait();
-            // a lane: four tokens of every `step`-th part; as many parts at once as the tokens leave lanes for
-            const int quads = p.M <= 8 ? 2 : (p.M <= 16 ? 4 : 8), step = 32 / quads, quad = lane & (quads - 1);
+            // A lane: four tokens of every `step`-th part, four or eight loads in flight whatever the number of parts.  (Unrolled by seven with
+            // the rest one at a time: 4.3 us at 3584 x 16 tokens and 8.3 at 4096 x 32, longer than the MMAs.  Parts of 128 columns, added up
+            // by the producer's warps: 0.15 us more for each of them, of 2.7 in a draft-sized layer.)
+            const int parts = p.H / kSsqCols, quads = p.M <= 8 ? 2 : (p.M <= 16 ? 4 : 8), step = 32 / quads, quad = lane & (quads - 1);
             float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 7
-            for (int part = lane / quads; part < p.H / 32; part += step) {
-                const float4 v = __ldcg(reinterpret_cast<const float4*>(p.ssq + part * kSsqPitch + quad * 4));
-                t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w;
+            constexpr int FLY = NT == 16 ? 4 : 8;
+#pragma unroll 1
+            for (int part = lane / quads; part < parts; part += FLY * step) {
+                float4 v[FLY];
+#pragma unroll
+                for (int i = 0; i < FLY; i++)
+                    v[i] = part + i * step < parts ? __ldcg(reinterpret_cast<const float4*>(p.ssq + (part + i * step) * kSsqPitch + quad * 4))
+                                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int i = 0; i < FLY; i++) { t.x += v[i].x; t.y += v[i].y; t.z += v[i].z; t.w += v[i].w; }
             }
+            __syncwarp();
             for (int o = 16; o >= quads; o >>= 1) {
                 t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
                 t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
@@ -478,7 +491,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                         if (bias != nullptr) x = __hadd(x, extra);
                         if (valid) p.y[(size_t)tok * p.N + n] = x;
                     } else if (KIND == D_HEAD) {
-                        const int rel = tok - rq * p.mr - (p.row_index ? p.row_index[rq] : 0);
+                        const int rel = tok - rq * p.mr - s_base[rq];
                         if (valid && rel >= 0 && rel < p.rows_out) p.y[(size_t)(rq * p.rows_out + rel) * p.N + n] = __float2half_rn(v.v[k]);
                     } else {
                         __half x = __float2half_rn(v.v[k]);
@@ -493,7 +506,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                             if (head < p.Hq) {
                                 p.y[(size_t)tok * p.N + n] = x;
                             } else {
-                                const int row = p.prefix[rq] + p.write_off + (tok - rq * p.mr);
+                                const int row = s_base[rq] + p.write_off + (tok - rq * p.mr);
                                 const int kvh = head - p.Hq - (rotate ? 0 : p.Hkv);
                                 if (row < p.cap) ((rotate ? p.kc : p.vc) + (size_t)rq * p.req_stride)[((size_t)kvh * p.cap + row) * p.hd + hi] = x;
                             }
@@ -501,13 +514,20 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                     }
                 }
                 if (KIND == D_RESID) {
+                    // sums over the warp's rows, halving the tokens a lane holds with the first steps: token lane / (32 / TQ) in the end
+                    float x = ss[0];
+                    if (TQ == 4) {
+                        const bool hi = lane & 16, odd = lane & 8;
+                        const float x0 = (hi ? ss[TQ - 2] : ss[0]) + __shfl_xor_sync(0xffffffffu, hi ? ss[0] : ss[TQ - 2], 16);
+                        const float x1 = (hi ? ss[TQ - 1] : ss[1]) + __shfl_xor_sync(0xffffffffu, hi ? ss[1] : ss[TQ - 1], 16);
+                        x = (odd ? x1 : x0) + __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 8);
+                    } else {
+                        const bool hi = lane & 16;
+                        x = (hi ? ss[1] : ss[0]) + __shfl_xor_sync(0xffffffffu, hi ? ss[0] : ss[1], 16);
+                    }
 #pragma unroll
-                    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-                        for (int k = 0; k < TQ; k++) ss[k] += __shfl_xor_sync(0xffffffffu, ss[k], o);
-#pragma unroll
-                    for (int k = 0; k < TQ; k++)
-                        if (lane == k && valid && tok0 + k < p.M) p.ssq[(n >> 5) * kSsqPitch + tok0 + k] = ss[k];
+                    for (int o = 16 / TQ; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+                    if ((lane & (32 / TQ - 1)) == 0 && valid && tok0 + lane / (32 / TQ) < p.M) p.ssq[(n >> 5) * kSsqPitch + tok0 + lane / (32 / TQ)] = x;
                 }
             }
         };
