@@ -100,23 +100,6 @@ __device__ __forceinline__ const T* listed(const void* const* entry) {
     return reinterpret_cast<const T*>(__ldcg(reinterpret_cast<const unsigned long long*>(entry)));
 }
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t cluster_size() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;\n" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
-__device__ __forceinline__ uint32_t peer_addr(uint32_t addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
 template <int TQ>
 __device__ __forceinline__ void st_async(uint32_t addr, const uint32_t* a, uint32_t bar) {
     if (TQ == 4)
@@ -124,9 +107,6 @@ __device__ __forceinline__ void st_async(uint32_t addr, const uint32_t* a, uint3
                      "r"(a[TQ - 2]), "r"(a[TQ - 1]), "r"(bar) : "memory");
     else
         asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];\n" ::"r"(addr), "r"(a[0]), "r"(a[1]), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void arrive_peer(uint32_t bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
 // Phase 0, with what the peers stored before they arrived; longer than their own waits take.
 __device__ __forceinline__ void inbox_wait(uint32_t bar, int polls, int* err, int code) {

@@ -88,21 +88,6 @@ struct GParams {
     int epilogue;
 };
 
-template <int C>
-__device__ __forceinline__ void tmem_ld(uint32_t (&r)[C], uint32_t addr) {
-    static_assert(C % 8 == 0 || C == 4, "columns");
-    if constexpr (C % 8 == 0) {
-#pragma unroll
-        for (int i = 0; i < C; i += 8)
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-                         : "=r"(r[i]), "=r"(r[i + 1]), "=r"(r[i + 2]), "=r"(r[i + 3]), "=r"(r[i + 4]), "=r"(r[i + 5]),
-                           "=r"(r[i + 6]), "=r"(r[i + 7]) : "r"(addr + i) : "memory");
-    } else {
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];\n"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-    }
-}
-
 struct GItem {
     int row_item, tok0, split, c_begin, nc;
 };
@@ -507,6 +492,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
 // ---- work split: token columns per item, row tiles behind one activation tile, K ranges
 struct GPlan {
     int S, NT, splits, cps, row_items, tok_items;
+    double cost;
 };
 
 size_t gemm_partial_bytes(const GPlan& pl) {
@@ -542,6 +528,43 @@ GPlan gemm_plan(int M, int N, int K, bool dual, int sms, size_t partial_room) {
                 if (cost < best_cost) { best_cost = cost; best = pl; }
                 if (tiles * splits >= 3LL * sms) break;
             }
+        }
+    }
+    best.cost = best_cost;
+    return best;
+}
+
+// The same for csrc/qmm_pair.cu (more than 128 rows), whose work is dealt to pairs of SMs; of the two kernels the cheaper one runs.  Fitted to
+// 26 shapes of 129 to 1024 rows: a chunk costs its MMAs, 4 cycles a token, or the expansion; an item that drains behind the last
+// MMAs 23 cycles a token; a K split 6600 and 12.7 cycles a token and range.  Pairs win where a weight is used by more than 128 tokens and
+// the K of an item is long (203 x 4096 x 14336: 42 -> 32 us, 517 x 6144 x 4096: 28 -> 23, 1024 x 4096 x 14336: 92 -> 85); where the start and the end
+// of a kernel are most of it, one CTA's shorter ones do (256 x 3584 x 3584: 13.4 against 16.4 us, 256 x 1024 x 1024: 6 against 10).
+size_t pair_partial_bytes(const PairPlan& pl) {
+    return pl.splits > 1 ? (size_t)pl.splits * pl.row_items * pl.tok_items * pl.NT * 2 * kTileRows * sizeof(float) : 0;
+}
+
+PairPlan pair_plan(int M, int N, int K, bool dual, int sms, size_t partial_room) {
+    PairPlan best{};
+    best.cost = 1e30;
+    if (M <= 128) return best;
+    const int nchunks = K / kChunkK, pairs = std::max(1, sms / 2), rows = dual ? kTileRows : 2 * kTileRows;
+    for (int t = (M + 255) / 256; t <= (M + 127) / 128; t++) {
+        PairPlan pl{};
+        pl.tok_items = t;
+        pl.NT = ((M + t - 1) / t + 31) / 32 * 32;
+        pl.row_items = (N + rows - 1) / rows;
+        const long long tiles = (long long)pl.row_items * t;
+        const double chunk = std::max(4.0 * pl.NT, 800.0);
+        for (int splits = 1; splits <= std::max(1, nchunks / 2); splits++) {
+            if (splits > 1 && (2 * tiles > kGemmTiles || splits > 32)) break;
+            pl.cps = (nchunks + splits - 1) / splits;
+            pl.splits = (nchunks + pl.cps - 1) / pl.cps;
+            if (pl.splits != splits) continue;
+            if (splits > 1 && pair_partial_bytes(pl) > partial_room) break;
+            const long long rounds = (tiles * splits + pairs - 1) / pairs;
+            const double cost = 9500 + rounds * (pl.cps * chunk + 1140) + 23.0 * pl.NT + (splits > 1 ? 6600 + rounds * splits * 12.7 * pl.NT : 0.0);
+            if (cost < best.cost) { best = pl; best.cost = cost; }
+            if (tiles * splits >= 3LL * pairs) break;
         }
     }
     return best;
@@ -580,13 +603,19 @@ int gemm_sms() {
 }
 
 size_t qmm_gemm_partial_bytes(int M, int N, int K, bool dual) {
-    return gemm_partial_bytes(gemm_plan(M, N, K, dual, gemm_sms(), (size_t)1 << 40));
+    const int sms = gemm_sms();
+    const size_t room = (size_t)1 << 40;
+    const GPlan one = gemm_plan(M, N, K, dual, sms, room);
+    const PairPlan two = pair_plan(M, N, K, dual, sms, room);
+    return std::max(gemm_partial_bytes(one), two.cost < 0.95 * one.cost ? pair_partial_bytes(two) : 0);
 }
 
 int qmm_gemm(const GemmArgs& a, cudaStream_t stream) {
     const bool dual = a.epilogue == B200_EPI_SILU_MUL, tiled = a.w_tiled != nullptr;
     const int sms = gemm_sms();
     const GPlan pl = gemm_plan(a.M, a.N, a.K, dual, sms, a.partial_bytes);
+    const PairPlan pairs = pair_plan(a.M, a.N, a.K, dual, sms, a.partial_bytes);
+    if (pairs.cost < 0.95 * pl.cost && a.epilogue != B200_EPI_F32 && (tiled || !dual)) return qmm_pair(a, pairs, stream);
     GParams p{};
     int rc = make_map_2d(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a.x, (uint64_t)a.K, (uint64_t)a.M, (uint64_t)a.K * 2, 64, (uint32_t)pl.NT,
                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);

@@ -33,6 +33,14 @@ inline void gemm_workspace(GemmArgs& a, void* workspace, size_t bytes) {
     a.partial_bytes = bytes - kCounterBytes;
 }
 
+// Work split of csrc/qmm_pair.cu: tokens per tile (a multiple of 32, at most 256), 256-row tiles, token tiles, K ranges of cps chunks; its cost
+// in cycles.
+struct PairPlan {
+    int NT, row_items, tok_items, splits, cps;
+    double cost;
+};
+int qmm_pair(const GemmArgs& a, const PairPlan& plan, cudaStream_t stream);
+
 int gemm_sms();                  // SMs of the current device
 size_t qmm_gemm_partial_bytes(int M, int N, int K, bool dual);
 

@@ -28,6 +28,21 @@ __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&d)[4][
                  "r"(d[2][0]), "r"(d[2][1]), "r"(d[2][2]), "r"(d[2][3]), "r"(d[3][0]), "r"(d[3][1]), "r"(d[3][2]), "r"(d[3][3]) : "memory");
 }
 
+template <int C>
+__device__ __forceinline__ void tmem_ld(uint32_t (&r)[C], uint32_t addr) {
+    static_assert(C % 8 == 0 || C == 4, "columns");
+    if constexpr (C % 8 == 0) {
+#pragma unroll
+        for (int i = 0; i < C; i += 8)
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                         : "=r"(r[i]), "=r"(r[i + 1]), "=r"(r[i + 2]), "=r"(r[i + 3]), "=r"(r[i + 4]), "=r"(r[i + 5]),
+                           "=r"(r[i + 6]), "=r"(r[i + 7]) : "r"(addr + i) : "memory");
+    } else {
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];\n"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+    }
+}
+
 // The thread's row of a chunk (16 packs, 128 k) -> its lane of the tile at `trow`, sixteen columns (32 k) at a time.  Streaming layout:
 // pack j of unit t is k group 4 j + t; ROWS (as quantised): pack t of unit j, its values still to be put side by side.  sc, bi: scale and
 // bias of the chunk's two groups of 64, in the low halves.
