@@ -108,18 +108,16 @@ __device__ __forceinline__ void st_async(uint32_t addr, const uint32_t* a, uint3
     else
         asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];\n" ::"r"(addr), "r"(a[0]), "r"(a[1]), "r"(bar) : "memory");
 }
-// Phase 0, with what the peers stored before they arrived; longer than their own waits take.
+// Phase 0 of a barrier that counts the bytes of the cluster's st.async into this CTA's shared memory; longer than the peers' own waits take.
+// No acquire from the cluster: the bytes counted are in this SM's shared memory, where no cache stands before them, and making the rest of
+// memory coherent between the SMs of a cluster took 0.3 us of every kernel.
 __device__ __forceinline__ void inbox_wait(uint32_t bar, int polls, int* err, int code) {
-    uint32_t ok = 0;
+    bool ok = false;
 #pragma unroll 1
     for (int i = 0; !ok && i < 4 * kFirmPolls; i++) {
-        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n selp.u32 %0, 1, 0, p;\n}\n"
-                     : "=r"(ok) : "r"(bar) : "memory");
+        ok = mbar_try_wait(bar, 0);
         if (i == 4 * polls) atomicCAS(err, 0, code);
     }
-}
-__device__ __forceinline__ void st_peer2(uint32_t addr, float x, float y) {
-    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};\n" ::"r"(addr), "f"(x), "f"(y) : "memory");
 }
 
 // ================================================================================ matmul kernel
@@ -216,7 +214,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = s_tmem;
     pdl_launch_dependents();
-    if (cs > 1) cluster_arrive();                                // (waited for before the first store to a peer)
+    if (cs > 1) cluster_arrive_relaxed();                        // (waited for before the first store to a peer)
 
     if (warp == kDeq) {
         // ------------------------------------------------------------------ weight producer: depends on nothing
@@ -300,6 +298,11 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
     } else if (warp == kDeq + 3) {
         // ------------------------------------------------------------------ sums of squares -> 1 / rms of each token
         // (by the dequant warps it held up every chunk behind the first three: 1.4 us at a hidden size of 3584)
+        // The epilogue's parameters are asked for ahead of the wait: read for the first time behind it, each line is a miss on the way.
+        asm volatile("" ::"l"(p.bias), "l"(p.wn), "l"(p.y), "l"(p.h), "l"(p.hw), "l"(p.ssq), "r"(p.H), "f"(p.eps), "r"(p.M), "r"(p.N), "r"(p.tiles), "l"(p.err), "r"(p.polls));
+        if (KIND == D_QKV)
+            asm volatile("" ::"l"(p.cs), "l"(p.kc), "l"(p.vc), "l"(p.prefix), "r"(p.Hq), "r"(p.Hkv), "r"(p.hd), "r"(p.cap), "r"(p.write_off), "r"(p.mr), "l"(p.req_stride));
+        if (KIND == D_HEAD) asm volatile("" ::"r"(p.mr), "l"(p.row_index), "r"(p.rows_out));
         if (KIND != D_RESID && KIND != D_PLAIN && KIND != D_ROWS) {
             // (both were there before the pass; read in the epilogue they were 0.5 us of every q|k|v kernel)
             if (KIND == D_QKV && lane < p.M / p.mr) s_base[lane] = __ldcg(p.prefix + lane);
@@ -381,6 +384,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                 if (KIND == D_QKV) extra2 = bias[tile * kTileRows + pr];
             }
             if (j0 < nq) ask(j0);
+            if (cs > 1) cluster_wait();                          // (the peers have started: while the last MMAs run)
 
             mbar_wait_reported(smem_u32(accfull + ab), (it >> 1) & 1, p.polls, p.err, 23);
             __syncwarp();
@@ -411,7 +415,6 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
             } else {
                 // A store into a peer's memory counts its bytes at the peer's barrier by itself: no fence, no arrival behind it.  TQ
                 // tokens a store: with one, the stores were what a pass of many tokens waited for (1.1 us for four more tokens).
-                cluster_wait();
                 const uint32_t in0 = smem_u32(inbox), inbar = smem_u32(&inboxfull);
                 uint32_t dst = (me * (C / TQ)) % cs, sl = (me * (C / TQ)) / cs;
 #pragma unroll
@@ -577,7 +580,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                 }
             } while (done < end);
         }
-        return;
+        if (warp < kEpi) return;
     }
     if (cs > 1) cluster_wait();
 }
@@ -683,12 +686,12 @@ __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_co
     if (threadIdx.x == 0) {
         asm volatile("prefetch.tensormap [%0];\n" ::"l"(&p.kvmap) : "memory");
         for (int s = 0; s < G::STAGES; s++) mbar_init(smem_u32(full + s), 1);
-        mbar_init(smem_u32(&inboxfull), cs * kAWarps);                         // every warp of the cluster
+        mbar_init(smem_u32(&inboxfull), 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
     pdl_launch_dependents();
-    if (cs > 1) cluster_arrive();
+    if (cs > 1) cluster_arrive_relaxed();
 
     const int prefix = p.prefix[req];
     const int nact = min((prefix + p.tail + kKeyBlock - 1) / kKeyBlock, p.nkb);
@@ -716,6 +719,10 @@ __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_co
     const int tile = warp / PT, part = warp % PT;
     const int lr = tile * 16 + g;                                       // this thread's rows: lr, lr + 8
     const bool v0 = lr < rows, v1 = lr + 8 < rows, busy = tile * 16 < rows && b0 < b1;
+    const int nslot = (rows + (int)cs - 1) / (int)cs, row_lo = (int)rank * nslot, mine_rows = min(nslot, rows - row_lo);     // rows this CTA finishes
+    if (cs > 1 && threadIdx.x == 0)                                     // what will be stored here: (max, sum) from all, outputs from those with keys
+        mbar_expect_tx(smem_u32(&inboxfull), max(mine_rows, 0) * ((int)cs * PT * 8 + min(nact, (int)cs) * HD * 4));
+    if (cs > 1) cluster_wait();                                         // the peers have started: they may be stored to
     pdl_wait();
     if (warp == kLoader) {
         if (elect_one()) {
@@ -863,27 +870,41 @@ __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_co
     l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
     l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
     l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-    const int nslot = (rows + (int)cs - 1) / (int)cs;
-    if (cs > 1) cluster_wait();
 #pragma unroll
     for (int hrow = 0; hrow < 2; hrow++) {
         const int row = lr + 8 * hrow;
         if (row < rows) {
             const uint32_t dst = row / nslot, sl = row - dst * nslot;    // (a warp's rows: mostly one CTA)
-            if (t == 0) st_peer2(peer_addr(sbase + G::INBOX_ML + ((rank * PT + part) * nslot + sl) * 8, dst), hrow ? mrun1 : mrun0, hrow ? l1 : l0);
-            if (busy) {
-                const uint32_t at = peer_addr(sbase + G::INBOX + ((rank * nslot + sl) * G::OP + part * ND * 8 + 2 * t) * 4, dst);
+            const uint32_t ml_at = sbase + G::INBOX_ML + ((rank * PT + part) * nslot + sl) * 8;
+            const uint32_t out_at = sbase + G::INBOX + ((rank * nslot + sl) * G::OP + part * ND * 8 + 2 * t) * 4;
+            const uint32_t ml[2] = {__float_as_uint(hrow ? mrun1 : mrun0), __float_as_uint(hrow ? l1 : l0)};
+            if (cs > 1) {                                                // (a store counts its own bytes at the peer's barrier)
+                const uint32_t bar = peer_addr(smem_u32(&inboxfull), dst), at = peer_addr(out_at, dst);
+                if (t == 0) st_async<2>(peer_addr(ml_at, dst), ml, bar);
+                if (busy) {
 #pragma unroll
-                for (int nd = 0; nd < ND; nd++) st_peer2(at + nd * 32, o[nd][2 * hrow], o[nd][2 * hrow + 1]);
+                    for (int nd = 0; nd < ND; nd++) {
+                        const uint32_t x[2] = {__float_as_uint(o[nd][2 * hrow]), __float_as_uint(o[nd][2 * hrow + 1])};
+                        st_async<2>(at + nd * 32, x, bar);
+                    }
+                }
+            } else {                                                     // (st.async belongs to clusters)
+                if (t == 0) asm volatile("st.shared.v2.b32 [%0], {%1, %2};\n" ::"r"(ml_at), "r"(ml[0]), "r"(ml[1]) : "memory");
+                if (busy) {
+#pragma unroll
+                    for (int nd = 0; nd < ND; nd++)
+                        asm volatile("st.shared.v2.f32 [%0], {%1, %2};\n" ::"r"(out_at + nd * 32), "f"(o[nd][2 * hrow]), "f"(o[nd][2 * hrow + 1]) : "memory");
+                }
             }
         }
     }
-    __syncwarp();
-    if (lane < (int)cs) arrive_peer(peer_addr(smem_u32(&inboxfull), lane));
-    inbox_wait(smem_u32(&inboxfull), p.polls, p.err, 25);
-    __syncwarp();
+    if (cs > 1) {
+        inbox_wait(smem_u32(&inboxfull), p.polls, p.err, 25);
+        __syncwarp();
+    } else {
+        __syncthreads();
+    }
     // ---- merge: one warp per row, CTAs in key order
-    const int row_lo = (int)rank * nslot, mine_rows = min(nslot, rows - row_lo);
 #pragma unroll 1
     for (int j = warp; j < mine_rows; j += kAWarps) {
         constexpr int C = HD / 32;

@@ -60,15 +60,15 @@ __device__ __forceinline__ uint32_t cluster_size() {
     asm volatile("mov.u32 %0, %%cluster_nctarank;\n" : "=r"(r));
     return r;
 }
+// Ahead of the first arrival or store at a peer, behind mbarrier inits (with their fence) that the block has synchronised on: nothing
+// else passes, so nothing else is waited for.
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ uint32_t peer_addr(uint32_t addr, uint32_t rank) {
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
-}
-__device__ __forceinline__ void arrive_peer(uint32_t bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
 // One lane of a converged warp.  A branch on this keeps the compiler's knowledge that everything else is warp-uniform, so the
 // descriptors and addresses of tcgen05.mma and of copies stay in uniform registers: an MMA issues every 19 cycles instead of

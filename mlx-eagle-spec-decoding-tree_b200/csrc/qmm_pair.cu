@@ -148,7 +148,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) qmm_pai
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
-    cluster_arrive();                                // the barriers of both are there before either is arrived at
+    cluster_arrive_relaxed();                        // the barriers of both are there before either is arrived at
     cluster_wait();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = s_tmem;
