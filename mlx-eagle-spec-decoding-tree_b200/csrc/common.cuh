@@ -52,6 +52,32 @@ inline void launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t 
     cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
+// A kernel of the chain: programmatic dependent launch, clusters of `cluster` CTAs along x.
+template <typename P>
+int launch_chain(void (*kern)(P), dim3 grid, int threads, size_t smem, int cluster, cudaStream_t stream, const P& p) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (g_use_pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        n++;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    cudaLaunchKernelEx(&cfg, kern, p);
+    return check_launch();
+}
+
 // Lets `kern` use `bytes` of dynamic shared memory: a per-device attribute, set once per device (`done`: one bit each, a static
 // of the caller's).
 // `whole`: prefer the largest shared-memory carve-out, for kernels meant to have two CTAs on an SM.

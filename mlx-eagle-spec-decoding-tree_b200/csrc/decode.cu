@@ -23,6 +23,7 @@
 
 #include "common.cuh"
 #include "decode.cuh"
+#include "flash.cuh"
 #include "pipeline.cuh"
 #include "qmm_common.cuh"
 #include "tensor_map.cuh"
@@ -108,18 +109,6 @@ __device__ __forceinline__ void st_async(uint32_t addr, const uint32_t* a, uint3
     else
         asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];\n" ::"r"(addr), "r"(a[0]), "r"(a[1]), "r"(bar) : "memory");
 }
-// Phase 0 of a barrier that counts the bytes of the cluster's st.async into this CTA's shared memory; longer than the peers' own waits take.
-// No acquire from the cluster: the bytes counted are in this SM's shared memory, where no cache stands before them, and making the rest of
-// memory coherent between the SMs of a cluster took 0.3 us of every kernel.
-__device__ __forceinline__ void inbox_wait(uint32_t bar, int polls, int* err, int code) {
-    bool ok = false;
-#pragma unroll 1
-    for (int i = 0; !ok && i < 4 * kFirmPolls; i++) {
-        ok = mbar_try_wait(bar, 0);
-        if (i == 4 * polls) atomicCAS(err, 0, code);
-    }
-}
-
 // ================================================================================ matmul kernel
 // Grid: 128-row tiles x cluster ranks; the cluster's CTAs share a tile's K range.  Each finishes its share of the token
 // columns: the others store their fp32 partial products for it straight into its shared memory and arrive at its barrier (a
@@ -630,12 +619,12 @@ __global__ void __launch_bounds__(256) embed_kernel(const int* __restrict__ toke
     }
 }
 
-// ================================================================================ attention
-// CTA = (key range, kv head, request, set of 32 query rows); a query row is (token, head of the group).  Four warps share a tile of 16
-// rows: each takes a quarter of a block's keys for the scores and, the probabilities exchanged through shared memory, 1 / PT of the
-// dims for the output, so partial outputs leave the CTA once per row.  (Each warp all dims for its keys sent PT times as much to
-// the peers, which took longer than the matmuls.)  All share the K/V blocks (TMA boxes, 128-byte swizzle).  The CTAs of a cluster
-// take neighbouring key ranges; each finishes its share of the rows, whose partial softmax states the others store into its shared
+// ================================================================================ attention of up to 16 query rows
+// (More of them, and long caches at head dim 128: csrc/flash.cu.)
+// CTA = (key range, kv head, request); a query row is (token, head of the group).  Four warps share the tile of 16
+// rows: each takes a quarter of a block's keys for the scores and, the probabilities exchanged through shared memory, a quarter of the
+// dims for the output, so partial outputs leave the CTA once per row.  All share the K/V blocks (TMA boxes, 128-byte swizzle).  The CTAs of a
+// cluster take neighbouring key ranges; each finishes its share of the rows, whose partial softmax states the others store into its shared
 // memory, merged in range order.  Committed blocks are asked for before the wait for the kernel that appends this pass's rows.
 struct DAttn {
     CUtensorMap kvmap;             // the cache as [rows][head_dim], 64 x 64 boxes
@@ -645,7 +634,6 @@ struct DAttn {
     const int* prefix;
     __half* out;                   // [M][Hq * HD]
     int Hq, Hkv, mr, tail, nkb;
-    int sets;                              // sets of query rows per kv head
     int row0, req_rows, cap, write_off;    // cache row of (this layer, K, head 0), rows of one request's cache
     float scale_log2;
     int* err;
@@ -655,34 +643,34 @@ struct DAttn {
 __device__ __forceinline__ uint32_t kv_swz(int r, int v) {     // 16-byte vector v of row r of a block (boxes of 8 vectors side by side)
     return (uint32_t)((v >> 3) * 8192 + r * 128 + (((v & 7) ^ (r & 7)) << 4));
 }
-constexpr int kAWarps = 8, kAParts = 4;            // warps of an attention CTA, warps that share a row tile
+constexpr int kAWarps = 4;                         // warps of an attention CTA: they share a row tile
 template <int HD>
 struct DAGeo {
-    static constexpr int ROWS = 16 * kAWarps / kAParts;                  // query rows of a CTA: tiles of 16
+    static constexpr int ROWS = 16;                                      // query rows of a CTA
     static constexpr int BLOCK = 2 * 64 * HD * 2;                        // K and V of 64 keys
     static constexpr int STAGES = HD == 128 ? 2 : 3;
     static constexpr int Q = STAGES * BLOCK;                             // queries [row][HD], 16-byte units swizzled
-    static constexpr int P = Q + ROWS * HD * 2;                          // probabilities of a block [tile][16][64], swizzled
+    static constexpr int P = Q + ROWS * HD * 2;                          // probabilities of a block [16][64], swizzled
     static constexpr int OP = HD + 4;                                    // floats per row of a partial output
     static constexpr int INBOX = P + ROWS * 128;                         // partial outputs [source CTA][row of this CTA][OP]
     static constexpr int INBOX_ML = INBOX + (ROWS + kMaxCluster) * OP * 4;       // and (max, sum) [source CTA][part][row]
-    static constexpr int SMEM = INBOX_ML + kAParts * (ROWS + kMaxCluster) * 8 + 1024;
+    static constexpr int SMEM = INBOX_ML + kAWarps * (ROWS + kMaxCluster) * 8 + 1024;
     static_assert(2 * (SMEM + 2048) <= 227 * 1024 && SMEM + DGeo<32>::SMEM + 4 * 1024 <= 227 * 1024, "two CTAs per SM, or one beside a matmul CTA");
 };
 
 template <int HD>
 __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_constant__ DAttn p) {
     using G = DAGeo<HD>;
-    constexpr int PT = kAParts;
+    constexpr int PT = kAWarps;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);
     __shared__ uint64_t full[G::STAGES], inboxfull;
-    __shared__ float s_max[kAWarps / PT][PT][16];
+    __shared__ float s_max[PT][16];
     const uint32_t sbase = smem_u32(smem);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const uint32_t rank = cluster_rank(), cs = cluster_size();
-    const int req = blockIdx.z, hk = (int)blockIdx.y / p.sets, set = (int)blockIdx.y - hk * p.sets;
+    const int req = blockIdx.z, hk = blockIdx.y;
     if (threadIdx.x == 0) {
         asm volatile("prefetch.tensormap [%0];\n" ::"l"(&p.kvmap) : "memory");
         for (int s = 0; s < G::STAGES; s++) mbar_init(smem_u32(full + s), 1);
@@ -709,16 +697,15 @@ __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_co
     };
     const int committed = min(b1, new0 / kKeyBlock);                    // blocks below it hold no row of this pass
     const int asked = max(b0, min(committed, b0 + G::STAGES));
-    constexpr int kLoader = kAWarps - 1;                                          // (the warp with the last rows, if it has any)
+    constexpr int kLoader = kAWarps - 1;
     if (warp == kLoader) {
         if (elect_one())
             for (int b = b0; b < asked; b++) load(b);
         __syncwarp();
     }
-    const int Gq = p.Hq / p.Hkv, QR = p.mr * Gq, row_base = set * G::ROWS, rows = min(G::ROWS, QR - row_base);
-    const int tile = warp / PT, part = warp % PT;
-    const int lr = tile * 16 + g;                                       // this thread's rows: lr, lr + 8
-    const bool v0 = lr < rows, v1 = lr + 8 < rows, busy = tile * 16 < rows && b0 < b1;
+    const int Gq = p.Hq / p.Hkv, rows = p.mr * Gq;
+    const int part = warp, lr = g;                                       // this thread's rows: lr, lr + 8
+    const bool v0 = lr < rows, v1 = lr + 8 < rows, busy = b0 < b1;
     const int nslot = (rows + (int)cs - 1) / (int)cs, row_lo = (int)rank * nslot, mine_rows = min(nslot, rows - row_lo);     // rows this CTA finishes
     if (cs > 1 && threadIdx.x == 0)                                     // what will be stored here: (max, sum) from all, outputs from those with keys
         mbar_expect_tx(smem_u32(&inboxfull), max(mine_rows, 0) * ((int)cs * PT * 8 + min(nact, (int)cs) * HD * 4));
@@ -737,13 +724,13 @@ __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_co
         const int r = i / (HD / 8), v = i % (HD / 8);
         uint4 q = make_uint4(0, 0, 0, 0);
         if (r < rows) {
-            const int tok = (row_base + r) / Gq;
-            q = __ldcg(reinterpret_cast<const uint4*>(p.q + (size_t)(req * p.mr + tok) * p.pitch + (size_t)(hk * Gq + row_base + r - tok * Gq) * HD) + v);
+            const int tok = r / Gq;
+            q = __ldcg(reinterpret_cast<const uint4*>(p.q + (size_t)(req * p.mr + tok) * p.pitch + (size_t)(hk * Gq + r - tok * Gq) * HD) + v);
         }
         *reinterpret_cast<uint4*>(smem + G::Q + r * HD * 2 + ((v ^ (r & 7)) << 4)) = q;
     }
-    const unsigned long long mk0 = v0 ? p.mask[req * p.mr + (row_base + lr) / Gq] : 0ull;
-    const unsigned long long mk1 = v1 ? p.mask[req * p.mr + (row_base + lr + 8) / Gq] : 0ull;
+    const unsigned long long mk0 = v0 ? p.mask[req * p.mr + lr / Gq] : 0ull;
+    const unsigned long long mk1 = v1 ? p.mask[req * p.mr + (lr + 8) / Gq] : 0ull;
     __syncthreads();
 
     constexpr int KT = 8 / PT;                                          // 8-key columns of a warp in the first matmul
@@ -755,8 +742,7 @@ __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_co
     const uint32_t arow = (uint32_t)(lane & 15), avec = (uint32_t)(lane >> 4);                           // fragments of Q and P
     const uint32_t krow_l = (uint32_t)(lane & 7), kvec_l = (uint32_t)(lane >> 3);                        // of K
     const uint32_t vrow_l = (uint32_t)(((lane >> 3) & 1) * 8 + (lane & 7)), vvec_l = (uint32_t)(lane >> 4);    // and of V
-    const uint32_t qaddr = sbase + G::Q + (tile * 16 + arow) * (HD * 2), paddr = sbase + G::P + tile * 2048;
-    auto tile_sync = [&]() { asm volatile("bar.sync %0, %1;\n" ::"r"(tile + 1), "n"(PT * 32) : "memory"); };
+    const uint32_t qaddr = sbase + G::Q + arow * (HD * 2), paddr = sbase + G::P;
 
 #pragma unroll 1
     for (int b = b0; b < b1; b++) {
@@ -812,16 +798,16 @@ __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_co
             mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
             mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
             if (t == 0) {
-                s_max[tile][part][g] = mx0;
-                s_max[tile][part][g + 8] = mx1;
+                s_max[part][g] = mx0;
+                s_max[part][g + 8] = mx1;
             }
-            tile_sync();
+            __syncthreads();
             mx0 = mrun0;
             mx1 = mrun1;
 #pragma unroll
             for (int i = 0; i < PT; i++) {
-                mx0 = fmaxf(mx0, s_max[tile][i][g]);
-                mx1 = fmaxf(mx1, s_max[tile][i][g + 8]);
+                mx0 = fmaxf(mx0, s_max[i][g]);
+                mx1 = fmaxf(mx1, s_max[i][g + 8]);
             }
             const float base0 = (mx0 == -INFINITY) ? 0.f : mx0;
             const float base1 = (mx1 == -INFINITY) ? 0.f : mx1;
@@ -836,13 +822,13 @@ __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_co
                 // the sum uses the rounded probabilities so that numerator and denominator agree
                 l0 += __low2float(h0) + __high2float(h0);
                 l1 += __low2float(h1) + __high2float(h1);
-                unsigned char* d = smem + G::P + tile * 2048 + g * 128 + (((part * KT + nt) ^ g) << 4) + t * 4;      // (rows g and g + 8: the same swizzle)
+                unsigned char* d = smem + G::P + g * 128 + (((part * KT + nt) ^ g) << 4) + t * 4;      // (rows g and g + 8: the same swizzle)
                 *reinterpret_cast<__half2*>(d) = h0;
                 *reinterpret_cast<__half2*>(d + 1024) = h1;
             }
 #pragma unroll
             for (int nd = 0; nd < ND; nd++) { o[nd][0] *= al0; o[nd][1] *= al0; o[nd][2] *= al1; o[nd][3] *= al1; }
-            tile_sync();
+            __syncthreads();
             // this warp's dims of the output, over all keys of the block
 #pragma unroll 2
             for (int ks = 0; ks < 4; ks++) {
@@ -930,7 +916,7 @@ __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_co
             }
         }
         const float inv = den > 0.f ? 1.f / den : 0.f;
-        const int gr = row_base + row_lo + j, tok = gr / Gq;
+        const int gr = row_lo + j, tok = gr / Gq;
         __half* dst = p.out + (size_t)(req * p.mr + tok) * p.Hq * HD + (size_t)(hk * Gq + gr - tok * Gq) * HD + lane * C;
         __align__(8) __half ov[C];
 #pragma unroll
@@ -941,32 +927,6 @@ __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_co
 }
 
 // ================================================================================ host
-// A kernel of the chain: programmatic dependent launch, clusters of `cluster` CTAs along x.
-template <typename P>
-int launch_chain(void (*kern)(P), dim3 grid, int threads, size_t smem, int cluster, cudaStream_t stream, const P& p) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    int n = 0;
-    if (g_use_pdl) {
-        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[n++].val.programmaticStreamSerializationAllowed = 1;
-    }
-    if (cluster > 1) {
-        attr[n].id = cudaLaunchAttributeClusterDimension;
-        attr[n].val.clusterDim.x = cluster;
-        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
-        n++;
-    }
-    cfg.attrs = attr;
-    cfg.numAttrs = n;
-    cudaLaunchKernelEx(&cfg, kern, p);
-    return check_launch();
-}
-
 // Cluster size along K for `tiles` row tiles of `nch` chunks, by a cost in microseconds fitted on B200 to passes of four model
 // shapes with 1 to 32 tokens (the choices are on average 0.09 us a kernel behind the best).  A chunk costs 0.2, one behind the
 // three that are expanded before the wait 0.125 more; a source of the reduction 0.08 and 0.0105 a token; two groups of tokens to
@@ -1007,19 +967,17 @@ int launch_dense(DenseParams& p, int split, cudaStream_t stream) {
     return rc != B200_OK ? rc : launch(tiles - rest, rest, rest_cs);
 }
 
-// Clusters of as many key ranges as still run at once, two CTAs to an SM (33 clusters of 8 fit, 71 of 4; at one CTA to an SM, with
-// 64 query rows in a CTA, 15 of 8: the sixteenth ran alone and doubled the time).  `split` as b200_forward_desc.attn_split_blocks.
+// Clusters of as many key ranges as still run at once, two CTAs to an SM.  `split` as b200_forward_desc.attn_split_blocks.
 template <int HD>
 int launch_attention(DAttn& a, int nreq, int split, cudaStream_t stream) {
     using G = DAGeo<HD>;
     static std::atomic<uint64_t> done{0};
     if (!allow_smem(attention_kernel<HD>, G::SMEM, done, true)) return check_launch();
-    a.sets = (a.mr * (a.Hq / a.Hkv) + G::ROWS - 1) / G::ROWS;
-    const int clusters = a.Hkv * a.sets * nreq;
+    const int clusters = a.Hkv * nreq;
     int cs = std::min(a.nkb, kMaxCluster);
     while (split >= 0 && cs > 1 && clusters > 8 * (32 / cs)) cs--;
     if (split > 0 && a.nkb < split) cs = 1;
-    return launch_chain(attention_kernel<HD>, dim3(cs, a.Hkv * a.sets, nreq), kAWarps * 32, G::SMEM, cs, stream, a);
+    return launch_chain(attention_kernel<HD>, dim3(cs, a.Hkv, nreq), kAWarps * 32, G::SMEM, cs, stream, a);
 }
 
 // TABLE: the kernels take a layer's pointers from the table in device memory, in stream order like everything else.  (Variants of
@@ -1046,15 +1004,22 @@ int run_chain(const ChainArgs& c, cudaStream_t st) {
     const size_t half_stride = (size_t)d->n_kv_heads * d->cache_rows * hd;
     p.req_stride = (size_t)d->n_layers * 2 * half_stride;
     p.row_index = d->row_index; p.rows_out = d->rows_out;
-    DAttn a{};
-    if ((rc = make_map_2d(&a.kvmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, d->kv_cache, hd, (uint64_t)nreq * d->n_layers * 2 * d->n_kv_heads * d->cache_rows,
-                          (uint64_t)hd * 2, 64, 64, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B)))
-        return rc;
-    a.q = static_cast<const __half*>(d->qkv); a.pitch = nqkv; a.mask = d->mask; a.prefix = d->prefix;
-    a.out = static_cast<__half*>(d->attn); a.Hq = d->n_heads; a.Hkv = d->n_kv_heads; a.mr = p.mr; a.tail = d->tail;
-    a.nkb = (d->cache_rows + kKeyBlock - 1) / kKeyBlock;
-    a.req_rows = d->n_layers * 2 * d->n_kv_heads * d->cache_rows;
-    a.cap = d->cache_rows; a.write_off = d->write_off; a.scale_log2 = d->attn_scale * kLog2e; a.err = c.err; a.polls = p.polls;
+    FlashArgs a{};
+    a.q = d->qkv; a.kv = d->kv_cache; a.kv_rows = (uint64_t)nreq * d->n_layers * 2 * d->n_kv_heads * d->cache_rows;
+    a.out = d->attn; a.tokens = M; a.Hq = d->n_heads; a.Hkv = d->n_kv_heads; a.hd = hd; a.cap = d->cache_rows;
+    a.scale_log2 = d->attn_scale * kLog2e; a.err = c.err; a.polls = p.polls;
+    a.mask = d->mask; a.prefix = d->prefix; a.nreq = nreq; a.mr = p.mr; a.tail = d->tail; a.write_off = d->write_off;
+    a.nkb = (d->cache_rows + 63) / 64; a.split = d->attn_split_blocks; a.req_rows = d->n_layers * 2 * d->n_kv_heads * d->cache_rows;
+    FlashPlan flash{};
+    if ((rc = flash_decode_plan(a, &flash)) != B200_OK) return rc;
+    DAttn one{};
+    one.kvmap = flash.kvmap; one.q = static_cast<const __half*>(d->qkv); one.pitch = nqkv; one.mask = d->mask; one.prefix = d->prefix;
+    one.out = static_cast<__half*>(d->attn); one.Hq = d->n_heads; one.Hkv = d->n_kv_heads; one.mr = p.mr; one.tail = d->tail; one.nkb = a.nkb;
+    one.req_rows = a.req_rows; one.cap = d->cache_rows; one.write_off = d->write_off; one.scale_log2 = a.scale_log2; one.err = c.err; one.polls = p.polls;
+    // Up to 16 query rows of a kv head (a token or two) mma.sync has the shorter chain: next token of the 0.5B shape 455 against 470 us, of the
+    // 7B shape (8 layers) 440 against 444; from 1000 rows on at head dim 128 the tensor memory's is (7B, 3000 cached: 480 against 487; 0.5B
+    // there 583 against 568).  Beyond 16 rows: 0.5B, 8 tokens, 300 cached 493 against 495, 3000 cached 605 against 666.
+    const bool few = p.mr * (d->n_heads / d->n_kv_heads) <= DAGeo<64>::ROWS && (hd == 64 || a.nkb <= 16);
 
     const void* const* layers = TABLE ? static_cast<const void* const*>(d->layer_table) : c.layers;      // (not read here with TABLE)
     auto given = [&](const void* const* L, int i) { return TABLE ? nullptr : L[i]; };
@@ -1078,8 +1043,11 @@ int run_chain(const ChainArgs& c, cudaStream_t st) {
             if ((rc = launch_dense<NT, TQ, D_QKV, TABLE>(p, c.splits[0], st)) != B200_OK) return rc;
         }
         if (on(2)) {
-            a.row0 = l * 2 * d->n_kv_heads * d->cache_rows;
-            if ((rc = hd == 128 ? launch_attention<128>(a, nreq, d->attn_split_blocks, st) : launch_attention<64>(a, nreq, d->attn_split_blocks, st)) != B200_OK) return rc;
+            const int row0 = l * 2 * d->n_kv_heads * d->cache_rows;
+            one.row0 = row0;
+            if (few) rc = hd == 128 ? launch_attention<128>(one, nreq, d->attn_split_blocks, st) : launch_attention<64>(one, nreq, d->attn_split_blocks, st);
+            else rc = flash_decode(a, flash, row0, st);
+            if (rc != B200_OK) return rc;
         }
         p.bias = nullptr;
         if (on(4)) {
