@@ -72,6 +72,8 @@ struct DenseParams {
     int H;
     float eps;
     int M, N, K;                  // N: output rows of each matrix
+    int pitch;                    // WIDE: of ssq
+    int base;                     // WIDE: first cache row of the pass
     int tile_lo, tiles;           // 128-row tiles (64 + 64 rows of gate and up): first and end
     int* err;
     int polls;                    // of a wait before it gives up
@@ -118,7 +120,8 @@ __device__ __forceinline__ void st_async(uint32_t addr, const uint32_t* a, uint3
 // follows in order.  Three chunks are expanded before the wait for the previous kernel: behind it
 // come the activation load (0.5 us), the MMAs (0.1 us a chunk) and the epilogue.  Code that runs once per kernel is kept short:
 // cold instructions cost 2 to 4 cycles each.
-template <int NT, int KIND, int TQ, bool TABLE = false>
+// WIDE (prompts): blockIdx.y counts tiles of NT tokens, each with CTAs of its own that stream and expand the weights for themselves.
+template <int NT, int KIND, int TQ, bool TABLE = false, bool WIDE = false>
 __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_constant__ DenseParams p) {
     using G = DGeo<NT, TQ>;
     using V = Vec<TQ>;
@@ -136,7 +139,8 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
     const int nit = cs > 1 ? 1 : (p.tiles - tile0 + tstep - 1) / tstep;                                   // this CTA's tiles: tile0, + tstep, ...
     const int nchunks = p.K / kChunkK;
     const int c_lo = nchunks * (int)rank / (int)cs, nc = nchunks * ((int)rank + 1) / (int)cs - c_lo;      // chunks of each
-    const int quads = (p.M + TQ - 1) / TQ, qslots = (quads + (int)cs - 1) / (int)cs;                      // groups of tokens, most of a CTA's
+    const int t0 = WIDE ? (int)blockIdx.y * NT : 0, M = WIDE ? min(NT, p.M - t0) : p.M, mr = WIDE ? M : p.mr;       // first token, tokens, of a request
+    const int quads = (M + TQ - 1) / TQ, qslots = (quads + (int)cs - 1) / (int)cs;                      // groups of tokens, most of a CTA's
     const int nq = quads > (int)rank ? (quads - (int)rank + (int)cs - 1) / (int)cs : 0;                   // this CTA finishes rank, rank + cs, ...
 
     if (threadIdx.x < 32) {                                      // (a thread a barrier: one thread for all took 400 cycles)
@@ -242,8 +246,8 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                 if (elect_one()) {
                     const uint32_t bar = smem_u32(xfull + slot), dst = smem_u32(ring + G::XOFF + slot * G::X);
                     mbar_expect_tx(bar, G::X);
-                    tma_box(dst, &p.xmap, (c_lo + c) * kChunkK, 0, bar);
-                    tma_box(dst + NT * 128, &p.xmap, (c_lo + c) * kChunkK + 64, 0, bar);
+                    tma_box(dst, &p.xmap, (c_lo + c) * kChunkK, t0, bar);
+                    tma_box(dst + NT * 128, &p.xmap, (c_lo + c) * kChunkK + 64, t0, bar);
                 }
                 __syncwarp();
                 if (++slot == (uint32_t)G::NX) { slot = 0; ph ^= 1; lap = true; }
@@ -294,13 +298,14 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         if (KIND == D_HEAD) asm volatile("" ::"r"(p.mr), "l"(p.row_index), "r"(p.rows_out));
         if (KIND != D_RESID && KIND != D_PLAIN && KIND != D_ROWS) {
             // (both were there before the pass; read in the epilogue they were 0.5 us of every q|k|v kernel)
-            if (KIND == D_QKV && lane < p.M / p.mr) s_base[lane] = __ldcg(p.prefix + lane);
-            if (KIND == D_HEAD && lane < p.M / p.mr) s_base[lane] = p.row_index != nullptr ? __ldcg(p.row_index + lane) : 0;
+            if (KIND == D_QKV && lane < M / mr) s_base[lane] = WIDE ? p.base + t0 : __ldcg(p.prefix + lane);
+            if (KIND == D_HEAD && lane < M / mr) s_base[lane] = p.row_index != nullptr ? __ldcg(p.row_index + lane) : 0;
             pdl_wait();
             // A lane: four tokens of every `step`-th part, four or eight loads in flight whatever the number of parts.  (Unrolled by seven with
             // the rest one at a time: 4.3 us at 3584 x 16 tokens and 8.3 at 4096 x 32, longer than the MMAs.  Parts of 128 columns, added up
             // by the producer's warps: 0.15 us more for each of them, of 2.7 in a draft-sized layer.)
-            const int parts = p.H / kSsqCols, quads = p.M <= 8 ? 2 : (p.M <= 16 ? 4 : 8), step = 32 / quads, quad = lane & (quads - 1);
+            const int pitch = WIDE ? p.pitch : kSsqPitch;
+            const int parts = p.H / kSsqCols, quads = M <= 8 ? 2 : (M <= 16 ? 4 : 8), step = 32 / quads, quad = lane & (quads - 1);
             float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
             constexpr int FLY = NT == 16 ? 4 : 8;
 #pragma unroll 1
@@ -308,7 +313,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                 float4 v[FLY];
 #pragma unroll
                 for (int i = 0; i < FLY; i++)
-                    v[i] = part + i * step < parts ? __ldcg(reinterpret_cast<const float4*>(p.ssq + (part + i * step) * kSsqPitch + quad * 4))
+                    v[i] = part + i * step < parts ? __ldcg(reinterpret_cast<const float4*>(p.ssq + (part + i * step) * pitch + t0 + quad * 4))
                                                    : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int i = 0; i < FLY; i++) { t.x += v[i].x; t.y += v[i].y; t.z += v[i].z; t.w += v[i].w; }
@@ -361,9 +366,9 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                 const int tok0 = TQ * ((int)rank + j * (int)cs);
 #pragma unroll
                 for (int k = 0; k < TQ; k++) {
-                    if (KIND == D_RESID && valid && tok0 + k < p.M)
-                        hres[k] = __ldcg(reinterpret_cast<const unsigned short*>(p.h) + (size_t)(tok0 + k) * p.N + n);
-                    if (KIND == D_QKV && rotate && tok0 + k < p.M) rot[k] = __ldcg(p.cs + (tok0 + k) * kCsPitch + (first ? hi : hi - half));
+                    if (KIND == D_RESID && valid && tok0 + k < M)
+                        hres[k] = __ldcg(reinterpret_cast<const unsigned short*>(p.h) + (size_t)(t0 + tok0 + k) * p.N + n);
+                    if (KIND == D_QKV && rotate && tok0 + k < M) rot[k] = __ldcg(p.cs + (t0 + tok0 + k) * kCsPitch + (first ? hi : hi - half));
                 }
             };
             if (it == 0) pdl_wait();
@@ -394,7 +399,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                 if (it > 0) consumer_sync(kEpi * 32);            // the tile before this one has been read
 #pragma unroll
                 for (int i = 0; i < C; i += TQ)
-                    if ((int)me * C + i < p.M) {
+                    if ((int)me * C + i < M) {
                         V x;
 #pragma unroll
                         for (int k = 0; k < TQ; k++) x.v[k] = __uint_as_float(a[i + k]);
@@ -408,7 +413,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                 uint32_t dst = (me * (C / TQ)) % cs, sl = (me * (C / TQ)) / cs;
 #pragma unroll
                 for (int i = 0; i < C; i += TQ) {
-                    if ((int)me * C + i < p.M)
+                    if ((int)me * C + i < M)
                         st_async<TQ>(peer_addr(in0 + ((rank * qslots + sl) * kTileRows + r) * (TQ * 4), dst), a + i, peer_addr(inbar, dst));
                     if (++dst == cs) { dst = 0; sl++; }
                 }
@@ -445,13 +450,13 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
 #pragma unroll
                 for (int k = 0; k < TQ; k++) {
                     const int tok = tok0 + k;
-                    if (tok >= p.M) break;
-                    const int rq = KIND == D_HEAD || KIND == D_QKV ? (p.mr == p.M ? 0 : tok / p.mr) : 0;
+                    if (tok >= M) break;
+                    const int rq = KIND == D_HEAD || KIND == D_QKV ? (mr == M ? 0 : tok / mr) : 0;
                     if (KIND == D_SILU) {
-                        if (valid) p.y[(size_t)tok * p.N + n] = __float2half_rn(silu_mul_f16(v.v[k], w.v[k]));
+                        if (valid) p.y[(size_t)(t0 + tok) * p.N + n] = __float2half_rn(silu_mul_f16(v.v[k], w.v[k]));
                     } else if (KIND == D_RESID) {
                         if (valid) {
-                            const size_t at = (size_t)tok * p.N + n;
+                            const size_t at = (size_t)(t0 + tok) * p.N + n;
                             const __half o = __hadd(__ushort_as_half(hres[k]), __float2half_rn(v.v[k]));
                             const float f = __half2float(o);
                             ss[k] = f * f;
@@ -463,7 +468,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                         if (bias != nullptr) x = __hadd(x, extra);
                         if (valid) p.y[(size_t)tok * p.N + n] = x;
                     } else if (KIND == D_HEAD) {
-                        const int rel = tok - rq * p.mr - s_base[rq];
+                        const int rel = tok - rq * mr - s_base[rq];
                         if (valid && rel >= 0 && rel < p.rows_out) p.y[(size_t)(rq * p.rows_out + rel) * p.N + n] = __float2half_rn(v.v[k]);
                     } else {
                         __half x = __float2half_rn(v.v[k]);
@@ -476,9 +481,9 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                         }
                         if (valid) {
                             if (head < p.Hq) {
-                                p.y[(size_t)tok * p.N + n] = x;
+                                p.y[(size_t)(t0 + tok) * p.N + n] = x;
                             } else {
-                                const int row = s_base[rq] + p.write_off + (tok - rq * p.mr);
+                                const int row = s_base[rq] + p.write_off + (tok - rq * mr);
                                 const int kvh = head - p.Hq - (rotate ? 0 : p.Hkv);
                                 if (row < p.cap) ((rotate ? p.kc : p.vc) + (size_t)rq * p.req_stride)[((size_t)kvh * p.cap + row) * p.hd + hi] = x;
                             }
@@ -499,7 +504,8 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                     }
 #pragma unroll
                     for (int o = 16 / TQ; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-                    if ((lane & (32 / TQ - 1)) == 0 && valid && tok0 + lane / (32 / TQ) < p.M) p.ssq[(n >> 5) * kSsqPitch + tok0 + lane / (32 / TQ)] = x;
+                    if ((lane & (32 / TQ - 1)) == 0 && valid && tok0 + lane / (32 / TQ) < M)
+                        p.ssq[(n >> 5) * (WIDE ? p.pitch : kSsqPitch) + t0 + tok0 + lane / (32 / TQ)] = x;
                 }
             }
         };
@@ -577,6 +583,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
 // ================================================================================ embedding
 // One CTA per token: dequantised embedding row -> h, h * w_norm, sums of squares per 32 columns, and the token's RoPE table.  The norm
 // weights may come from the layer table (`wn_entry`).
+// The attention of a short prompt takes a tree's mask words and committed length, which come from here, too.
 // The next kernel is let go only behind the wait: everything before the pass (tree kernels, KV compaction, other programs'
 // writes) is then complete before any kernel of the pass starts, which may so read committed K/V rows, and the layer table, ahead
 // of its own wait.
@@ -584,11 +591,15 @@ __global__ void __launch_bounds__(256) embed_kernel(const int* __restrict__ toke
                                                     const __half* __restrict__ sc, const __half* __restrict__ bi, const __half* wn,
                                                     __half* __restrict__ h, __half* __restrict__ hw, float* __restrict__ ssq,
                                                     float2* __restrict__ cs, const float* __restrict__ inv_freq, float scaling, int H, int V,
-                                                    int half_hd, const void* const* wn_entry) {
+                                                    int half_hd, const void* const* wn_entry, int pitch, int pos0, unsigned long long* mask, int* prefix) {
     pdl_wait();
     pdl_launch_dependents();
     if (wn_entry != nullptr) wn = listed<__half>(wn_entry);
     const int m = blockIdx.x, units = H / 8;
+    if (mask != nullptr && threadIdx.x == 0) {                      // a causal pass behind pos0 rows
+        mask[m] = (2ull << m) - 1;
+        if (m == 0) *prefix = pos0;
+    }
     const int tok = min(max(tokens[m], 0), V - 1);
     for (int u = threadIdx.x; u < ((units + 31) & ~31); u += 256) {
         float ss = 0.f;
@@ -610,11 +621,11 @@ __global__ void __launch_bounds__(256) embed_kernel(const int* __restrict__ toke
         }
         ss += __shfl_xor_sync(0xffffffffu, ss, 1);
         ss += __shfl_xor_sync(0xffffffffu, ss, 2);
-        if (u < units && (u & 3) == 0) ssq[(u >> 2) * kSsqPitch + m] = ss;
+        if (u < units && (u & 3) == 0) ssq[(u >> 2) * pitch + m] = ss;
     }
     if ((int)threadIdx.x < half_hd) {
         float s, c;
-        sincosf((scaling * inv_freq[threadIdx.x]) * (float)pos[m], &s, &c);
+        sincosf((scaling * inv_freq[threadIdx.x]) * (float)(pos != nullptr ? pos[m] : pos0 + m), &s, &c);
         cs[m * kCsPitch + threadIdx.x] = make_float2(c, s);
     }
 }
@@ -946,23 +957,23 @@ int plan_cluster(int tiles, int nch, int tokens, int group) {
     return best;
 }
 
-template <int NT, int TQ, int KIND, bool TABLE = false>
+template <int NT, int TQ, int KIND, bool TABLE = false, bool WIDE = false>
 int launch_dense(DenseParams& p, int split, cudaStream_t stream) {
     static std::atomic<uint64_t> done{0};
-    if (!allow_smem(dense_kernel<NT, KIND, TQ, TABLE>, DGeo<NT, TQ>::SMEM, done, KIND != D_ROWS)) return check_launch();
+    if (!allow_smem(dense_kernel<NT, KIND, TQ, TABLE, WIDE>, DGeo<NT, TQ>::SMEM, done, KIND != D_ROWS)) return check_launch();
     const int nch = p.K / kChunkK;
-    const int tiles = KIND == D_SILU ? p.N / 64 : (p.N + kTileRows - 1) / kTileRows;
-    const int cs = split > 0 && split <= std::min(kMaxCluster, nch) ? split : plan_cluster(tiles, nch, p.M, TQ);
+    const int tiles = KIND == D_SILU ? p.N / 64 : (p.N + kTileRows - 1) / kTileRows, wide = WIDE ? (p.M + NT - 1) / NT : 1;
+    const int cs = split > 0 && split <= std::min(kMaxCluster, nch) ? split : plan_cluster(tiles * wide, nch, std::min(p.M, NT), TQ);
     constexpr int cap = 296;
     auto launch = [&](int lo, int n, int cluster) {
         p.tile_lo = lo;
         p.tiles = lo + n;
-        return launch_chain(dense_kernel<NT, KIND, TQ, TABLE>, dim3(cluster > 1 ? n * cluster : std::min(n, cap)), kDThreads, DGeo<NT, TQ>::SMEM, cluster, stream, p);
+        return launch_chain(dense_kernel<NT, KIND, TQ, TABLE, WIDE>, dim3(cluster > 1 ? n * cluster : std::min(n, cap), wide), kDThreads, DGeo<NT, TQ>::SMEM, cluster, stream, p);
     };
     // Whole waves of tiles, then what is left over as a launch of its own with K split over clusters: alone it would take as long
     // as a whole wave.
     const int rest = cs == 1 && tiles > cap ? tiles % cap : 0, rest_cs = rest > 0 ? std::min({cap / rest, kMaxCluster, nch}) : 1;
-    if (rest_cs < 2) return launch(0, tiles, cs);
+    if (WIDE || rest_cs < 2) return launch(0, tiles, cs);
     const int rc = launch(0, tiles - rest, 1);
     return rc != B200_OK ? rc : launch(tiles - rest, rest, rest_cs);
 }
@@ -1026,7 +1037,7 @@ int run_chain(const ChainArgs& c, cudaStream_t st) {
     if (on(0) || TABLE) {                                       // (what makes the table safe to read ahead of a kernel's wait)
         launch_kernel(embed_kernel, dim3(M), dim3(256), 0, st, d->tokens, d->pos, d->embed_wq, static_cast<const __half*>(d->embed_scales),
                       static_cast<const __half*>(d->embed_biases), static_cast<const __half*>(given(layers, 6)), p.h, p.hw, p.ssq, c.cs, d->inv_freq,
-                      d->rope_scaling, H, d->vocab, hd / 2, TABLE ? layers + 6 : nullptr);
+                      d->rope_scaling, H, d->vocab, hd / 2, TABLE ? layers + 6 : nullptr, kSsqPitch, 0, static_cast<unsigned long long*>(nullptr), static_cast<int*>(nullptr));
         if ((rc = check_launch()) != B200_OK) return rc;
     }
     for (int l = 0; l < d->n_layers; l++) {
@@ -1073,6 +1084,46 @@ int run_chain(const ChainArgs& c, cudaStream_t st) {
     return B200_OK;
 }
 
+// The layers of a prompt pass: as run_chain, in tiles of 32 tokens.
+int run_prompt(const ChainPrompt& c, cudaStream_t st) {
+    const b200_prefill_desc* d = c.d;
+    const int n = d->n, H = d->hidden, I = d->intermediate, hd = d->head_dim, nq = d->n_heads * hd, nqkv = (d->n_heads + 2 * d->n_kv_heads) * hd;
+    CUtensorMap hw_map, attn_map, act_map;
+    auto xmap = [&](CUtensorMap* m, const void* x, int width) {
+        return make_map_2d(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x, width, n, (uint64_t)width * 2, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+    };
+    int rc;
+    if ((rc = xmap(&hw_map, d->xn, H)) || (rc = xmap(&attn_map, d->attn, nq)) || (rc = xmap(&act_map, d->act, I))) return rc;
+    DenseParams p{};
+    p.ssq = c.ssq; p.pitch = (n + 31) / 32 * 32; p.H = H; p.eps = d->rms_eps; p.M = p.mr = n; p.err = c.err; p.polls = wait_polls(kWaitPolls, kFirmPolls / 2);
+    p.h = static_cast<__half*>(d->h); p.hw = static_cast<__half*>(d->xn);
+    p.cs = c.cs; p.base = d->off; p.Hq = d->n_heads; p.Hkv = d->n_kv_heads; p.hd = hd; p.cap = d->cache_rows;
+    const size_t half = (size_t)d->n_kv_heads * d->cache_rows * hd;
+    launch_kernel(embed_kernel, dim3(n), dim3(256), 0, st, d->tokens, static_cast<const int*>(nullptr), d->embed_wq, static_cast<const __half*>(d->embed_scales),
+                  static_cast<const __half*>(d->embed_biases), static_cast<const __half*>(d->layers[6]), p.h, p.hw, p.ssq, c.cs, d->inv_freq, d->rope_scaling, H, d->vocab,
+                  hd / 2, static_cast<const void* const*>(nullptr), p.pitch, d->off, c.mask, c.prefix);
+    if ((rc = check_launch()) != B200_OK) return rc;
+    for (int l = 0; l < d->n_layers; l++) {
+        const void* const* L = d->layers + (size_t)l * 8;       // qkv, qkv bias, o, gate, up, down, input norm, post norm
+        auto weights = [&](int i, int count) {
+            for (int j = 0; j < count; j++) p.w[j] = static_cast<const unsigned char*>(L[i + j]);
+        };
+        p.xmap = hw_map; weights(0, 1); p.bias = static_cast<const __half*>(L[1]); p.y = static_cast<__half*>(d->qkv); p.N = nqkv; p.K = H;
+        p.kc = static_cast<__half*>(d->kv_cache) + (size_t)l * 2 * half;
+        p.vc = p.kc + half;
+        if ((rc = launch_dense<32, 4, D_QKV, false, true>(p, 0, st)) != B200_OK) return rc;
+        if ((rc = c.attention(c.context, l * 2 * d->n_kv_heads * d->cache_rows, st)) != B200_OK) return rc;
+        p.bias = nullptr;
+        p.xmap = attn_map; weights(2, 1); p.wn = static_cast<const __half*>(L[7]); p.N = H; p.K = nq;
+        if ((rc = launch_dense<32, 4, D_RESID, false, true>(p, 0, st)) != B200_OK) return rc;
+        p.xmap = hw_map; weights(3, 2); p.y = static_cast<__half*>(d->act); p.N = I; p.K = H;
+        if ((rc = launch_dense<32, 4, D_SILU, false, true>(p, 0, st)) != B200_OK) return rc;
+        p.xmap = act_map; weights(5, 1); p.wn = static_cast<const __half*>(l + 1 < d->n_layers ? L[8 + 6] : d->final_norm); p.N = H; p.K = I;
+        if ((rc = launch_dense<32, 4, D_RESID, false, true>(p, 0, st)) != B200_OK) return rc;
+    }
+    return B200_OK;
+}
+
 template <int NT, int TQ>
 int run_matmul(const ChainMatmul& c, cudaStream_t st) {
     DenseParams p{};
@@ -1103,6 +1154,8 @@ template <bool TABLE>
 static int forward_chain_rows(const ChainArgs& a, cudaStream_t stream) {
     return a.d->M <= 8 ? run_chain<16, 2, TABLE>(a, stream) : (a.d->M <= 16 ? run_chain<16, 4, TABLE>(a, stream) : run_chain<32, 4, TABLE>(a, stream));
 }
+
+int chain_prompt(const ChainPrompt& c, cudaStream_t st) { return run_prompt(c, st); }
 
 int forward_chain(const ChainArgs& a, cudaStream_t stream) {
     return a.layers != nullptr ? forward_chain_rows<false>(a, stream) : forward_chain_rows<true>(a, stream);

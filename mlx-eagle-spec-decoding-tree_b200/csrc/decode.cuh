@@ -17,6 +17,19 @@ struct ChainArgs {
 
 int forward_chain(const ChainArgs& a, cudaStream_t stream);
 
+// The layers of a prompt pass (embedding to the last layer's h) through the chain's kernels, tiles of 32 tokens side by side.
+struct ChainPrompt {
+    const b200_prefill_desc* d;  // checked; xn holds h * w_norm
+    int* err;
+    float* ssq;                  // [hidden / 32][tokens rounded up to 32]
+    float2* cs;                  // [tokens][64]
+    unsigned long long* mask;    // [tokens], at most 64, and committed length for the attention; or NULL
+    int* prefix;
+    int (*attention)(const void* context, int row0, cudaStream_t stream);
+    const void* context;
+};
+int chain_prompt(const ChainPrompt& c, cudaStream_t stream);
+
 // y[M][N] = x[M][K] . W^T (+ bias), M <= 32, by the chain's matmul kernel on its own.  W in the streaming layout, or as quantised
 // (packs, with 4-byte aligned scales and biases).
 struct ChainMatmul {

@@ -11,6 +11,7 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "decode.cuh"
 #include "flash.cuh"
 #include "pipeline.cuh"
 #include "qmm_common.cuh"
@@ -172,6 +173,28 @@ int launch_attention(const FlashArgs& a, const FlashPlan& plan, int row0, cudaSt
     return check_launch();
 }
 
+// The chain's kernels for prompts: 5 a layer and not 8, but every tile of 32 tokens expands the weights for itself.  Against chunks of weights
+// (128 x 128) times token tiles a layer: 0.5B shape (910 chunks) 33 tokens 805 -> 640 us, 61 836 -> 659, 128 947 -> 876; 1B (3712) 61 781 ->
+// 651, 96 852 -> 833, 128 886 against 968; 7B (14224; 4 layers) 61 321 against 369.
+constexpr int kChainPromptTokens = 128;
+bool chain_prompt_wins(const b200_prefill_desc* d) {
+    auto chunks = [](long long n, long long k) { return (n + 127) / 128 * (k / 128); };
+    const int nq = d->n_heads * d->head_dim;
+    const long long layer = chunks(nq + 2ll * d->n_kv_heads * d->head_dim, d->hidden) + chunks(d->hidden, nq) + chunks(2ll * d->intermediate, d->hidden) +
+                            chunks(d->hidden, d->intermediate);
+    return d->n <= kChainPromptTokens && layer * ((d->n + 31) / 32) <= 11200;
+}
+// Its scratch, and that of the attention when that is a tree's.
+struct ChainScratch {
+    size_t cs, ssq, mask, bytes;
+    ChainScratch(int hidden, int n) {
+        cs = 0;
+        ssq = cs + (size_t)n * 64 * sizeof(float2);
+        mask = ssq + (size_t)(hidden / 32) * ((n + 31) / 32 * 32) * sizeof(float);
+        bytes = mask + 64 * sizeof(unsigned long long) + 16;       // and the committed length
+    }
+};
+
 int norm_rows(const b200_prefill_desc* d, void* x, const void* w, void* y, int rows, bool embed, cudaStream_t st) {
     launch_kernel(norm_rows_kernel, dim3(rows), dim3(kNormThreads), 0, st, static_cast<__half*>(x), static_cast<const __half*>(w),
                   static_cast<__half*>(y), d->hidden, d->rms_eps, embed ? d->tokens : nullptr, d->embed_wq,
@@ -227,26 +250,50 @@ int b200_prefill(const b200_prefill_desc* d, void* stream) {
     const int nblk = (d->off + n + kKeyBlock - 1) / kKeyBlock;
     a.splits = std::max(1, std::min({148 / items, nblk / 4, 16}));
     const size_t per_split = (size_t)d->n_heads * n * (hd + 2) * sizeof(float);
-    while (a.splits > 1 && a.splits * per_split + 16 > ga.partial_bytes) a.splits--;
-    a.part_ml = static_cast<float*>(ga.partial);
+    const ChainScratch scratch(H, n);
+    const size_t chain = chain_prompt_wins(d) && scratch.bytes <= ga.partial_bytes ? scratch.bytes : 0;      // (ahead of the ranges' partial states)
+    while (a.splits > 1 && chain + a.splits * per_split + 16 > ga.partial_bytes) a.splits--;
+    a.part_ml = ga.partial ? static_cast<float*>(ga.partial) + chain / sizeof(float) : nullptr;
     a.part_o = a.part_ml ? a.part_ml + (((size_t)a.splits * d->n_heads * n * 2 + 3) & ~(size_t)3) : nullptr;
 
-    rc = norm_rows(d, d->h, d->layers[6], d->xn, n, true, st);
-    for (int l = 0; l < d->n_layers && rc == B200_OK; l++) {
-        const void* const* L = d->layers + (size_t)l * 8;       // qkv, qkv bias, o, gate, up, down, input norm, post norm
-        __half* kc = static_cast<__half*>(d->kv_cache) + (size_t)l * 2 * half;
-        __half* vc = kc + half;
-        rc = gemm(d->xn, L[0], nullptr, L[1], nullptr, d->qkv, n, nqkv, H, B200_EPI_NONE);
-        if (rc != B200_OK) break;
-        launch_kernel(rope_append_kernel, dim3(n), dim3(256), 0, st, static_cast<__half*>(d->qkv), d->inv_freq, d->rope_scaling, kc, vc, d->off,
-                      d->n_heads, d->n_kv_heads, hd, d->cache_rows);
-        if ((rc = check_launch()) != B200_OK) break;
-        if ((rc = launch_attention(a, flash, l * 2 * d->n_kv_heads * d->cache_rows, st)) != B200_OK) break;
-        if ((rc = gemm(d->attn, L[2], nullptr, nullptr, d->h, d->h, n, H, nq, B200_EPI_RESIDUAL)) != B200_OK) break;
-        if ((rc = norm_rows(d, d->h, L[7], d->xn, n, false, st)) != B200_OK) break;
-        if ((rc = gemm(d->xn, L[3], L[4], nullptr, nullptr, d->act, n, I, H, B200_EPI_SILU_MUL)) != B200_OK) break;
-        if ((rc = gemm(d->act, L[5], nullptr, nullptr, d->h, d->h, n, H, I, B200_EPI_RESIDUAL)) != B200_OK) break;
-        if (l + 1 < d->n_layers) rc = norm_rows(d, d->h, L[8 + 6], d->xn, n, false, st);
+    // Few tokens of a small model: the chain of the 32-row passes, whose kernels norm, RoPE and append themselves.
+    if (chain > 0) {
+        unsigned char* const at = static_cast<unsigned char*>(ga.partial);
+        ChainPrompt c{};
+        c.d = d; c.err = ga.err;
+        c.cs = reinterpret_cast<float2*>(at + scratch.cs);
+        c.ssq = reinterpret_cast<float*>(at + scratch.ssq);
+        struct Attention { const FlashArgs* a; const FlashPlan* plan; bool tree; } attention{&a, &flash, n <= 64 && a.splits > 1};
+        if (attention.tree) {                                      // key ranges by the CTAs of a cluster, merged in the same kernel
+            c.mask = reinterpret_cast<unsigned long long*>(at + scratch.mask);
+            c.prefix = reinterpret_cast<int*>(c.mask + 64);
+            a.mask = c.mask; a.prefix = c.prefix; a.nreq = 1; a.mr = a.tail = n; a.nkb = (d->cache_rows + kKeyBlock - 1) / kKeyBlock;
+            if ((rc = flash_decode_plan(a, &flash)) != B200_OK) return rc;
+        }
+        c.attention = [](const void* p, int row0, cudaStream_t stream) {
+            const Attention* x = static_cast<const Attention*>(p);
+            return x->tree ? flash_decode(*x->a, *x->plan, row0, stream) : launch_attention(*x->a, *x->plan, row0, stream);
+        };
+        c.context = &attention;
+        rc = chain_prompt(c, st);
+    } else {
+        rc = norm_rows(d, d->h, d->layers[6], d->xn, n, true, st);
+        for (int l = 0; l < d->n_layers && rc == B200_OK; l++) {
+            const void* const* L = d->layers + (size_t)l * 8;       // qkv, qkv bias, o, gate, up, down, input norm, post norm
+            __half* kc = static_cast<__half*>(d->kv_cache) + (size_t)l * 2 * half;
+            __half* vc = kc + half;
+            rc = gemm(d->xn, L[0], nullptr, L[1], nullptr, d->qkv, n, nqkv, H, B200_EPI_NONE);
+            if (rc != B200_OK) break;
+            launch_kernel(rope_append_kernel, dim3(n), dim3(256), 0, st, static_cast<__half*>(d->qkv), d->inv_freq, d->rope_scaling, kc, vc, d->off,
+                          d->n_heads, d->n_kv_heads, hd, d->cache_rows);
+            if ((rc = check_launch()) != B200_OK) break;
+            if ((rc = launch_attention(a, flash, l * 2 * d->n_kv_heads * d->cache_rows, st)) != B200_OK) break;
+            if ((rc = gemm(d->attn, L[2], nullptr, nullptr, d->h, d->h, n, H, nq, B200_EPI_RESIDUAL)) != B200_OK) break;
+            if ((rc = norm_rows(d, d->h, L[7], d->xn, n, false, st)) != B200_OK) break;
+            if ((rc = gemm(d->xn, L[3], L[4], nullptr, nullptr, d->act, n, I, H, B200_EPI_SILU_MUL)) != B200_OK) break;
+            if ((rc = gemm(d->act, L[5], nullptr, nullptr, d->h, d->h, n, H, I, B200_EPI_RESIDUAL)) != B200_OK) break;
+            if (l + 1 < d->n_layers) rc = norm_rows(d, d->h, L[8 + 6], d->xn, n, false, st);
+        }
     }
     if (rc != B200_OK || d->head_out == 0) return rc;
     const int rows = d->head_out == 1 ? n : 1;
