@@ -938,20 +938,27 @@ __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_co
 }
 
 // ================================================================================ host
-// Cluster size along K for `tiles` row tiles of `nch` chunks, by a cost in microseconds fitted on B200 to passes of four model
-// shapes with 1 to 32 tokens (the choices are on average 0.09 us a kernel behind the best).  A chunk costs 0.2, one behind the
-// three that are expanded before the wait 0.125 more; a source of the reduction 0.08 and 0.0105 a token; two groups of tokens to
-// finish 0.24; CTAs beyond one per SM take the room of the next kernel's, which then starts later.  Clusters beyond what fits at
-// once into eight GPCs of at least 16 SMs, two CTAs each, run as a second wave (36 clusters of 7 or 48 of 6 added 2 to 8 us a
-// kernel): not taken.
-int plan_cluster(int tiles, int nch, int tokens, int group) {
+// Cluster size along K for `tiles` row tiles of `nch` chunks, by a cost (in chunks) fitted on B200 to passes of four model shapes with 1, 8, 16
+// and 32 tokens, one kernel's size changed at a time around the choice: a chunk, one behind the three that are expanded before the wait as
+// much again; a source of the reduction 0.38 and 0.007 a token; clusters that nearly fill what runs at once (eight GPCs of at least 16 SMs,
+// two CTAs each) start late, and beyond it run as a second wave (36 clusters of 7 or 48 of 6 added 2 to 8 us a kernel): not taken, nor eights
+// of more than 28 tiles (32 x 112 chunks: + 0.7 to 1.7 us).  On average 0.02 us a kernel behind the best of the 64 cases.  (The terms fitted
+// when an exchange cost 0.5 us more kept to half the cluster: 24 x 16 chunks, 32 tokens - 2.2 us with 8 instead of 4, 128 x 16 - 2.8 with 2
+// instead of none.)
+// A matmul on its own (`alone`) has nothing but its like before and behind it, which come up where a CTA leaves them room: there fewer
+// and longer CTAs are better (4096 x 4096, 8 rows: 6.3 us with 4, 7.2 with 7), in microseconds: a chunk 0.2, behind the third 0.125 more, a
+// source of the reduction 0.08 and 0.0105 a token, two groups of tokens to finish 0.24.
+int plan_cluster(int tiles, int nch, int tokens, int group, bool alone) {
     int best = 1;
     double best_cost = 1e30;
     const int groups = (tokens + group - 1) / group;
-    for (int cs = 1; cs <= kMaxCluster && cs <= nch && (cs == 1 || tiles <= 8 * (32 / cs)); cs++) {
+    for (int cs = 1; cs <= kMaxCluster && cs <= nch && (cs == 1 || tiles <= 8 * (32 / cs)) && (cs < 8 || tiles <= 28 || alone); cs++) {
         const int ctas = tiles * cs, n = ((nch + cs - 1) / cs) * ((ctas + 295) / 296);
-        const double cost = n * 0.2 + std::max(0, n - 3) * 0.125 + (cs > 1 ? 0.5 + (0.08 + 0.0105 * tokens) * cs : 0.0) +
-                            0.24 * (((groups + cs - 1) / cs + 1) / 2) + (ctas > 148 ? std::min(ctas - 148, 148) * 0.018 : 0.0);
+        const double second = std::min(std::max(ctas - 148, 0), 148) / 148.0;
+        const double cost = alone ? n * 0.2 + std::max(0, n - 3) * 0.125 + (cs > 1 ? 0.5 + (0.08 + 0.0105 * tokens) * cs : 0.0) +
+                                        0.24 * (((groups + cs - 1) / cs + 1) / 2) + second * 2.66
+                                  : n + std::max(0, n - 3) + (0.38 + 0.007 * tokens) * cs +
+                                        (cs > 1 ? std::max(0.0, tiles / (8.0 * (32 / cs)) - 0.8) * 8.4 : 0.0);
         if (cost < best_cost - 1e-9) { best_cost = cost; best = cs; }
     }
     return best;
@@ -963,7 +970,7 @@ int launch_dense(DenseParams& p, int split, cudaStream_t stream) {
     if (!allow_smem(dense_kernel<NT, KIND, TQ, TABLE, WIDE>, DGeo<NT, TQ>::SMEM, done, KIND != D_ROWS)) return check_launch();
     const int nch = p.K / kChunkK;
     const int tiles = KIND == D_SILU ? p.N / 64 : (p.N + kTileRows - 1) / kTileRows, wide = WIDE ? (p.M + NT - 1) / NT : 1;
-    const int cs = split > 0 && split <= std::min(kMaxCluster, nch) ? split : plan_cluster(tiles * wide, nch, std::min(p.M, NT), TQ);
+    const int cs = split > 0 && split <= std::min(kMaxCluster, nch) ? split : plan_cluster(tiles * wide, nch, std::min(p.M, NT), TQ, KIND == D_PLAIN || KIND == D_ROWS);
     constexpr int cap = 296;
     auto launch = [&](int lo, int n, int cluster) {
         p.tile_lo = lo;
