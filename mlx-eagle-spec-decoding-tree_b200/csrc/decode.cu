@@ -948,20 +948,36 @@ __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_co
 // of more than 28 tiles (32 x 112 chunks: + 0.7 to 1.7 us).  On average 0.02 us a kernel behind the best of the 64 cases.  (The terms fitted
 // when an exchange cost 0.5 us more kept to half the cluster: 24 x 16 chunks, 32 tokens - 2.2 us with 8 instead of 4, 128 x 16 - 2.8 with 2
 // instead of none.)
-// A matmul on its own (`alone`) has nothing but its like before and behind it, which come up where a CTA leaves them room: there fewer
-// and longer CTAs are better (4096 x 4096, 8 rows: 6.3 us with 4, 7.2 with 7), in microseconds: a chunk 0.2, behind the third 0.125 more, a
-// source of the reduction 0.08 and 0.0105 a token, two groups of tokens to finish 0.24.
-int plan_cluster(int tiles, int nch, int tokens, int group, bool alone) {
+int plan_cluster(int tiles, int nch, int tokens) {
+    int best = 1;
+    double best_cost = 1e30;
+    for (int cs = 1; cs <= kMaxCluster && cs <= nch && (cs == 1 || tiles <= 8 * (32 / cs)) && (cs < 8 || tiles <= 28); cs++) {
+        const int n = ((nch + cs - 1) / cs) * ((tiles * cs + 295) / 296);
+        const double cost = n + std::max(0, n - 3) + (0.38 + 0.007 * tokens) * cs + (cs > 1 ? std::max(0.0, tiles / (8.0 * (32 / cs)) - 0.8) * 8.4 : 0.0);
+        if (cost < best_cost - 1e-9) { best_cost = cost; best = cs; }
+    }
+    return best;
+}
+// Clusters of 1 .. 8 CTAs that find SMs of their own (148 SMs in GPCs of 16 to 20; cudaOccupancyMaxActiveClusters at one CTA per SM).
+constexpr int kOwnSms[kMaxCluster + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+
+// The same for a matmul on its own, which has nothing but its like before and behind it: in microseconds but for a constant, fitted to 37
+// shapes from 128 x 256 to 8192 x 8192 of 1 to 32 rows with every size; 0.2 % behind the best of each on average, 7 % at most.
+// Re-laid-out weights: a chunk 0.2, behind the third 0.055 more, a source of the reduction 0.04, two groups of tokens to finish 0.29; a CTA that
+// shares its SM comes up later, up to 1.2.  (With the terms of exchanges half a microsecond dearer: 32 x 896 x 896 3.7 us in threes, 3.0 in
+// sevens; 32 x 512 x 2048 3.7, 3.3 in eights; 8 x 256 x 512 2.8, 2.1 in fours.)
+// As quantised nothing is expanded before the wait, and two CTAs of an SM then work at the same time: each takes nearly twice as long (2560 x
+// 9728: 9.2 us in sixes, 120 CTAs, 11.8 in sevens, 140 CTAs).  (Before: 8 x 512 x 2048 4.5 in fours, 3.7 in eights; 16 x 896 x 896 4.0 and 3.4.)
+int plan_alone(int tiles, int nch, int tokens, int group, bool as_quantised) {
     int best = 1;
     double best_cost = 1e30;
     const int groups = (tokens + group - 1) / group;
-    for (int cs = 1; cs <= kMaxCluster && cs <= nch && (cs == 1 || tiles <= 8 * (32 / cs)) && (cs < 8 || tiles <= 28 || alone); cs++) {
-        const int ctas = tiles * cs, n = ((nch + cs - 1) / cs) * ((ctas + 295) / 296);
-        const double second = std::min(std::max(ctas - 148, 0), 148) / 148.0;
-        const double cost = alone ? n * 0.2 + std::max(0, n - 3) * 0.125 + (cs > 1 ? 0.5 + (0.08 + 0.0105 * tokens) * cs : 0.0) +
-                                        0.24 * (((groups + cs - 1) / cs + 1) / 2) + second * 2.66
-                                  : n + std::max(0, n - 3) + (0.38 + 0.007 * tokens) * cs +
-                                        (cs > 1 ? std::max(0.0, tiles / (8.0 * (32 / cs)) - 0.8) * 8.4 : 0.0);
+    for (int cs = 1; cs <= kMaxCluster && cs <= nch && (cs == 1 || tiles <= 8 * (32 / cs)); cs++) {
+        const int n = ((nch + cs - 1) / cs) * ((tiles * cs + 295) / 296), finish = ((groups + cs - 1) / cs + 1) / 2;
+        const bool shared = tiles > kOwnSms[cs];
+        const double part = std::min(1.0, std::max(0.0, (double)tiles / kOwnSms[cs] - 1));
+        const double cost = as_quantised ? n * (shared ? 0.38 : 0.2) + (cs > 1 ? 0.17 : 0) + 0.003 * cs + 0.05 * finish + 0.2 * part
+                                         : n * 0.2 + std::max(0, n - 3) * 0.055 + (cs > 1 ? 0.04 * cs : 0) + 0.29 * finish + (shared ? 0.07 : 0) + 1.18 * part;
         if (cost < best_cost - 1e-9) { best_cost = cost; best = cs; }
     }
     return best;
@@ -973,7 +989,9 @@ int launch_dense(DenseParams& p, int split, cudaStream_t stream) {
     if (!allow_smem(dense_kernel<NT, KIND, TQ, TABLE, WIDE, FAST>, DGeo<NT, TQ>::SMEM, done, KIND != D_ROWS)) return check_launch();
     const int nch = p.K / kChunkK;
     const int tiles = KIND == D_SILU ? p.N / 64 : (p.N + kTileRows - 1) / kTileRows, wide = WIDE ? (p.M + NT - 1) / NT : 1;
-    const int cs = split > 0 && split <= std::min(kMaxCluster, nch) ? split : plan_cluster(tiles * wide, nch, std::min(p.M, NT), TQ, KIND == D_PLAIN || KIND == D_ROWS);
+    const int cs = split > 0 && split <= std::min(kMaxCluster, nch) ? split
+                   : KIND == D_PLAIN || KIND == D_ROWS                ? plan_alone(tiles, nch, p.M, TQ, KIND == D_ROWS)
+                                                                      : plan_cluster(tiles * wide, nch, std::min(p.M, NT));
     constexpr int cap = 296;
     auto launch = [&](int lo, int n, int cluster) {
         p.tile_lo = lo;
@@ -1155,6 +1173,25 @@ int run_matmul(const ChainMatmul& c, cudaStream_t st) {
 }
 
 }  // namespace
+
+// Against the large-M kernel, over the shapes above, us here / there.  The clusters add up K without going through memory and the CTAs are
+// half as large, which counts for more the fewer chunks an SM has; its four groups of dequant warps against three win with many.
+// Re-laid-out: up to 2047 chunks (32 rows: 896 x 896 3.0 / 3.9, 4096 x 4096 6.5 / 8.4, 5120 x 5120 7.8 / 9.4, 32000 x 1024 8.7 / 9.3; 16384 x
+// 2048 7.7 to 8.8 / 7.8 to 8.3), and where it has to split K, which it does through memory, up to 4096 (32 x 4096 x 8192 9.2 / 10.8, 32 x 8192
+// x 8192 13.6 / 17.6; 18944 x 3584 12.4 to 14.4 / 11.9 to 12.5, 3584 x 18944 the same).
+// As quantised, where weights have to wait, scales are to be fetched and pairs reordered: always up to 320 chunks (32 rows: 896 x 896 3.7 /
+// 4.8, 512 x 2048 4.2 / 6.3; the smallest only up to 16 rows, 128 x 256 2.7 / 2.9, 32 rows 3.4 / 3.0), up to 1024 if no SM has two CTAs of
+// it (32 x 4608 x 3584 8.8 / 9.2), up to 2048 if moreover K is split and most SMs have one (8 x 4096 x 8192 10.6 / 11.7, 5120 x 5120 9.5 /
+// 10.5; 6144 x 4096 with 96 CTAs the same, 16384 x 2048 10.3 / 9.2, 6144 x 6144 12.1 / 11.5).
+bool chain_matmul_wins(int M, int N, int K, bool as_quantised) {
+    if (M > 32) return false;
+    const int tiles = (N + kTileRows - 1) / kTileRows, nch = K / kChunkK;
+    const long long chunks = (long long)tiles * nch;
+    if (!as_quantised) return chunks < 2048 || (tiles <= 64 && chunks <= 4096);
+    if (chunks < (M <= 16 ? 1 : 8) || chunks > 2048) return false;
+    const int cs = plan_alone(tiles, nch, M, M <= 8 ? 2 : 4, true);
+    return chunks <= 320 || (tiles <= kOwnSms[cs] && (chunks <= 1024 || (cs > 1 && tiles * cs >= 108)));
+}
 
 int chain_matmul(const ChainMatmul& c, cudaStream_t st) {
     return c.M <= 8 ? run_matmul<16, 2>(c, st) : (c.M <= 16 ? run_matmul<16, 4>(c, st) : run_matmul<32, 4>(c, st));
