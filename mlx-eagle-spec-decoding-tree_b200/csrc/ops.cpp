@@ -114,23 +114,30 @@ PyObject* rope_positions(PyObject* const* a, Py_ssize_t n) {
     return THPVariable_Wrap(std::move(y));
 }
 
-// layer_pointers(layers, table) -> 0: `table` (address of [layers][8] pointers in the order of b200_forward_desc.layer_table) holds
+// layer_pointers(layers, table[, changes]) -> 0: `table` (address of [layers][8] pointers in the order of b200_forward_desc.layer_table) holds
 // the device pointers of the layers already, 1: it does now, -1: a layer is not as it should be (no re-laid-out weights, say).
-// Runs ahead of every pass, so that a pass never sees the address of a tensor that has been replaced: ~0.3 us a layer.
+// Runs ahead of every pass, so that a pass never sees the address of a tensor that has been replaced: ~0.3 us a layer.  `changes` (address
+// of 64 bits) becomes a number that is another one once a re-laid-out matrix has been written in place.
 PyObject* layer_pointers(PyObject*, PyObject* const* a, Py_ssize_t n) {
     static PyObject* const linears[] = {PyUnicode_InternFromString("qkv"), PyUnicode_InternFromString("o"), PyUnicode_InternFromString("gate"),
                                         PyUnicode_InternFromString("up"), PyUnicode_InternFromString("down")};
     static PyObject* const norms[] = {PyUnicode_InternFromString("input_norm"), PyUnicode_InternFromString("post_norm")};
     static PyObject* const tiled = PyUnicode_InternFromString("tiled");
     static PyObject* const bias = PyUnicode_InternFromString("bias");
-    void** table = n == 2 && (PyList_Check(a[0]) || PyTuple_Check(a[0])) ? static_cast<void**>(PyLong_AsVoidPtr(a[1])) : nullptr;
+    void** table = (n == 2 || n == 3) && (PyList_Check(a[0]) || PyTuple_Check(a[0])) ? static_cast<void**>(PyLong_AsVoidPtr(a[1])) : nullptr;
+    uint64_t* changes = table != nullptr && n == 3 ? static_cast<uint64_t*>(PyLong_AsVoidPtr(a[2])) : nullptr;
     if (PyErr_Occurred()) return nullptr;
     if (table == nullptr) return PyLong_FromLong(-1);
+    uint64_t versions = 0;
     bool plain = true, same = true;
     auto put = [&](PyObject* t, bool optional) {              // (borrowed, may be NULL)
         void* q = nullptr;
         if (t == nullptr || !THPVariable_Check(t)) plain = plain && optional && t == Py_None;
-        else q = THPVariable_Unpack(t).data_ptr();
+        else {
+            const at::Tensor& x = THPVariable_Unpack(t);
+            q = x.data_ptr();
+            versions = versions * 31 + (x.is_inference() ? 0 : x._version());
+        }
         same = same && *table == q;
         *table++ = q;
     };
@@ -155,6 +162,7 @@ PyObject* layer_pointers(PyObject*, PyObject* const* a, Py_ssize_t n) {
     } catch (const std::exception&) {                            // (a tensor without storage)
         plain = false;
     }
+    if (changes != nullptr) *changes = versions;
     return PyLong_FromLong(!plain ? -1 : (same ? 0 : 1));
 }
 

@@ -198,18 +198,24 @@ class QLinear:
         self.in_features = wq.shape[1] * 8
         self.group_size, self.bits = 64, 4
         self.tiled = None
-        self.scales_fast = False
+        self._fast_of = None
 
     def relayout(self, keep_rowmajor: bool = False):
         """Build the streaming layout of this layer's weights; drop the row-major tensors unless asked."""
         self._nbytes = self.nbytes()
-        # a shard's persistent kernel expands nibbles with a shorter, bit-identical sequence when every scale's fp16
+        # a pass's kernels expand nibbles with a shorter, bit-identical sequence when every scale's fp16
         # exponent field is in 1..10 (2^-14 <= |s| < 2^-4); recorded here, while the scales are still at hand
         e = (self.scales.view(torch.int16).to(torch.int32) >> 10) & 31
-        self.scales_fast = bool(((e >= 1) & (e <= 10)).all())
         self.tiled = qk.relayout(self.weight, self.scales, self.biases)
+        ok = not self.tiled.is_inference() and bool(((e >= 1) & (e <= 10)).all())      # (an inference tensor does not count its changes)
+        self._fast_of = (self.tiled, self.tiled._version) if ok else None
         if not keep_rowmajor:
             self.weight = self.scales = self.biases = None
+
+    @property
+    def scales_fast(self) -> bool:
+        """Every scale is known to allow the short expansion: of the tensor that ``relayout`` made, neither replaced nor written since."""
+        return self._fast_of is not None and self._fast_of[0] is self.tiled and self._fast_of[1] == self.tiled._version
 
     def nbytes(self) -> int:
         if self.weight is None:
@@ -558,9 +564,13 @@ class Model:
         False if a layer has no re-laid-out weights."""
         n = self.args.num_hidden_layers
         if self._layers_host is None:
-            self._layers_host = (ctypes.c_void_p * (8 * n))()
-        state = _lib.ops().layer_pointers(self.layers, ctypes.addressof(self._layers_host)) if len(self.layers) == n else -1
+            self._layers_host, self._layer_changes = (ctypes.c_void_p * (8 * n))(), ctypes.c_uint64()
+        before = self._layer_changes.value
+        state = _lib.ops().layer_pointers(self.layers, ctypes.addressof(self._layers_host),
+                                          ctypes.addressof(self._layer_changes)) if len(self.layers) == n else -1
         if state == 0 and self._layer_table is not None:
+            if self._layer_changes.value != before:      # (written in place)
+                self._layers_fast = self._all_fast()
             return True
         self._graphs.clear()                             # (a graph has the layers' pointers in it)
         self._layer_table = None
@@ -568,15 +578,18 @@ class Model:
             self._fuse_fits = self._pf_fits = False
             return False
         self._layer_table = torch.tensor([p or 0 for p in self._layers_host], dtype=torch.int64).to(self.device)
-        self._layers_fast = all(lw[k].scales_fast for lw in self.layers for k in ("qkv", "o", "gate", "up", "down"))
+        self._layers_fast = self._all_fast()
         return True
 
+    def _all_fast(self) -> bool:
+        return all(lw[k].scales_fast for lw in self.layers for k in ("qkv", "o", "gate", "up", "down"))
+
     def weight_addresses(self) -> bytes:
-        """Where this model's weights are now, for whoever keeps graphs of its passes."""
+        """Where this model's weights are now, and whether they allow the short expansion, for whoever keeps graphs of its passes."""
         linears, others = [self.embed, self.lm_head], [self.norm, self.inv_freqs]
         layers = b""
         if self.can_fuse():
-            layers = bytes(self._layers_host)
+            layers = bytes(self._layers_host) + bytes([self._layers_fast and self.lm_head.scales_fast and self.fast_dequant])
         else:
             linears += [lw[k] for lw in self.layers for k in ("qkv", "o", "gate", "up", "down")]
             others += [lw[k] for lw in self.layers for k in ("input_norm", "post_norm")]

@@ -1,0 +1,41 @@
+"""The short nibble expansion is chosen for weights that `relayout` found to allow it.  Weights that take their place afterwards, as
+another tensor or written over the old one, are expanded as they need: with passes launched one by one and with graphs of them."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("which", ["layer", "head"])
+@pytest.mark.parametrize("how", ["replaced", "written"])
+def test_weights_that_change_after_relayout(be, cuda, how, which):
+    args = be.shape_preset("tiny-qwen2")
+    m = be.Model.random_init(args, seed=5, device=cuda, gen_device="cpu")
+    lin = m.layers[1]["down"] if which == "layer" else m.lm_head
+    packed = [t.clone() for t in (lin.weight, lin.scales, lin.biases)]
+    packed[1][3:40] = 0.25                               # beyond the range
+    packed[1][41] = 0.0
+    wide = be.qmm_kernel.relayout(*packed)
+    m.relayout()
+    tokens = torch.arange(7, dtype=torch.int32, device=cuda)[None]
+    cache = m.make_cache(128)
+
+    def run():
+        cache.offset = 0
+        return m(tokens, cache).clone()
+
+    for _ in range(2 * m._graphs.AFTER):
+        before = run()
+    assert m._scales_fast is True
+    kept = m.weight_addresses()
+    if how == "replaced":
+        lin.tiled = wide
+    else:
+        lin.tiled.copy_(wide)
+    got = [run() for _ in range(2 * m._graphs.AFTER)]
+    assert m._scales_fast is False and m.weight_addresses() != kept
+    m.fast_dequant = False
+    want = run()
+    m.check_fused_error()
+    assert torch.isfinite(want).all() and not torch.equal(want, before)
+    assert all(torch.equal(g, want) for g in got)        # the same kernels: the same bits
