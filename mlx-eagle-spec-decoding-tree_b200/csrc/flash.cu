@@ -235,16 +235,16 @@ __global__ void __launch_bounds__(FGeo<HD, DECODE>::THREADS) flash_kernel(const 
                 for (int x = 0; x < HD / 64; x++) tma_box3(sbase + x * G::QBOX, &p.qmap, x * 64, hk * p.G + hs * p.heads, tok_base, smem_u32(&qfull));
             }
             __syncwarp();
-            mbar_wait_reported(smem_u32(&qfull), 0, p.polls, p.err, 30);
+            mbar_wait_reported(smem_u32(&qfull), 0, p.polls, p.err, 28);
             scores(0);
 #pragma unroll 1
             for (int i = 0; i < nb; i++) {
                 if (i + 1 < nb) {
-                    if (i > 0) mbar_wait_reported(smem_u32(&pvdone), (i - 1) & 1, p.polls, p.err, 30);      // (its probabilities stand where the scores go)
+                    if (i > 0) mbar_wait_reported(smem_u32(&pvdone), (i - 1) & 1, p.polls, p.err, 28);      // (its probabilities stand where the scores go)
                     scores(i + 1);
                 }
                 mbar_wait_reported(smem_u32(vfull + i % ST), (i / ST) & 1, p.polls, p.err, 29);
-                mbar_wait_reported(smem_u32(pready + (i & 1)), (i >> 1) & 1, p.polls, p.err, 30);
+                mbar_wait_reported(smem_u32(pready + (i & 1)), (i >> 1) & 1, p.polls, p.err, 28);
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 __syncwarp();
                 if (elect_one()) {
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(FGeo<HD, DECODE>::THREADS) flash_kernel(const 
                 vis = c >= kKeyBlock ? ~0ull : (c <= 0 ? 0ull : (1ull << c) - 1);
             }
             const uint32_t seen = (uint32_t)(vis >> (KEYS * part));
-            mbar_wait_reported(smem_u32(sfull + (i & 1)), (i >> 1) & 1, p.polls, p.err, 31);
+            mbar_wait_reported(smem_u32(sfull + (i & 1)), (i >> 1) & 1, p.polls, p.err, 27);
             __syncwarp();
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             uint32_t raw[KEYS];
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(FGeo<HD, DECODE>::THREADS) flash_kernel(const 
             }
             l = l * al + (sum[0] + sum[1]);
             if (rescale) {
-                mbar_wait_reported(smem_u32(&pvdone), (i - 1) & 1, p.polls, p.err, 31);
+                mbar_wait_reported(smem_u32(&pvdone), (i - 1) & 1, p.polls, p.err, 27);
                 __syncwarp();
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 #pragma unroll
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(FGeo<HD, DECODE>::THREADS) flash_kernel(const 
 #pragma unroll
         for (int j = 1; j < PT; j++) l += s_part[nb & 1][j][r];
         if (nb > 0) {
-            mbar_wait_reported(smem_u32(&ofull), 0, p.polls, p.err, 31);
+            mbar_wait_reported(smem_u32(&ofull), 0, p.polls, p.err, 27);
             __syncwarp();
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         }
