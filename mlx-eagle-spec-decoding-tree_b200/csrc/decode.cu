@@ -6,7 +6,7 @@
 //                          E  down_proj matmul + residual                 | vocabulary projection
 //
 // Why a chain and not one persistent kernel: a kernel of such a chain whose every CTA reads what all CTAs of its predecessor
-// wrote costs 1.0 us, the load included; a device-wide barrier of 148 CTAs took 1.5 to 2.3 us and the first loads behind it
+// wrote costs 1.0 to 1.3 us, the load included; a device-wide barrier of 148 CTAs took 1.5 to 2.3 us and the first loads behind it
 // another 1.1.  A CTA here keeps to half of an SM (512 threads, 64 registers each, ~95 KB of shared memory, 256 columns of tensor memory), so
 // the next kernel's CTAs become resident beside it and stream and expand their first weights before its results are there.
 //
@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                     if (done >= kGroups) mbar_wait_reported(smem_u32(tfree + me), tph, p.polls, p.err, 24);
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                     __syncwarp();
-                    expand_row<KIND == D_ROWS>(u, sc, bi, fast, trow + me * kTileCols);
+                    expand_row<KIND == D_ROWS, KIND == D_PLAIN && NT == 32>(u, sc, bi, fast, trow + me * kTileCols);
                     asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
                     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                     __syncwarp();
@@ -961,10 +961,10 @@ int plan_cluster(int tiles, int nch, int tokens) {
 // Clusters of 1 .. 8 CTAs that find SMs of their own (148 SMs in GPCs of 16 to 20; cudaOccupancyMaxActiveClusters at one CTA per SM).
 constexpr int kOwnSms[kMaxCluster + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
 
-// The same for a matmul on its own, which has nothing but its like before and behind it: in microseconds but for a constant, fitted to 37
-// shapes from 128 x 256 to 8192 x 8192 of 1 to 32 rows with every size; 0.2 % behind the best of each on average, 7 % at most.
-// Re-laid-out weights: a chunk 0.2, behind the third 0.055 more, a source of the reduction 0.04, two groups of tokens to finish 0.29; a CTA that
-// shares its SM comes up later, up to 1.2.  (With the terms of exchanges half a microsecond dearer: 32 x 896 x 896 3.7 us in threes, 3.0 in
+// The same for a matmul on its own, which has nothing but its like before and behind it: in microseconds but for a constant, fitted to 40
+// shapes from 128 x 256 to 8192 x 8192 of 1 to 32 rows with every size; 0.3 % behind the best of each on average, 6 % at most.
+// Re-laid-out weights: a chunk 0.2, behind the third 0.05 more, a source of the reduction 0.04, two groups of tokens to finish 0.2; a CTA that
+// shares its SM comes up 0.1 to 1.4 later.  (With the terms of exchanges half a microsecond dearer: 32 x 896 x 896 3.7 us in threes, 3.0 in
 // sevens; 32 x 512 x 2048 3.7, 3.3 in eights; 8 x 256 x 512 2.8, 2.1 in fours.)
 // As quantised nothing is expanded before the wait, and two CTAs of an SM then work at the same time: each takes nearly twice as long (2560 x
 // 9728: 9.2 us in sixes, 120 CTAs, 11.8 in sevens, 140 CTAs).  (Before: 8 x 512 x 2048 4.5 in fours, 3.7 in eights; 16 x 896 x 896 4.0 and 3.4.)
@@ -977,7 +977,7 @@ int plan_alone(int tiles, int nch, int tokens, int group, bool as_quantised) {
         const bool shared = tiles > kOwnSms[cs];
         const double part = std::min(1.0, std::max(0.0, (double)tiles / kOwnSms[cs] - 1));
         const double cost = as_quantised ? n * (shared ? 0.38 : 0.2) + (cs > 1 ? 0.17 : 0) + 0.003 * cs + 0.05 * finish + 0.2 * part
-                                         : n * 0.2 + std::max(0, n - 3) * 0.055 + (cs > 1 ? 0.04 * cs : 0) + 0.29 * finish + (shared ? 0.07 : 0) + 1.18 * part;
+                                         : n * 0.2 + std::max(0, n - 3) * 0.05 + (cs > 1 ? 0.04 * cs : 0) + 0.2 * finish + (shared ? 0.1 : 0) + 1.3 * part;
         if (cost < best_cost - 1e-9) { best_cost = cost; best = cs; }
     }
     return best;

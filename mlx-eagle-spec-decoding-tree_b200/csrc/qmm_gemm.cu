@@ -23,6 +23,8 @@
 // ~700 of 1024 slots per scheduler.  With few tokens the weight stream is the bound: 18.4 KB per chunk are ~800 cycles of
 // an SM's share of HBM.
 //
+// Beyond 128 tokens csrc/qmm_pair.cu, whose CTAs work in pairs on a tile, runs where it is cheaper (pair_plan below).
+//
 // Where the tiles alone would leave SMs idle the K range is cut across CTAs; the last CTA of a tile adds the fp32 partial
 // products in split order (deterministic).  Every wait is bounded; one that runs out sets the error word.  No copy uses cluster multicast.
 #include <cuda.h>
@@ -462,7 +464,7 @@ __global__ void __launch_bounds__(kGThreads, 1) qmm_gemm_kernel(const __grid_con
                     bi2[0] = bv; bi2[1] = bv >> 16;
                 }
                 const bool fast = __all_sync(0xffffffffu, fast_scale(sc2[0]) && fast_scale(sc2[1]));
-                expand_row<LAYOUT == W_ROWS>(u, sc2, bi2, fast, trow);
+                expand_row<LAYOUT == W_ROWS, LAYOUT == W_ROWS && NT == 128>(u, sc2, bi2, fast, trow);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(pempty + slot));       // the packs are in registers
                 asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");

@@ -45,15 +45,15 @@ __device__ __forceinline__ void tmem_ld(uint32_t (&r)[C], uint32_t addr) {
 
 // The thread's row of a chunk (16 packs, 128 k) -> its lane of the tile at `trow`, sixteen columns (32 k) at a time.  Streaming layout:
 // pack j of unit t is k group 4 j + t; ROWS (as quantised): pack t of unit j, its values still to be put side by side.  sc, bi: scale and
-// bias of the chunk's two groups of 64, in the low halves.
-template <bool ROWS>
+// bias of the chunk's two groups of 64, in the low halves; WORDS: doubled as words.
+template <bool ROWS, bool WORDS = false>
 __device__ __forceinline__ void expand_row(const uint4 (&u)[4], const uint32_t (&sc)[2], const uint32_t (&bi)[2], bool fast, uint32_t trow) {
     auto expand = [&](auto fast_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            __half2 s2 = dup_half((unsigned short)sc[j >> 1]);
-            const __half2 b2 = dup_half((unsigned short)bi[j >> 1]);
+            __half2 s2 = WORDS ? dup_half_of_word(sc[j >> 1]) : dup_half((unsigned short)sc[j >> 1]);
+            const __half2 b2 = WORDS ? dup_half_of_word(bi[j >> 1]) : dup_half((unsigned short)bi[j >> 1]);
             if (FAST) s2 = scale_times_2_20(s2);
             uint32_t d[4][4];
 #pragma unroll
