@@ -3,8 +3,10 @@
 //   embedding + input norm | per layer: q|k|v matmul (+ bias) -> RoPE + KV append -> causal attention -> o_proj matmul
 //   (+ residual) -> norm -> gate/up matmul (SiLU(gate) * up) -> down matmul (+ residual) -> norm | vocabulary projection
 //
-// The matmuls are csrc/qmm_gemm.cu (one weight read per 128 tokens, from L2 after the first); the element-wise steps that
-// do not fit their epilogues are the kernels below.  Rounding points are those of the 32-row path's per-op kernels: norm ->
+// The matmuls are csrc/qmm_gemm.cu and, beyond 128 tokens where it is cheaper, csrc/qmm_pair.cu, attention is csrc/flash.cu; the
+// element-wise steps that do not fit their epilogues are the kernels below (8B shape, 1024 tokens: 17 of 420 us a layer; their waits hidden
+// behind the matmul before them, nothing was gained: such a pass runs at the power limit).  Up to 128 tokens of a small model go
+// through the kernels of csrc/decode.cu instead.  Rounding points are those of the 32-row path's per-op kernels: norm ->
 // fp16, product -> fp16, + bias / + residual in fp16, SiLU(gate) * up with fp16 results, probabilities -> fp16.
 // Replaces the chunk loop of mlx_eagle.py:522-535 over mlx_llama.py:231-249.
 #include <algorithm>
