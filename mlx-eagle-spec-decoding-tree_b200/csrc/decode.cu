@@ -586,7 +586,6 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
 // ================================================================================ embedding
 // One CTA per token: dequantised embedding row -> h, h * w_norm, sums of squares per 32 columns, and the token's RoPE table.  The norm
 // weights may come from the layer table (`wn_entry`).
-// The attention of a short prompt takes a tree's mask words and committed length, which come from here, too.
 // The next kernel is let go only behind the wait: everything before the pass (tree kernels, KV compaction, other programs'
 // writes) is then complete before any kernel of the pass starts, which may so read committed K/V rows, and the layer table, ahead
 // of its own wait.
@@ -594,15 +593,11 @@ __global__ void __launch_bounds__(256) embed_kernel(const int* __restrict__ toke
                                                     const __half* __restrict__ sc, const __half* __restrict__ bi, const __half* wn,
                                                     __half* __restrict__ h, __half* __restrict__ hw, float* __restrict__ ssq,
                                                     float2* __restrict__ cs, const float* __restrict__ inv_freq, float scaling, int H, int V,
-                                                    int half_hd, const void* const* wn_entry, int pitch, int pos0, unsigned long long* mask, int* prefix) {
+                                                    int half_hd, const void* const* wn_entry, int pitch, int pos0) {
     pdl_wait();
     pdl_launch_dependents();
     if (wn_entry != nullptr) wn = listed<__half>(wn_entry);
     const int m = blockIdx.x, units = H / 8;
-    if (mask != nullptr && threadIdx.x == 0) {                      // a causal pass behind pos0 rows
-        mask[m] = (2ull << m) - 1;
-        if (m == 0) *prefix = pos0;
-    }
     const int tok = min(max(tokens[m], 0), V - 1);
     for (int u = threadIdx.x; u < ((units + 31) & ~31); u += 256) {
         float ss = 0.f;
@@ -1065,7 +1060,7 @@ int run_chain(const ChainArgs& c, cudaStream_t st) {
     if (on(0) || TABLE) {                                       // (what makes the table safe to read ahead of a kernel's wait)
         launch_kernel(embed_kernel, dim3(M), dim3(256), 0, st, d->tokens, d->pos, d->embed_wq, static_cast<const __half*>(d->embed_scales),
                       static_cast<const __half*>(d->embed_biases), static_cast<const __half*>(given(layers, 6)), p.h, p.hw, p.ssq, c.cs, d->inv_freq,
-                      d->rope_scaling, H, d->vocab, hd / 2, TABLE ? layers + 6 : nullptr, kSsqPitch, 0, static_cast<unsigned long long*>(nullptr), static_cast<int*>(nullptr));
+                      d->rope_scaling, H, d->vocab, hd / 2, TABLE ? layers + 6 : nullptr, kSsqPitch, 0);
         if ((rc = check_launch()) != B200_OK) return rc;
     }
     for (int l = 0; l < d->n_layers; l++) {
@@ -1129,7 +1124,7 @@ int run_prompt(const ChainPrompt& c, cudaStream_t st) {
     const size_t half = (size_t)d->n_kv_heads * d->cache_rows * hd;
     launch_kernel(embed_kernel, dim3(n), dim3(256), 0, st, d->tokens, static_cast<const int*>(nullptr), d->embed_wq, static_cast<const __half*>(d->embed_scales),
                   static_cast<const __half*>(d->embed_biases), static_cast<const __half*>(d->layers[6]), p.h, p.hw, p.ssq, c.cs, d->inv_freq, d->rope_scaling, H, d->vocab,
-                  hd / 2, static_cast<const void* const*>(nullptr), p.pitch, d->off, c.mask, c.prefix);
+                  hd / 2, static_cast<const void* const*>(nullptr), p.pitch, d->off);
     if ((rc = check_launch()) != B200_OK) return rc;
     for (int l = 0; l < d->n_layers; l++) {
         const void* const* L = d->layers + (size_t)l * 8;       // qkv, qkv bias, o, gate, up, down, input norm, post norm

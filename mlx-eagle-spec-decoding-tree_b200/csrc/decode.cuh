@@ -23,8 +23,6 @@ struct ChainPrompt {
     int* err;
     float* ssq;                  // [hidden / 32][tokens rounded up to 32]
     float2* cs;                  // [tokens][64]
-    unsigned long long* mask;    // [tokens], at most 64, and committed length for the attention; or NULL
-    int* prefix;
     int (*attention)(const void* context, int row0, cudaStream_t stream);
     const void* context;
 };

@@ -145,8 +145,9 @@ __global__ void __launch_bounds__(FGeo<HD, DECODE>::THREADS) flash_kernel(const 
     pdl_launch_dependents();
     if (DECODE && cs > 1) cluster_arrive_relaxed();
 
-    // (decode: the committed length was there before the pass; what reads it is complete before any kernel of the pass starts)
-    const int prefix = DECODE ? p.prefix[req] : p.off;
+    // Mask and committed length are read ahead of the wait for the kernel before this one: where they are given as memory, that was written
+    // before the pass, and what wrote it is complete before any kernel of the pass starts.  A causal pass has them by value (`off`).
+    const int prefix = DECODE && p.prefix != nullptr ? p.prefix[req] : p.off;
     int b0, b1;                                                          // this CTA's key blocks
     if (DECODE) {
         const int nact = min((prefix + p.tail + kKeyBlock - 1) / kKeyBlock, p.nkb);
@@ -270,7 +271,7 @@ __global__ void __launch_bounds__(FGeo<HD, DECODE>::THREADS) flash_kernel(const 
         if (DECODE && cs > 1) cluster_wait();
         unsigned long long mk = 0;                                       // the tail rows this row sees
         if (DECODE && valid) {
-            mk = p.mask[tok_base + t];
+            mk = p.mask != nullptr ? p.mask[tok_base + t] : (2ull << (ts * p.T + t)) - 1;
             if (p.tail < 64) mk &= (1ull << p.tail) - 1;
         }
         const int lim = p.off + ts * p.T + t;                            // prompt: the last key this row sees

@@ -17,7 +17,8 @@ struct FlashArgs {
     float scale_log2;
     int* err;
     int polls;
-    // the decode chain: `mr` tokens of each of `nreq` requests over prefix[request] committed rows, tail rows by bit mask
+    // the decode chain: `mr` tokens of each of `nreq` requests over prefix[request] committed rows, tail rows by bit mask.  Both are read before
+    // the kernel ahead of the attention has ended, so nothing in the pass may write them: NULL for a causal pass of one request behind `off` rows.
     const unsigned long long* mask;
     const int* prefix;
     int nreq, mr, tail, write_off, nkb, split;

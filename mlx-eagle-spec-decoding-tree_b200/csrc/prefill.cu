@@ -186,14 +186,13 @@ bool chain_prompt_wins(const b200_prefill_desc* d) {
                             chunks(d->hidden, d->intermediate);
     return d->n <= kChainPromptTokens && layer * ((d->n + 31) / 32) <= 11200;
 }
-// Its scratch, and that of the attention when that is a tree's.
+// Its scratch.
 struct ChainScratch {
-    size_t cs, ssq, mask, bytes;
+    size_t cs, ssq, bytes;
     ChainScratch(int hidden, int n) {
         cs = 0;
         ssq = cs + (size_t)n * 64 * sizeof(float2);
-        mask = ssq + (size_t)(hidden / 32) * ((n + 31) / 32 * 32) * sizeof(float);
-        bytes = mask + 64 * sizeof(unsigned long long) + 16;       // and the committed length
+        bytes = ssq + (size_t)(hidden / 32) * ((n + 31) / 32 * 32) * sizeof(float);
     }
 };
 
@@ -267,9 +266,7 @@ int b200_prefill(const b200_prefill_desc* d, void* stream) {
         c.ssq = reinterpret_cast<float*>(at + scratch.ssq);
         struct Attention { const FlashArgs* a; const FlashPlan* plan; bool tree; } attention{&a, &flash, n <= 64 && a.splits > 1};
         if (attention.tree) {                                      // key ranges by the CTAs of a cluster, merged in the same kernel
-            c.mask = reinterpret_cast<unsigned long long*>(at + scratch.mask);
-            c.prefix = reinterpret_cast<int*>(c.mask + 64);
-            a.mask = c.mask; a.prefix = c.prefix; a.nreq = 1; a.mr = a.tail = n; a.nkb = (d->cache_rows + kKeyBlock - 1) / kKeyBlock;
+            a.nreq = 1; a.mr = a.tail = n; a.nkb = (d->cache_rows + kKeyBlock - 1) / kKeyBlock;
             if ((rc = flash_decode_plan(a, &flash)) != B200_OK) return rc;
         }
         c.attention = [](const void* p, int row0, cudaStream_t stream) {

@@ -50,3 +50,25 @@ def test_without_scratch_the_large_kernels_run(be, cuda):
     m.check_fused_error()
     for a, b in zip(small, full):
         assert ((a - b).abs() <= 2.0 ** -6 * b.abs() + 1e-2).all()
+
+
+@pytest.mark.parametrize("n,off", [(33, 700), (64, 448), (64, 1500)])
+def test_attention_over_a_filled_cache_takes_nothing_from_scratch(be, cuda, n, off):
+    """It starts while kernels two before it may still run, so mask and committed length come by value: the pass writes none of
+    them (the scratch behind rotations and sums of squares stays as it was), and what the scratch held changes no bit."""
+    m = _model(be, cuda, *SHAPES[1])
+    hidden = m.args.hidden_size
+    tokens = torch.randint(0, 520, (n,), generator=torch.Generator().manual_seed(n))[None].to(cuda)
+    want = _run(be, m, tokens, off, False, True)
+    used = 4096 + n * 64 * 8 + hidden // 32 * ((n + 31) // 32 * 32) * 4
+    for fill in (0, 255, 1):
+        m._pf_buf["ws"][4096:].fill_(fill)
+        got = _run(be, m, tokens, off, False, True)
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+        m._pf_buf["ws"][4096:].fill_(fill)
+        cache = m.make_cache(64 * ((off + n + 63) // 64))
+        cache.offset = off
+        assert m.can_prefill_large_m()
+        m._prefill_large_m(tokens[0].int(), cache, off, None, 0)
+        assert (m._pf_buf["ws"][used:] == fill).all()
+    m.check_fused_error()
