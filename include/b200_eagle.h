@@ -238,7 +238,8 @@ int b200_tree_attention(const void* q, int q_stride, const void* kcache, const v
  * hw, attn, act are scratch in a layout of the kernels' own and need 32*width halves each, width = hidden,
  * n_heads*head_dim, intermediate.  kv_cache is
  * [n_layers][2][n_kv_heads][cache_rows][head_dim] fp16; the K/V rows of the M new tokens are written
- * to cache row prefix[0]+write_off+m.  Output row r of logits belongs to token row_index[0]+r
+ * to cache row prefix[0]+write_off+m; rows from prefix[0]+tail on may hold anything, those before it finite numbers,
+ * shown to a token or not.  Output row r of logits belongs to token row_index[0]+r
  * (row_index may be NULL = 0).  RMSNorm is folded into the adjacent matmuls (h*w is rounded to fp16,
  * the per-token 1/rms multiplies the fp32 accumulator), which differs from the per-op kernels by
  * input-rounding noise only.
@@ -414,7 +415,7 @@ typedef struct b200_prefill_desc {
     void* attn;                 /* [n][n_heads * head_dim] */
     void* act;                  /* [n][intermediate] */
     void* logits;               /* [n or 1][vocab] */
-    void* kv_cache;             /* [n_layers][2][n_kv_heads][cache_rows][head_dim] */
+    void* kv_cache;             /* [n_layers][2][n_kv_heads][cache_rows][head_dim]; rows from off + n on may hold anything */
     void* workspace;            /* as b200_qmm_gemm's; what exceeds 4 KiB holds partial sums (16 MiB serve every size well) */
     size_t workspace_bytes;
 } b200_prefill_desc;

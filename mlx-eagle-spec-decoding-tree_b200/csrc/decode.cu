@@ -760,6 +760,12 @@ __global__ void __launch_bounds__(kAWarps * 32) attention_kernel(const __grid_co
         __syncwarp();
         if (busy) {
             const uint32_t sk = sbase + st * G::BLOCK, sv = sk + (HD / 64) * 8192;
+            if (b == b1 - 1)                                             // rows of V past the last: 0 x Inf or NaN would be NaN
+#pragma unroll 1
+                for (int k = (prefix + p.tail - b * kKeyBlock) * 8 + (int)threadIdx.x; k < kKeyBlock * 8; k += kAWarps * 32)
+#pragma unroll
+                    for (int x = 0; x < HD / 64; x++)
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};\n" ::"r"(sv + x * 8192 + k * 16), "r"(0) : "memory");
             // scores of this warp's keys
             const int k0 = part * KT * 8;
             float s[KT][4], s1[KT][4];                                   // (even and odd steps apart: chains of half the length)

@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(FGeo<HD, DECODE>::THREADS) flash_kernel(const 
         b0 = (int)blockIdx.z * per;
         b1 = min(b0 + per, all);
     }
-    const int nb = max(b1 - b0, 0);
+    const int nb = max(b1 - b0, 0), end = DECODE ? prefix + p.tail : p.off + p.n;      // (first cache row that is nobody's)
     const int nslot = (rows + (int)cs - 1) / (int)cs, row_lo = (int)rank * nslot, mine_rows = min(nslot, rows - row_lo);    // rows this CTA finishes
     if (DECODE && cs > 1 && threadIdx.x == 0)                            // what the cluster will copy here
         mbar_expect_tx(smem_u32(&inboxfull), max(mine_rows, 0) * (int)cs * G::OP * 4);
@@ -245,6 +245,18 @@ __global__ void __launch_bounds__(FGeo<HD, DECODE>::THREADS) flash_kernel(const 
                     scores(i + 1);
                 }
                 mbar_wait_reported(smem_u32(vfull + i % ST), (i / ST) & 1, p.polls, p.err, 29);
+                if (i == nb - 1 && end < (b0 + nb) * kKeyBlock) {        // (while the block's softmax runs)
+                    // The box reaches past the last row: there is what the cache, or the next head's, holds there.  Its probabilities are 0, and
+                    // 0 x Inf or NaN would be NaN in every row.
+                    const uint32_t v = sbase + G::KV0 + (i % ST) * 2 * G::HALF + G::HALF;
+#pragma unroll 1
+                    for (int k = (end - (b0 + i) * kKeyBlock) * 8 + lane; k < kKeyBlock * 8; k += 32)
+#pragma unroll
+                        for (int x = 0; x < HD / 64; x++)
+                            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};\n" ::"r"(v + x * 8192 + k * 16), "r"(0) : "memory");
+                    fence_proxy_async();
+                    __syncwarp();
+                }
                 mbar_wait_reported(smem_u32(pready + (i & 1)), (i >> 1) & 1, p.polls, p.err, 28);
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 __syncwarp();
