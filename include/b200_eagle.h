@@ -320,7 +320,8 @@ typedef struct b200_forward_desc {
     int scales_in_fast_range;   /* non-zero: EVERY group scale of every matrix of layer_table and of lm_head_tiled has its
                                  * fp16 exponent field in 1..10 (2^-14 <= |scale| < 2^-4, never zero or subnormal): the
                                  * kernel then expands the nibbles with a shorter instruction sequence that gives the
-                                 * same bits.  0 is always safe. */
+                                 * same bits, and is not asked again whether it may: with scales outside the range the
+                                 * results are wrong.  0 is always safe. */
     int tp_two_shot;            /* exchange of the row-parallel layers (o_proj, down_proj); the same value on every rank,
                                  * the same bits whichever form runs; zero the exchange buffers when switching.
                                  * 0 = the library's choice (the push form).

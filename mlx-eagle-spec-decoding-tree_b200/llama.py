@@ -201,16 +201,25 @@ class QLinear:
         self._fast_of = None
 
     def relayout(self, keep_rowmajor: bool = False):
-        """Build the streaming layout of this layer's weights; drop the row-major tensors unless asked."""
+        """Build the streaming layout of this layer's weights; drop the row-major tensors unless asked.
+
+        Passes trust what is found here about the scales for as long as ``tiled`` is the same tensor and torch has counted no change
+        of it.  A write that torch does not count (through ``.data``, DLPack, ``__cuda_array_interface__`` or a kernel of the
+        caller's) needs ``weights_changed()`` before the next pass: scales outside 2^-14 .. 2^-4 would be expanded wrongly."""
         self._nbytes = self.nbytes()
-        # a pass's kernels expand nibbles with a shorter, bit-identical sequence when every scale's fp16
-        # exponent field is in 1..10 (2^-14 <= |s| < 2^-4); recorded here, while the scales are still at hand
-        e = (self.scales.view(torch.int16).to(torch.int32) >> 10) & 31
         self.tiled = qk.relayout(self.weight, self.scales, self.biases)
-        ok = not self.tiled.is_inference() and bool(((e >= 1) & (e <= 10)).all())      # (an inference tensor does not count its changes)
-        self._fast_of = (self.tiled, self.tiled._version) if ok else None
+        self.weights_changed()
         if not keep_rowmajor:
             self.weight = self.scales = self.biases = None
+
+    def weights_changed(self):
+        """Look at the scales of the re-laid-out weights again (waits for the device).  For a layer of a ``Model``:
+        ``Model.weights_changed``, which also lets go of what was made for the old ones."""
+        # a pass's kernels expand nibbles with a shorter, bit-identical sequence when every scale's fp16
+        # exponent field is in 1..10 (2^-14 <= |s| < 2^-4)
+        e = (qk.tiled_scales(self.tiled, self.out_features, self.in_features).view(torch.int16).to(torch.int32) >> 10) & 31
+        ok = not self.tiled.is_inference() and bool(((e >= 1) & (e <= 10)).all())      # (an inference tensor does not count its changes)
+        self._fast_of = (self.tiled, self.tiled._version) if ok else None
 
     @property
     def scales_fast(self) -> bool:
@@ -580,6 +589,16 @@ class Model:
         self._layer_table = torch.tensor([p or 0 for p in self._layers_host], dtype=torch.int64).to(self.device)
         self._layers_fast = self._all_fast()
         return True
+
+    def weights_changed(self):
+        """To be called between passes once re-laid-out weights have been written in a way that torch does not count (``.data``, DLPack,
+        ``__cuda_array_interface__``, a kernel of the caller's).  Their scales are looked at again, which waits for the device;
+        decoders capture their step anew with the next request if the outcome is another one."""
+        for q in [lw[k] for lw in self.layers for k in ("qkv", "o", "gate", "up", "down")] + [self.lm_head]:
+            if q.tiled is not None:
+                q.weights_changed()
+        if self._layer_table is not None:                # (else gathered ahead of the next pass)
+            self._layers_fast = self._all_fast()
 
     def _all_fast(self) -> bool:
         return all(lw[k].scales_fast for lw in self.layers for k in ("qkv", "o", "gate", "up", "down"))

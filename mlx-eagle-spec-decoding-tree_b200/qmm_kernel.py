@@ -144,6 +144,13 @@ def relayout(w, s, b) -> torch.Tensor:
     return out
 
 
+def tiled_scales(wt, n, k) -> torch.Tensor:
+    """The scales ``(n, k / 64)`` of re-laid-out weights: of every record of 16 rows x 128 k, 1024 bytes of packs are followed by two
+    (scale, bias) pairs a row; blocks of 64 rows, their chunks of 128 k, four records each."""
+    pairs = wt.view(-1, k // 128, 4, 1152)[..., 1024:].view(torch.float16).unflatten(-1, (16, 2, 2))[..., 0]
+    return pairs.permute(0, 2, 3, 1, 4).reshape(-1, k // 64)[:n]
+
+
 def matmul_tiled(x, wt, n, *, epilogue=EPI_NONE, wt2=None, bias=None, extra=None, out=None):
     """``x (M<=32, K) @ W.T`` on re-laid-out weights ``wt`` (from ``relayout``) of ``n`` output rows."""
     if epilogue == EPI_NONE and out is None and isinstance(x, torch.Tensor):
