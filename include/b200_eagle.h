@@ -242,7 +242,8 @@ int b200_tree_attention(const void* q, int q_stride, const void* kcache, const v
  * shown to a token or not.  Output row r of logits belongs to token row_index[0]+r
  * (row_index may be NULL = 0).  RMSNorm is folded into the adjacent matmuls (h*w is rounded to fp16,
  * the per-token 1/rms multiplies the fp32 accumulator), which differs from the per-op kernels by
- * input-rounding noise only.
+ * input-rounding noise only while h*w fits fp16: |h*w| of 65520 and more is Inf, where the per-op kernels and b200_prefill
+ * norm h in fp32 first, and a token whose h*w is mostly below 2^-14 loses bits.
  *
  * workspace: b200_forward_workspace_bytes bytes, the first 4352 bytes zero before the first use (the
  * kernel restores that state).  Int word 2 of the workspace is an error flag: non-zero after a launch

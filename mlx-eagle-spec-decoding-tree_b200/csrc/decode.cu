@@ -39,7 +39,7 @@ constexpr int kEpi = 8;                          // of which these run the epilo
 constexpr int kDThreads = (kDeq + 4) * 32;       // + weight producer, activation producer, MMA issuer, sums of squares
 constexpr int kTmem = 256;                       // columns a CTA takes: two CTAs share an SM
 constexpr int kMaxCluster = 8;
-constexpr int kSsqPitch = 32, kSsqCols = 32, kCsPitch = 64, kKeyBlock = 64;
+constexpr int kSsqPitch = 32, kSsqCols = 32, kKeyBlock = 64;
 
 enum { D_QKV = 0, D_RESID = 1, D_SILU = 2, D_HEAD = 3, D_PLAIN = 4, D_ROWS = 5 };      // the last two: y = x W^T (+ bias), a matmul on its own; D_ROWS: W as quantised
 
@@ -72,8 +72,6 @@ struct DenseParams {
     int H;
     float eps;
     int M, N, K;                  // N: output rows of each matrix
-    int pitch;                    // WIDE: of ssq
-    int base;                     // WIDE: first cache row of the pass
     int tile_lo, tiles;           // 128-row tiles (64 + 64 rows of gate and up): first and end
     int* err;
     int polls;                    // of a wait before it gives up
@@ -82,7 +80,7 @@ struct DenseParams {
     __half* kc;                   // this layer's K and V of request 0
     __half* vc;
     const int* prefix;
-    int Hq, Hkv, hd, cap, write_off, mr;
+    int Hq, Hkv, hd, cap, write_off, mr;      // WIDE: write_off is the first cache row of the pass
     size_t req_stride;            // halves between the caches of two requests
     // D_ROWS: packs [N][K / 8] as rows of bytes, boxes of 64 bytes x 128 rows, 64-byte swizzle; scales and biases [N][K / 64]
     CUtensorMap wmap;
@@ -120,7 +118,8 @@ __device__ __forceinline__ void st_async(uint32_t addr, const uint32_t* a, uint3
 // follows in order.  Three chunks are expanded before the wait for the previous kernel: behind it
 // come the activation load (0.5 us), the MMAs (0.1 us a chunk) and the epilogue.  Code that runs once per kernel is kept short:
 // cold instructions cost 2 to 4 cycles each.
-// WIDE (prompts): blockIdx.y counts tiles of NT tokens, each with CTAs of its own that stream and expand the weights for themselves.
+// WIDE (prompts): blockIdx.y counts tiles of NT tokens, each with CTAs of its own that stream and expand the weights for themselves.  The input
+// is normed already, in fp32 by a kernel of its own as in longer prompts: h * w_norm before 1 / rms, in fp16, has less of a range.
 // FAST: every scale is known to allow the short expansion (b200_forward_desc.scales_in_fast_range).  Asking every chunk, with the long
 // expansion at hand, made the 18944 x 3584 pair 18.6 us and not 17.7, the vocabulary projection of the 7B shape 74 and not 68.
 template <int NT, int KIND, int TQ, bool TABLE = false, bool WIDE = false, bool FAST = false>
@@ -135,6 +134,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
     __shared__ __align__(16) float s_rs[32];                                   // 1 / rms per token
     __shared__ int s_base[32];                                                 // per request: committed rows (D_QKV), first row of logits (D_HEAD)
 
+    constexpr bool NORMED = !WIDE && KIND != D_RESID && KIND != D_PLAIN && KIND != D_ROWS;               // the input is h * w_norm: scale by 1 / rms
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank(), cs = cluster_size();
     const int tile0 = p.tile_lo + blockIdx.x / (int)cs, tstep = gridDim.x / (int)cs;
@@ -298,15 +298,14 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         if (KIND == D_QKV)
             asm volatile("" ::"l"(p.cs), "l"(p.kc), "l"(p.vc), "l"(p.prefix), "r"(p.Hq), "r"(p.Hkv), "r"(p.hd), "r"(p.cap), "r"(p.write_off), "r"(p.mr), "l"(p.req_stride));
         if (KIND == D_HEAD) asm volatile("" ::"r"(p.mr), "l"(p.row_index), "r"(p.rows_out));
-        if (KIND != D_RESID && KIND != D_PLAIN && KIND != D_ROWS) {
+        if (NORMED) {
             // (both were there before the pass; read in the epilogue they were 0.5 us of every q|k|v kernel)
-            if (KIND == D_QKV && lane < M / mr) s_base[lane] = WIDE ? p.base + t0 : __ldcg(p.prefix + lane);
+            if (KIND == D_QKV && lane < M / mr) s_base[lane] = __ldcg(p.prefix + lane);
             if (KIND == D_HEAD && lane < M / mr) s_base[lane] = p.row_index != nullptr ? __ldcg(p.row_index + lane) : 0;
             pdl_wait();
             // A lane: four tokens of every `step`-th part, four or eight loads in flight whatever the number of parts.  (Unrolled by seven with
             // the rest one at a time: 4.3 us at 3584 x 16 tokens and 8.3 at 4096 x 32, longer than the MMAs.  Parts of 128 columns, added up
             // by the producer's warps: 0.15 us more for each of them, of 2.7 in a draft-sized layer.)
-            const int pitch = WIDE ? p.pitch : kSsqPitch;
             const int parts = p.H / kSsqCols, quads = M <= 8 ? 2 : (M <= 16 ? 4 : 8), step = 32 / quads, quad = lane & (quads - 1);
             float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
             constexpr int FLY = NT == 16 ? 4 : 8;
@@ -315,7 +314,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                 float4 v[FLY];
 #pragma unroll
                 for (int i = 0; i < FLY; i++)
-                    v[i] = part + i * step < parts ? __ldcg(reinterpret_cast<const float4*>(p.ssq + (part + i * step) * pitch + t0 + quad * 4))
+                    v[i] = part + i * step < parts ? __ldcg(reinterpret_cast<const float4*>(p.ssq + (part + i * step) * kSsqPitch + quad * 4))
                                                    : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int i = 0; i < FLY; i++) { t.x += v[i].x; t.y += v[i].y; t.z += v[i].z; t.w += v[i].w; }
@@ -345,7 +344,6 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
         const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
         // (Four threads of a quarter-warp read the same banks: swapping units between threads to halve that took more issue slots, 16
         // selects a chunk, than the reads took cycles.)
-        constexpr bool NORMED = KIND != D_RESID && KIND != D_PLAIN && KIND != D_ROWS;                 // the input is h * w_norm: scale by 1 / rms
         const __half* const wn = TABLE && KIND == D_RESID && p.tv != nullptr ? listed<__half>(p.tv) : p.wn;
         const __half* const bias = TABLE && KIND == D_QKV ? listed<__half>(p.tv) : p.bias;
         // ---- one finished tile: accumulators -> inbox of the CTA that finishes each token -> output
@@ -374,7 +372,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                 }
             };
             if (it == 0) pdl_wait();
-            if (KIND == D_RESID && valid) extra = wn[n];
+            if (KIND == D_RESID && !WIDE && valid) extra = wn[n];
             if ((KIND == D_QKV || KIND == D_PLAIN || KIND == D_ROWS) && valid && bias != nullptr) {
                 extra = bias[n];
                 if (KIND == D_QKV) extra2 = bias[tile * kTileRows + pr];
@@ -463,7 +461,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                             const float f = __half2float(o);
                             ss[k] = f * f;
                             p.h[at] = o;
-                            p.hw[at] = __hmul(o, extra);
+                            if (!WIDE) p.hw[at] = __hmul(o, extra);
                         }
                     } else if (KIND == D_PLAIN || KIND == D_ROWS) {
                         __half x = __float2half_rn(v.v[k]);
@@ -485,14 +483,14 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
                             if (head < p.Hq) {
                                 p.y[(size_t)(t0 + tok) * p.N + n] = x;
                             } else {
-                                const int row = s_base[rq] + p.write_off + (tok - rq * mr);
+                                const int row = (WIDE ? t0 : s_base[rq]) + p.write_off + (tok - rq * mr);
                                 const int kvh = head - p.Hq - (rotate ? 0 : p.Hkv);
                                 if (row < p.cap) ((rotate ? p.kc : p.vc) + (size_t)rq * p.req_stride)[((size_t)kvh * p.cap + row) * p.hd + hi] = x;
                             }
                         }
                     }
                 }
-                if (KIND == D_RESID) {
+                if (KIND == D_RESID && !WIDE) {
                     // sums over the warp's rows, halving the tokens a lane holds with the first steps: token lane / (32 / TQ) in the end
                     float x = ss[0];
                     if (TQ == 4) {
@@ -507,7 +505,7 @@ __global__ void __launch_bounds__(kDThreads, 2) dense_kernel(const __grid_consta
 #pragma unroll
                     for (int o = 16 / TQ; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
                     if ((lane & (32 / TQ - 1)) == 0 && valid && tok0 + lane / (32 / TQ) < M)
-                        p.ssq[(n >> 5) * (WIDE ? p.pitch : kSsqPitch) + t0 + tok0 + lane / (32 / TQ)] = x;
+                        p.ssq[(n >> 5) * kSsqPitch + tok0 + lane / (32 / TQ)] = x;
                 }
             }
         };
@@ -593,7 +591,7 @@ __global__ void __launch_bounds__(256) embed_kernel(const int* __restrict__ toke
                                                     const __half* __restrict__ sc, const __half* __restrict__ bi, const __half* wn,
                                                     __half* __restrict__ h, __half* __restrict__ hw, float* __restrict__ ssq,
                                                     float2* __restrict__ cs, const float* __restrict__ inv_freq, float scaling, int H, int V,
-                                                    int half_hd, const void* const* wn_entry, int pitch, int pos0) {
+                                                    int half_hd, const void* const* wn_entry) {
     pdl_wait();
     pdl_launch_dependents();
     if (wn_entry != nullptr) wn = listed<__half>(wn_entry);
@@ -619,11 +617,11 @@ __global__ void __launch_bounds__(256) embed_kernel(const int* __restrict__ toke
         }
         ss += __shfl_xor_sync(0xffffffffu, ss, 1);
         ss += __shfl_xor_sync(0xffffffffu, ss, 2);
-        if (u < units && (u & 3) == 0) ssq[(u >> 2) * pitch + m] = ss;
+        if (u < units && (u & 3) == 0) ssq[(u >> 2) * kSsqPitch + m] = ss;
     }
     if ((int)threadIdx.x < half_hd) {
         float s, c;
-        sincosf((scaling * inv_freq[threadIdx.x]) * (float)(pos != nullptr ? pos[m] : pos0 + m), &s, &c);
+        sincosf((scaling * inv_freq[threadIdx.x]) * (float)pos[m], &s, &c);
         cs[m * kCsPitch + threadIdx.x] = make_float2(c, s);
     }
 }
@@ -1066,7 +1064,7 @@ int run_chain(const ChainArgs& c, cudaStream_t st) {
     if (on(0) || TABLE) {                                       // (what makes the table safe to read ahead of a kernel's wait)
         launch_kernel(embed_kernel, dim3(M), dim3(256), 0, st, d->tokens, d->pos, d->embed_wq, static_cast<const __half*>(d->embed_scales),
                       static_cast<const __half*>(d->embed_biases), static_cast<const __half*>(given(layers, 6)), p.h, p.hw, p.ssq, c.cs, d->inv_freq,
-                      d->rope_scaling, H, d->vocab, hd / 2, TABLE ? layers + 6 : nullptr, kSsqPitch, 0);
+                      d->rope_scaling, H, d->vocab, hd / 2, TABLE ? layers + 6 : nullptr);
         if ((rc = check_launch()) != B200_OK) return rc;
     }
     for (int l = 0; l < d->n_layers; l++) {
@@ -1113,41 +1111,39 @@ int run_chain(const ChainArgs& c, cudaStream_t st) {
     return B200_OK;
 }
 
-// The layers of a prompt pass: as run_chain, in tiles of 32 tokens.
+// The layers of a prompt pass: as run_chain, in tiles of 32 tokens side by side, with the norms as kernels between them.
 int run_prompt(const ChainPrompt& c, cudaStream_t st) {
     const b200_prefill_desc* d = c.d;
     const int n = d->n, H = d->hidden, I = d->intermediate, hd = d->head_dim, nq = d->n_heads * hd, nqkv = (d->n_heads + 2 * d->n_kv_heads) * hd;
-    CUtensorMap hw_map, attn_map, act_map;
+    CUtensorMap xn_map, attn_map, act_map;
     auto xmap = [&](CUtensorMap* m, const void* x, int width) {
         return make_map_2d(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x, width, n, (uint64_t)width * 2, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
     };
     int rc;
-    if ((rc = xmap(&hw_map, d->xn, H)) || (rc = xmap(&attn_map, d->attn, nq)) || (rc = xmap(&act_map, d->act, I))) return rc;
+    if ((rc = xmap(&xn_map, d->xn, H)) || (rc = xmap(&attn_map, d->attn, nq)) || (rc = xmap(&act_map, d->act, I))) return rc;
     DenseParams p{};
-    p.ssq = c.ssq; p.pitch = (n + 31) / 32 * 32; p.H = H; p.eps = d->rms_eps; p.M = p.mr = n; p.err = c.err; p.polls = wait_polls(kWaitPolls, kFirmPolls / 2);
-    p.h = static_cast<__half*>(d->h); p.hw = static_cast<__half*>(d->xn);
-    p.cs = c.cs; p.base = d->off; p.Hq = d->n_heads; p.Hkv = d->n_kv_heads; p.hd = hd; p.cap = d->cache_rows;
+    p.M = p.mr = n; p.err = c.err; p.polls = wait_polls(kWaitPolls, kFirmPolls / 2);
+    p.h = static_cast<__half*>(d->h);
+    p.cs = c.cs; p.write_off = d->off; p.Hq = d->n_heads; p.Hkv = d->n_kv_heads; p.hd = hd; p.cap = d->cache_rows;
     const size_t half = (size_t)d->n_kv_heads * d->cache_rows * hd;
-    launch_kernel(embed_kernel, dim3(n), dim3(256), 0, st, d->tokens, static_cast<const int*>(nullptr), d->embed_wq, static_cast<const __half*>(d->embed_scales),
-                  static_cast<const __half*>(d->embed_biases), static_cast<const __half*>(d->layers[6]), p.h, p.hw, p.ssq, c.cs, d->inv_freq, d->rope_scaling, H, d->vocab,
-                  hd / 2, static_cast<const void* const*>(nullptr), p.pitch, d->off);
-    if ((rc = check_launch()) != B200_OK) return rc;
     for (int l = 0; l < d->n_layers; l++) {
         const void* const* L = d->layers + (size_t)l * 8;       // qkv, qkv bias, o, gate, up, down, input norm, post norm
         auto weights = [&](int i, int count) {
             for (int j = 0; j < count; j++) p.w[j] = static_cast<const unsigned char*>(L[i + j]);
         };
-        p.xmap = hw_map; weights(0, 1); p.bias = static_cast<const __half*>(L[1]); p.y = static_cast<__half*>(d->qkv); p.N = nqkv; p.K = H;
+        if ((rc = c.norm(c.context, L[6], l == 0, st)) != B200_OK) return rc;
+        p.xmap = xn_map; weights(0, 1); p.bias = static_cast<const __half*>(L[1]); p.y = static_cast<__half*>(d->qkv); p.N = nqkv; p.K = H;
         p.kc = static_cast<__half*>(d->kv_cache) + (size_t)l * 2 * half;
         p.vc = p.kc + half;
         if ((rc = launch_dense<32, 4, D_QKV, false, true>(p, 0, st)) != B200_OK) return rc;
         if ((rc = c.attention(c.context, l * 2 * d->n_kv_heads * d->cache_rows, st)) != B200_OK) return rc;
         p.bias = nullptr;
-        p.xmap = attn_map; weights(2, 1); p.wn = static_cast<const __half*>(L[7]); p.N = H; p.K = nq;
+        p.xmap = attn_map; weights(2, 1); p.N = H; p.K = nq;
         if ((rc = launch_dense<32, 4, D_RESID, false, true>(p, 0, st)) != B200_OK) return rc;
-        p.xmap = hw_map; weights(3, 2); p.y = static_cast<__half*>(d->act); p.N = I; p.K = H;
+        if ((rc = c.norm(c.context, L[7], false, st)) != B200_OK) return rc;
+        p.xmap = xn_map; weights(3, 2); p.y = static_cast<__half*>(d->act); p.N = I; p.K = H;
         if ((rc = launch_dense<32, 4, D_SILU, false, true>(p, 0, st)) != B200_OK) return rc;
-        p.xmap = act_map; weights(5, 1); p.wn = static_cast<const __half*>(l + 1 < d->n_layers ? L[8 + 6] : d->final_norm); p.N = H; p.K = I;
+        p.xmap = act_map; weights(5, 1); p.N = H; p.K = I;
         if ((rc = launch_dense<32, 4, D_RESID, false, true>(p, 0, st)) != B200_OK) return rc;
     }
     return B200_OK;

@@ -17,12 +17,14 @@ struct ChainArgs {
 
 int forward_chain(const ChainArgs& a, cudaStream_t stream);
 
+constexpr int kCsPitch = 64;     // (cos, sin) of a token
+
 // The layers of a prompt pass (embedding to the last layer's h) through the chain's kernels, tiles of 32 tokens side by side.
 struct ChainPrompt {
-    const b200_prefill_desc* d;  // checked; xn holds h * w_norm
+    const b200_prefill_desc* d;  // checked
     int* err;
-    float* ssq;                  // [hidden / 32][tokens rounded up to 32]
-    float2* cs;                  // [tokens][64]
+    const float2* cs;            // [tokens][kCsPitch], written by the first norm
+    int (*norm)(const void* context, const void* weights, bool first, cudaStream_t stream);      // h -> xn; first: tokens -> h, too
     int (*attention)(const void* context, int row0, cudaStream_t stream);
     const void* context;
 };

@@ -6,8 +6,8 @@
 // The matmuls are csrc/qmm_gemm.cu and, beyond 128 tokens where it is cheaper, csrc/qmm_pair.cu, attention is csrc/flash.cu; the
 // element-wise steps that do not fit their epilogues are the kernels below (8B shape, 1024 tokens: 17 of 420 us a layer; their waits hidden
 // behind the matmul before them, nothing was gained: such a pass runs at the power limit).  Up to 128 tokens of a small model go
-// through the kernels of csrc/decode.cu instead.  Rounding points are those of the 32-row path's per-op kernels: norm ->
-// fp16, product -> fp16, + bias / + residual in fp16, SiLU(gate) * up with fp16 results, probabilities -> fp16.
+// through the matmuls of csrc/decode.cu instead, which RoPE and append themselves.  Rounding points are those of the 32-row path's
+// per-op kernels either way: norm (fp32) -> fp16, product -> fp16, + bias / + residual in fp16, SiLU(gate) * up with fp16 results, probabilities -> fp16.
 // Replaces the chunk loop of mlx_eagle.py:522-535 over mlx_llama.py:231-249.
 #include <algorithm>
 #include <atomic>
@@ -89,6 +89,97 @@ __global__ void __launch_bounds__(kNormThreads) norm_rows_kernel(__half* __restr
             }
             *reinterpret_cast<uint4*>(y + (size_t)row * H + u * 8) = *reinterpret_cast<const uint4*>(o);
         }
+    }
+}
+
+// The same between the kernels of csrc/decode.cu, a row a CTA.  The next of them comes up and expands its first weights while this one
+// waits, but for the first of a pass (FIRST: with `tokens`), which lets it go behind the wait, like embed_kernel there, and makes the
+// tokens' rotations.  What bounds it: start, one load and code that runs for the first time, 1.2 us a norm (61 tokens of the 0.5B shape
+// 660 -> 719 us with norms that the matmuls on both sides shared before, as in passes of up to 32 tokens, and whose products with h did not
+// always fit fp16).  One to four warps for a row of 896: a warp and four rows a CTA 796, norm weights asked for behind the wait 754.
+struct ChainNorm {
+    __half* x;
+    const __half* w;
+    __half* y;
+    int H;
+    float eps;
+    const int* tokens;
+    const uint32_t* wq;
+    const __half* sc;
+    const __half* bi;
+    int V;
+    float2* cs;                    // [n][kCsPitch]
+    const float* inv_freq;
+    float scaling;
+    int off, half_hd;
+};
+template <bool FIRST, int UNITS>                                  // UNITS: 16-byte units of a thread
+__global__ void __launch_bounds__(kNormThreads) chain_norm_kernel(const ChainNorm p) {
+    const int row = blockIdx.x, units = p.H / 8;
+    __half* const xr = p.x + (size_t)row * p.H;
+    uint4 v[UNITS], w[UNITS];
+    auto weights = [&]() {
+#pragma unroll
+        for (int i = 0; i < UNITS; i++) {
+            const int u = threadIdx.x + i * blockDim.x;
+            w[i] = u < units ? __ldg(reinterpret_cast<const uint4*>(p.w + u * 8)) : make_uint4(0, 0, 0, 0);
+        }
+    };
+    if (!FIRST) {
+        pdl_launch_dependents();
+        weights();                                               // (there before the pass)
+    }
+    pdl_wait();
+    if (FIRST) {
+        pdl_launch_dependents();
+        weights();
+        if ((int)threadIdx.x < p.half_hd) {
+            float s, c;
+            sincosf((p.scaling * p.inv_freq[threadIdx.x]) * (float)(p.off + row), &s, &c);
+            p.cs[row * kCsPitch + threadIdx.x] = make_float2(c, s);
+        }
+    }
+    const int tok = FIRST ? min(max(p.tokens[row], 0), p.V - 1) : 0;
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < UNITS; i++) {
+        const int u = threadIdx.x + i * blockDim.x;
+        v[i] = make_uint4(0, 0, 0, 0);
+        if (u < units) {
+            if (FIRST) {
+                const uint32_t pk = p.wq[(size_t)tok * units + u];
+                const __half s = p.sc[(size_t)tok * (p.H / 64) + (u >> 3)], b = p.bi[(size_t)tok * (p.H / 64) + (u >> 3)];
+                __half* o = reinterpret_cast<__half*>(&v[i]);
+#pragma unroll
+                for (int j = 0; j < 8; j++) o[j] = __hfma(__int2half_rn((int)((pk >> (4 * j)) & 0xfu)), s, b);
+                *reinterpret_cast<uint4*>(xr + u * 8) = v[i];
+            } else {
+                v[i] = __ldcg(reinterpret_cast<const uint4*>(xr + u * 8));
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < UNITS; i++) {
+        const __half2* h = reinterpret_cast<const __half2*>(&v[i]);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float2 f = __half22float2(h[j]);
+            ss += f.x * f.x + f.y * f.y;
+        }
+    }
+    const float inv = rsqrtf(block_sum(ss) / (float)p.H + p.eps);
+#pragma unroll
+    for (int i = 0; i < UNITS; i++) {
+        const int u = threadIdx.x + i * blockDim.x;
+        const __half2* h = reinterpret_cast<const __half2*>(&v[i]);
+        const __half2* g = reinterpret_cast<const __half2*>(&w[i]);
+        __align__(16) __half2 o[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float2 f = __half22float2(h[j]), gf = __half22float2(g[j]);
+            o[j] = __floats2half2_rn((f.x * inv) * gf.x, (f.y * inv) * gf.y);
+        }
+        if (u < units) *reinterpret_cast<uint4*>(p.y + (size_t)row * p.H + u * 8) = *reinterpret_cast<const uint4*>(o);
     }
 }
 
@@ -175,9 +266,10 @@ int launch_attention(const FlashArgs& a, const FlashPlan& plan, int row0, cudaSt
     return check_launch();
 }
 
-// The chain's kernels for prompts: 5 a layer and not 8, but every tile of 32 tokens expands the weights for itself.  Against chunks of weights
-// (128 x 128) times token tiles a layer: 0.5B shape (910 chunks) 33 tokens 805 -> 640 us, 61 836 -> 659, 128 947 -> 876; 1B (3712) 61 781 ->
-// 651, 96 852 -> 833, 128 886 against 968; 7B (14224; 4 layers) 61 321 against 369.
+// The chain's kernels for prompts: clusters add up K without going through memory, but every tile of 32 tokens expands the weights for itself.
+// Against chunks of weights (128 x 128) times token tiles a layer, large kernels and these, us: 0.5B shape (910 chunks) 33 tokens 839, 677; 64 861,
+// 687; 128 972, 894.  1B (3712) 64 800, 663; 65 839, 820; 128 900, 978.  8 layers of 2856 chunks 64 374, 314; 96 398, 398; 128 425, 448.  4 layers
+// of the 7B shape (14224) 64 325, 355.
 constexpr int kChainPromptTokens = 128;
 bool chain_prompt_wins(const b200_prefill_desc* d) {
     auto chunks = [](long long n, long long k) { return (n + 127) / 128 * (k / 128); };
@@ -186,20 +278,20 @@ bool chain_prompt_wins(const b200_prefill_desc* d) {
                             chunks(d->hidden, d->intermediate);
     return d->n <= kChainPromptTokens && layer * ((d->n + 31) / 32) <= 11200;
 }
-// Its scratch.
-struct ChainScratch {
-    size_t cs, ssq, bytes;
-    ChainScratch(int hidden, int n) {
-        cs = 0;
-        ssq = cs + (size_t)n * 64 * sizeof(float2);
-        bytes = ssq + (size_t)(hidden / 32) * ((n + 31) / 32 * 32) * sizeof(float);
-    }
-};
-
 int norm_rows(const b200_prefill_desc* d, void* x, const void* w, void* y, int rows, bool embed, cudaStream_t st) {
     launch_kernel(norm_rows_kernel, dim3(rows), dim3(kNormThreads), 0, st, static_cast<__half*>(x), static_cast<const __half*>(w),
                   static_cast<__half*>(y), d->hidden, d->rms_eps, embed ? d->tokens : nullptr, d->embed_wq,
                   static_cast<const __half*>(d->embed_scales), static_cast<const __half*>(d->embed_biases), d->vocab);
+    return check_launch();
+}
+
+int chain_norm(const b200_prefill_desc* d, const void* w, float2* cs, bool first, cudaStream_t st) {
+    const ChainNorm p{static_cast<__half*>(d->h), static_cast<const __half*>(w), static_cast<__half*>(d->xn), d->hidden, d->rms_eps, d->tokens, d->embed_wq,
+                      static_cast<const __half*>(d->embed_scales), static_cast<const __half*>(d->embed_biases), d->vocab, cs, d->inv_freq, d->rope_scaling, d->off,
+                      d->head_dim / 2};
+    const dim3 threads(d->hidden <= 1024 ? 128 : kNormThreads);
+    if (d->hidden <= 8 * kNormThreads) launch_kernel(first ? chain_norm_kernel<true, 1> : chain_norm_kernel<false, 1>, dim3(d->n), threads, 0, st, p);
+    else launch_kernel(first ? chain_norm_kernel<true, 4> : chain_norm_kernel<false, 4>, dim3(d->n), threads, 0, st, p);
     return check_launch();
 }
 
@@ -251,29 +343,35 @@ int b200_prefill(const b200_prefill_desc* d, void* stream) {
     const int nblk = (d->off + n + kKeyBlock - 1) / kKeyBlock;
     a.splits = std::max(1, std::min({148 / items, nblk / 4, 16}));
     const size_t per_split = (size_t)d->n_heads * n * (hd + 2) * sizeof(float);
-    const ChainScratch scratch(H, n);
-    const size_t chain = chain_prompt_wins(d) && scratch.bytes <= ga.partial_bytes ? scratch.bytes : 0;      // (ahead of the ranges' partial states)
+    const size_t rotations = (size_t)n * kCsPitch * sizeof(float2), chain = chain_prompt_wins(d) && rotations <= ga.partial_bytes ? rotations : 0;      // (ahead of the ranges' partial states)
     while (a.splits > 1 && chain + a.splits * per_split + 16 > ga.partial_bytes) a.splits--;
     a.part_ml = ga.partial ? static_cast<float*>(ga.partial) + chain / sizeof(float) : nullptr;
     a.part_o = a.part_ml ? a.part_ml + (((size_t)a.splits * d->n_heads * n * 2 + 3) & ~(size_t)3) : nullptr;
 
-    // Few tokens of a small model: the chain of the 32-row passes, whose kernels norm, RoPE and append themselves.
+    // Few tokens of a small model: the matmuls and attention of the 32-row passes, whose kernels RoPE and append themselves.
     if (chain > 0) {
-        unsigned char* const at = static_cast<unsigned char*>(ga.partial);
+        struct Context {
+            const b200_prefill_desc* d;
+            float2* cs;
+            const FlashArgs* a;
+            const FlashPlan* plan;
+            bool tree;
+        } context{d, static_cast<float2*>(ga.partial), &a, &flash, n <= 64 && a.splits > 1};
         ChainPrompt c{};
-        c.d = d; c.err = ga.err;
-        c.cs = reinterpret_cast<float2*>(at + scratch.cs);
-        c.ssq = reinterpret_cast<float*>(at + scratch.ssq);
-        struct Attention { const FlashArgs* a; const FlashPlan* plan; bool tree; } attention{&a, &flash, n <= 64 && a.splits > 1};
-        if (attention.tree) {                                      // key ranges by the CTAs of a cluster, merged in the same kernel
+        c.d = d; c.err = ga.err; c.cs = context.cs;
+        if (context.tree) {                                        // key ranges by the CTAs of a cluster, merged in the same kernel
             a.nreq = 1; a.mr = a.tail = n; a.nkb = (d->cache_rows + kKeyBlock - 1) / kKeyBlock;
             if ((rc = flash_decode_plan(a, &flash)) != B200_OK) return rc;
         }
+        c.norm = [](const void* p, const void* w, bool first, cudaStream_t stream) {
+            const Context* x = static_cast<const Context*>(p);
+            return chain_norm(x->d, w, x->cs, first, stream);
+        };
         c.attention = [](const void* p, int row0, cudaStream_t stream) {
-            const Attention* x = static_cast<const Attention*>(p);
+            const Context* x = static_cast<const Context*>(p);
             return x->tree ? flash_decode(*x->a, *x->plan, row0, stream) : launch_attention(*x->a, *x->plan, row0, stream);
         };
-        c.context = &attention;
+        c.context = &context;
         rc = chain_prompt(c, st);
     } else {
         rc = norm_rows(d, d->h, d->layers[6], d->xn, n, true, st);

@@ -72,3 +72,48 @@ def test_attention_over_a_filled_cache_takes_nothing_from_scratch(be, cuda, n, o
         m._prefill_large_m(tokens[0].int(), cache, off, None, 0)
         assert (m._pf_buf["ws"][used:] == fill).all()
     m.check_fused_error()
+
+
+def _ranged(be, cuda, shape, embed, norms, group=None):
+    """A model whose embedding (the first 64 columns, or all) and norm weights there are multiplied before the re-layout."""
+    heads, kv, hd, hidden, inter, kind = shape
+    args = be.ModelArgs(model_type=kind, hidden_size=hidden, num_hidden_layers=2, intermediate_size=inter, num_attention_heads=heads,
+                        num_key_value_heads=kv, head_dim=hd, rms_norm_eps=1e-6, vocab_size=520, tie_word_embeddings=False)
+    m = be.Model.random_init(args, seed=4, device=cuda, gen_device="cpu")
+    cols = slice(None) if group is None else slice(group, group + 1)
+    m.embed.scales[:, cols].mul_(embed)
+    m.embed.biases[:, cols].mul_(embed)
+    for w in [lw[k] for lw in m.layers for k in ("input_norm", "post_norm")]:
+        w.view(-1, 64)[cols].mul_(norms)
+    return m.relayout()
+
+
+@pytest.mark.parametrize("n,off", [(33, 0), (61, 700), (128, 64)])
+@pytest.mark.parametrize("shape", SHAPES[1:], ids=lambda s: "x".join(map(str, s)))
+def test_residual_times_norm_weight_beyond_fp16(be, cuda, shape, n, off):
+    """A prompt's activations are normed in fp32: with a group of 64 residuals of 4e3 and more under norm weights of 8 some of
+    their products do not fit fp16, what is normed (up to 8 sqrt(hidden)) does."""
+    m = _ranged(be, cuda, shape, 2e5, 8.0, group=0)
+    first, span = (t[:, 0].float().abs().max() for t in (m.embed.biases, m.embed.scales))      # (a nibble of 0 is the bias)
+    assert first + 15 * span < 65504 and 8 * first > 65504
+    tokens = torch.randint(0, 520, (n,), generator=torch.Generator().manual_seed(n))[None].to(cuda)
+    got, want = (_run(be, m, tokens, off, False, large) for large in (True, False))
+    m.prefill_large_m = True
+    m.check_fused_error()
+    for a, b in zip(got, want):
+        assert torch.isfinite(a).all() and ((a - b).abs() <= 2.0 ** -6 * b.abs() + 1e-2).all()
+
+
+@pytest.mark.parametrize("n,off", [(33, 0), (61, 700), (128, 64)])
+def test_residual_times_norm_weight_below_fp16(be, cuda, n, off):
+    """Residuals of 1.2e-3 under norm weights of 2^-12: their product, 3e-7, is five steps of fp16's smallest.  Normed it is 2e-4, which both
+    paths round alike; keys and values, rms 1e-4 or more, are rounded to steps of 2^-24, a relative 3e-4 in the worst case."""
+    m = _ranged(be, cuda, SHAPES[2], 1.0 / 16, 2.0 ** -12)
+    tokens = torch.randint(0, 520, (n,), generator=torch.Generator().manual_seed(n))[None].to(cuda)
+    got, want = (_run(be, m, tokens, off, False, large)[1][:, :, :, off:] for large in (True, False))
+    m.prefill_large_m = True
+    m.check_fused_error()
+    for i in range(2):
+        for j in range(2):
+            a, b = got[i, j].double(), want[i, j].double()
+            assert b.pow(2).mean().sqrt() > 1e-5 and (a - b).norm() <= 2.0 ** -8 * b.norm()
