@@ -183,8 +183,9 @@ __global__ void __launch_bounds__(FGeo<HD, DECODE>::THREADS) flash_kernel(const 
         __syncwarp();
         if (DECODE && cs > 1) cluster_wait();                            // (the peers have started)
         pdl_wait();
-        if (early < first && elect_one()) {
-            asm volatile("fence.proxy.async;\n" ::: "memory");                  // rows appended by the previous kernel's ordinary stores
+        if (elect_one()) {
+            // The previous kernel appended rows by ordinary stores.  (On a long cache they are asked for further down only.)
+            asm volatile("fence.proxy.async;\n" ::: "memory");
 #pragma unroll 1
             for (int i = 2 * early; i < 2 * first; i++) load(i >> 1, i & 1);
         }
@@ -231,6 +232,7 @@ __global__ void __launch_bounds__(FGeo<HD, DECODE>::THREADS) flash_kernel(const 
         if (nb > 0) {
             // (the queries, too: the warp that copies has the last blocks to ask for)
             if (elect_one()) {
+                asm volatile("fence.proxy.async;\n" ::: "memory");              // (ordinary stores of the previous kernel)
                 mbar_expect_tx(smem_u32(&qfull), p.T * p.heads * HD * 2);
 #pragma unroll
                 for (int x = 0; x < HD / 64; x++) tma_box3(sbase + x * G::QBOX, &p.qmap, x * 64, hk * p.G + hs * p.heads, tok_base, smem_u32(&qfull));

@@ -73,3 +73,23 @@ def test_prompt_pass_equals_per_op_kernels(be, cuda, shape, n, off, growing):
     m.prefill_large_m = True
     m.check_fused_error()
     _close(zip(*out))
+
+
+@pytest.mark.parametrize("cached", [40, 3000, 3070])
+@pytest.mark.parametrize("rows", [10, 32])
+def test_rows_of_the_pass_are_read_as_just_written(be, cuda, rows, cached):
+    """K, V and queries come in by copies that the previous kernel's ordinary stores have to be fenced for, on a long cache behind the blocks
+    asked for ahead.  A pass over rows that held another pass's, and the same again over its own: the same bits."""
+    m = _model(be, cuda, *SHAPES[2])
+    tm = torch.ones(rows, rows, dtype=torch.bool).tril()
+    cache = _cache(m, cached, rows)
+    g = torch.Generator().manual_seed(cached)
+
+    def run(tokens):
+        cache.offset = cached
+        return be.eagle.tree_decoding(tokens, tm, tm.sum(1) - 1, m, cache)[0].clone()
+
+    for _ in range(100):
+        tokens = torch.randint(0, 264, (rows,), generator=g)[None]
+        assert torch.equal(run(tokens), run(tokens))
+    m.check_fused_error()
