@@ -204,8 +204,8 @@ class QLinear:
         """Build the streaming layout of this layer's weights; drop the row-major tensors unless asked.
 
         Passes trust what is found here about the scales for as long as ``tiled`` is the same tensor and torch has counted no change
-        of it.  A write that torch does not count (through ``.data``, DLPack, ``__cuda_array_interface__`` or a kernel of the
-        caller's) needs ``weights_changed()`` before the next pass: scales outside 2^-14 .. 2^-4 would be expanded wrongly."""
+        of it.  A write that torch does not count (through ``.data``, a view of another type made in inference mode, DLPack,
+        ``__cuda_array_interface__`` or a kernel of the caller's) needs ``weights_changed()`` before the next pass: scales outside 2^-14 .. 2^-4 would be expanded wrongly."""
         self._nbytes = self.nbytes()
         self.tiled = qk.relayout(self.weight, self.scales, self.biases)
         self.weights_changed()
@@ -218,7 +218,7 @@ class QLinear:
         # a pass's kernels expand nibbles with a shorter, bit-identical sequence when every scale's fp16
         # exponent field is in 1..10 (2^-14 <= |s| < 2^-4)
         e = (qk.tiled_scales(self.tiled, self.out_features, self.in_features).view(torch.int16).to(torch.int32) >> 10) & 31
-        ok = not self.tiled.is_inference() and bool(((e >= 1) & (e <= 10)).all())      # (an inference tensor does not count its changes)
+        ok = not self.tiled.is_inference() and bool(((e >= 1) & (e <= 10)).all())      # (a caller's inference tensor does not count its changes)
         self._fast_of = (self.tiled, self.tiled._version) if ok else None
 
     @property

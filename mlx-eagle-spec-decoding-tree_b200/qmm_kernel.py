@@ -137,7 +137,8 @@ def relayout(w, s, b) -> torch.Tensor:
     _check_size("scales", s, torch.float16, n * k // 64)
     _check_size("biases", b, torch.float16, n * k // 64)
     w = w.contiguous()
-    out = torch.empty(_lib.lib().b200_qmm_tiled_bytes(n, k), dtype=torch.uint8, device=w.device)
+    with torch.inference_mode(False):            # (torch counts no changes of a tensor that it makes in inference mode)
+        out = torch.empty(_lib.lib().b200_qmm_tiled_bytes(n, k), dtype=torch.uint8, device=w.device)
     rc = _lib.lib().b200_qmm_relayout(_lib.ptr(w), _lib.ptr(s), _lib.ptr(b), _lib.ptr(out), n, k,
                                       _lib.stream_ptr(w.device))
     _lib.check(rc, "b200_qmm_relayout")

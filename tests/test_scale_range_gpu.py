@@ -85,3 +85,30 @@ def test_weights_written_past_torch(be, cuda, which):
     m.weights_changed()
     assert all(torch.equal(run(), before[0]) for _ in range(passes)) and m._scales_fast is True and m.weight_addresses() == kept
     m.check_fused_error()
+
+
+def test_weights_relaid_in_inference_mode(be, cuda):
+    """They allow the short expansion like any, and writes are seen there, too."""
+    m = be.Model.random_init(be.shape_preset("tiny-qwen2"), seed=5, device=cuda, gen_device="cpu")
+    lin = m.layers[1]["down"]
+    packed = [t.clone() for t in (lin.weight, lin.scales, lin.biases)]
+    packed[1][3:40] = 0.25
+    wide = be.qmm_kernel.relayout(*packed)
+    tokens = torch.arange(7, dtype=torch.int32, device=cuda)[None]
+    cache = m.make_cache(128)
+
+    def run():
+        cache.offset = 0
+        return m(tokens, cache).clone()
+
+    with torch.inference_mode():
+        m.relayout()
+        before = run()
+        assert m._scales_fast is True
+        lin.tiled.copy_(wide)
+        got = run()
+        assert m._scales_fast is False
+    m.fast_dequant = False
+    want = run()
+    m.check_fused_error()
+    assert torch.equal(got, want) and not torch.equal(want, before)
