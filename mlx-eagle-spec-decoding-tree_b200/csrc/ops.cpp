@@ -114,30 +114,28 @@ PyObject* rope_positions(PyObject* const* a, Py_ssize_t n) {
     return THPVariable_Wrap(std::move(y));
 }
 
-// layer_pointers(layers, table[, changes]) -> 0: `table` (address of [layers][8] pointers in the order of b200_forward_desc.layer_table) holds
+// layer_pointers(layers, table[, fast]) -> 0: `table` (address of [layers][8] pointers in the order of b200_forward_desc.layer_table) holds
 // the device pointers of the layers already, 1: it does now, -1: a layer is not as it should be (no re-laid-out weights, say).
-// Runs ahead of every pass, so that a pass never sees the address of a tensor that has been replaced: ~0.3 us a layer.  `changes` (address
-// of 64 bits) becomes a number that is another one once a re-laid-out matrix has been written in place.
+// Runs ahead of every pass, so that a pass never sees the address of a tensor that has been replaced: ~0.35 us a layer.  `fast` (address of 32
+// bits) becomes 1 if every re-laid-out matrix is known to allow the short expansion as it is now, as QLinear.scales_fast, 0 if not.  (Asked
+// for every pass like the addresses: a matrix that has taken the place of one that was freed can have its address and its count of changes.)
 PyObject* layer_pointers(PyObject*, PyObject* const* a, Py_ssize_t n) {
     static PyObject* const linears[] = {PyUnicode_InternFromString("qkv"), PyUnicode_InternFromString("o"), PyUnicode_InternFromString("gate"),
                                         PyUnicode_InternFromString("up"), PyUnicode_InternFromString("down")};
     static PyObject* const norms[] = {PyUnicode_InternFromString("input_norm"), PyUnicode_InternFromString("post_norm")};
     static PyObject* const tiled = PyUnicode_InternFromString("tiled");
     static PyObject* const bias = PyUnicode_InternFromString("bias");
+    static PyObject* const fast_of = PyUnicode_InternFromString("_fast_of");
     void** table = (n == 2 || n == 3) && (PyList_Check(a[0]) || PyTuple_Check(a[0])) ? static_cast<void**>(PyLong_AsVoidPtr(a[1])) : nullptr;
-    uint64_t* changes = table != nullptr && n == 3 ? static_cast<uint64_t*>(PyLong_AsVoidPtr(a[2])) : nullptr;
+    uint32_t* fast = table != nullptr && n == 3 ? static_cast<uint32_t*>(PyLong_AsVoidPtr(a[2])) : nullptr;
     if (PyErr_Occurred()) return nullptr;
     if (table == nullptr) return PyLong_FromLong(-1);
-    uint64_t versions = 0;
-    bool plain = true, same = true;
+    if (fast != nullptr) *fast = 0;
+    bool plain = true, same = true, all_fast = fast != nullptr;
     auto put = [&](PyObject* t, bool optional) {              // (borrowed, may be NULL)
         void* q = nullptr;
         if (t == nullptr || !THPVariable_Check(t)) plain = plain && optional && t == Py_None;
-        else {
-            const at::Tensor& x = THPVariable_Unpack(t);
-            q = x.data_ptr();
-            versions = versions * 31 + (x.is_inference() ? 0 : x._version());
-        }
+        else q = THPVariable_Unpack(t).data_ptr();
         same = same && *table == q;
         *table++ = q;
     };
@@ -145,6 +143,14 @@ PyObject* layer_pointers(PyObject*, PyObject* const* a, Py_ssize_t n) {
         PyObject* t = o == nullptr ? nullptr : PyObject_GetAttr(o, name);
         if (t == nullptr) PyErr_Clear();
         put(t, optional);
+        if (name == tiled && all_fast) {                         // (the tensor looked at, its count of changes then)
+            PyObject* of = t == nullptr ? nullptr : PyObject_GetAttr(o, fast_of);
+            if (of == nullptr) PyErr_Clear();
+            all_fast = of != nullptr && PyTuple_Check(of) && PyTuple_GET_SIZE(of) == 2 && PyTuple_GET_ITEM(of, 0) == t && THPVariable_Check(t) &&
+                       !THPVariable_Unpack(t).is_inference() && PyLong_AsLongLong(PyTuple_GET_ITEM(of, 1)) == (long long)THPVariable_Unpack(t)._version();
+            if (PyErr_Occurred()) PyErr_Clear();                 // (no number there)
+            Py_XDECREF(of);
+        }
         Py_XDECREF(t);                                           // (the layer still holds it)
     };
     try {
@@ -162,7 +168,7 @@ PyObject* layer_pointers(PyObject*, PyObject* const* a, Py_ssize_t n) {
     } catch (const std::exception&) {                            // (a tensor without storage)
         plain = false;
     }
-    if (changes != nullptr) *changes = versions;
+    if (fast != nullptr) *fast = plain && all_fast;
     return PyLong_FromLong(!plain ? -1 : (same ? 0 : 1));
 }
 

@@ -357,7 +357,8 @@ class Model:
         self.fused = True                                # b200_forward when possible
         self._fwd_ws = None
         self._fwd_ws_key = None
-        self._layers_host = self._layer_table = None     # device pointers of the layers: kept up to date by _gather_layers()
+        # device pointers of the layers, and whether all allow the short expansion: kept up to date by _gather_layers()
+        self._layers_host = self._layer_table = self._layers_fast = None
         self.tp: Optional[TensorParallel] = None         # set by shard(): this model is one shard of a tensor-parallel model
         self.vocab_offset = 0
         self.part32 = None
@@ -369,7 +370,7 @@ class Model:
         self.tp_two_shot = 0                             # tensor-parallel exchange: 0 library's choice (push), 1 two-step, 2 pull behind a hierarchical barrier, 3 push, 4 pull
         self.prefill_large_m = True                      # prompts beyond 32 tokens through b200_prefill
         self._pf_buf, self._pf_fits = None, False        # buffers of that path, made on first use
-        self._scales_fast, self._layers_fast, self._fuse_fits = None, None, False
+        self._scales_fast, self._fuse_fits = None, False
         self._graphs = _Graphs()
         self.fwd = FwdInputs(self.device)
 
@@ -573,13 +574,10 @@ class Model:
         False if a layer has no re-laid-out weights."""
         n = self.args.num_hidden_layers
         if self._layers_host is None:
-            self._layers_host, self._layer_changes = (ctypes.c_void_p * (8 * n))(), ctypes.c_uint64()
-        before = self._layer_changes.value
+            self._layers_host, self._layers_fast = (ctypes.c_void_p * (8 * n))(), ctypes.c_uint32()
         state = _lib.ops().layer_pointers(self.layers, ctypes.addressof(self._layers_host),
-                                          ctypes.addressof(self._layer_changes)) if len(self.layers) == n else -1
+                                          ctypes.addressof(self._layers_fast)) if len(self.layers) == n else -1
         if state == 0 and self._layer_table is not None:
-            if self._layer_changes.value != before:      # (written in place)
-                self._layers_fast = self._all_fast()
             return True
         self._graphs.clear()                             # (a graph has the layers' pointers in it)
         self._layer_table = None
@@ -587,7 +585,6 @@ class Model:
             self._fuse_fits = self._pf_fits = False
             return False
         self._layer_table = torch.tensor([p or 0 for p in self._layers_host], dtype=torch.int64).to(self.device)
-        self._layers_fast = self._all_fast()
         return True
 
     def weights_changed(self):
@@ -597,18 +594,13 @@ class Model:
         for q in [lw[k] for lw in self.layers for k in ("qkv", "o", "gate", "up", "down")] + [self.lm_head]:
             if q.tiled is not None:
                 q.weights_changed()
-        if self._layer_table is not None:                # (else gathered ahead of the next pass)
-            self._layers_fast = self._all_fast()
-
-    def _all_fast(self) -> bool:
-        return all(lw[k].scales_fast for lw in self.layers for k in ("qkv", "o", "gate", "up", "down"))
 
     def weight_addresses(self) -> bytes:
         """Where this model's weights are now, and whether they allow the short expansion, for whoever keeps graphs of its passes."""
         linears, others = [self.embed, self.lm_head], [self.norm, self.inv_freqs]
         layers = b""
         if self.can_fuse():
-            layers = bytes(self._layers_host) + bytes([self._layers_fast and self.lm_head.scales_fast and self.fast_dequant])
+            layers = bytes(self._layers_host) + bytes([bool(self._layers_fast.value and self.lm_head.scales_fast and self.fast_dequant)])
         else:
             linears += [lw[k] for lw in self.layers for k in ("qkv", "o", "gate", "up", "down")]
             others += [lw[k] for lw in self.layers for k in ("input_norm", "post_norm")]
@@ -631,7 +623,7 @@ class Model:
         d.final_norm, d.lm_head_tiled, d.layer_table = p(self.norm), p(self.lm_head.tiled), p(self._layer_table)
         d.h, d.hw, d.qkv, d.attn, d.act = p(self.h), p(self.hw), p(self.qkv), p(self.xt_attn), p(self.xt_act)
         d.grid_ctas, d.phase_mask, d.attn_split_blocks = self.grid_ctas, self.phase_mask, self.attn_split_blocks
-        self._scales_fast = self._layers_fast and self.lm_head.scales_fast
+        self._scales_fast = bool(self._layers_fast.value and self.lm_head.scales_fast)
         d.scales_in_fast_range = 1 if (self._scales_fast and self.fast_dequant) else 0
         if self.tp is not None:
             d.tp_world, d.tp_rank, d.head_rows = self.tp.world, self.tp.rank, self.vocab_local

@@ -112,3 +112,39 @@ def test_weights_relaid_in_inference_mode(be, cuda):
     want = run()
     m.check_fused_error()
     assert torch.equal(got, want) and not torch.equal(want, before)
+
+
+def test_weights_where_freed_ones_were(be, cuda):
+    """A layer that is made anew once the old one has been let go can have its addresses: its own scales decide."""
+    m = be.Model.random_init(be.shape_preset("tiny-qwen2"), seed=5, device=cuda, gen_device="cpu")
+    old = m.layers[1]["down"]
+    packed = [t.clone() for t in (old.weight, old.scales, old.biases)]
+    packed[1][3:40] = 0.25
+    m.relayout()
+    tokens = torch.arange(7, dtype=torch.int32, device=cuda)[None]
+    cache = m.make_cache(128)
+
+    def run():
+        cache.offset = 0
+        return m(tokens, cache).clone()
+
+    for _ in range(2 * m._graphs.AFTER):
+        before = run()
+    assert m._scales_fast is True
+    at = old.tiled.data_ptr()
+    new = be.llama.QLinear(*packed)
+    del m.layers[1]["down"], old
+    spare = []
+    while True:                                          # (the allocator may have other blocks of this size first)
+        new.relayout(keep_rowmajor=True)
+        if new.tiled.data_ptr() == at or len(spare) > 1000:
+            break
+        spare.append(new.tiled)
+    assert new.tiled.data_ptr() == at
+    m.layers[1]["down"] = new
+    got = [run() for _ in range(2 * m._graphs.AFTER)]
+    assert m._scales_fast is False
+    m.fast_dequant = False
+    want = run()
+    m.check_fused_error()
+    assert not torch.equal(want, before) and all(torch.equal(g, want) for g in got)

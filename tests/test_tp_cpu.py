@@ -81,6 +81,41 @@ def test_layer_pointers_follow_the_layers(be):
     assert walk(model.layers, at) == -1
 
 
+def test_layer_pointers_say_whether_the_scales_that_were_looked_at_are_there(be):
+    """Of the very tensor that stands in the layer, with as many changes as then: one in its place may have its address, and its count."""
+    import ctypes
+    model = be.Model.random_init(be.shape_preset("tiny-qwen2"), seed=3, device="cpu")
+    walk = be._lib.ops().layer_pointers
+    table, fast = (ctypes.c_void_p * (8 * len(model.layers)))(), ctypes.c_uint32(7)
+    ask = lambda: (walk(model.layers, ctypes.addressof(table), ctypes.addressof(fast)), fast.value)
+    assert ask() == (-1, 0)
+    for lw in model.layers:
+        for k in ("qkv", "o", "gate", "up", "down"):
+            lw[k].tiled = torch.zeros(16)
+            lw[k]._fast_of = (lw[k].tiled, 0)
+    lin = model.layers[1]["down"]
+    assert ask() == (1, 1) and ask() == (0, 1) and lin.scales_fast
+    lin.tiled.zero_()                                            # (written)
+    assert ask() == (0, 0) and not lin.scales_fast
+    lin._fast_of = (lin.tiled, 1)
+    assert ask() == (0, 1) and lin.scales_fast
+    other = be.llama.QLinear(lin.weight, lin.scales, lin.biases)
+    other.tiled = lin.tiled[:]                                   # (another tensor: same address, same count)
+    model.layers[1]["down"] = other
+    assert other.tiled._version == 1 and ask() == (0, 0) and not other.scales_fast
+    for of in (None, (), (other.tiled, "1"), (other.tiled,), 1):
+        other._fast_of = of
+        assert ask() == (0, 0)
+    del other._fast_of
+    assert ask() == (0, 0)
+    other._fast_of = (other.tiled, 1)
+    assert ask() == (0, 1)
+    with torch.inference_mode():
+        other.tiled = torch.zeros(16)
+    other._fast_of = (other.tiled, 0)
+    assert ask() == (1, 0)
+
+
 def test_the_timeline_of_a_model_that_is_no_shard_is_refused(be):
     full = be.Model.random_init(be.shape_preset("tiny-qwen2"), seed=3, device="cpu")
     with pytest.raises(be._lib.B200Error, match="shard"):        # (its passes have no device-wide barriers to stamp)
