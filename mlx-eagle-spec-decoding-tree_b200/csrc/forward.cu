@@ -1541,6 +1541,12 @@ __device__ __forceinline__ void attn_bp_consume(const FwdParams& p, Ctx& c, cons
                     }
                     __syncwarp();
                 }
+                if (key0 + kKeyBlock > a.total) {          // rows of V past the last: the box has whatever is there, and 0 x Inf or NaN is NaN
+#pragma unroll 1
+                    for (int idx = (a.total - key0) * VPR + lane; idx < kKeyBlock * VPR; idx += 32)
+                        *reinterpret_cast<uint4*>(myslot + NBX * kBox + swz(idx / VPR, idx % VPR)) = make_uint4(0, 0, 0, 0);
+                    __syncwarp();
+                }
                 const bool all_visible = key0 + kKeyBlock <= prefix;      // committed rows: no mask needed
 #pragma unroll
                 for (int half = 0; half < 2; half++) {         // 32 keys at a time keeps the scores in 16 registers

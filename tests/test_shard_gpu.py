@@ -90,6 +90,27 @@ def test_shard_kernel_equals_per_op_kernels(be, cuda, name, form):
     p.check()
 
 
+@pytest.mark.parametrize("room", [0, 70])
+@pytest.mark.parametrize("name", ["tiny-qwen2", "tiny-llama"])
+def test_cache_rows_behind_the_last_do_not_reach_the_results(be, cuda, name, room):
+    """They may hold anything, the next head's rows where the cache's are no multiple of a key block among it."""
+    p = _Pair(be, cuda, be.shape_preset(name), PUSH)
+    for rows, cached, split in [(1, 62, 0), (1, 64, 0), (17, 300, -1), (9, 600, 3), (32, 90, 0)]:
+        tokens = torch.randint(0, p.model.args.vocab_size, (1, rows), generator=torch.Generator().manual_seed(rows))
+        p.shard.attn_split_blocks = split
+
+        def run(behind):
+            _, cache = p.caches(max(64, cached + rows + room), cached)
+            cache.data[:, :, :, cached:] = behind
+            return p.shard(tokens, cache).clone(), cache.data[:, :, :, :cached + rows].clone()
+
+        want = run(0.0)
+        assert all(torch.isfinite(t).all() for t in want)
+        for behind in (float("nan"), float("inf"), -65504.0):
+            assert all(torch.equal(a, b) for a, b in zip(run(behind), want))
+    p.check()
+
+
 @pytest.mark.parametrize("form", [PUSH, PULL])
 @pytest.mark.parametrize("world", [4, 8])
 def test_shard_kernel_at_the_shapes_of_a_large_model(be, cuda, world, form):
