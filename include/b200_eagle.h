@@ -322,7 +322,8 @@ typedef struct b200_forward_desc {
                                  * fp16 exponent field in 1..10 (2^-14 <= |scale| < 2^-4, never zero or subnormal): the
                                  * kernel then expands the nibbles with a shorter instruction sequence that gives the
                                  * same bits, and is not asked again whether it may: with scales outside the range the
-                                 * results are wrong.  0 is always safe. */
+                                 * results are wrong.  0 is always safe.  A pass that takes its layers from the table in
+                                 * device memory (no B200_LAYERS_ON_HOST) asks for every chunk of weights whatever is said here. */
     int tp_two_shot;            /* exchange of the row-parallel layers (o_proj, down_proj); the same value on every rank,
                                  * the same bits whichever form runs; zero the exchange buffers when switching.
                                  * 0 = the library's choice (the push form).

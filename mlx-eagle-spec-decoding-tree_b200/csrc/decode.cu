@@ -1054,9 +1054,11 @@ int run_chain(const ChainArgs& c, cudaStream_t st) {
     one.kvmap = flash.kvmap; one.q = static_cast<const __half*>(d->qkv); one.pitch = nqkv; one.mask = d->mask; one.prefix = d->prefix;
     one.out = static_cast<__half*>(d->attn); one.Hq = d->n_heads; one.Hkv = d->n_kv_heads; one.mr = p.mr; one.tail = d->tail; one.nkb = a.nkb;
     one.req_rows = a.req_rows; one.cap = d->cache_rows; one.write_off = d->write_off; one.scale_log2 = a.scale_log2; one.err = c.err; one.polls = p.polls;
-    // Up to 16 query rows of a kv head (a token or two) mma.sync has the shorter chain: next token of the 0.5B shape 455 against 470 us, of the
-    // 7B shape (8 layers) 440 against 444; from 1000 rows on at head dim 128 the tensor memory's is (7B, 3000 cached: 480 against 487; 0.5B
-    // there 583 against 568).  Beyond 16 rows: 0.5B, 8 tokens, 300 cached 493 against 495, 3000 cached 605 against 666.
+    // Up to 16 query rows of a kv head (a token or two) mma.sync has the shorter chain: next token of the 0.5B shape 455 against 470 us, there 568
+    // against 583 with 3000 cached.  At head dim 128 the tensor memory's wins on many cached rows (8 layers of the 7B shape behind 100, 900, 3000,
+    // 12000 of them: mma.sync 423, 432, 465, 617 us, the other 425, 430, 453, 559); how many there are only the device knows, so the cache's
+    // capacity decides, and few rows in a large cache take up to 1 % longer.  Beyond 16 rows: 0.5B, 8 tokens, 300 cached 493 against 495, 3000 cached
+    // 605 against 666.
     const bool few = p.mr * (d->n_heads / d->n_kv_heads) <= DAGeo<64>::ROWS && (hd == 64 || a.nkb <= 16);
 
     const void* const* layers = TABLE ? static_cast<const void* const*>(d->layer_table) : c.layers;      // (not read here with TABLE)

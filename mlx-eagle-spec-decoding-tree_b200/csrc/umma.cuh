@@ -1,5 +1,5 @@
-// Pieces shared by the two matmul kernels on the fifth-generation tensor cores (csrc/decode.cu, csrc/qmm_gemm.cu): matrix descriptor,
-// completion of MMAs, and the expansion of a weight row's packs into a tensor-memory tile.
+// Pieces shared by the kernels on the fifth-generation tensor cores (matmuls: csrc/decode.cu, csrc/qmm_gemm.cu, csrc/qmm_pair.cu; attention:
+// csrc/flash.cu): matrix descriptor, completion of MMAs, and the expansion of a weight row's packs into a tensor-memory tile.
 #pragma once
 
 #include <type_traits>

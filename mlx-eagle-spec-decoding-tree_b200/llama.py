@@ -673,7 +673,7 @@ class Model:
             code = int(word)
             if code != 0:
                 word.zero_()
-                raise _lib.B200Error(f"b200_prefill: a bounded wait ran out inside a matmul (code {code})")
+                raise _lib.B200Error(f"b200_prefill: a bounded wait ran out inside a kernel of the pass (code {code})")
         if not self.can_fuse():
             code = qk.stream_error(self.device)
             if code != 0:
