@@ -208,16 +208,19 @@ class QLinear:
         ``__cuda_array_interface__`` or a kernel of the caller's) needs ``weights_changed()`` before the next pass: scales outside 2^-14 .. 2^-4 would be expanded wrongly."""
         self._nbytes = self.nbytes()
         self.tiled = qk.relayout(self.weight, self.scales, self.biases)
-        self.weights_changed()
+        self._look_at(self.scales)
         if not keep_rowmajor:
             self.weight = self.scales = self.biases = None
 
     def weights_changed(self):
         """Look at the scales of the re-laid-out weights again (waits for the device).  For a layer of a ``Model``:
         ``Model.weights_changed``, which also lets go of what was made for the old ones."""
+        self._look_at(qk.tiled_scales(self.tiled, self.out_features, self.in_features))
+
+    def _look_at(self, scales):
         # a pass's kernels expand nibbles with a shorter, bit-identical sequence when every scale's fp16
         # exponent field is in 1..10 (2^-14 <= |s| < 2^-4)
-        e = (qk.tiled_scales(self.tiled, self.out_features, self.in_features).view(torch.int16).to(torch.int32) >> 10) & 31
+        e = (scales.view(torch.int16).to(torch.int32) >> 10) & 31
         ok = not self.tiled.is_inference() and bool(((e >= 1) & (e <= 10)).all())      # (a caller's inference tensor does not count its changes)
         self._fast_of = (self.tiled, self.tiled._version) if ok else None
 
