@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(kNormThreads) norm_rows_kernel(__half* __restr
 // waits, but for the first of a pass (FIRST: with `tokens`), which lets it go behind the wait, like embed_kernel there, and makes the
 // tokens' rotations.  What bounds it: start, one load and code that runs for the first time, 1.2 us a norm (61 tokens of the 0.5B shape
 // 660 -> 722 us with norms that the matmuls on both sides shared before, as in passes of up to 32 tokens, and whose products with h did not
-// always fit fp16).  One to four warps for a row of 896: a warp and four rows a CTA 796, norm weights asked for behind the wait 754.
+// always fit fp16).  A warp a row, four rows a CTA: 796; norm weights asked for behind the wait: 754.
 struct ChainNorm {
     __half* x;
     const __half* w;

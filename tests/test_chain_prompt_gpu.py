@@ -117,3 +117,15 @@ def test_residual_times_norm_weight_below_fp16(be, cuda, n, off):
         for j in range(2):
             a, b = got[i, j].double(), want[i, j].double()
             assert b.pow(2).mean().sqrt() > 1e-5 and (a - b).norm() <= 2.0 ** -8 * b.norm()
+
+
+@pytest.mark.parametrize("tail", [1, 6, 32, 33])
+def test_last_tokens_of_a_prompt_longer_than_a_pass(be, cuda, tail):
+    """They are a pass of their own, through these kernels behind the rows of the large ones."""
+    m = _model(be, cuda, *SHAPES[1])
+    tokens = torch.randint(0, 520, (be.llama.PREFILL_ROWS + tail,), generator=torch.Generator().manual_seed(tail))[None].to(cuda)
+    got, want = (_run(be, m, tokens, 0, False, large) for large in (True, False))
+    m.prefill_large_m = True
+    m.check_fused_error()
+    for a, b in zip(got, want):
+        assert ((a - b).abs() <= 2.0 ** -6 * b.abs() + 1e-2).all()
